@@ -13,6 +13,7 @@
 // --fmad=false: only the explicit fma() calls fuse, in the same places the CPU
 // oracle fuses, so both round identically.
 #include "pm_common.cuh"
+#include "pm_sum6.cuh"
 #include "pm_tail.cuh"
 
 #include <algorithm>
@@ -143,6 +144,57 @@ __global__ void k_resnorm_split(LevelView L, unsigned long long* out)
     block_umax_store(v, out);
 }
 
+// Two compact cells 2 t2, 2 t2 + 1 of one colour of row (j, k) of a split level whose
+// rows hold an even number of them: their neighbour sums from the other colour's array
+// (16-byte loads; the two cells share one x neighbour), cell u of the pair being
+// i = 4 t2 + 2 u + q.
+__device__ __forceinline__ double2 pair_at(const double* a, unsigned at)
+{
+    return __ldg(reinterpret_cast<const double2*>(a + at));
+}
+
+__device__ __forceinline__ unsigned pair_row(unsigned n, unsigned j, unsigned k) { return (j + n * k) * (n >> 1); }
+
+__device__ __forceinline__ double2 pair_sums(int n, const double* __restrict__ other, unsigned t2, int j, int k,
+                                             int q, bool on_int)
+{
+    const unsigned half = (unsigned)n >> 1, ih = 2 * t2;
+    const int jm = j == 0 ? n - 1 : j - 1, jp = j == n - 1 ? 0 : j + 1;
+    const int km = k == 0 ? n - 1 : k - 1, kp = k == n - 1 ? 0 : k + 1;
+    const unsigned r0 = pair_row(n, j, k);
+    const double2 c = pair_at(other, r0 + ih);
+    const double2 ym = pair_at(other, pair_row(n, jm, k) + ih), yp = pair_at(other, pair_row(n, jp, k) + ih);
+    const double2 zm = pair_at(other, pair_row(n, j, km) + ih), zp = pair_at(other, pair_row(n, j, kp) + ih);
+    const double e = __ldg(other + r0 + (q ? (ih + 2 == half ? 0u : ih + 2) : (ih == 0 ? half - 1 : ih - 1)));
+    const double x0 = q ? c.x : e, x1 = q ? c.y : c.x, x2 = q ? e : c.y;
+    const double nb0[6] = {x0, x1, ym.x, yp.x, zm.x, zp.x};
+    const double nb1[6] = {x1, x2, ym.y, yp.y, zm.y, zp.y};
+    return make_double2(sum6(nb0, on_int), sum6(nb1, on_int));
+}
+
+// k_resnorm_split by pairs of each colour
+__global__ void __launch_bounds__(256) k_resnorm_split2(LevelView L, unsigned long long* out)
+{
+    const int n = L.n;
+    const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    unsigned long long v = 0;
+    if (t2 < (unsigned)n >> 2 && j < n) {
+        const unsigned t = pair_row(n, j, k) + 2 * t2;
+        const bool on_int = sum6_on_int();
+#pragma unroll
+        for (int color = 0; color < 2; ++color) {
+            const double2 s = pair_sums(n, color ? L.phi_r : L.phi_b, t2, j, k, (j + k + color) & 1, on_int);
+            const double2 c = pair_at(color ? L.phi_b : L.phi_r, t), b = pair_at(color ? L.beta_b : L.beta_r, t);
+            const unsigned long long r0 = absbits(b.x - fma(s.x, kSixth, -c.x));
+            const unsigned long long r1 = absbits(b.y - fma(s.y, kSixth, -c.y));
+            v = max(v, max(r0, r1));
+        }
+    }
+    block_umax_store(v, out);
+}
+
 // the same over the red cells only: one thread per red cell of the split level
 __global__ void k_resnorm_red(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
                               const double* __restrict__ beta_r, unsigned long long* out)
@@ -207,6 +259,30 @@ __global__ void k_resnorm_red_sweep(int n, const double* __restrict__ phi_r,
     block_umax_store(v, out);
 }
 
+// k_resnorm_red_sweep by pairs
+__global__ void __launch_bounds__(256) k_resnorm_red_sweep2(int n, const double* __restrict__ phi_r,
+                                                            const double* __restrict__ phi_b,
+                                                            const double* __restrict__ beta_r,
+                                                            double* __restrict__ next_r, unsigned long long* out)
+{
+    pdl_wait();
+    pdl_trigger();
+    const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    unsigned long long v = 0;
+    if (t2 < (unsigned)n >> 2 && j < n) {
+        const unsigned t = pair_row(n, j, k) + 2 * t2;
+        const double2 s = pair_sums(n, phi_b, t2, j, k, (j + k) & 1, sum6_on_int());
+        const double2 c = pair_at(phi_r, t), b = pair_at(beta_r, t);
+        const unsigned long long r0 = absbits(b.x - fma(s.x, kSixth, -c.x));
+        const unsigned long long r1 = absbits(b.y - fma(s.y, kSixth, -c.y));
+        v = max(r0, r1);
+        *reinterpret_cast<double2*>(next_r + t) = make_double2(fma(s.x, kSixth, -b.x), fma(s.y, kSixth, -b.y));
+    }
+    block_umax_store(v, out);
+}
+
 __global__ void k_resnorm_nat(LevelView L, unsigned long long* out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -247,6 +323,23 @@ __global__ void __launch_bounds__(256) k_gsrb(int n, int color, double* __restri
     mine[t] = fma(s, kSixth, -beta[t]);
 }
 
+// k_gsrb by pairs
+__global__ void __launch_bounds__(256) k_gsrb2(int n, int color, double* __restrict__ mine,
+                                               const double* __restrict__ other,
+                                               const double* __restrict__ beta)
+{
+    pdl_wait();
+    pdl_trigger();
+    const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (t2 >= (unsigned)n >> 2 || j >= n) return;
+    const unsigned t = pair_row(n, j, k) + 2 * t2;
+    const double2 b = pair_at(beta, t);
+    const double2 s = pair_sums(n, other, t2, j, k, (j + k + color) & 1, sum6_on_int());
+    *reinterpret_cast<double2*>(mine + t) = make_double2(fma(s.x, kSixth, -b.x), fma(s.y, kSixth, -b.y));
+}
+
 // coarse beta = 1/2 of the 8 fine residuals (summed dk, dj, di); coarse phi = 0
 // RED = 1 after pre-smoothing (the last half sweep was black): the black
 // children's residuals are round-off by construction and count as 0, so the 4 red
@@ -273,6 +366,35 @@ __global__ void k_restrict(LevelView F, LevelView Cv)
                     s = s + resid_at(F, 2 * I + di, 2 * J + dj, 2 * K + dk);
     *lv_ptr<double>(Cv.beta_r, Cv.beta_b, nc, Cv.split, I, J, K) = s * 0.5;
     *lv_ptr<double>(Cv.phi_r, Cv.phi_b, nc, Cv.split, I, J, K) = 0.0;
+}
+
+// k_restrict<1> by pairs: two coarse cells 2 t2, 2 t2 + 1 of a row per thread, whose
+// red children in a fine row are the row's red pair 2 t2, 2 t2 + 1
+__global__ void __launch_bounds__(256) k_restrict_red2(LevelView F, LevelView Cv)
+{
+    pdl_wait();
+    pdl_trigger();
+    const int n = F.n, nc = Cv.n;
+    const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;
+    const int J = blockIdx.y * blockDim.y + threadIdx.y;
+    const int K = blockIdx.z;
+    if (t2 >= (unsigned)nc >> 1 || J >= nc) return;
+    const bool on_int = sum6_on_int();
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 1
+    for (int d = 0; d < 4; ++d) {
+        const int j = 2 * J + (d & 1), k = 2 * K + (d >> 1);
+        const unsigned t = pair_row(n, j, k) + 2 * t2;
+        const double2 b = pair_at(F.beta_r, t), c = pair_at(F.phi_r, t);
+        const double2 s = pair_sums(n, F.phi_b, t2, j, k, (j + k) & 1, on_int);
+        acc.x = acc.x + (b.x - fma(s.x, kSixth, -c.x));
+        acc.y = acc.y + (b.y - fma(s.y, kSixth, -c.y));
+    }
+    const int I = 2 * (int)t2;
+    *lv_ptr<double>(Cv.beta_r, Cv.beta_b, nc, Cv.split, I, J, K) = acc.x * 0.5;
+    *lv_ptr<double>(Cv.beta_r, Cv.beta_b, nc, Cv.split, I + 1, J, K) = acc.y * 0.5;
+    *lv_ptr<double>(Cv.phi_r, Cv.phi_b, nc, Cv.split, I, J, K) = 0.0;
+    *lv_ptr<double>(Cv.phi_r, Cv.phi_b, nc, Cv.split, I + 1, J, K) = 0.0;
 }
 
 // k_prolong for a split fine level over a split coarse level with
@@ -488,6 +610,13 @@ __global__ void k_beta_from_natural(LevelView L, const double* __restrict__ in)
     *lv_ptr<double>(L.beta_r, L.beta_b, n, L.split, i, j, k) = in[cidx(i, j, k, n)];
 }
 
+// Levels of at least this edge work by pairs of cells, their sums on the integer pipes
+// (pm_sum6.cuh): there the FP64 pipe is the bound (128^3: a half sweep 16.4 -> 12.3 us,
+// a whole solve 3.21 -> 2.82 ms).  On 64^3 a half sweep is latency: integer sums gave
+// a ten-step 64^3 run 23.8 ms against 24.0 ms, and with them on every level 25.4 ms.
+constexpr int kPairMinEdge = 128;
+inline bool by_pairs(const Level& l) { return l.split && l.n >= kPairMinEdge && l.n % 4 == 0; }
+
 inline unsigned norm_blocks(Ctx& c, long long cnt)
 {
     long long b = (cnt + kThreads - 1) / kThreads;
@@ -498,13 +627,14 @@ inline unsigned norm_blocks(Ctx& c, long long cnt)
 nyxpm_status gsrb_sweep(Ctx& c, const Level& l, int fine, int black_only = 0)
 {
     const long long half_cells = (long long)l.n * l.n * l.n / 2;
-    const Geo g = geo3(l.n / 2, l.n, l.n);
+    const bool pairs = by_pairs(l);
+    const Geo g = geo3(pairs ? l.n / 4 : l.n / 2, l.n, l.n);
     for (int color = black_only ? 1 : 0; color < 2; ++color) {
         double* mine = color ? l.phi_b : l.phi_r;
         const double* other = color ? l.phi_r : l.phi_b;
         const double* beta = color ? l.beta_b : l.beta_r;
         prof_begin(c);
-        launch_pdl(c, k_gsrb, dim3(g.grid), dim3(g.block), l.n, color, mine, other, beta);
+        launch_pdl(c, pairs ? k_gsrb2 : k_gsrb, dim3(g.grid), dim3(g.block), l.n, color, mine, other, beta);
         prof_end(c, NYXPM_ST_SMOOTH, 24.0 * half_cells, fine);
     }
     return check_launch(c, "gsrb");
@@ -562,10 +692,11 @@ nyxpm_status vcycle(Ctx& c, Box& b, size_t li, int red_done = 0)
     const long long ncf = (long long)f.n * f.n * f.n;
     const bool quads = f.split && (f.n / 2) % 4 == 0;
     {
-        const Geo g = geo3(cl.n, cl.n, cl.n);
+        const bool pairs = c.p.nu1 > 0 && by_pairs(f);
+        const Geo g = geo3(pairs ? cl.n / 2 : cl.n, cl.n, cl.n);
         prof_begin(c);
         if (c.p.nu1 > 0)
-            launch_pdl(c, k_restrict<1>, dim3(g.grid), dim3(g.block), view(f), view(cl));
+            launch_pdl(c, pairs ? k_restrict_red2 : k_restrict<1>, dim3(g.grid), dim3(g.block), view(f), view(cl));
         else
             launch_pdl(c, k_restrict<0>, dim3(g.grid), dim3(g.block), view(f), view(cl));
         prof_end(c, NYXPM_ST_RESTRICT, 16.0 * ncf + 16.0 * ncc);
@@ -604,8 +735,9 @@ nyxpm_status launch_resnorm(Ctx& c, Box& b, int slot, int red_only)
         const Geo g = geo3(l.n / 2, l.n, l.n);
         k_resnorm_red<<<g.grid, g.block, 0, c.stream>>>(l.n, l.phi_r, l.phi_b, l.beta_r, b.norms + slot);
     } else if (l.split) {
-        const Geo g = geo3(l.n / 2, l.n, l.n);
-        k_resnorm_split<<<g.grid, g.block, 0, c.stream>>>(view(l), b.norms + slot);
+        const bool pairs = by_pairs(l);
+        const Geo g = geo3(pairs ? l.n / 4 : l.n / 2, l.n, l.n);
+        (pairs ? k_resnorm_split2 : k_resnorm_split)<<<g.grid, g.block, 0, c.stream>>>(view(l), b.norms + slot);
     } else {
         const Geo g = geo3(l.n, l.n, l.n);
         k_resnorm_nat<<<g.grid, g.block, 0, c.stream>>>(view(l), b.norms + slot);
@@ -702,10 +834,11 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
             nyxpm_status s;
             if ((s = vcycle(c, b, 0, fuse && !first ? 1 : 0)) != NYXPM_OK) return s;
             if (fuse) {
-                const Geo g = geo3(L0.n / 2, L0.n, L0.n);
+                const bool pairs = by_pairs(L0);
+                const Geo g = geo3(pairs ? L0.n / 4 : L0.n / 2, L0.n, L0.n);
                 prof_begin(c);
                 cudaMemsetAsync(b.norms + 1, 0, sizeof(unsigned long long), c.stream);
-                launch_pdl(c, k_resnorm_red_sweep, dim3(g.grid), dim3(g.block), L0.n, L0.phi_r, L0.phi_b, L0.beta_r,
+                launch_pdl(c, pairs ? k_resnorm_red_sweep2 : k_resnorm_red_sweep, dim3(g.grid), dim3(g.block), L0.n, L0.phi_r, L0.phi_b, L0.beta_r,
                                                                       b.phi_r_spare, b.norms + 1);
                 prof_end(c, NYXPM_ST_NORM, 16.0 * nc);
                 if ((s = check_launch(c, "red norm + sweep")) != NYXPM_OK) return s;
