@@ -64,6 +64,10 @@ typedef struct nyxpm_params {
     int mg_fused_edge;      /* the FP32 V-cycle levels of at most this many cells per edge
                                (the FP64 ones of at most half as many, below the finest) run
                                as one launch (one CTA per box) per V-cycle, same results;
+                               with any value above 0 and nu1, nu2 > 0, a single box's FP32
+                               levels of at most 64 and FP64 levels of at most 32 cells per
+                               edge run as one launch of a 16-CTA cluster where their planes
+                               fit in its shared memory, same results;
                                0: one launch per pass on every level (default 16) */
 } nyxpm_params;
 

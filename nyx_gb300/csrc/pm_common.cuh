@@ -441,7 +441,8 @@ struct Box {
     double* planes = nullptr;          // n plane sums
     double* scal = nullptr;            // [0] mean
     unsigned long long* norms = nullptr;   // [0] ||rhs||inf, [1] ||r||inf, [2] bad uploads,
-                                           // [3] time-step limit, [4] mixed: max |e|
+                                           // [3] time-step limit, [4] mixed: max |e|,
+                                           // [5] .. [7] a cluster solve's result
     unsigned long long* h_norms = nullptr; // pinned host mirror
     double* G = nullptr;               // bottom Green's function (smoother units)
     float* Gf = nullptr;               // the same in FP32 (mixed inner V-cycles)
@@ -479,6 +480,8 @@ struct Ctx {
     // multigrid kernels launched with programmatic dependent launch (off with
     // the environment variable NYXPM_NO_PDL set, for comparison)
     int pdl = 1;
+    // the cluster kernels of the FP64 and FP32 forms can run here: -1 not asked yet
+    int cluster_d = -1, cluster_f = -1;
     // the first error a launch_pdl returned since the last check_launch
     cudaError_t launch_error = cudaSuccess;
 };

@@ -12,6 +12,7 @@
 //
 // FP32 arithmetic is compiled with multiply-add contraction (the default): this
 // form is checked against the FP64 oracle by a stated tolerance, not bitwise.
+#include "pm_cluster.cuh"
 #include "pm_common.cuh"
 #include "pm_prolong.cuh"
 #include "pm_restrict.cuh"
@@ -1169,6 +1170,103 @@ __global__ void __launch_bounds__(kTailThreads) k_vcycle_tail_f(TailF A)
     vcycle_tail<float>(A.lv, A.nl, A.nu1, A.nu2, A.Gf, A.nb, r, g, A.nu1 > 0);
 }
 
+// An FP32 V-cycle, or a whole defect-correction solve, of small levels by one cluster
+// (pm_cluster.cuh).
+// one V-cycle from a zero guess: the right-hand side and the correction of L in global memory
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_f(ClArgs<float> A, LevelViewF L)
+{
+    extern __shared__ __align__(16) float cl_mem_f[];
+    __shared__ ClShared<float> S;
+    cl_setup(A, S, cl_mem_f);
+    pdl_wait();
+    pdl_trigger();
+    cl_load_green(A, S);
+    cl_load(S.lv[0], L, false);
+    cl_barrier();
+    cl_vcycle(A, S, cl_mem_f, true);
+    cl_store(S.lv[0], L);
+}
+
+struct ClSolveArgs {
+    double *phi_r, *phi_b;          // FP64 solution
+    const float *r_r, *r_b;         // high words of the residual
+    float *rl_r, *rl_b;             // low words
+    int inner, first, max_it;       // iterations made so far, limit
+    double rel_tol, target;         // target < 0: rel_tol times the larger of norms[0], norms[1]
+    int zero_guess;                 // ||r0|| is norms[0]
+    float c_hi, c_lo;
+    unsigned long long* norms;      // out: [5] ||r||, [6] iterations | 2^32 if r has to be
+                                    // recomputed from phi, [7] the error bound
+};
+
+// mixed_solve's iterations: inner V-cycles from e = 0 for the residual's high words,
+// phi += e and the double-float update of the residual (k_mx_correct), until the tracked
+// residual and its error bound meet the target.  Where the bound could hide the
+// tolerance the kernel stops, the host recomputes the residual from phi and calls again.
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_f(ClArgs<float> A, ClSolveArgs P)
+{
+    extern __shared__ __align__(16) float cl_mem_f[];
+    __shared__ ClShared<float> S;
+    cl_setup(A, S, cl_mem_f);
+    pdl_wait();
+    pdl_trigger();
+    const double bnorm = __longlong_as_double((long long)P.norms[0]);
+    const double r0 = P.zero_guess ? bnorm : __longlong_as_double((long long)P.norms[1]);
+    const double target = P.target >= 0.0 ? P.target : P.rel_tol * (bnorm < r0 ? r0 : bnorm);
+    double r = r0, err = 0.0;
+    int it = P.first, again = 0;
+    if (P.target >= 0.0 || !(r0 <= target)) {
+        const ClLevel<float>& F = S.lv[0];
+        const int n = F.n, half = n >> 1, plane = n * half, total = plane * F.np;
+        const size_t o = (size_t)F.p0 * plane;
+        cl_load_green(A, S);
+        cl_copy(F.beta_r, P.r_r + o, total);
+        cl_copy(F.beta_b, P.r_b + o, total);
+        cl_barrier();
+        for (it = P.first + 1;; ++it) {
+            for (int v = 0; v < P.inner; ++v) cl_vcycle(A, S, cl_mem_f, v == 0);
+            float vmax = 0.f, emax = 0.f;
+            for (int t = threadIdx.x; t < total; t += blockDim.x) {
+                int ih, j, q;
+                cl_split(t, half, n, ih, j, q);
+#pragma unroll
+                for (int color = 0; color < 2; ++color) {
+                    float* const* z = color ? F.zr : F.zb;
+                    const int odd = (j + F.p0 + q + color) & 1;
+                    const int ihm = odd ? ih : (ih == 0 ? half - 1 : ih - 1);
+                    const int ihp = odd ? (ih == half - 1 ? 0 : ih + 1) : ih;
+                    const int jm = j == 0 ? n - 1 : j - 1, jp = j == n - 1 ? 0 : j + 1;
+                    const float v[6] = {z[q + 1][j * half + ihm], z[q + 1][j * half + ihp], z[q + 1][jm * half + ih],
+                                        z[q + 1][jp * half + ih], z[q][j * half + ih], z[q + 2][j * half + ih]};
+                    const float em = (color ? F.phi_b : F.phi_r)[t];
+                    float* hi = (color ? F.beta_b : F.beta_r) + t;
+                    float* lo = (color ? P.rl_b : P.rl_r) + o + t;
+                    float rh = *hi, rl = *lo;
+                    df_residual_update(v, em, P.c_hi, P.c_lo, rh, rl);
+                    *hi = rh;
+                    *lo = rl;
+                    double* p = (color ? P.phi_b : P.phi_r) + o + t;
+                    *p = *p + f32_to_f64(em);
+                    vmax = fmaxf(vmax, fabsf(rh));
+                    emax = fmaxf(emax, fabsf(em));
+                }
+            }
+            cl_norm_put(S, 0, absbits(f32_to_f64(vmax)));
+            cl_norm_put(S, 1, absbits(f32_to_f64(emax)));
+            cl_barrier();
+            r = __longlong_as_double((long long)cl_norm_get(S, 0));
+            err = __dadd_rn(err, __dmul_rn(kDfUpdateErr, __longlong_as_double((long long)cl_norm_get(S, 1))));
+            if (err > 0.5 * target && r == r) again = 1;
+            if (again || r != r || __dadd_rn(r, err) <= target || it >= P.max_it) break;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        P.norms[5] = absbits(r);
+        P.norms[6] = (unsigned long long)(unsigned)it | ((unsigned long long)again << 32);
+        P.norms[7] = absbits(err);
+    }
+}
+
 // FP32 gravity vector from the FP64 phi: the difference in FP64, the scaling in FP32
 // (one float4 {gx, gy, gz, 0} per cell: a CIC corner is one 16-byte load)
 __global__ void k_mx_grav(LevelView L, float half_dxi, float* g)
@@ -1356,6 +1454,16 @@ nyxpm_status vcycle_tail_f(Ctx& c, Box& b, size_t li)
     return check_launch(c, "fused coarse V-cycle f32");
 }
 
+// whether the levels from li on are taken by one cluster, and how they lie in it
+bool cluster_fits_f(Ctx& c, const Box& b, size_t li, ClArgs<float>& A)
+{
+    if (!cl_args<float>(c, b, li, A)) return false;
+    if (c.cluster_f < 0)
+        c.cluster_f = cl_prepare(k_cluster_vcycle_f, cl_max_bytes<float>()) &&
+                      cl_prepare(k_cluster_solve_f, cl_max_bytes<float>());
+    return c.cluster_f > 0;
+}
+
 bool tail_fits(const Ctx& c, const Box& b, size_t li)
 {
     return c.p.mg_fused_edge > 0 && b.levels[li].n <= c.p.mg_fused_edge &&
@@ -1379,6 +1487,13 @@ nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false)
             cudaMemsetAsync(f.fphi_r, 0, cnt * sizeof(float), c.stream);
         }
         fresh = false;
+    }
+    ClArgs<float> ca;
+    if (li > 0 && cluster_fits_f(c, b, li, ca)) {
+        prof_begin(c);
+        launch_cluster(c, k_cluster_vcycle_f, ca.elems * sizeof(float), ca, viewf(f));
+        prof_end(c, NYXPM_ST_SMOOTH, 16.0 * f.n * f.n * f.n);
+        return check_launch(c, "cluster V-cycle f32");
     }
     if (tail_fits(c, b, li)) return vcycle_tail_f(c, b, li);
     if (li + 1 == b.levels.size()) {
@@ -1743,6 +1858,34 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
         cudaMemcpyAsync(b.h_norms, b.norms, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                         c.stream);
     }
+    // a small box: the iterations in one cluster launch (until the residual has to be
+    // recomputed from phi)
+    ClArgs<float> ca;
+    const bool in_cluster = incremental && cluster_fits_f(c, b, 0, ca);
+    auto cluster_solve = [&](int first, double goal) -> nyxpm_status {
+        ClSolveArgs P;
+        P.phi_r = l0.phi_r;
+        P.phi_b = l0.phi_b;
+        P.r_r = l0.fbeta_r;
+        P.r_b = l0.fbeta_b;
+        P.rl_r = b.r_lo;
+        P.rl_b = b.r_lo + nc / 2;
+        P.inner = c.p.mixed_inner_vcycles;
+        P.first = first;
+        P.max_it = c.p.max_vcycles;
+        P.rel_tol = c.p.rel_tol;
+        P.target = goal;
+        P.zero_guess = zero_guess;
+        P.c_hi = (float)(1.0 / 6.0);
+        P.c_lo = (float)(1.0 / 6.0 - (double)P.c_hi);
+        P.norms = b.norms;
+        prof_begin(c);
+        launch_cluster(c, k_cluster_solve_f, ca.elems * sizeof(float), ca, P);
+        prof_end(c, NYXPM_ST_SMOOTH, 0);
+        cudaMemcpyAsync(b.h_norms, b.norms, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.stream);
+        return check_launch(c, "mixed cluster solve");
+    };
+    if (in_cluster && (st = cluster_solve(0, -1.0)) != NYXPM_OK) return st;
     if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
     const double bnorm = read_norm(b, 0);
     const double r0 = (zero_guess && incremental) ? bnorm : read_norm(b, 1);
@@ -1751,7 +1894,34 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
     double err = 0.0;   // bound on |tracked residual - residual of phi|
     int it = 0, inner = 0;
     nyxpm_status result = NYXPM_OK;
-    if (!(r0 <= target)) {
+    if (in_cluster) {
+        for (;;) {
+            r = read_norm(b, 5);
+            err = read_norm(b, 7);
+            it = (int)(b.h_norms[6] & 0xffffffffULL);
+            if (b.h_norms[6] >> 32) {
+                if ((st = launch_mx_resid(c, b, true)) != NYXPM_OK) return st;
+                cudaMemcpyAsync(b.h_norms + 1, b.norms + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                c.stream);
+                if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
+                r = read_norm(b, 1);
+                err = 0.0;
+            }
+            inner = it * c.p.mixed_inner_vcycles;
+            if (r != r) {
+                c.err = "mixed defect correction residual is NaN";
+                return NYXPM_NOT_CONVERGED;
+            }
+            if (r + err <= target) break;
+            if (it >= c.p.max_vcycles) {
+                result = NYXPM_NOT_CONVERGED;
+                c.err = "defect correction reached max_vcycles above tolerance";
+                break;
+            }
+            if ((st = cluster_solve(it, target)) != NYXPM_OK) return st;
+            if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
+        }
+    } else if (!(r0 <= target)) {
         auto iteration = [&]() -> nyxpm_status {
             // inner FP32 solve of L e = r from e = 0, phi += e, the new residual
             nyxpm_status s;

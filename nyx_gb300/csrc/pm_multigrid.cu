@@ -12,6 +12,7 @@
 // arithmetic uses 3-D launch geometry instead of integer division.  Built with
 // --fmad=false: only the explicit fma() calls fuse, in the same places the CPU
 // oracle fuses, so both round identically.
+#include "pm_cluster.cuh"
 #include "pm_common.cuh"
 #include "pm_sum6.cuh"
 #include "pm_tail.cuh"
@@ -557,6 +558,92 @@ __global__ void __launch_bounds__(kTailThreadsD) k_vcycle_tail_d(TailD A)
     vcycle_tail<double>(A.lv, A.nl, A.nu1, A.nu2, A.G, A.nb, r, g, A.nu1 > 0);
 }
 
+// A V-cycle, or a whole solve, of small levels by one cluster (pm_cluster.cuh).
+// one V-cycle from a zero guess: the right-hand side and the correction of L in global memory
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_d(ClArgs<double> A, LevelView L)
+{
+    extern __shared__ __align__(16) double cl_mem_d[];
+    __shared__ ClShared<double> S;
+    cl_setup(A, S, cl_mem_d);
+    pdl_wait();
+    pdl_trigger();
+    cl_load_green(A, S);
+    cl_load(S.lv[0], L, false);
+    cl_barrier();
+    cl_vcycle(A, S, cl_mem_d, true);
+    cl_store(S.lv[0], L);
+}
+
+// the same with both in natural layout
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_nat_d(ClArgs<double> A, const double* __restrict__ beta,
+                                                                     double* __restrict__ e)
+{
+    extern __shared__ __align__(16) double cl_mem_d[];
+    __shared__ ClShared<double> S;
+    cl_setup(A, S, cl_mem_d);
+    pdl_wait();
+    pdl_trigger();
+    cl_load_green(A, S);
+    const ClLevel<double>& L = S.lv[0];
+    const int n = L.n, half = n >> 1, total = n * n * L.np;
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        int i, j, q;
+        cl_split(t, n, n, i, j, q);
+        ((i + j + L.p0 + q) & 1 ? L.beta_b : L.beta_r)[(i >> 1) + half * (j + n * q)] = beta[(size_t)L.p0 * n * n + t];
+    }
+    cl_barrier();
+    cl_vcycle(A, S, cl_mem_d, true);
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        int i, j, q;
+        cl_split(t, n, n, i, j, q);
+        e[(size_t)L.p0 * n * n + t] = ((i + j + L.p0 + q) & 1 ? L.phi_b : L.phi_r)[(i >> 1) + half * (j + n * q)];
+    }
+}
+
+// The V-cycles of a solve from phi (level 0) until ||r||_inf <= rel_tol max(norms[0],
+// norms[1]) = rel_tol max(||beta||, ||r0||), with the red-cell norm of mg_solve's loop:
+// norms[5] = ||r||, norms[6] = the number of V-cycles.  Every CTA sees the same norms, so
+// all leave the loop together.
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_d(ClArgs<double> A, LevelView L, double rel_tol,
+                                                                int max_vcycles, unsigned long long* norms)
+{
+    extern __shared__ __align__(16) double cl_mem_d[];
+    __shared__ ClShared<double> S;
+    cl_setup(A, S, cl_mem_d);
+    pdl_wait();
+    pdl_trigger();
+    const double bnorm = __longlong_as_double((long long)norms[0]), r0 = __longlong_as_double((long long)norms[1]);
+    const double target = rel_tol * (bnorm < r0 ? r0 : bnorm);
+    double r = r0;
+    int it = 0;
+    if (!(r0 <= target)) {
+        const ClLevel<double>& F = S.lv[0];
+        const int n = F.n, half = n >> 1, total = half * n * F.np;
+        cl_load_green(A, S);
+        cl_load(F, L, true);
+        cl_barrier();
+        for (it = 1;; ++it) {
+            cl_vcycle(A, S, cl_mem_d, false);
+            unsigned long long v = 0;
+            for (int t = threadIdx.x; t < total; t += blockDim.x) {
+                int ih, j, q;
+                cl_split(t, half, n, ih, j, q);
+                const double s = cl_sum<double>(F.zb, n, q + 1, j, ih, (j + F.p0 + q) & 1);
+                v = max(v, absbits(F.beta_r[t] - fma(s, kSixth, -F.phi_r[t])));
+            }
+            cl_norm_put(S, it & 1, v);
+            cl_barrier();
+            r = __longlong_as_double((long long)cl_norm_get(S, it & 1));
+            if (r <= target || r != r || it >= max_vcycles) break;
+        }
+        cl_store(F, L);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        norms[5] = absbits(r);
+        norms[6] = (unsigned long long)it;
+    }
+}
+
 // g_d(c) = 0.5*((phi_c - phi_{c-e_d})*dxi + (phi_{c+e_d} - phi_c)*dxi), second product fused;
 // component-major output
 __global__ void k_grav(LevelView L, double dxi, double* g)
@@ -650,6 +737,18 @@ bool tail_fits_d(const Ctx& c, const Box& b, size_t li)
            b.levels.size() - li <= (size_t)kMaxTail;
 }
 
+// whether the levels from li on are taken by one cluster, and how they lie in it
+bool cluster_fits_d(Ctx& c, const Box& b, size_t li, ClArgs<double>& A)
+{
+    if (!cl_args<double>(c, b, li, A)) return false;
+    if (c.cluster_d < 0) {
+        const size_t most = cl_max_bytes<double>();
+        c.cluster_d = cl_prepare(k_cluster_vcycle_d, most) && cl_prepare(k_cluster_vcycle_nat_d, most) &&
+                      cl_prepare(k_cluster_solve_d, most);
+    }
+    return c.cluster_d > 0;
+}
+
 nyxpm_status vcycle_tail_d(Ctx& c, Box& b, size_t li)
 {
     TailD A;
@@ -677,6 +776,13 @@ nyxpm_status vcycle(Ctx& c, Box& b, size_t li, int red_done = 0)
 {
     nyxpm_status st;
     const Level& f = b.levels[li];
+    ClArgs<double> ca;
+    if (li > 0 && cluster_fits_d(c, b, li, ca)) {
+        prof_begin(c);
+        launch_cluster(c, k_cluster_vcycle_d, ca.elems * sizeof(double), ca, view(f));
+        prof_end(c, NYXPM_ST_SMOOTH, 32.0 * f.n * f.n * f.n);
+        return check_launch(c, "cluster V-cycle");
+    }
     if (tail_fits_d(c, b, li)) return vcycle_tail_d(c, b, li);
     if (li + 1 == b.levels.size()) {
         prof_begin(c);
@@ -812,7 +918,17 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
     prof_end(c, NYXPM_ST_NORM, 8.0 * nc);
     if ((st = check_launch(c, "rhs norm")) != NYXPM_OK) return st;
     if ((st = launch_resnorm(c, b, 1, 0)) != NYXPM_OK) return st;
-    cudaMemcpyAsync(b.h_norms, b.norms, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+    // a small box: the whole solve in one cluster launch
+    ClArgs<double> ca;
+    const bool in_cluster = cluster_fits_d(c, b, 0, ca);
+    if (in_cluster) {
+        prof_begin(c);
+        launch_cluster(c, k_cluster_solve_d, ca.elems * sizeof(double), ca, view(l0), c.p.rel_tol, c.p.max_vcycles,
+                       b.norms);
+        prof_end(c, NYXPM_ST_SMOOTH, 0);
+        if ((st = check_launch(c, "cluster solve")) != NYXPM_OK) return st;
+    }
+    cudaMemcpyAsync(b.h_norms, b.norms, (in_cluster ? 7 : 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                     c.stream);
     if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "solve sync");
     const double bnorm = read_norm(b, 0);
@@ -828,7 +944,18 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
     // goes on (the next V-cycle then starts at its black half sweep).
     Level& L0 = b.levels[0];
     const bool fuse = red_only && c.p.nu1 > 0 && L0.split && b.phi_r_spare;
-    if (!(r0 <= target)) {
+    if (in_cluster) {
+        r = read_norm(b, 5);
+        it = (int)b.h_norms[6];
+        if (r != r) {
+            c.err = "multigrid residual is NaN";
+            return NYXPM_NOT_CONVERGED;
+        }
+        if (!(r <= target)) {
+            result = NYXPM_NOT_CONVERGED;
+            c.err = "multigrid reached max_vcycles above tolerance";
+        }
+    } else if (!(r0 <= target)) {
         bool first = true;
         auto iteration = [&]() -> nyxpm_status {
             nyxpm_status s;
@@ -918,6 +1045,13 @@ nyxpm_status mg_vcycle_zero(Ctx& c, Box& b, const double* beta_nat, double* e_na
     nyxpm_status st;
     const long long nc = (long long)b.n * b.n * b.n;
     const Geo g = geo3(b.n, b.n, b.n);
+    ClArgs<double> ca;
+    if (cluster_fits_d(c, b, 0, ca)) {
+        prof_begin(c);
+        launch_cluster(c, k_cluster_vcycle_nat_d, ca.elems * sizeof(double), ca, beta_nat, e_nat);
+        prof_end(c, NYXPM_ST_SMOOTH, 16.0 * nc);
+        return check_launch(c, "cluster V-cycle");
+    }
     prof_begin(c);
     k_beta_from_natural<<<g.grid, g.block, 0, c.stream>>>(view(b.levels[0]), beta_nat);
     prof_end(c, NYXPM_ST_RHS, 16.0 * nc);
