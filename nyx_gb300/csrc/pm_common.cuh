@@ -21,7 +21,21 @@
 
 #include "../../include/nyxpm.h"
 
+#include <unistd.h>
+
 namespace nyxpm {
+
+// One write to every page of a host buffer that a device-to-host copy will fill.  On a
+// host whose page tables the GPU shares, a copy into pages the process has not touched
+// yet takes a GPU page fault for each (measured 1.4 to 25 GB/s against 190 GB/s into
+// touched pages); the host faults them in at 30 to 40 GB/s.
+inline void touch_pages(void* p, size_t bytes)
+{
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = static_cast<volatile char*>(p);
+    for (size_t o = 0; o < bytes; o += page) c[o] = 0;
+    if (bytes) c[bytes - 1] = 0;
+}
 
 constexpr int kMaxBottom = 8;          // largest coarsest-grid edge (solved exactly)
 // A deposit key with more particles than this is summed by a whole warp in
