@@ -18,6 +18,7 @@
 // Like nyxpm_deposit it refuses non-finite positions: the key pass counts them,
 // and the call reads the count back before it returns.
 // Built with --fmad=false like the other FP64 units.
+#include "pm_cluster.cuh"
 #include "pm_common.cuh"
 
 #include <cmath>
@@ -35,6 +36,11 @@ constexpr long long kNaMaxParticles = 262144;
 constexpr int kNaScanT = 512, kNaScanIPT = 8, kNaScanTile = kNaScanT * kNaScanIPT;
 constexpr long long kNaTiles = (kNaMaxCells + kNaScanTile - 1) / kNaScanTile;
 
+// Up to this many particles and cells the sort is one cluster launch (na_sort), beyond it
+// ten launches over the whole chip.  Measured, a call from the host, particles on a
+// lattice: 8^3 77 -> 40 us, 32^3 95 -> 61 us, 48^3 112 -> 87 us; 64^3 with 262,144 particles 134 us by launches,
+// 136 by the cluster, 155 before the deposit below.
+constexpr long long kNaClusterMax = 131072;
 // scratch layout, each part rounded up to 256 bytes
 constexpr size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kOffCount = 0;
@@ -51,6 +57,11 @@ constexpr size_t kScratchBytes = kOffZ + up256(8 * kNaMaxParticles);
 
 // the scratch: every call shares it, and it keeps the last call's contents
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
+
+// the cluster sort (declared here for its launch attribute)
+__global__ void na_sort(int np, int n, double dxi, const double* __restrict__ x, const double* __restrict__ y,
+                        const double* __restrict__ z, int* key, int* count, int* start, int* perm, int* long_list,
+                        int* long_count, int* bad);
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
@@ -93,6 +104,8 @@ nyxpm_status scratch_address(cudaStream_t stream, unsigned char** out, int* sm_c
             sms = 1;
         }
         g_sm_count[dev] = sms > 0 ? sms : 1;
+        if (cudaFuncSetAttribute(na_sort, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            cudaGetLastError();   // the launch reports it
     }
     *out = g_scratch_addr[dev];
     *sm_count = g_sm_count[dev];
@@ -281,10 +294,6 @@ __global__ void na_gather(long long np, const int* __restrict__ perm, const doub
     zs[s] = z[q];
 }
 
-constexpr int kTx = 8, kTy = 8, kTz = 8;
-constexpr int kKx = kTx + 1, kKy = kTy + 1, kKz = kTz + 1;
-constexpr int kNKeys = kKx * kKy * kKz;
-
 __device__ __forceinline__ void na_add_weights(int q, int n, double dxi,
                                                const double* __restrict__ x,
                                                const double* __restrict__ y,
@@ -306,72 +315,235 @@ __device__ __forceinline__ void na_add_weights(int q, int n, double dxi,
                 s[cx + 2 * cy + 4 * cz] = s[cx + 2 * cy + 4 * cz] + (sx[cx] * sy[cy]) * sz[cz];
 }
 
-// A key longer than a warp, summed in the order the allocating deposit sums it
-// with a whole warp: 32 lane partials (lane l: particles l, l+32, ... in order)
-// combined by the xor butterfly 16, 8, 4, 2, 1.  Here one thread does it: the
-// butterfly's result is the pairwise tree over the lanes taken in bit-reversed
-// order, built with a stack of finished subtrees (a binary counter).
-__device__ void na_long_key(int b0, int e, int n, double dxi, const double* __restrict__ x,
-                            const double* __restrict__ y, const double* __restrict__ z,
-                            double out[8])
+// ---------------------------------------------------------------------------
+// The whole counting sort by one cluster of 16 CTAs: counts to zero, keys, exclusive
+// scan, scatter, segments back in particle order, a cluster barrier between two steps.
+// As launches the steps were ten kernels of 2 to 4 us each (their own time and the host's)
+// for a few microseconds of work.  The particles are not permuted: the deposit reads them
+// through perm.  Same keys, counts and order as the kernels above.
+// ---------------------------------------------------------------------------
+constexpr int kNaThreads = 1024;
+constexpr int kNaSeg = 512;   // longer segments are ranked by a block
+
+// Corner sums of the keys longer than a warp, a warp each: lane l sums particles l, l + 32,
+// ... and an xor butterfly adds the lanes, as nyxpm_deposit sums them.  Key K's sums go to
+// heavy[8 slot], slot = count[K] (the counts are zero after the scatter).  perm null: the
+// particles are in sorted order.
+__device__ __forceinline__ void na_heavy_keys(int warp, int warps, int n, double dxi, const double* x, const double* y,
+                                              const double* z, const int* perm, const int* start,
+                                              const int* long_list, int longs, int* count, double* heavy)
 {
-    double stack[6][8];
-    int depth = 0;
-    for (int t = 0; t < 32; ++t) {
-        const int lane = (int)(__brev((unsigned)t) >> 27);
-        double* p = stack[depth++];
-        for (int c = 0; c < 8; ++c) p[c] = 0.0;
-        for (int q = b0 + lane; q < e; q += 32) na_add_weights(q, n, dxi, x, y, z, p);
-        for (int v = t + 1; (v & 1) == 0; v >>= 1) {
-            for (int c = 0; c < 8; ++c) stack[depth - 2][c] = stack[depth - 2][c] + stack[depth - 1][c];
-            --depth;
+    const int lane = threadIdx.x & 31;
+    for (int li = warp; li < longs; li += warps) {
+        const int K = long_list[li], e = start[K + 1];
+        double s[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int q = start[K] + lane; q < e; q += 32) na_add_weights(perm ? perm[q] : q, n, dxi, x, y, z, s);
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) s[c] = s[c] + __shfl_xor_sync(0xffffffffu, s[c], off);
+        if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) heavy[8 * li + c] = s[c];
+            count[K] = li;
         }
     }
-    for (int c = 0; c < 8; ++c) out[c] = stack[0][c];
 }
 
-// per-key partial sums of the 8 corner weights, then cell sums in a fixed order
-__global__ void __launch_bounds__(256) na_deposit(int n, double dxi, double scale,
-                                                  const double* __restrict__ x,
-                                                  const double* __restrict__ y,
-                                                  const double* __restrict__ z,
-                                                  const int* __restrict__ start, double* rho)
+__global__ void __launch_bounds__(256) na_heavy(int n, double dxi, const double* x, const double* y, const double* z,
+                                                const int* start, const int* long_list, const int* long_count,
+                                                int* count, double* heavy)
 {
-    __shared__ double part[kNKeys * 8];
-    const int i0 = blockIdx.x * kTx, j0 = blockIdx.y * kTy, k0 = blockIdx.z * kTz;
-    for (int kl = threadIdx.x; kl < kNKeys; kl += blockDim.x) {
-        const int ki = kl % kKx, kj = (kl / kKx) % kKy, kk = kl / (kKx * kKy);
-        const long long K = cidx(wrapi(i0 + ki, n), wrapi(j0 + kj, n), wrapi(k0 + kk, n), n);
-        double s[8];
-        const int b0 = start[K], e = start[K + 1];
-        if (e - b0 > 32) {
-            na_long_key(b0, e, n, dxi, x, y, z, s);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) s[c] = 0.0;
-            for (int q = b0; q < e; ++q) na_add_weights(q, n, dxi, x, y, z, s);
-        }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) part[kl * 8 + c] = s[c];
-    }
-    __syncthreads();
-    for (int cl = threadIdx.x; cl < kTx * kTy * kTz; cl += blockDim.x) {
-        const int ci = cl % kTx, cj = (cl / kTx) % kTy, ck = cl / (kTx * kTy);
-        const int i = i0 + ci, j = j0 + cj, k = k0 + ck;
-        if (i >= n || j >= n || k >= n) continue;
-        double acc = 0.0;
-#pragma unroll
-        for (int dk = 0; dk < 2; ++dk)
-#pragma unroll
-            for (int dj = 0; dj < 2; ++dj)
-#pragma unroll
-                for (int di = 0; di < 2; ++di) {
-                    const int kl = (ci + di) + kKx * ((cj + dj) + kKy * (ck + dk));
-                    acc = acc + part[kl * 8 + (1 - di) + 2 * (1 - dj) + 4 * (1 - dk)];
-                }
-        rho[cidx(i, j, k, n)] = acc * scale;
+    na_heavy_keys((blockIdx.x * 256 + threadIdx.x) >> 5, gridDim.x * 8, n, dxi, x, y, z, nullptr, start, long_list,
+                  *long_count, count, heavy);
+}
+
+// segment s .. s + len of perm into ascending order, by the calling group of `width`
+// threads, t the thread's number in it; tmp: scratch of the same extent
+__device__ __forceinline__ void na_rank(const int* perm, int* tmp, int s, int len, int t, int width)
+{
+    for (int i = t; i < len; i += width) {
+        const int v = perm[s + i];
+        int rank = 0;
+        for (int u = 0; u < len; ++u) rank += perm[s + u] < v;
+        tmp[s + rank] = v;
     }
 }
+
+__global__ void __launch_bounds__(kNaThreads, 1) na_sort(int np, int n, double dxi, const double* __restrict__ x,
+                                                         const double* __restrict__ y, const double* __restrict__ z,
+                                                         int* key, int* count, int* start, int* perm, int* long_list,
+                                                         int* long_count, int* bad)
+{
+    __shared__ int part[kClCtas];
+    const int rank = cl_rank(), lane = threadIdx.x & 31;
+    const int nc = n * n * n, gt = rank * kNaThreads + threadIdx.x;
+    constexpr int kAll = kClCtas * kNaThreads;
+    for (int c = gt; c < nc; c += kAll) count[c] = 0;
+    if (gt == 0) *long_count = 0;
+    if (gt == 1) *bad = 0;
+    cl_barrier();
+    for (int q = gt; q < np; q += kAll) {
+        const double px = x[q], py = y[q], pz = z[q];
+        if (!(isfinite(px) && isfinite(py) && isfinite(pz))) atomicAdd(bad, 1);
+        double f;
+        const int K = (int)cidx(na_key1(px, dxi, n, &f), na_key1(py, dxi, n, &f), na_key1(pz, dxi, n, &f), n);
+        key[q] = K;
+        atomicAdd(count + K, 1);
+    }
+    cl_barrier();
+    // scan: each thread a run of consecutive cells, each CTA a slice
+    const int ipt = (nc + kAll - 1) / kAll, c0 = gt * ipt;
+    int sum = 0;
+    for (int i = 0; i < ipt; ++i)
+        if (c0 + i < nc) sum += count[c0 + i];
+    int total;
+    int run = na_block_scan(sum, &total);
+    if (threadIdx.x < kClCtas) *cl_map(&part[rank], (int)threadIdx.x) = total;
+    cl_barrier();
+    for (int c = 0; c < rank; ++c) run += part[c];
+    for (int i = 0; i < ipt; ++i)
+        if (c0 + i < nc) {
+            start[c0 + i] = run;
+            run += count[c0 + i];
+        }
+    if (gt == 0) start[nc] = np;
+    cl_barrier();
+    for (int q = gt; q < np; q += kAll) {
+        const int K = key[q];
+        perm[start[K] + atomicSub(count + K, 1) - 1] = q;
+    }
+    cl_barrier();
+    for (int K = gt; K < nc; K += kAll) {
+        const int s = start[K], len = start[K + 1] - s;
+        if (len > 32) long_list[atomicAdd(long_count, 1)] = K;
+        else if (len > 1) sort_short_segment(perm, s, len);
+    }
+    cl_barrier();
+    const int longs = *(volatile int*)long_count;
+    for (int li = gt >> 5; li < longs; li += kAll >> 5) {
+        const int s = start[long_list[li]], len = start[long_list[li] + 1] - s;
+        if (len > kNaSeg) continue;
+        na_rank(perm, key, s, len, lane, 32);
+        __syncwarp();
+        for (int i = lane; i < len; i += 32) perm[s + i] = key[s + i];
+    }
+    for (int li = rank; li < longs; li += kClCtas) {
+        const int s = start[long_list[li]], len = start[long_list[li] + 1] - s;
+        if (len <= kNaSeg) continue;
+        __syncthreads();
+        na_rank(perm, key, s, len, threadIdx.x, kNaThreads);
+        __syncthreads();
+        for (int i = threadIdx.x; i < len; i += kNaThreads) perm[s + i] = key[s + i];
+    }
+    cl_barrier();
+    // the ranks' scratch (key) takes the long keys' sums
+    na_heavy_keys(gt >> 5, kAll >> 5, n, dxi, x, y, z, perm, start, long_list, longs, count,
+                  reinterpret_cast<double*>(key));
+}
+
+// Tiles of 8 x 8 x 4 cells, one block each: the eight corner sums of every key of the
+// tile's 9 x 9 x 5 window (a long key's from na_heavy_keys), then the cells.  The weights
+// are bound by the FP64 pipe, which one thread with a key of 32 particles keeps waiting
+// 35 us; so a warp takes 32 keys, numbers their particles densely over its lanes, one lane
+// computes one particle's weights into shared memory, and eight lanes per key, one per
+// corner, add them in sorted order (k_deposit_keys does the same).  Four planes, not
+// eight: 32^3 would be 64 tiles for 152 SMs.  The particles are perm's (null: in place).
+constexpr int kTx = 8, kTy = 8, kTz = 4;
+constexpr int kKx = kTx + 1, kKy = kTy + 1, kKz = kTz + 1;
+constexpr int kNKeys = kKx * kKy * kKz;
+constexpr int kDepWarps = 8;
+
+__global__ void __launch_bounds__(32 * kDepWarps) na_deposit(int n, double dxi, double scale,
+                                                             const double* __restrict__ x,
+                                                             const double* __restrict__ y,
+                                                             const double* __restrict__ z,
+                                                             const int* __restrict__ perm,
+                                                             const int* __restrict__ start,
+                                                             const int* __restrict__ slot,
+                                                             const double* __restrict__ heavy, double* rho)
+{
+    __shared__ double part[kNKeys * 8];
+    __shared__ double wbuf[kDepWarps][32][8];
+    pdl_wait();
+    pdl_trigger();
+    constexpr unsigned full = 0xffffffffu;
+    const int i0 = blockIdx.x * kTx, j0 = blockIdx.y * kTy, k0 = blockIdx.z * kTz;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, corner = lane & 7;
+    for (int kl0 = 32 * wid; kl0 < kNKeys; kl0 += 32 * kDepWarps) {
+        const int kl = kl0 + lane;
+        int b0 = 0, cnt = 0;
+        if (kl < kNKeys) {
+            const int ki = kl % kKx, kj = (kl / kKx) % kKy, kk = kl / (kKx * kKy);
+            const int K = (int)cidx(wrapi(i0 + ki, n), wrapi(j0 + kj, n), wrapi(k0 + kk, n), n);
+            b0 = start[K];
+            cnt = start[K + 1] - b0;
+            const bool longer = cnt > kDepositLanes;
+            const double* h = heavy + 8LL * (longer ? slot[K] : 0);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) part[kl * 8 + c] = longer ? h[c] : 0.0;
+            if (longer) cnt = 0;
+        }
+        const int incl = na_warp_scan(cnt), excl = incl - cnt;
+        const int total = __shfl_sync(full, incl, 31);
+        __syncwarp();
+        for (int base = 0; base < total; base += 32) {
+            // the lane whose key holds particle number q: the first whose inclusive count exceeds q
+            const int q = base + lane;
+            int o = 0;
+#pragma unroll
+            for (int bit = 16; bit >= 1; bit >>= 1) {
+                const int v = __shfl_sync(full, incl, o + bit - 1);
+                if (v <= q) o += bit;
+            }
+            const int ob0 = __shfl_sync(full, b0, o & 31), oex = __shfl_sync(full, excl, o & 31);
+            if (q < total) {
+                const int s = ob0 + (q - oex), p = perm ? perm[s] : s;
+                double fx, fy, fz;
+                na_key1(x[p], dxi, n, &fx);
+                na_key1(y[p], dxi, n, &fy);
+                na_key1(z[p], dxi, n, &fz);
+                const double sx[2] = {1.0 - fx, fx};
+                const double sy[2] = {1.0 - fy, fy};
+                const double sz[2] = {1.0 - fz, fz};
+#pragma unroll
+                for (int c = 0; c < 8; ++c) wbuf[wid][lane][c] = (sx[c & 1] * sy[(c >> 1) & 1]) * sz[c >> 2];
+            }
+            __syncwarp();
+            // eight rounds of four keys x eight corners
+#pragma unroll 1
+            for (int r = 0; r < 8; ++r) {
+                const int ow = 4 * r + (lane >> 3);
+                const int oi = __shfl_sync(full, incl, ow), oe = __shfl_sync(full, excl, ow);
+                const int lo = max(oe, base) - base, hi = min(oi, base + 32) - base;
+                if (lo < hi) {
+                    double a = part[(kl0 + ow) * 8 + corner];
+                    for (int t = lo; t < hi; ++t) a = a + wbuf[wid][t][corner];
+                    part[(kl0 + ow) * 8 + corner] = a;
+                }
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    const int cl = threadIdx.x;   // one cell per thread
+    const int ci = cl % kTx, cj = (cl / kTx) % kTy, ck = cl / (kTx * kTy);
+    const int i = i0 + ci, j = j0 + cj, k = k0 + ck;
+    if (i >= n || j >= n || k >= n) return;
+    double acc = 0.0;
+#pragma unroll
+    for (int dk = 0; dk < 2; ++dk)
+#pragma unroll
+        for (int dj = 0; dj < 2; ++dj)
+#pragma unroll
+            for (int di = 0; di < 2; ++di) {
+                const int kl = (ci + di) + kKx * ((cj + dj) + kKy * (ck + dk));
+                acc = acc + part[kl * 8 + (1 - di) + 2 * (1 - dj) + 4 * (1 - dk)];
+            }
+    rho[cidx(i, j, k, n)] = acc * scale;
+}
+
+static_assert(kTx * kTy * kTz == 32 * kDepWarps, "one cell per thread");
 
 }  // namespace
 
@@ -419,22 +591,50 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
     const double scale = mass * (1.0 / (dx * dx * dx));
     const unsigned pb = (unsigned)((np + 255) / 256);
     const unsigned cb = (unsigned)((nc + 255) / 256);
-    const int ntiles = (nc + kNaScanTile - 1) / kNaScanTile;
-    // the counts, the long-segment counter and the non-finite count must start at
-    // zero: the array keeps whatever the previous call (or an interrupted one) left
-    na_zero<<<cb, 256, 0, s>>>(count, nc);
-    na_zero<<<1, 32, 0, s>>>(long_count, 2);
-    na_keys<<<pb, 256, 0, s>>>(np, n, dxi, d_x, d_y, d_z, key, count, bad);
-    na_scan_reduce<<<ntiles, kNaScanT, 0, s>>>(count, nc, tiles);
-    na_scan_top<<<1, 1024, 0, s>>>(tiles, ntiles);
-    na_scan_down<<<ntiles, kNaScanT, 0, s>>>(count, nc, tiles, start);
-    na_scatter<<<pb, 256, 0, s>>>(np, key, start, count, perm);
-    na_fix_short<<<cb, 256, 0, s>>>(nc, start, perm, long_list, long_count);
-    na_fix_long<<<2 * sm_count, 512, 0, s>>>(start, long_list, long_count, perm, key);
-    na_gather<<<pb, 256, 0, s>>>(np, perm, d_x, d_y, d_z, xs, ys, zs);
     const dim3 grid((n + kTx - 1) / kTx, (n + kTy - 1) / kTy, (n + kTz - 1) / kTz);
-    na_deposit<<<grid, 256, 0, s>>>(n, dxi, scale, xs, ys, zs, start, d_rho);
-    const cudaError_t e = cudaGetLastError();
+    cudaError_t e;
+    if (np <= kNaClusterMax && nc <= kNaClusterMax) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kClCtas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kClCtas);
+        cfg.blockDim = dim3(kNaThreads);
+        cfg.stream = s;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, na_sort, (int)np, n, dxi, d_x, d_y, d_z, key, count, start, perm, long_list,
+                               long_count, bad);
+        if (e == cudaSuccess) {
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.gridDim = grid;
+            cfg.blockDim = dim3(256);
+            e = cudaLaunchKernelEx(&cfg, na_deposit, n, dxi, scale, d_x, d_y, d_z,
+                                   (const int*)perm, (const int*)start, (const int*)count, (const double*)key, d_rho);
+        }
+    } else {
+        const int ntiles = (nc + kNaScanTile - 1) / kNaScanTile;
+        // the counts, the long-segment counter and the non-finite count must start at
+        // zero: the array keeps whatever the previous call (or an interrupted one) left
+        na_zero<<<cb, 256, 0, s>>>(count, nc);
+        na_zero<<<1, 32, 0, s>>>(long_count, 2);
+        na_keys<<<pb, 256, 0, s>>>(np, n, dxi, d_x, d_y, d_z, key, count, bad);
+        na_scan_reduce<<<ntiles, kNaScanT, 0, s>>>(count, nc, tiles);
+        na_scan_top<<<1, 1024, 0, s>>>(tiles, ntiles);
+        na_scan_down<<<ntiles, kNaScanT, 0, s>>>(count, nc, tiles, start);
+        na_scatter<<<pb, 256, 0, s>>>(np, key, start, count, perm);
+        na_fix_short<<<cb, 256, 0, s>>>(nc, start, perm, long_list, long_count);
+        na_fix_long<<<2 * sm_count, 512, 0, s>>>(start, long_list, long_count, perm, key);
+        na_gather<<<pb, 256, 0, s>>>(np, perm, d_x, d_y, d_z, xs, ys, zs);
+        na_heavy<<<4 * sm_count, 256, 0, s>>>(n, dxi, xs, ys, zs, start, long_list, long_count, count, (double*)key);
+        na_deposit<<<grid, 256, 0, s>>>(n, dxi, scale, xs, ys, zs, nullptr, start, count,
+                                                                   (const double*)key, d_rho);
+        e = cudaSuccess;
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    else cudaGetLastError();
     if (e != cudaSuccess) {
         if (errbuf && errlen) std::snprintf(errbuf, errlen, "kernel launch failed: %s", cudaGetErrorString(e));
         return NYXPM_CUDA_ERROR;
