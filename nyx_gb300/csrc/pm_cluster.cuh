@@ -15,7 +15,9 @@
 // launch.  Whole solves from phi = 0: FP64 32^3 0.83 -> 0.55 ms, FP32 32^3 0.63 -> 0.28,
 // 64^3 0.80 -> 0.59 ms.  The limits on the edge: FP32 64^3 is what 16 CTAs' shared memory
 // holds; FP64 issues at 19 clocks per warp instruction and SM, so that 16 SMs smooth 48^3
-// in 6 us, twice a launch over the whole chip.
+// in 6 us, twice a launch over the whole chip.  (Integer sums, pm_sum6.cuh, lose here: on
+// coarse levels some lane of a warp nearly always needs the FP64 additions as well, a
+// 32^3 solve took 0.64 ms.)
 //
 // Every cell's arithmetic is that of the per-pass kernels (k_gsrb, k_restrict<1>,
 // k_prolong<1> and their FP32 forms), in the same order, so the bits are theirs.
@@ -289,6 +291,63 @@ __device__ __forceinline__ void cl_restrict(const ClLevel<T>& F, const ClLevel<T
     }
 }
 
+// the same, two coarse cells of a row at a time (half % 4 == 0): their red children in a
+// fine row are a pair of the row
+__device__ __forceinline__ void cl_restrict2(const ClLevel<float>& F, const ClLevel<float>* C, float* solo)
+{
+    const int n = F.n, half = n >> 1, nc = n >> 1, chalf = nc >> 1, plane = nc * chalf;
+    const int K0 = (F.p0 + 1) >> 1, nK = ((F.p0 + F.np + 1) >> 1) - K0;
+    const int total = chalf * nc * nK;
+    constexpr float sixth = 1.0f / 6.0f;
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        int t2, J, K;
+        cl_split(t, chalf, nc, t2, J, K);
+        K += K0;
+        const int c2 = 2 * t2;
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int dk = 0; dk < 2; ++dk)
+#pragma unroll
+            for (int dj = 0; dj < 2; ++dj) {
+                const int j = 2 * J + dj, q = 2 * K + dk - F.p0 + 1, odd = (dj + dk) & 1;
+                const int jm = j == 0 ? n - 1 : j - 1, jp = j == n - 1 ? 0 : j + 1;
+                const float* row = F.zb[q] + j * half;
+                auto pair = [&](const float* a) { return *reinterpret_cast<const float2*>(a + c2); };
+                const float2 c = pair(row), ym = pair(F.zb[q] + jm * half), yp = pair(F.zb[q] + jp * half);
+                const float2 zm = pair(F.zb[q - 1] + j * half), zp = pair(F.zb[q + 1] + j * half);
+                const float2 b = pair(F.br[q] + j * half), m = pair(F.zr[q] + j * half);
+                const float e = row[odd ? (c2 + 2 == half ? 0 : c2 + 2) : (c2 == 0 ? half - 1 : c2 - 1)];
+                const float x0 = odd ? c.x : e, x1 = odd ? c.y : c.x, x2 = odd ? e : c.y;
+                s0 = s0 + (b.x - fmaf(((((x0 + x1) + ym.x) + yp.x) + zm.x) + zp.x, sixth, -m.x));
+                s1 = s1 + (b.y - fmaf(((((x1 + x2) + ym.y) + yp.y) + zm.y) + zp.y, sixth, -m.y));
+            }
+        // coarse cells 2 t2 (colour of J + K) and 2 t2 + 1, both at compact t2
+        const int even_black = (J + K) & 1, o = t2 + chalf * J;
+        float *be, *bo;
+        int c = 0;
+        if (C) {
+            c = cl_owner(K, nc);
+            const int at = (K - cl_first(c, nc)) * plane + o;
+            be = (even_black ? C->beta_b : C->beta_r) + at;
+            bo = (even_black ? C->beta_r : C->beta_b) + at;
+        } else {
+            be = solo + (2 + even_black) * nc * plane + K * plane + o;
+            bo = solo + (3 - even_black) * nc * plane + K * plane + o;
+        }
+        *cl_map(be, c) = s0 * 0.5f;
+        *cl_map(bo, c) = s1 * 0.5f;
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void cl_restrict_any(const ClLevel<T>& F, const ClLevel<T>* C, T* solo)
+{
+    if constexpr (sizeof(T) == 4) {
+        if ((F.n & 7) == 0) return cl_restrict2(F, C, solo);
+    }
+    cl_restrict<T>(F, C, solo);
+}
+
 // the coarse planes a slab's prolongation reads, (p0 >> 1) - 1 on, into this CTA
 template <typename T>
 __device__ __forceinline__ void cl_stage(const ClLevel<T>& F, const ClLevel<T>* C, T* solo, T* stage, int cap)
@@ -296,17 +355,23 @@ __device__ __forceinline__ void cl_stage(const ClLevel<T>& F, const ClLevel<T>* 
     const int nc = F.n >> 1, chalf = nc >> 1, plane = nc * chalf;
     if (F.np == 0) return;
     const int Kf = (F.p0 >> 1) - 1, nK = ((F.p0 + F.np - 1) >> 1) + 1 - Kf + 1;
-    for (int t = threadIdx.x; t < 2 * nK * plane; t += blockDim.x) {
-        const int color = t >= nK * plane ? 1 : 0, u = t - color * nK * plane;
-        const int k = u / plane, o = u - k * plane, K = (Kf + k + nc) % nc;
-        T v;
+    // whole 16-byte words where a plane is a number of them
+    constexpr int kW = 16 / sizeof(T);
+    const int w = plane % kW == 0 ? kW : 1, pw = plane / w;
+    for (int t = threadIdx.x; t < 2 * nK * pw; t += blockDim.x) {
+        int o, k, color;
+        cl_split(t, pw, nK, o, k, color);
+        const int K = (Kf + k + nc) % nc;
+        const T* src;
         if (C) {
             const int c = cl_owner(K, nc);
-            v = *cl_map((color ? C->phi_b : C->phi_r) + (K - cl_first(c, nc)) * plane + o, c);
+            src = cl_map((color ? C->phi_b : C->phi_r) + (K - cl_first(c, nc)) * plane + o * w, c);
         } else {
-            v = *cl_map(solo + color * nc * plane + K * plane + o, 0);
+            src = cl_map(solo + color * nc * plane + K * plane + o * w, 0);
         }
-        stage[color * cap + u] = v;
+        T* dst = stage + color * cap + k * plane + o * w;
+        if (w == kW) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
+        else *dst = *src;
     }
 }
 
@@ -408,7 +473,7 @@ __device__ __forceinline__ void cl_vcycle(const ClArgs<T>& A, ClShared<T>& S, T*
             cl_barrier();
         }
         const bool last = l + 1 == A.nd;
-        cl_restrict<T>(S.lv[l], last ? nullptr : &S.lv[l + 1], S.solo[0].base);
+        cl_restrict_any<T>(S.lv[l], last ? nullptr : &S.lv[l + 1], S.solo[0].base);
         cl_barrier();
     }
     if (rank == 0) vcycle_solo<T>(S.solo, A.ns, A.nu1, A.nu2, S.g, A.nb, mem + A.stage, true);
