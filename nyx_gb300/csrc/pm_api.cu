@@ -462,30 +462,33 @@ nyxpm_status nyxpm_box_upload(nyxpm_ctx* c, nyxpm_box* b, const double* pos, con
     CHECK_BOX(c, b);
     if (!pos || !vel) return fail(c, NYXPM_INVALID_ARG, "null pos/vel");
     const int64_t np = b->np;
-    double total = 0.0;
-    if (mass) {
-        for (int64_t q = 0; q < np; ++q) {
-            if (!(mass[q] >= 0) || !std::isfinite(mass[q])) return fail(c, NYXPM_INVALID_ARG, "bad mass");
-            total = total + mass[q];
-        }
-    } else {
-        if (!(mass_scalar >= 0) || !std::isfinite(mass_scalar)) return fail(c, NYXPM_INVALID_ARG, "bad mass");
-        total = mass_scalar * (double)np;
-    }
-    b->uniform_mass = mass ? 0 : 1;
-    b->mscalar = mass ? 0.0 : mass_scalar;
-    b->mass_offset = total / (b->L * b->L * b->L);
+    if (!mass && (!(mass_scalar >= 0) || !std::isfinite(mass_scalar))) return fail(c, NYXPM_INVALID_ARG, "bad mass");
+    // the copies into the staging area run while the host adds up the masses
     double* d_pos = b->staging;
     double* d_vel = b->staging + 3 * np;
     cudaMemcpyAsync(d_pos, pos, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(d_vel, vel, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, c->stream);
     const double* d_mass = nullptr;
+    double total = mass_scalar * (double)np;
     if (mass) {
         double* dm = b->staging + 6 * np;
         cudaMemcpyAsync(dm, mass, sizeof(double) * np, cudaMemcpyHostToDevice, c->stream);
         d_mass = dm;
+        bool ok = true;
+        total = 0.0;
+        for (int64_t q = 0; q < np; ++q) {
+            ok = ok && mass[q] >= 0 && std::isfinite(mass[q]);
+            total = total + mass[q];
+        }
+        if (!ok) {
+            cudaStreamSynchronize(c->stream);   // the caller's arrays are the caller's again
+            return fail(c, NYXPM_INVALID_ARG, "bad mass");
+        }
     }
     TRY(check_launch(*c, "upload copy"));
+    b->uniform_mass = mass ? 0 : 1;
+    b->mscalar = mass ? 0.0 : mass_scalar;
+    b->mass_offset = total / (b->L * b->L * b->L);
     cudaMemsetAsync(b->norms + 2, 0, sizeof(unsigned long long), c->stream);
     if (b->prec == NYXPM_MIXED) TRY(mixed_unpack(*c, *b, d_pos, d_vel, d_mass));
     else TRY(launch_unpack(*c, *b, d_pos, d_vel, d_mass));
@@ -859,13 +862,19 @@ nyxpm_status nyxpm_est_time_step(nyxpm_ctx* c, nyxpm_box* b, double cfl, double 
     }
     if (!b->have_phi && !b->g_from_caller)
         return fail(c, NYXPM_INVALID_ARG, "no field: solve, step, set phi or set the gravity vector first");
-    TRY(b->prec == NYXPM_MIXED ? mixed_est_dt(*c, *b, cfl, a) : launch_est_dt(*c, *b, cfl, a));
-    cudaMemcpyAsync(b->h_norms + 3, b->norms + 3, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+    TRY(b->prec == NYXPM_MIXED ? mixed_est_dt(*c, *b) : launch_est_dt(*c, *b));
+    cudaMemcpyAsync(b->h_norms + 3, b->norms + 3, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                     c->stream);
     TRY(check_launch(*c, "time-step readback"));
     TRY(nyxpm_synchronize(c));
-    const unsigned long long bits = ~b->h_norms[3];
-    std::memcpy(dt, &bits, sizeof(double));
+    double v, g2;
+    std::memcpy(&v, &b->h_norms[3], sizeof(double));
+    std::memcpy(&g2, &b->h_norms[5], sizeof(double));
+    const double um = v * (b->dxi / a), ga = std::sqrt(g2);
+    double limit = 1.0e50;
+    if (um > 0) limit = std::min(limit, cfl / um);
+    if (ga > 0) limit = std::min(limit, 1.0 / std::sqrt(ga * b->dxi));
+    *dt = limit;
     return NYXPM_OK;
 }
 

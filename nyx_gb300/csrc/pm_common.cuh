@@ -161,6 +161,13 @@ __host__ __device__ inline unsigned long long absbits(double v)
 #endif
 }
 
+// the same, a NaN counting as 0
+__device__ __forceinline__ unsigned long long number_bits(double v)
+{
+    const unsigned long long u = absbits(v);
+    return u > 0x7ff0000000000000ULL ? 0ULL : u;
+}
+
 // block max of bits into *out (blocks are whole warps)
 __device__ inline void block_umax_store(unsigned long long v, unsigned long long* out)
 {
@@ -455,7 +462,7 @@ struct Box {
     double* planes = nullptr;          // n plane sums
     double* scal = nullptr;            // [0] mean
     unsigned long long* norms = nullptr;   // [0] ||rhs||inf, [1] ||r||inf, [2] bad uploads,
-                                           // [3] time-step limit, [4] mixed: max |e|,
+                                           // [3], [5] time-step limit, [4] mixed: max |e|,
                                            // [5] .. [7] a cluster solve's result
     unsigned long long* h_norms = nullptr; // pinned host mirror
     double* G = nullptr;               // bottom Green's function (smoother units)
@@ -554,9 +561,9 @@ nyxpm_status launch_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur,
                          int do_wrap);
 
 nyxpm_status launch_make_rhs(Ctx& c, Box& b, double a);
-// particle time-step limit into norms[3] (as ~bits of the minimum dt)
-nyxpm_status launch_est_dt(Ctx& c, Box& b, double cfl, double a);
-nyxpm_status mixed_est_dt(Ctx& c, Box& b, double cfl, double a);
+// the particle time-step limit's maxima: |v_d| into norms[3], |g|^2 into norms[5]
+nyxpm_status launch_est_dt(Ctx& c, Box& b);
+nyxpm_status mixed_est_dt(Ctx& c, Box& b);
 double beta_scale(const Box& b);  // (h*h)/6 of level 0: rhs -> smoother units
 nyxpm_status launch_zero_phi(Ctx& c, Box& b);
 nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info);

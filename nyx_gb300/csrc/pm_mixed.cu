@@ -1638,34 +1638,29 @@ nyxpm_status launch_mx_update(Ctx& c, Box& b)
     return check_launch(c, "mixed update");
 }
 
-// particle time-step limit of the mixed form: the same formula as the FP64
-// form (NyxParticleContainer.H:329-465), from the FP32 velocities and the FP32
-// gravity vector the kicks use, evaluated in FP64; the cell is the particle's
-// stored cell (floor(x*dxi)).  out must start at 0 (complemented-bits max).
-__global__ void __launch_bounds__(256) k_mx_est_dt(long long np, int n, double dxi, double adxi,
-                                                   double cfl, const int* __restrict__ cell,
+// particle time-step limit of the mixed form: the same formula and maxima as the FP64
+// form (k_est_dt), from the FP32 velocities and the FP32 gravity vector the kicks use,
+// widened; the cell is the particle's stored cell (floor(x*dxi)).
+__global__ void __launch_bounds__(256) k_mx_est_dt(long long np, int n, const int* __restrict__ cell,
                                                    const float* __restrict__ vx,
                                                    const float* __restrict__ vy,
                                                    const float* __restrict__ vz,
                                                    const float* __restrict__ g,
-                                                   unsigned long long* out)
+                                                   unsigned long long* out_v, unsigned long long* out_g)
 {
-    double best = 1.0e50;
+    unsigned long long gmax = 0;
+    float vmax = 0.f;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < np;
          q += (long long)gridDim.x * blockDim.x) {
         const int cq = cell[q];
-        const double ux = fabs((double)vx[q]) * adxi, uy = fabs((double)vy[q]) * adxi,
-                     uz = fabs((double)vz[q]) * adxi;
-        const double um = fmax(fmax(ux, uy), uz);
-        double dtp = um > 0 ? cfl / um : 1.0e50;
+        vmax = fmaxf(vmax, fmaxf(fmaxf(fabsf(vx[q]), fabsf(vy[q])), fabsf(vz[q])));
         const long long c = cidx(cell_i(cq), cell_j(cq), cell_k(cq), n);
         const float4 gc = __ldg(reinterpret_cast<const float4*>(g) + c);
         const double gx = gc.x, gy = gc.y, gz = gc.z;
-        const double ga = sqrt((gx * gx + gy * gy) + gz * gz);
-        if (ga > 0) dtp = fmin(dtp, 1.0 / sqrt(ga * dxi));
-        best = fmin(best, dtp);
+        gmax = max(gmax, number_bits((gx * gx + gy * gy) + gz * gz));
     }
-    block_umax_store(~(unsigned long long)__double_as_longlong(best), out);
+    block_umax_store(number_bits(f32_to_f64(vmax)), out_v);
+    block_umax_store(gmax, out_g);
 }
 
 }  // namespace
@@ -2004,12 +1999,13 @@ nyxpm_status mixed_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur, 
     return check_launch(c, "mixed kick");
 }
 
-nyxpm_status mixed_est_dt(Ctx& c, Box& b, double cfl, double a)
+nyxpm_status mixed_est_dt(Ctx& c, Box& b)
 {
     cudaMemsetAsync(b.norms + 3, 0, sizeof(unsigned long long), c.stream);
+    cudaMemsetAsync(b.norms + 5, 0, sizeof(unsigned long long), c.stream);
     const unsigned blocks = std::min(blocks_for(b.np), (unsigned)(c.sm_count * 8));
-    k_mx_est_dt<<<blocks, kThreads, 0, c.stream>>>(b.np, b.n, b.dxi, b.dxi / a, cfl, b.cell, b.fvx,
-                                                    b.fvy, b.fvz, b.g32, b.norms + 3);
+    k_mx_est_dt<<<blocks, kThreads, 0, c.stream>>>(b.np, b.n, b.cell, b.fvx, b.fvy, b.fvz, b.g32, b.norms + 3,
+                                                    b.norms + 5);
     c.launches += 1;
     return check_launch(c, "mixed time-step estimate");
 }
