@@ -36,6 +36,7 @@
 // per cell, ghost cell, record or particle.
 // Built with --fmad=false: only the explicit fma() calls fuse.
 #include "pm_common.cuh"
+#include "pm_sum6.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -56,12 +57,29 @@ constexpr double kSixth = 1.0 / 6.0;
 __constant__ double kAmrProlongW[8] = {0.421875, 0.140625, 0.140625, 0.046875,
                                        0.140625, 0.046875, 0.046875, 0.015625};
 
+// n / d for n < 2^31 as a product and a shift: m = floor(2^sh / d) + 1 with
+// sh = 31 + ceil(log2 d) (Granlund & Montgomery 1994); a cell's number is divided twice
+// in every kernel over fine cells
+struct Divisor {
+    unsigned m;
+    int sh;
+    __host__ void set(unsigned d)
+    {
+        int l = 0;
+        while ((1ull << l) < d) ++l;
+        sh = 31 + l;
+        m = (unsigned)((1ull << sh) / d + 1);
+    }
+    __host__ __device__ unsigned div(unsigned n) const { return (unsigned)(((unsigned long long)n * m) >> sh); }
+};
+
 struct ABox {
     int lev;
     int lo[3], hi[3];
     int d[3];          // padded extents
     int pbox;          // the coarser box holding this box's parents (-1: level 0; -2: several)
     long long off;     // first padded cell in the composite layout
+    Divisor nx, hx, ny;   // by the cells of a row, half of them, the rows of a plane
 };
 
 struct ACell {
@@ -92,12 +110,17 @@ struct AFace {
 struct AFRec {
     long long C;
     int first, count;
+    int lev, pad;      // C's level
 };
 
 struct APar {
     long long pc;      // parent's composite index
     int sx, sxy;       // strides of the parent's box (0: the parent is on level 0)
 };
+
+// flags of a valid cell
+constexpr unsigned char kCovered = 1;    // by the next finer level
+constexpr unsigned char kRefluxed = 2;   // uncovered, beside a covered cell: its residual is refluxed
 
 struct BoxTab {
     const ABox* box;
@@ -346,6 +369,8 @@ __global__ void k_amr_scalef(long long nc, const ACell* __restrict__ cells, cons
 __global__ void k_amr_sum8(long long nr, const ARRec* __restrict__ r, const double* __restrict__ src, double s,
                            double* dst)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nr) return;
     const ARRec R = r[t];
@@ -376,7 +401,7 @@ __global__ void k_amr_usum0(long long n3, const double* __restrict__ rho, const 
                             double mo, double* out)
 {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const double v = (q < n3 && !cov[q]) ? rho[q] - mo : 0.0;
+    const double v = (q < n3 && !(cov[q] & kCovered)) ? rho[q] - mo : 0.0;
     block_add(v, out);
 }
 
@@ -385,7 +410,7 @@ __global__ void k_amr_usumf(long long nc, const ACell* __restrict__ cells, const
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0.0;
-    if (t < nc && !cov[cells[t].q]) v = rho[cells[t].q] - mo;
+    if (t < nc && !(cov[cells[t].q] & kCovered)) v = rho[cells[t].q] - mo;
     block_add(v, out);
 }
 
@@ -422,6 +447,8 @@ __global__ void k_amr_betaf(long long nc, const ACell* __restrict__ cells, const
 // ghost cells: f[dst] = sum of w * f[src] over the ghost's stencil (sources are valid cells)
 __global__ void k_amr_ghost(long long ng, const AGhost* __restrict__ gh, const AEnt* __restrict__ ent, double* f)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ng) return;
     const AGhost G = gh[t];
@@ -448,33 +475,66 @@ __global__ void k_amr_ghost3(long long ng, const AGhost* __restrict__ gh, const 
     f2[G.dst] = v2;
 }
 
-// out = rhs - (s/6 - u), s the 6 neighbours in the order xm + xp, ym, yp, zm, zp
-__global__ void k_amr_resid0(int n, const double* __restrict__ u, const double* __restrict__ rhs, double* out)
+// max |f| * inv_scale over the uncovered cells into out (as the bits of a
+// non-negative double): a block maximum, then one atomic per block
+__device__ __forceinline__ void block_umax(unsigned long long v, unsigned long long* out)
 {
+    __shared__ unsigned long long part[kT / 32];
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, off);
+        v = o > v ? o : v;
+    }
+    const unsigned tid = threadIdx.x + blockDim.x * threadIdx.y;   // blocks of kT threads
+    if ((tid & 31) == 0) part[tid >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int w = 1; w < kT / 32; ++w) v = part[w] > v ? part[w] : v;
+        if (v != 0ULL) atomicMax(out, v);
+    }
+}
+
+// (the maximum is taken over the bit patterns: equal to the maximum of the
+// non-negative values, and a NaN, whose bits are above every number's, wins)
+__device__ __forceinline__ unsigned long long umax_bits(unsigned long long v, double x)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    return u > v ? u : v;
+}
+
+// The composite residual of level 0, out = rhs - (s/6 - u), s the 6 neighbours in the order
+// xm + xp, ym, yp, zm, zp, and the maximum of |out| inv_scale over the cells that are
+// neither covered nor refluxed into norm.  INT: sums on the integer pipes (pm_sum6.cuh).
+template <bool INT>
+__global__ void __launch_bounds__(kT) k_amr_resid0(int n, const double* __restrict__ u, const double* __restrict__ rhs,
+                                                   const unsigned char* __restrict__ cov, double inv_scale, double* out,
+                                                   unsigned long long* norm)
+{
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
-    if (i >= n || j >= n) return;
-    const int im = i == 0 ? n - 1 : i - 1, ip = i == n - 1 ? 0 : i + 1;
-    const int jm = j == 0 ? n - 1 : j - 1, jp = j == n - 1 ? 0 : j + 1;
-    const int km = k == 0 ? n - 1 : k - 1, kp = k == n - 1 ? 0 : k + 1;
-    double s = u[cidx(im, j, k, n)] + u[cidx(ip, j, k, n)];
-    s = s + u[cidx(i, jm, k, n)];
-    s = s + u[cidx(i, jp, k, n)];
-    s = s + u[cidx(i, j, km, n)];
-    s = s + u[cidx(i, j, kp, n)];
-    const long long q = cidx(i, j, k, n);
-    out[q] = rhs[q] - fma(s, kSixth, -u[q]);
+    unsigned long long v = 0ULL;
+    if (i < n && j < n) {
+        const int im = i == 0 ? n - 1 : i - 1, ip = i == n - 1 ? 0 : i + 1;
+        const int jm = j == 0 ? n - 1 : j - 1, jp = j == n - 1 ? 0 : j + 1;
+        const int km = k == 0 ? n - 1 : k - 1, kp = k == n - 1 ? 0 : k + 1;
+        const double nb[6] = {u[cidx(im, j, k, n)], u[cidx(ip, j, k, n)], u[cidx(i, jm, k, n)],
+                              u[cidx(i, jp, k, n)], u[cidx(i, j, km, n)], u[cidx(i, j, kp, n)]};
+        const long long q = cidx(i, j, k, n);
+        const double r = rhs[q] - fma(sum6(nb, INT && sum6_on_int()), kSixth, -u[q]);
+        out[q] = r;
+        if (cov[q] == 0) v = umax_bits(v, fabs(r) * inv_scale);
+    }
+    block_umax(v, norm);
 }
 
+template <bool INT>
 __device__ __forceinline__ double nbr_fine(const double* __restrict__ u, long long q, long long sx, long long sxy)
 {
-    double s = u[q - 1] + u[q + 1];
-    s = s + u[q - sx];
-    s = s + u[q + sx];
-    s = s + u[q - sxy];
-    s = s + u[q + sxy];
-    return s;
+    const double nb[6] = {u[q - 1], u[q + 1], u[q - sx], u[q + sx], u[q - sxy], u[q + sxy]};
+    return sum6(nb, INT && sum6_on_int());
 }
 
 // Fine cells are numbered box by box (x fastest), boxes in level order;
@@ -504,9 +564,9 @@ __device__ __forceinline__ long long fine_cell(const ABox* __restrict__ boxes, c
     // a box holds fewer than 2^31 cells: 32-bit index arithmetic
     const unsigned r = (unsigned)(g - pref[b]);
     const unsigned nx = (unsigned)(B.hi[0] - B.lo[0] + 1), ny = (unsigned)(B.hi[1] - B.lo[1] + 1);
-    const unsigned row = r / nx;
+    const unsigned row = B.nx.div(r);
     const int u = (int)(r - row * nx);
-    const unsigned k = row / ny;
+    const unsigned k = B.ny.div(row);
     const int j = (int)(row - k * ny);
     return box_idx(B, B.lo[0] + u, B.lo[1] + j, B.lo[2] + (int)k);
 }
@@ -520,9 +580,9 @@ __device__ __forceinline__ long long fine_color_cell(const ABox* __restrict__ bo
     const ABox& B = boxes[b];
     const unsigned r = (unsigned)(g - (pref[b] >> 1));
     const unsigned hx = (unsigned)(B.hi[0] - B.lo[0] + 1) >> 1, ny = (unsigned)(B.hi[1] - B.lo[1] + 1);
-    const unsigned row = r / hx;
+    const unsigned row = B.hx.div(r);
     const int tp = (int)(r - row * hx);
-    const unsigned kk = row / ny;
+    const unsigned kk = B.ny.div(row);
     const int j = B.lo[1] + (int)(row - kk * ny), k = B.lo[2] + (int)kk;
     const int i = B.lo[0] + 2 * tp + ((col - B.lo[0] - j - k) & 1);
     if (ijk) {
@@ -533,54 +593,117 @@ __device__ __forceinline__ long long fine_color_cell(const ABox* __restrict__ bo
     return box_idx(B, i, j, k);
 }
 
-// out = rhs - (s/6 - u) on the n fine cells from box b0
-__global__ void k_amr_residf(long long n, int b0, int nb, const long long* __restrict__ pref,
-                             const ABox* __restrict__ boxes, const double* __restrict__ u,
-                             const double* __restrict__ rhs, double* out)
+// the composite residual and its norm on the n fine cells from box b0, as k_amr_resid0
+template <bool INT>
+__global__ void __launch_bounds__(kT) k_amr_residf(long long n, int b0, int nb, const long long* __restrict__ pref,
+                                                   const ABox* __restrict__ boxes, const double* __restrict__ u,
+                                                   const double* __restrict__ rhs,
+                                                   const unsigned char* __restrict__ cov,
+                                                   const double* __restrict__ inv_scale, double* out,
+                                                   unsigned long long* norm)
+{
+    pdl_wait();
+    pdl_trigger();
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long v = 0ULL;
+    if (t < n) {
+        int b;
+        const long long q = fine_cell(boxes, pref, b0, nb, t, b);
+        const long long sx = boxes[b].d[0], sxy = (long long)boxes[b].d[0] * boxes[b].d[1];
+        const double r = rhs[q] - fma(nbr_fine<INT>(u, q, sx, sxy), kSixth, -u[q]);
+        out[q] = r;
+        if (cov[q] == 0) v = umax_bits(v, fabs(r) * inv_scale[boxes[b].lev]);
+    }
+    block_umax(v, norm);
+}
+
+// out = rhs - (s/6 - u) alone (nu1 = 0: the restriction takes every child's residual)
+__global__ void k_amr_resid_all(long long n, int b0, int nb, const long long* __restrict__ pref,
+                                const ABox* __restrict__ boxes, const double* __restrict__ u,
+                                const double* __restrict__ rhs, double* out)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int b;
     const long long q = fine_cell(boxes, pref, b0, nb, t, b);
     const long long sx = boxes[b].d[0], sxy = (long long)boxes[b].d[0] * boxes[b].d[1];
-    out[q] = rhs[q] - fma(nbr_fine(u, q, sx, sxy), kSixth, -u[q]);
+    out[q] = rhs[q] - fma(nbr_fine<false>(u, q, sx, sxy), kSixth, -u[q]);
 }
 
-// one colour of a Gauss-Seidel sweep on the n colour cells from box b0
-__global__ void k_amr_gsrbf(long long n, int b0, int nb, const long long* __restrict__ pref,
-                            const ABox* __restrict__ boxes, int col, double* e, const double* __restrict__ R)
+// The restriction after pre-smoothing: R of a covered coarse cell = half the sum of its
+// children's residuals.  The last half sweep was black, so the black children's residuals
+// are its round-off; the 4 red children are summed in (dk, dj) order, as the single-level
+// restriction does.  One pass in place of a residual array and a pass over it.
+template <bool INT>
+__global__ void __launch_bounds__(kT) k_amr_restrict_red(long long nr, const ARRec* __restrict__ recs,
+                                                         const double* __restrict__ e, double* R)
 {
+    pdl_wait();
+    pdl_trigger();
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nr) return;
+    const ARRec r = recs[t];
+    double s = 0.0;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        const int dj = c & 1, dk = c >> 1;
+        const long long q = r.c0 + (dj ^ dk) + (long long)dj * r.sx + (long long)dk * r.sxy;
+        s = s + (R[q] - fma(nbr_fine<INT>(e, q, r.sx, r.sxy), kSixth, -e[q]));
+    }
+    R[r.P] = s * 0.5;
+}
+
+// one colour of a Gauss-Seidel sweep on the n colour cells from box b0; zero: the first red
+// half sweep from e = 0 (e is not read)
+template <bool INT>
+__global__ void __launch_bounds__(kT) k_amr_gsrbf(long long n, int b0, int nb, const long long* __restrict__ pref,
+                                                  const ABox* __restrict__ boxes, int col, int zero, double* e,
+                                                  const double* __restrict__ R)
+{
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int b;
     const long long q = fine_color_cell(boxes, pref, b0, nb, t, col, b);
     const long long sx = boxes[b].d[0], sxy = (long long)boxes[b].d[0] * boxes[b].d[1];
-    e[q] = fma(nbr_fine(e, q, sx, sxy), kSixth, -R[q]);
+    e[q] = fma(zero ? 0.0 : nbr_fine<INT>(e, q, sx, sxy), kSixth, -R[q]);
 }
 
-// R(C) -= ((sum_k (u(f_k) - u(g_k))) / 2 - (u(N) - u(C))) / 6 at each coarse/fine face of C
-__global__ void k_amr_reflux(long long nr, const AFRec* __restrict__ recs, const AFace* __restrict__ faces,
-                             const double* __restrict__ u, double* R)
+// R(C) -= ((sum_k (u(f_k) - u(g_k))) / 2 - (u(N) - u(C))) / 6 at each coarse/fine face of C;
+// with norm, the maximum of |R| inv_scale over these cells into it
+__global__ void __launch_bounds__(kT) k_amr_reflux(long long nr, const AFRec* __restrict__ recs,
+                                                   const AFace* __restrict__ faces, const double* __restrict__ u,
+                                                   double* R, const double* __restrict__ inv_scale,
+                                                   unsigned long long* norm)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nr) return;
-    const AFRec r = recs[t];
-    double v = R[r.C];
-    for (int f = r.first; f < r.first + r.count; ++f) {
-        const AFace& F = faces[f];
-        double s = u[F.f[0]] - u[F.g[0]];
-        s = s + (u[F.f[1]] - u[F.g[1]]);
-        s = s + (u[F.f[2]] - u[F.g[2]]);
-        s = s + (u[F.f[3]] - u[F.g[3]]);
-        v = v - (((s * 0.5) - (u[F.N] - u[r.C])) * kSixth);
+    unsigned long long m = 0ULL;
+    if (t < nr) {
+        const AFRec r = recs[t];
+        double v = R[r.C];
+        for (int f = r.first; f < r.first + r.count; ++f) {
+            const AFace& F = faces[f];
+            double s = u[F.f[0]] - u[F.g[0]];
+            s = s + (u[F.f[1]] - u[F.g[1]]);
+            s = s + (u[F.f[2]] - u[F.g[2]]);
+            s = s + (u[F.f[3]] - u[F.g[3]]);
+            v = v - (((s * 0.5) - (u[F.N] - u[r.C])) * kSixth);
+        }
+        R[r.C] = v;
+        m = umax_bits(m, fabs(v) * inv_scale[r.lev]);
     }
-    R[r.C] = v;
+    if (norm) block_umax(m, norm);
 }
 
 // e += the trilinear prolongation of the coarser level's e
 __global__ void k_amr_prolong(long long nc, const ACell* __restrict__ cells, const APar* __restrict__ par, int n0,
                               double* e)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nc) return;
     const ACell c = cells[t];
@@ -608,6 +731,8 @@ __global__ void k_amr_prolong(long long nc, const ACell* __restrict__ cells, con
 __global__ void k_amr_prolong_black(long long n, int b0, int nb, const long long* __restrict__ pref,
                                     const ABox* __restrict__ boxes, int n0, double* e)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int b, c[3];
@@ -636,34 +761,10 @@ __global__ void k_amr_prolong_black(long long n, int b0, int nb, const long long
 
 __global__ void k_amr_add(long long n, double* phi, const double* __restrict__ e)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q < n) phi[q] = phi[q] + e[q];
-}
-
-// max |f| * inv_scale over the uncovered cells into out (as the bits of a
-// non-negative double): a block maximum, then one atomic per block
-__device__ __forceinline__ void block_umax(unsigned long long v, unsigned long long* out)
-{
-    __shared__ unsigned long long part[kT / 32];
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, off);
-        v = o > v ? o : v;
-    }
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = part[w] > v ? part[w] : v;
-        if (v != 0ULL) atomicMax(out, v);
-    }
-}
-
-// (the maximum is taken over the bit patterns: equal to the maximum of the
-// non-negative values, and a NaN, whose bits are above every number's, wins)
-__device__ __forceinline__ unsigned long long umax_bits(unsigned long long v, double x)
-{
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    return u > v ? u : v;
 }
 
 __global__ void k_amr_absmax0(long long n3, const double* __restrict__ f, const unsigned char* __restrict__ cov,
@@ -671,7 +772,7 @@ __global__ void k_amr_absmax0(long long n3, const double* __restrict__ f, const 
 {
     unsigned long long v = 0ULL;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n3; q += (long long)gridDim.x * blockDim.x)
-        if (!cov[q]) v = umax_bits(v, fabs(f[q]) * inv_scale);
+        if (!(cov[q] & kCovered)) v = umax_bits(v, fabs(f[q]) * inv_scale);
     block_umax(v, out);
 }
 
@@ -684,7 +785,7 @@ __global__ void k_amr_absmaxf(long long n, int b0, int nb, const long long* __re
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         int b;
         const long long q = fine_cell(boxes, pref, b0, nb, t, b);
-        if (!cov[q]) v = umax_bits(v, fabs(f[q]) * inv_scale[boxes[b].lev]);
+        if (!(cov[q] & kCovered)) v = umax_bits(v, fabs(f[q]) * inv_scale[boxes[b].lev]);
     }
     block_umax(v, out);
 }
@@ -778,6 +879,7 @@ struct nyxpm_amr {
     unsigned long long* norms = nullptr;     // [0] ||beta||, [1] ||r||, [2] move errors
     unsigned long long* h_norms = nullptr;
     nyxpm_box* mg = nullptr;                 // level 0's multigrid hierarchy
+    IterGraph iter_graph;                    // a composite V-cycle, its residual and the norm's copy
     std::vector<void*> allocs;
 };
 
@@ -958,7 +1060,7 @@ nyxpm_status build_lists(nyxpm_ctx* c, nyxpm_amr* a)
         A.frec[l].first = (long long)frec.size();
         auto faces_of = [&](int i, int j, int k, long long C) {
             if (Bd.covered(l - 1, i, j, k)) return;
-            AFRec r{C, (int)face.size(), 0};
+            AFRec r{C, (int)face.size(), 0, l - 1, 0};
             const int n = A.n0 << (l - 1);
             for (int d = 0; d < 3; ++d)
                 for (int s = -1; s <= 1; s += 2) {
@@ -985,7 +1087,10 @@ nyxpm_status build_lists(nyxpm_ctx* c, nyxpm_amr* a)
                     face.push_back(F);
                     r.count += 1;
                 }
-            if (r.count > 0) frec.push_back(r);
+            if (r.count > 0) {
+                frec.push_back(r);
+                cov[C] |= kRefluxed;
+            }
         };
         if (l - 1 == 0) {
             for (int k = 0; k < n0; ++k)
@@ -1015,11 +1120,15 @@ nyxpm_status build_lists(nyxpm_ctx* c, nyxpm_amr* a)
 // ---------------------------------------------------------------------------
 // launch sequences
 // ---------------------------------------------------------------------------
+// passes over at least this many cells sum on the integer pipes (the FP64 pipe bounds them;
+// smaller ones are latency, as on the single level)
+inline bool on_int(long long cells) { return cells >= (1LL << 20); }
+
 nyxpm_status ghost_fill(Ctx& c, nyxpm_amr& A, double* f, const Range& r)
 {
     if (r.count == 0) return NYXPM_OK;
     prof_begin(c);
-    k_amr_ghost<<<nblk(r.count), kT, 0, c.stream>>>(r.count, A.d_ghost + r.first, A.d_ent, f);
+    launch_pdl(c, k_amr_ghost, dim3(nblk(r.count)), dim3(kT), r.count, A.d_ghost + r.first, A.d_ent, f);
     prof_end(c, NYXPM_ST_SMOOTH, 40.0 * r.count);
     return check_launch(c, "ghost fill");
 }
@@ -1028,8 +1137,8 @@ nyxpm_status avg_down(Ctx& c, nyxpm_amr& A, double* f)
 {
     for (int l = A.nlev - 1; l >= 1; --l) {
         prof_begin(c);
-        k_amr_sum8<<<nblk(A.rrec[l].count), kT, 0, c.stream>>>(A.rrec[l].count, A.d_rrec + A.rrec[l].first, f,
-                                                                 0.125, f);
+        launch_pdl(c, k_amr_sum8, dim3(nblk(A.rrec[l].count)), dim3(kT), A.rrec[l].count, A.d_rrec + A.rrec[l].first,
+                   f, 0.125, f);
         prof_end(c, NYXPM_ST_RESTRICT, 96.0 * A.rrec[l].count);
     }
     return check_launch(c, "average down");
@@ -1068,32 +1177,29 @@ nyxpm_status comp_resid(Ctx& c, nyxpm_amr& A, int slot)
     const long long n3 = (long long)A.n0 * A.n0 * A.n0;
     if ((st = avg_down(c, A, A.phi)) != NYXPM_OK) return st;
     if ((st = ghost_fill(c, A, A.phi, A.all_ghost1)) != NYXPM_OK) return st;
-    const Geo g = geo3(A.n0, A.n0, A.n0);
+    cudaMemsetAsync(A.norms + slot, 0, sizeof(unsigned long long), c.stream);
+    const Geo g = geo3(A.n0, A.n0, A.n0, kT);
     prof_begin(c);
-    k_amr_resid0<<<g.grid, g.block, 0, c.stream>>>(A.n0, A.phi, A.beta, A.R);
-    prof_end(c, NYXPM_ST_NORM, 24.0 * n3);
+    if (g.block.x * g.block.y == kT) {
+        launch_pdl(c, on_int(n3) ? k_amr_resid0<true> : k_amr_resid0<false>, dim3(g.grid), dim3(g.block), A.n0, A.phi,
+                   A.beta, A.d_cov, A.inv_scale[0], A.R, A.norms + slot);
+    } else {   // a tiny level 0: whole blocks of kT threads all the same
+        launch_pdl(c, k_amr_resid0<false>, dim3(1, 1, A.n0), dim3(kT / 16, 16), A.n0, A.phi, A.beta, A.d_cov,
+                   A.inv_scale[0], A.R, A.norms + slot);
+    }
+    prof_end(c, NYXPM_ST_NORM, 25.0 * n3);
     if (A.fine_cells.count) {
         prof_begin(c);
-        k_amr_residf<<<nblk(A.fine_cells.count), kT, 0, c.stream>>>(A.fine_cells.count, 0, (int)A.boxes.size(),
-                                                                     A.d_pref, A.d_boxes, A.phi, A.beta, A.R);
-        prof_end(c, NYXPM_ST_NORM, 48.0 * A.fine_cells.count);
+        launch_pdl(c, on_int(A.fine_cells.count) ? k_amr_residf<true> : k_amr_residf<false>,
+                   dim3(nblk(A.fine_cells.count)), dim3(kT), A.fine_cells.count, 0, (int)A.boxes.size(), A.d_pref,
+                   A.d_boxes, A.phi, A.beta, A.d_cov, A.d_level + 8, A.R, A.norms + slot);
+        prof_end(c, NYXPM_ST_NORM, 49.0 * A.fine_cells.count);
     }
     if (A.all_frec.count) {
         prof_begin(c);
-        k_amr_reflux<<<nblk(A.all_frec.count), kT, 0, c.stream>>>(A.all_frec.count, A.d_frec, A.d_face, A.phi,
-                                                                   A.R);
+        launch_pdl(c, k_amr_reflux, dim3(nblk(A.all_frec.count)), dim3(kT), A.all_frec.count, A.d_frec, A.d_face, A.phi,
+                   A.R, A.d_level + 8, A.norms + slot);
         prof_end(c, NYXPM_ST_NORM, 96.0 * A.all_frec.count);
-    }
-    cudaMemsetAsync(A.norms + slot, 0, sizeof(unsigned long long), c.stream);
-    prof_begin(c);
-    k_amr_absmax0<<<norm_grid(c, n3), kT, 0, c.stream>>>(n3, A.R, A.d_cov, A.inv_scale[0], A.norms + slot);
-    prof_end(c, NYXPM_ST_NORM, 9.0 * n3);
-    if (A.fine_cells.count) {
-        prof_begin(c);
-        k_amr_absmaxf<<<norm_grid(c, A.fine_cells.count), kT, 0, c.stream>>>(
-            A.fine_cells.count, 0, (int)A.boxes.size(), A.d_pref, A.d_boxes, A.R, A.d_cov, A.d_level + 8,
-            A.norms + slot);
-        prof_end(c, NYXPM_ST_NORM, 33.0 * A.fine_cells.count);
     }
     return check_launch(c, "composite residual");
 }
@@ -1103,17 +1209,21 @@ nyxpm_status comp_resid(Ctx& c, nyxpm_amr& A, int slot)
 // not change while level l smooths: the interpolated ghosts are filled once, at
 // the start (fill_interp; not on the way down, where every coarser correction
 // and so every such ghost is still zero), the copies before each colour.
+// On the way down (fill_interp = 0) the level's correction is zero on entry: the first red
+// half sweep reads nothing of it.
 nyxpm_status smooth_level(Ctx& c, nyxpm_amr& A, int l, int nsweeps, int fill_interp)
 {
     nyxpm_status st;
     const long long half = A.cells[l].count / 2;
     for (int s = 0; s < nsweeps; ++s)
         for (int col = 0; col < 2; ++col) {
-            const bool all = fill_interp && s == 0 && col == 0;
-            if ((st = ghost_fill(c, A, A.e, all ? A.ghost1[l] : A.ghost1_same[l])) != NYXPM_OK) return st;
+            const bool first = s == 0 && col == 0, zero = first && !fill_interp;
+            if (!zero &&
+                (st = ghost_fill(c, A, A.e, first ? A.ghost1[l] : A.ghost1_same[l])) != NYXPM_OK)
+                return st;
             prof_begin(c);
-            k_amr_gsrbf<<<nblk(half), kT, 0, c.stream>>>(half, A.tab.first[l], A.tab.count[l], A.d_pref, A.d_boxes,
-                                                         col, A.e, A.R);
+            launch_pdl(c, on_int(half) && !zero ? k_amr_gsrbf<true> : k_amr_gsrbf<false>, dim3(nblk(half)), dim3(kT),
+                       half, A.tab.first[l], A.tab.count[l], A.d_pref, A.d_boxes, col, zero ? 1 : 0, A.e, A.R);
             prof_end(c, NYXPM_ST_SMOOTH, 24.0 * half, 1);
         }
     return check_launch(c, "fine smoother");
@@ -1129,18 +1239,25 @@ nyxpm_status vcycle(nyxpm_ctx* cx, nyxpm_amr& A)
         if ((st = smooth_level(c, A, l, nu1, 0)) != NYXPM_OK) return st;
         if ((st = ghost_fill(c, A, A.e, A.ghost1_same[l])) != NYXPM_OK) return st;
         const Range& r = A.cells[l];
-        prof_begin(c);
-        k_amr_residf<<<nblk(r.count), kT, 0, c.stream>>>(r.count, A.tab.first[l], A.tab.count[l], A.d_pref,
-                                                         A.d_boxes, A.e, A.R, A.T);
-        prof_end(c, NYXPM_ST_RESTRICT, 48.0 * r.count);
-        prof_begin(c);
-        k_amr_sum8<<<nblk(A.rrec[l].count), kT, 0, c.stream>>>(A.rrec[l].count, A.d_rrec + A.rrec[l].first, A.T,
-                                                                 0.5, A.R);
-        prof_end(c, NYXPM_ST_RESTRICT, 96.0 * A.rrec[l].count);
+        const Range& rr = A.rrec[l];
+        if (nu1 > 0) {
+            prof_begin(c);
+            launch_pdl(c, on_int(r.count / 2) ? k_amr_restrict_red<true> : k_amr_restrict_red<false>,
+                       dim3(nblk(rr.count)), dim3(kT), rr.count, A.d_rrec + rr.first, A.e, A.R);
+            prof_end(c, NYXPM_ST_RESTRICT, 24.0 * r.count);
+        } else {
+            prof_begin(c);
+            k_amr_resid_all<<<nblk(r.count), kT, 0, c.stream>>>(r.count, A.tab.first[l], A.tab.count[l], A.d_pref,
+                                                                A.d_boxes, A.e, A.R, A.T);
+            prof_end(c, NYXPM_ST_RESTRICT, 48.0 * r.count);
+            prof_begin(c);
+            launch_pdl(c, k_amr_sum8, dim3(nblk(rr.count)), dim3(kT), rr.count, A.d_rrec + rr.first, A.T, 0.5, A.R);
+            prof_end(c, NYXPM_ST_RESTRICT, 96.0 * rr.count);
+        }
         if (A.frec[l].count) {
             prof_begin(c);
-            k_amr_reflux<<<nblk(A.frec[l].count), kT, 0, c.stream>>>(A.frec[l].count, A.d_frec + A.frec[l].first,
-                                                                      A.d_face, A.e, A.R);
+            launch_pdl(c, k_amr_reflux, dim3(nblk(A.frec[l].count)), dim3(kT), A.frec[l].count,
+                       A.d_frec + A.frec[l].first, A.d_face, A.e, A.R, A.d_level + 8, nullptr);
             prof_end(c, NYXPM_ST_RESTRICT, 96.0 * A.frec[l].count);
         }
         if ((st = check_launch(c, "composite restriction")) != NYXPM_OK) return st;
@@ -1153,19 +1270,19 @@ nyxpm_status vcycle(nyxpm_ctx* cx, nyxpm_amr& A)
         const Range& r = A.cells[l];
         prof_begin(c);
         if (nu2 > 0 && A.prolong_black_ok[l]) {
-            k_amr_prolong_black<<<nblk(r.count / 2), kT, 0, c.stream>>>(r.count / 2, A.tab.first[l], A.tab.count[l],
-                                                                       A.d_pref, A.d_boxes, A.n0, A.e);
+            launch_pdl(c, k_amr_prolong_black, dim3(nblk(r.count / 2)), dim3(kT), r.count / 2, A.tab.first[l],
+                       A.tab.count[l], A.d_pref, A.d_boxes, A.n0, A.e);
             prof_end(c, NYXPM_ST_PROLONG, 48.0 * r.count);
         } else {
-            k_amr_prolong<<<nblk(r.count), kT, 0, c.stream>>>(r.count, A.d_cells + r.first, A.d_par + r.first, A.n0,
-                                                              A.e);
+            launch_pdl(c, k_amr_prolong, dim3(nblk(r.count)), dim3(kT), r.count, A.d_cells + r.first,
+                       A.d_par + r.first, A.n0, A.e);
             prof_end(c, NYXPM_ST_PROLONG, 96.0 * r.count);
         }
         if ((st = check_launch(c, "composite prolongation")) != NYXPM_OK) return st;
         if ((st = smooth_level(c, A, l, nu2, 1)) != NYXPM_OK) return st;
     }
     prof_begin(c);
-    k_amr_add<<<nblk(A.ntot), kT, 0, c.stream>>>(A.ntot, A.phi, A.e);
+    launch_pdl(c, k_amr_add, dim3(nblk(A.ntot)), dim3(kT), A.ntot, A.phi, A.e);
     prof_end(c, NYXPM_ST_PROLONG, 24.0 * A.ntot);
     return check_launch(c, "composite update");
 }
@@ -1231,11 +1348,17 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
     int it = 0;
     nyxpm_status result = NYXPM_OK;
     if (r0 > target) {
-        for (it = 1; it <= c.p.max_vcycles; ++it) {
-            if ((st = vcycle(cx, A)) != NYXPM_OK) return st;
-            if ((st = comp_resid(c, A, 1)) != NYXPM_OK) return st;
+        // the launches never change: captured once, replayed (run_iteration)
+        auto iteration = [&]() -> nyxpm_status {
+            nyxpm_status s;
+            if ((s = vcycle(cx, A)) != NYXPM_OK) return s;
+            if ((s = comp_resid(c, A, 1)) != NYXPM_OK) return s;
             cudaMemcpyAsync(A.h_norms + 1, A.norms + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                             c.stream);
+            return check_launch(c, "norm copy");
+        };
+        for (it = 1; it <= c.p.max_vcycles; ++it) {
+            if ((st = run_iteration(c, A.iter_graph, iteration)) != NYXPM_OK) return st;
             if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "multilevel solve sync");
             r = read_bits(A.h_norms, 1);
             if (r != r) {
@@ -1384,6 +1507,9 @@ nyxpm_status nyxpm_amr_create(nyxpm_ctx* c, int n0, double L, int nlev, const in
                 for (int d = 0; d < 3; ++d) sep = sep || B.hi[d] < O.lo[d] || O.hi[d] < B.lo[d];
                 if (!sep) return cleanup(afail(c, NYXPM_INVALID_ARG, "boxes of one level overlap"));
             }
+            B.nx.set(B.hi[0] - B.lo[0] + 1);
+            B.hx.set((B.hi[0] - B.lo[0] + 1) / 2);
+            B.ny.set(B.hi[1] - B.lo[1] + 1);
             B.off = off;
             off += (long long)B.d[0] * B.d[1] * B.d[2];
             a->boxes.push_back(B);
@@ -1477,6 +1603,7 @@ nyxpm_status nyxpm_amr_destroy(nyxpm_ctx* c, nyxpm_amr* a)
     if (!c) return NYXPM_INVALID_ARG;
     if (!a) return NYXPM_OK;
     cudaStreamSynchronize(c->stream);
+    if (a->iter_graph.exec) cudaGraphExecDestroy(a->iter_graph.exec);
     for (void* q : a->allocs) cudaFree(q);
     if (a->h_norms) cudaFreeHost(a->h_norms);
     if (a->mg) nyxpm_box_destroy(c, a->mg);

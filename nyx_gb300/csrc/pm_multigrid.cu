@@ -687,14 +687,21 @@ __global__ void k_from_natural(LevelView L, const double* __restrict__ in)
     *lv_ptr<double>(L.phi_r, L.phi_b, n, L.split, i, j, k) = in[cidx(i, j, k, n)];
 }
 
-__global__ void k_beta_from_natural(LevelView L, const double* __restrict__ in)
+// the right-hand side of a correction solve from natural layout; with red, also the red half
+// sweep that opens it from phi = 0
+__global__ void k_beta_from_natural(LevelView L, const double* __restrict__ in, int red)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = L.n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
     if (i >= n || j >= n) return;
-    *lv_ptr<double>(L.beta_r, L.beta_b, n, L.split, i, j, k) = in[cidx(i, j, k, n)];
+    const double b = in[cidx(i, j, k, n)];
+    *lv_ptr<double>(L.beta_r, L.beta_b, n, L.split, i, j, k) = b;
+    if (red && ((i + j + k) & 1) == 0)
+        *lv_ptr<double>(L.phi_r, L.phi_b, n, L.split, i, j, k) = fma(0.0, kSixth, -b);
 }
 
 // Levels of at least this edge work by pairs of cells, their sums on the integer pipes
@@ -1052,11 +1059,14 @@ nyxpm_status mg_vcycle_zero(Ctx& c, Box& b, const double* beta_nat, double* e_na
         prof_end(c, NYXPM_ST_SMOOTH, 16.0 * nc);
         return check_launch(c, "cluster V-cycle");
     }
+    // (black cells are written before they are read)
+    const Level& l0 = b.levels[0];
+    const int red = l0.split && c.p.nu1 > 0 && !tail_fits_d(c, b, 0) ? 1 : 0;
     prof_begin(c);
-    k_beta_from_natural<<<g.grid, g.block, 0, c.stream>>>(view(b.levels[0]), beta_nat);
+    launch_pdl(c, k_beta_from_natural, dim3(g.grid), dim3(g.block), view(l0), beta_nat, red);
     prof_end(c, NYXPM_ST_RHS, 16.0 * nc);
-    if ((st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
-    if ((st = vcycle(c, b, 0)) != NYXPM_OK) return st;
+    if (!red && (st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
+    if ((st = vcycle(c, b, 0, red)) != NYXPM_OK) return st;
     return launch_phi_to_natural(c, b, e_nat);
 }
 
