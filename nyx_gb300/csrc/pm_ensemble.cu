@@ -141,6 +141,8 @@ __device__ __forceinline__ int key_frac(int ci, float o, int n, float* f)
 __global__ void e_load_step(int nbox, const EStep* __restrict__ st, const EDesc* __restrict__ D,
                             EState* S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox) return;
     const double a_old = st[b].a_old, a_new = st[b].a_new, dt = st[b].dt;
@@ -167,6 +169,8 @@ __global__ void __launch_bounds__(kPT, 4) e_kick(const Item* __restrict__ items,
                                                const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                int phase, int bucket)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         // by reference: a copy indexed by the runtime phase would live in local memory
@@ -258,6 +262,8 @@ __global__ void __launch_bounds__(kPT) e_keys(const Item* __restrict__ items, in
                                                const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                int bucket)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -283,6 +289,8 @@ __global__ void __launch_bounds__(kPT) e_scatter(const Item* __restrict__ items,
                                                   const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                   int bucket)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         if (!S[it.box].active) continue;
@@ -300,6 +308,8 @@ __global__ void __launch_bounds__(kPT, 8) e_gather(const Item* __restrict__ item
                                                  const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                  int bucket)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -325,6 +335,8 @@ __global__ void __launch_bounds__(kPT, 8) e_gather(const Item* __restrict__ item
 // flip the current particle buffer of every active box (after the gather)
 __global__ void e_flip(int nbox, EState* S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox || !S[b].active) return;
     S[b].parity ^= 1;
@@ -368,6 +380,8 @@ __global__ void __launch_bounds__(kScanT) e_scan_reduce(const Item* __restrict__
                                                         const EDesc* __restrict__ D,
                                                         const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         if (!S[it.box].active) continue;  // uniform across the block
@@ -386,6 +400,8 @@ __global__ void __launch_bounds__(kScanT) e_scan_reduce(const Item* __restrict__
 
 __global__ void e_scan_top(int nbox, const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x;
     if (b >= nbox || !S[b].active) return;
     const EDesc& d = D[b];
@@ -406,6 +422,8 @@ __global__ void __launch_bounds__(kScanT) e_scan_down(const Item* __restrict__ i
                                                       const EDesc* __restrict__ D,
                                                       const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         if (!S[it.box].active) continue;
@@ -435,6 +453,8 @@ __global__ void __launch_bounds__(256) e_fix_short(const Item* __restrict__ item
                                                     const EDesc* __restrict__ D,
                                                     const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         if (!S[it.box].active) continue;
@@ -455,6 +475,8 @@ constexpr int kLongSmem = 12288;
 
 __global__ void e_fix_long(int nbox, const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int sv[kLongSmem];
     for (int b = 0; b < nbox; ++b) {
         if (!S[b].active) continue;
@@ -486,6 +508,8 @@ __global__ void e_fix_long(int nbox, const EDesc* __restrict__ D, const EState* 
 
 __global__ void e_sort_reset(int nbox, const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox || !S[b].active) return;
     *D[b].long_count = 0;
@@ -498,6 +522,8 @@ template <int TX, int TY, int TZ>
 __global__ void __launch_bounds__(256) e_deposit(const Item* __restrict__ items, int nitems,
                                                  const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     constexpr int KX = TX + 1, KY = TY + 1, KZ = TZ + 1, NK = KX * KY * KZ;
     // corner-major: a warp's consecutive keys (or cells) touch consecutive banks
     __shared__ float part[NK * 8];
@@ -576,6 +602,8 @@ __device__ __forceinline__ void kahan_add(double& s, double& c, double v)
 __global__ void __launch_bounds__(256) e_rowsum(const Item* __restrict__ items, int nitems,
                                                 const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
@@ -602,6 +630,8 @@ __global__ void __launch_bounds__(256) e_rowsum(const Item* __restrict__ items, 
 // per-box mean (one block per box); also opens the solve of every active box
 __global__ void e_mean(int nbox, const EDesc* __restrict__ D, EState* S, double ggrav)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ double ss[32];
     const int b = blockIdx.x;
     if (b >= nbox || !S[b].active) return;
@@ -635,6 +665,8 @@ __global__ void __launch_bounds__(256) e_make_beta(const Item* __restrict__ item
                                                    const EDesc* __restrict__ D,
                                                    const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -694,6 +726,8 @@ __global__ void __launch_bounds__(256) e_resid(const Item* __restrict__ items, i
                                                const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                int low_words)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -734,6 +768,8 @@ __global__ void __launch_bounds__(256, 5) e_resid_v(const Item* __restrict__ ite
                                                  const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                  int low_words)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
@@ -812,6 +848,8 @@ __global__ void __launch_bounds__(256, 5) e_resid_v(const Item* __restrict__ ite
 // residual plus the bound meets the target
 __global__ void e_flags(int nbox, const EDesc* __restrict__ D, EState* S, double rel_tol, int mode)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox) return;
     EState& st = S[b];
@@ -861,6 +899,8 @@ __global__ void e_loop_cond(int nbox, const EState* __restrict__ S, int* loop, i
 
 __global__ void e_count_inner(int nbox, EState* S, int cycles)
 {
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nbox) return;
     if (S[b].active && S[b].solve_active) S[b].inner += cycles;
@@ -874,6 +914,8 @@ __global__ void __launch_bounds__(256) e_correct(const Item* __restrict__ items,
                                                  const EDesc* __restrict__ D,
                                                  const EState* __restrict__ S, float c_hi, float c_lo)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -975,6 +1017,8 @@ __global__ void __launch_bounds__(256) e_correct_v(const Item* __restrict__ item
                                                    const EDesc* __restrict__ D,
                                                    const EState* __restrict__ S, float c_hi, float c_lo)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
@@ -1052,6 +1096,8 @@ __global__ void __launch_bounds__(256) e_zero_inner(const Item* __restrict__ ite
                                                     const EDesc* __restrict__ D,
                                                     const EState* __restrict__ S, int all)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -1077,6 +1123,8 @@ __global__ void __launch_bounds__(256) e_gsrb_zero(const Item* __restrict__ item
                                                    const EDesc* __restrict__ D,
                                                    const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState& st = S[it.box];
@@ -1099,6 +1147,8 @@ __global__ void __launch_bounds__(256) e_gsrb_zero_v(const Item* __restrict__ it
                                                      const EDesc* __restrict__ D,
                                                      const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
@@ -1130,6 +1180,8 @@ __global__ void __launch_bounds__(256) e_gsrb_zero_v(const Item* __restrict__ it
 __global__ void __launch_bounds__(256) e_update(const Item* __restrict__ items, int nitems,
                                                 const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -1153,6 +1205,8 @@ __global__ void __launch_bounds__(256) e_gsrb(const Item* __restrict__ items, in
                                               const EDesc* __restrict__ D, const EState* __restrict__ S,
                                               int color)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -1197,6 +1251,8 @@ __global__ void __launch_bounds__(256, 6) e_gsrb4(const Item* __restrict__ items
                                                const EDesc* __restrict__ D,
                                                const EState* __restrict__ S, int color)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
@@ -1279,6 +1335,8 @@ __device__ __forceinline__ float resid_f(const ELevel& L, int i, int j, int k)
 __global__ void __launch_bounds__(256) e_restrict(const Item* __restrict__ items, int nitems,
                                                   const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -1359,6 +1417,8 @@ __global__ void __launch_bounds__(256) e_restrict4(const Item* __restrict__ item
                                                    const EDesc* __restrict__ D,
                                                    const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int R = blockDim.y;
@@ -1405,6 +1465,8 @@ __global__ void __launch_bounds__(256, 5) e_restrict4_red(const Item* __restrict
                                                        const EDesc* __restrict__ D,
                                                        const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int R = blockDim.y;
@@ -1448,6 +1510,8 @@ __global__ void __launch_bounds__(256) e_prolong(const Item* __restrict__ items,
                                                  const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                  int black)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -1492,6 +1556,8 @@ __global__ void __launch_bounds__(256) e_prolong4(const Item* __restrict__ items
                                                   const EDesc* __restrict__ D,
                                                   const EState* __restrict__ S, int black)
 {
+    pdl_wait();
+    pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
@@ -1613,6 +1679,8 @@ __global__ void __launch_bounds__(256, 4) e_prolong4_black(const Item* __restric
                                                           const EDesc* __restrict__ D,
                                                           const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -1630,30 +1698,65 @@ __global__ void __launch_bounds__(256, 4) e_prolong4_black(const Item* __restric
     }
 }
 
-// the coarse end of every box's V-cycle (levels tail_l .. bottom), one CTA per
-// box: the per-pass kernels' arithmetic (pm_tail.cuh), so the same bits
-__global__ void __launch_bounds__(kTailThreads) e_tail(int nbox, const EDesc* __restrict__ D,
-                                                       const EState* __restrict__ S, int nu1, int nu2)
+// The coarse end of every box's V-cycle (levels tail_l .. bottom), one CTA per box: the
+// per-pass kernels' arithmetic (pm_tail.cuh), so the same bits.  Levels of up to 16^3
+// with pre- and post-smoothing are cycled in shared memory (vcycle_solo).
+constexpr int kETailThreads = 512;
+constexpr int kETailLevels = 2 * (16 * 16 * 16 + 8 * 8 * 8 + 4 * 4 * 4);   // no level chain from 16 down holds more
+constexpr int kETailGreen = 7 * 7 * 7, kETailTmp = 16 * 16 * 16 / 2;
+
+__global__ void __launch_bounds__(kETailThreads) e_tail(int nbox, const EDesc* __restrict__ D,
+                                                        const EState* __restrict__ S, int nu1, int nu2)
 {
-    __shared__ float r[kMaxBottom * kMaxBottom * kMaxBottom];
-    __shared__ float g[kMaxBottom * kMaxBottom * kMaxBottom];
+    pdl_wait();
+    pdl_trigger();
+    __shared__ __align__(16) float mem[kETailLevels + kETailTmp + kETailGreen];
+    __shared__ SoloLevel<float> solo[kMaxTail];
     const int b = blockIdx.x;
     if (b >= nbox) return;
     if (!(S[b].active && S[b].solve_active)) return;
     const EDesc& d = D[b];
-    LevelViewF lv[kMaxTail];
     const int nl = d.nlev - d.tail_l;
+    const ELevel& top = d.lv[d.tail_l];
+    if (top.split && top.n <= 16 && nu1 > 0 && nu2 > 0) {
+        const int half = top.n * top.n * top.n / 2;
+        float *tmp = mem + kETailLevels, *g = tmp + kETailTmp;
+        if (threadIdx.x == 0) {
+            float* at = mem;
+            for (int l = 0; l < nl; ++l) {
+                const int n = d.lv[d.tail_l + l].n;
+                solo[l] = SoloLevel<float>{n, at};
+                at += 2 * n * n * n;
+            }
+        }
+        for (int t = threadIdx.x; t < half; t += blockDim.x) {
+            mem[2 * half + t] = top.beta_r[t];
+            mem[3 * half + t] = top.beta_b[t];
+            if (d.tail_l == 0) mem[half + t] = top.phi_b[t];   // a whole V-cycle: from the present correction
+        }
+        for (int t = threadIdx.x; t < d.nb * d.nb * d.nb; t += blockDim.x) g[t] = d.Gf[t];
+        __syncthreads();
+        vcycle_solo<float>(solo, nl, nu1, nu2, g, d.nb, tmp, d.tail_l > 0);
+        for (int t = threadIdx.x; t < half; t += blockDim.x) {
+            top.phi_r[t] = mem[t];
+            top.phi_b[t] = mem[half + t];
+        }
+        return;
+    }
+    LevelViewF lv[kMaxTail];
     for (int l = 0; l < nl; ++l) {
         const ELevel& e = d.lv[d.tail_l + l];
         lv[l] = LevelViewF{e.n, e.split, e.phi_r, e.phi_b, e.beta_r, e.beta_b};
     }
-    vcycle_tail<float>(lv, nl, nu1, nu2, d.Gf, d.nb, r, g, nu1 > 0);
+    vcycle_tail<float>(lv, nl, nu1, nu2, d.Gf, d.nb, mem, mem + kMaxBottom * kMaxBottom * kMaxBottom, nu1 > 0);
 }
 
 // FP32 gravity vector from the FP64 phi (level-0 rows, natural coordinates)
 __global__ void __launch_bounds__(256) e_grav(const Item* __restrict__ items, int nitems,
                                               const EDesc* __restrict__ D, const EState* __restrict__ S)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         if (!S[it.box].active) continue;
@@ -2233,50 +2336,50 @@ void enqueue_solve_head(nyxpm_ctx* c, nyxpm_ensemble* E)
     EState* S = E->d_state;
     const unsigned bb = (unsigned)((nbox + 127) / 128);
     ep_begin(c);
-    e_sort_reset<<<bb, 128, 0, s>>>(nbox, D, S);
-    e_keys<<<pgrid(E, E->r_part.cnt), kPT, 0, s>>>(it + E->r_part.off, E->r_part.cnt, D, S,
+    launch_pdl(*c, e_sort_reset, dim3(bb), dim3(128), nbox, D, S);
+    launch_pdl(*c, e_keys, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), it + E->r_part.off, E->r_part.cnt, D, S,
                                                    E->tune.sort_bucket);
     ep_end(c, NYXPM_ST_KEYS);
     ep_begin(c);
-    e_scan_reduce<<<pgrid(E, E->r_scan.cnt), kScanT, 0, s>>>(it + E->r_scan.off, E->r_scan.cnt, D, S);
-    e_scan_top<<<nbox, 1024, 0, s>>>(nbox, D, S);
-    e_scan_down<<<pgrid(E, E->r_scan.cnt), kScanT, 0, s>>>(it + E->r_scan.off, E->r_scan.cnt, D, S);
+    launch_pdl(*c, e_scan_reduce, dim3(pgrid(E, E->r_scan.cnt)), dim3(kScanT), it + E->r_scan.off, E->r_scan.cnt, D, S);
+    launch_pdl(*c, e_scan_top, dim3(nbox), dim3(1024), nbox, D, S);
+    launch_pdl(*c, e_scan_down, dim3(pgrid(E, E->r_scan.cnt)), dim3(kScanT), it + E->r_scan.off, E->r_scan.cnt, D, S);
     ep_end(c, NYXPM_ST_SCAN);
     ep_begin(c);
-    e_scatter<<<pgrid(E, E->r_part.cnt), kPT, 0, s>>>(it + E->r_part.off, E->r_part.cnt, D, S,
+    launch_pdl(*c, e_scatter, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), it + E->r_part.off, E->r_part.cnt, D, S,
                                                       E->tune.sort_bucket);
-    e_fix_short<<<pgrid(E, E->r_keys.cnt), 256, 0, s>>>(it + E->r_keys.off, E->r_keys.cnt, D, S);
-    e_fix_long<<<E->sm * 2, 512, 0, s>>>(nbox, D, S);
+    launch_pdl(*c, e_fix_short, dim3(pgrid(E, E->r_keys.cnt)), dim3(256), it + E->r_keys.off, E->r_keys.cnt, D, S);
+    launch_pdl(*c, e_fix_long, dim3(E->sm * 2), dim3(512), nbox, D, S);
     ep_end(c, NYXPM_ST_SCATTER);
     ep_begin(c);
-    e_gather<<<pgrid(E, E->r_part.cnt), kPT, 0, s>>>(it + E->r_part.off, E->r_part.cnt, D, S,
+    launch_pdl(*c, e_gather, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), it + E->r_part.off, E->r_part.cnt, D, S,
                                                      E->tune.sort_bucket);
-    e_flip<<<bb, 128, 0, s>>>(nbox, S);
+    launch_pdl(*c, e_flip, dim3(bb), dim3(128), nbox, S);
     ep_end(c, NYXPM_ST_GATHER);
     ep_begin(c);
     const unsigned gt = pgrid(E, E->r_tile.cnt, 4);
     if (E->tune.deposit_tile == 1)
-        e_deposit<8, 8, 4><<<gt, 256, 0, s>>>(it + E->r_tile.off, E->r_tile.cnt, D, S);
+        launch_pdl(*c, e_deposit<8, 8, 4>, dim3(gt), dim3(256), it + E->r_tile.off, E->r_tile.cnt, D, S);
     else if (E->tune.deposit_tile == 2)
-        e_deposit<16, 8, 4><<<gt, 256, 0, s>>>(it + E->r_tile.off, E->r_tile.cnt, D, S);
+        launch_pdl(*c, e_deposit<16, 8, 4>, dim3(gt), dim3(256), it + E->r_tile.off, E->r_tile.cnt, D, S);
     else
-        e_deposit<8, 8, 8><<<gt, 256, 0, s>>>(it + E->r_tile.off, E->r_tile.cnt, D, S);
+        launch_pdl(*c, e_deposit<8, 8, 8>, dim3(gt), dim3(256), it + E->r_tile.off, E->r_tile.cnt, D, S);
     ep_end(c, NYXPM_ST_DEPOSIT);
     ep_begin(c);
-    e_rowsum<<<pgrid(E, E->r_rows_rho.cnt), 256, 0, s>>>(it + E->r_rows_rho.off, E->r_rows_rho.cnt, D, S);
+    launch_pdl(*c, e_rowsum, dim3(pgrid(E, E->r_rows_rho.cnt)), dim3(256), it + E->r_rows_rho.off, E->r_rows_rho.cnt, D, S);
     const double ggrav = -4.0 * M_PI * c->p.gconst;
-    e_mean<<<nbox, 512, 0, s>>>(nbox, D, S, ggrav);
+    launch_pdl(*c, e_mean, dim3(nbox), dim3(512), nbox, D, S, ggrav);
     const dim3 rb(32, E->tune.smooth_rows);
     const auto& r0 = E->r_rows_split[0];
-    e_make_beta<<<pgrid(E, r0.cnt), rb, 0, s>>>(it + r0.off, r0.cnt, D, S);
+    launch_pdl(*c, e_make_beta, dim3(pgrid(E, r0.cnt)), dim3(rb), it + r0.off, r0.cnt, D, S);
     {
         const auto& cv = E->r_correct_vec;
         const auto& cr = E->r_correct_rest;
-        if (cv.cnt) e_resid_v<<<pgrid(E, cv.cnt), rb, 0, s>>>(it + cv.off, cv.cnt, D, S, 1);
-        if (cr.cnt) e_resid<<<pgrid(E, cr.cnt), rb, 0, s>>>(it + cr.off, cr.cnt, D, S, 1);
+        if (cv.cnt) launch_pdl(*c, e_resid_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S, 1);
+        if (cr.cnt) launch_pdl(*c, e_resid, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, 1);
         c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
     }
-    e_flags<<<bb, 128, 0, s>>>(nbox, D, S, c->p.rel_tol, 1);
+    launch_pdl(*c, e_flags, dim3(bb), dim3(128), nbox, D, S, c->p.rel_tol, 1);
     ep_end(c, NYXPM_ST_RHS);
     c->launches += 16;
 }
@@ -2305,8 +2408,8 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
             const auto& cv = E->r_correct_vec;
             const auto& cr = E->r_correct_rest;
             ep_begin(c);
-            if (cv.cnt) e_gsrb_zero_v<<<pgrid(E, cv.cnt), rb, 0, s>>>(it + cv.off, cv.cnt, D, S);
-            if (cr.cnt) e_gsrb_zero<<<pgrid(E, cr.cnt), rb, 0, s>>>(it + cr.off, cr.cnt, D, S);
+            if (cv.cnt) launch_pdl(*c, e_gsrb_zero_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S);
+            if (cr.cnt) launch_pdl(*c, e_gsrb_zero, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S);
             c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
             ep_end(c, NYXPM_ST_SMOOTH);
             c->launches += 1;
@@ -2314,11 +2417,11 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
         }
         ep_begin(c);
         if (rv.cnt) {
-            e_gsrb4<<<pgrid(E, rv.cnt), rb, 0, s>>>(it + rv.off, rv.cnt, D, S, color);
+            launch_pdl(*c, e_gsrb4, dim3(pgrid(E, rv.cnt)), dim3(rb), it + rv.off, rv.cnt, D, S, color);
             c->launches += 1;
         }
         if (rr.cnt) {
-            e_gsrb<<<pgrid(E, rr.cnt), rb, 0, s>>>(it + rr.off, rr.cnt, D, S, color);
+            launch_pdl(*c, e_gsrb, dim3(pgrid(E, rr.cnt)), dim3(rb), it + rr.off, rr.cnt, D, S, color);
             c->launches += 1;
         }
         ep_end(c, NYXPM_ST_SMOOTH);
@@ -2335,16 +2438,16 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
                 const auto& qr = E->r_restrict_row[l + 1];
                 ep_begin(c);
                 if (qv.cnt && c->p.nu1 > 0)
-                    e_restrict4_red<<<pgrid(E, qv.cnt), rb, 0, s>>>(it + qv.off, qv.cnt, D, S);
+                    launch_pdl(*c, e_restrict4_red, dim3(pgrid(E, qv.cnt)), dim3(rb), it + qv.off, qv.cnt, D, S);
                 else if (qv.cnt)
-                    e_restrict4<<<pgrid(E, qv.cnt), rb, 0, s>>>(it + qv.off, qv.cnt, D, S);
-                if (qr.cnt) e_restrict<<<pgrid(E, qr.cnt), rb, 0, s>>>(it + qr.off, qr.cnt, D, S);
+                    launch_pdl(*c, e_restrict4, dim3(pgrid(E, qv.cnt)), dim3(rb), it + qv.off, qv.cnt, D, S);
+                if (qr.cnt) launch_pdl(*c, e_restrict, dim3(pgrid(E, qr.cnt)), dim3(rb), it + qr.off, qr.cnt, D, S);
                 ep_end(c, NYXPM_ST_RESTRICT);
                 c->launches += (qv.cnt ? 1 : 0) + (qr.cnt ? 1 : 0) - 1;
                 c->launches += 1;
             }
             ep_begin(c);
-            e_tail<<<nbox, kTailThreads, 0, s>>>(nbox, D, S, c->p.nu1, c->p.nu2);
+            launch_pdl(*c, e_tail, dim3(nbox), dim3(kETailThreads), nbox, D, S, c->p.nu1, c->p.nu2);
             ep_end(c, NYXPM_ST_BOTTOM);
             c->launches += 1;
             for (int l = E->max_lev - 2; l >= 0; --l) {
@@ -2358,14 +2461,14 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
                 if (black && E->tune.prolong_quad) {
                     const auto& pq = E->r_prolong_quad[l];
                     const auto& pe = E->r_prolong_rest[l];
-                    if (pq.cnt) e_prolong4_black<<<pgrid(E, pq.cnt, 4), 256, 0, s>>>(it + pq.off, pq.cnt, D, S);
-                    if (pe.cnt) e_prolong4<<<pgrid(E, pe.cnt), rb, 0, s>>>(it + pe.off, pe.cnt, D, S, black);
+                    if (pq.cnt) launch_pdl(*c, e_prolong4_black, dim3(pgrid(E, pq.cnt, 4)), dim3(256), it + pq.off, pq.cnt, D, S);
+                    if (pe.cnt) launch_pdl(*c, e_prolong4, dim3(pgrid(E, pe.cnt)), dim3(rb), it + pe.off, pe.cnt, D, S, black);
                     nk += (pq.cnt ? 1 : 0) + (pe.cnt ? 1 : 0);
                 } else {
-                    if (pv.cnt) e_prolong4<<<pgrid(E, pv.cnt), rb, 0, s>>>(it + pv.off, pv.cnt, D, S, black);
+                    if (pv.cnt) launch_pdl(*c, e_prolong4, dim3(pgrid(E, pv.cnt)), dim3(rb), it + pv.off, pv.cnt, D, S, black);
                     nk += pv.cnt ? 1 : 0;
                 }
-                if (pr.cnt) e_prolong<<<pgrid(E, pr.cnt), rb, 0, s>>>(it + pr.off, pr.cnt, D, S, black);
+                if (pr.cnt) launch_pdl(*c, e_prolong, dim3(pgrid(E, pr.cnt)), dim3(rb), it + pr.off, pr.cnt, D, S, black);
                 ep_end(c, NYXPM_ST_PROLONG);
                 c->launches += nk + (pr.cnt ? 1 : 0) - 1;
                 for (int sw = 0; sw < c->p.nu2; ++sw)
@@ -2375,26 +2478,26 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
         }
         const auto& r0 = E->r_rows_split[0];
         ep_begin(c);
-        e_count_inner<<<bb, 128, 0, s>>>(nbox, S, E->tune.inner_vcycles);
+        launch_pdl(*c, e_count_inner, dim3(bb), dim3(128), nbox, S, E->tune.inner_vcycles);
         if (first && o == 0) {
-            e_update<<<pgrid(E, r0.cnt), rb, 0, s>>>(it + r0.off, r0.cnt, D, S);
+            launch_pdl(*c, e_update, dim3(pgrid(E, r0.cnt)), dim3(rb), it + r0.off, r0.cnt, D, S);
             const auto& cv = E->r_correct_vec;
             const auto& cr = E->r_correct_rest;
-            if (cv.cnt) e_resid_v<<<pgrid(E, cv.cnt), rb, 0, s>>>(it + cv.off, cv.cnt, D, S, 1);
-            if (cr.cnt) e_resid<<<pgrid(E, cr.cnt), rb, 0, s>>>(it + cr.off, cr.cnt, D, S, 1);
+            if (cv.cnt) launch_pdl(*c, e_resid_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S, 1);
+            if (cr.cnt) launch_pdl(*c, e_resid, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, 1);
             c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
         } else {
             const float c_hi = (float)(1.0 / 6.0);
             const float c_lo = (float)(1.0 / 6.0 - (double)c_hi);
             const auto& cv = E->r_correct_vec;
             const auto& cr = E->r_correct_rest;
-            if (cv.cnt) e_correct_v<<<pgrid(E, cv.cnt), rb, 0, s>>>(it + cv.off, cv.cnt, D, S, c_hi, c_lo);
-            if (cr.cnt) e_correct<<<pgrid(E, cr.cnt), rb, 0, s>>>(it + cr.off, cr.cnt, D, S, c_hi, c_lo);
+            if (cv.cnt) launch_pdl(*c, e_correct_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S, c_hi, c_lo);
+            if (cr.cnt) launch_pdl(*c, e_correct, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, c_hi, c_lo);
             c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
-            e_zero_inner<<<pgrid(E, r0.cnt), rb, 0, s>>>(it + r0.off, r0.cnt, D, S,
+            launch_pdl(*c, e_zero_inner, dim3(pgrid(E, r0.cnt)), dim3(rb), it + r0.off, r0.cnt, D, S,
                                                           c->p.nu1 > 0 ? 0 : 1);
         }
-        e_flags<<<bb, 128, 0, s>>>(nbox, D, S, c->p.rel_tol, (first && o == 0) ? 2 : 0);
+        launch_pdl(*c, e_flags, dim3(bb), dim3(128), nbox, D, S, c->p.rel_tol, (first && o == 0) ? 2 : 0);
         ep_end(c, NYXPM_ST_NORM);
         c->launches += 4;
     }
@@ -2405,7 +2508,7 @@ void enqueue_grav(nyxpm_ctx* c, nyxpm_ensemble* E)
     const dim3 rb(32, E->tune.smooth_rows);
     const auto& r0 = E->r_rows_split[0];
     ep_begin(c);
-    e_grav<<<pgrid(E, r0.cnt), rb, 0, c->stream>>>(E->d_items + r0.off, r0.cnt, E->d_desc, E->d_state);
+    launch_pdl(*c, e_grav, dim3(pgrid(E, r0.cnt)), dim3(rb), E->d_items + r0.off, r0.cnt, E->d_desc, E->d_state);
     ep_end(c, NYXPM_ST_KICK);
     c->launches += 1;
 }
@@ -2413,7 +2516,7 @@ void enqueue_grav(nyxpm_ctx* c, nyxpm_ensemble* E)
 void enqueue_kick(nyxpm_ctx* c, nyxpm_ensemble* E, int phase)
 {
     ep_begin(c);
-    e_kick<<<pgrid(E, E->r_part.cnt), kPT, 0, c->stream>>>(E->d_items + E->r_part.off, E->r_part.cnt,
+    launch_pdl(*c, e_kick, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), E->d_items + E->r_part.off, E->r_part.cnt,
                                                             E->d_desc, E->d_state, phase,
                                                             E->tune.sort_bucket);
     ep_end(c, NYXPM_ST_KICK);
@@ -2424,7 +2527,7 @@ void enqueue_load(nyxpm_ctx* c, nyxpm_ensemble* E, const EStep* host_src)
 {
     const int nbox = (int)E->slots.size();
     cudaMemcpyAsync(E->d_step, host_src, nbox * sizeof(EStep), cudaMemcpyHostToDevice, c->stream);
-    e_load_step<<<(nbox + 127) / 128, 128, 0, c->stream>>>(nbox, E->d_step, E->d_desc, E->d_state);
+    launch_pdl(*c, e_load_step, dim3((nbox + 127) / 128), dim3(128), nbox, E->d_step, E->d_desc, E->d_state);
     c->launches += 1;
 }
 
