@@ -2914,13 +2914,13 @@ nyxpm_status nyxpm_ensemble_download(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, 
     ETRY(pull_state(c, E));
     const EDesc& d = E->slots[slot].desc;
     const long long np = d.np, piece = piece_of(d);
+    touch_pages(pos, 24 * np);
+    touch_pages(vel, 24 * np);
     cudaMemsetAsync(d.norms + 2, 0, sizeof(unsigned long long), c->stream);
     for (long long q0 = 0; q0 < np; q0 += piece) {
         const long long m = std::min(piece, np - q0);
         e_pack<<<(unsigned)((np + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, np, d.dx, parr(d, E->h_state[slot].parity),
                                                                         d.beta_r, d.beta_b, d.norms + 2);
-        touch_pages(pos + 3 * q0, 24 * m);
-        touch_pages(vel + 3 * q0, 24 * m);
         cudaMemcpyAsync(pos + 3 * q0, d.beta_r, 24 * m, cudaMemcpyDeviceToHost, c->stream);
         cudaMemcpyAsync(vel + 3 * q0, d.beta_b, 24 * m, cudaMemcpyDeviceToHost, c->stream);
     }
