@@ -377,7 +377,7 @@ nyxpm_status nyxpm_box_create(nyxpm_ctx* c, int n, double L, int64_t np, nyxpm_p
     ALLOC(b->nat, nc);
     ALLOC(b->rows, (size_t)n * n);
     ALLOC(b->planes, n);
-    ALLOC(b->scal, 4);
+    ALLOC(b->scal, 40);
     ALLOC(b->norms, 8);
     ALLOC(b->staging, 7 * (size_t)np + 1);
     if (cudaMallocHost(&b->h_norms, 8 * sizeof(unsigned long long)) != cudaSuccess) {
@@ -421,6 +421,7 @@ nyxpm_status nyxpm_box_create(nyxpm_ctx* c, int n, double L, int64_t np, nyxpm_p
     cudaMemcpyAsync(b->G, G.data(), sizeof(double) * G.size(), cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(b->Gf, Gf.data(), sizeof(float) * Gf.size(), cudaMemcpyHostToDevice, c->stream);
     cudaMemsetAsync(b->cell_count, 0, sizeof(int) * nc, c->stream);
+    cudaMemsetAsync(b->scal, 0, 40 * sizeof(double), c->stream);
     for (const Level& l : b->levels) {
         const size_t cnt = (size_t)l.n * l.n * l.n;
         if (l.split) {

@@ -485,7 +485,7 @@ struct Box {
     double* nat = nullptr;             // n^3 natural-layout scratch for phi in/out
     double* rows = nullptr;            // n^2 row sums
     double* planes = nullptr;          // n plane sums
-    double* scal = nullptr;            // [0] mean
+    double* scal = nullptr;            // [0] mean; mixed: [4] .. [35] its partial sums, [36] their ticket
     unsigned long long* norms = nullptr;   // [0] ||rhs||inf, [1] ||r||inf, [2] bad uploads,
                                            // [3], [5] time-step limit, [4] mixed: max |e|,
                                            // [5] .. [7] a cluster solve's result

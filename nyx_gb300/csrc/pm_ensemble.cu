@@ -25,6 +25,7 @@
 #include "pm_common.cuh"
 #include "pm_prolong.cuh"
 #include "pm_restrict.cuh"
+#include "pm_sum6.cuh"
 #include "pm_tail.cuh"
 
 #include <algorithm>
@@ -764,7 +765,7 @@ __global__ void __launch_bounds__(256) e_resid(const Item* __restrict__ items, i
 // e_correct_v's items: one task per compact pair of one row (k_mx_resid2's
 // pattern: paired FP64 loads, the neighbour sum in nbr_sum_split's order), so
 // small boxes fill the block; the same bits as e_resid.
-__global__ void __launch_bounds__(256, 5) e_resid_v(const Item* __restrict__ items, int nitems,
+__global__ void __launch_bounds__(256, 4) e_resid_v(const Item* __restrict__ items, int nitems,
                                                  const EDesc* __restrict__ D, const EState* __restrict__ S,
                                                  int low_words)
 {
@@ -772,6 +773,7 @@ __global__ void __launch_bounds__(256, 5) e_resid_v(const Item* __restrict__ ite
     pdl_trigger();
     const int nthreads = blockDim.x * blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    const bool on_int = sum6_on_int();
     for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
         const Item it = items[w];
         const EState st = S[it.box];
@@ -813,16 +815,9 @@ __global__ void __launch_bounds__(256, 5) e_resid_v(const Item* __restrict__ ite
                 const double2 zp = __ldg(reinterpret_cast<const double2*>(other + row(j, kp) + ih));
                 const double2 b = __ldg(reinterpret_cast<const double2*>(beta + t));
                 const double2 m = __ldg(reinterpret_cast<const double2*>(mine + t));
-                double s0 = xm0 + xp0;
-                s0 = s0 + ym.x;
-                s0 = s0 + yp.x;
-                s0 = s0 + zm.x;
-                s0 = s0 + zp.x;
-                double s1 = xm1 + xp1;
-                s1 = s1 + ym.y;
-                s1 = s1 + yp.y;
-                s1 = s1 + zm.y;
-                s1 = s1 + zp.y;
+                const double nb0[6] = {xm0, xp0, ym.x, yp.x, zm.x, zp.x};
+                const double nb1[6] = {xm1, xp1, ym.y, yp.y, zm.y, zp.y};
+                const double s0 = sum6(nb0, on_int), s1 = sum6(nb1, on_int);
                 const double r0v = b.x - fma(s0, kSixth, -m.x);
                 const double r1v = b.y - fma(s1, kSixth, -m.y);
                 const float h0 = f64_to_f32_rn(r0v), h1 = f64_to_f32_rn(r1v);

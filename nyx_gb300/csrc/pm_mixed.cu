@@ -16,6 +16,7 @@
 #include "pm_common.cuh"
 #include "pm_prolong.cuh"
 #include "pm_restrict.cuh"
+#include "pm_sum6.cuh"
 #include "pm_tail.cuh"
 
 #include <algorithm>
@@ -419,24 +420,30 @@ __global__ void k_mx_rowsum(int n, const float* __restrict__ rho, double mo, dou
     if (lane == 0) rows[row] = s - (double)n * mo;
 }
 
-__global__ void k_mx_mean(int n, double dx, double L, const double* __restrict__ rows, double* scal)
+// Compensated sum of the n^2 row sums: 1024 strided partials, a halving tree over each 32
+// of them, and those 32 sums in order by whichever block ends last (ticket wraps to 0).
+// The partials are a chain of FP64 additions each, and one SM's FP64 pipe took 83 us for
+// them at 256^3; a block of 32 threads each on 32 SMs takes 17 us.
+constexpr int kMeanBlocks = 32;
+
+__global__ void __launch_bounds__(32) k_mx_mean(int n, double dx, double L, const double* __restrict__ rows,
+                                                double* part, unsigned* ticket, double* scal)
 {
-    // one block: compensated sum of the n^2 row sums
-    __shared__ double ss[32];
     double s = 0.0, c = 0.0;
-    for (long long r = threadIdx.x; r < (long long)n * n; r += blockDim.x) kahan_add(s, c, rows[r]);
+    for (long long r = blockIdx.x * 32 + threadIdx.x; r < (long long)n * n; r += 32 * kMeanBlocks)
+        kahan_add(s, c, rows[r]);
     s -= c;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if (lane == 0) ss[w] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0, tc = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) kahan_add(t, tc, ss[q]);
-        t -= tc;
-        scal[0] = (t * (dx * dx * dx)) / (L * L * L);
-    }
+    if (threadIdx.x != 0) return;
+    part[blockIdx.x] = s;
+    __threadfence();
+    if (atomicInc(ticket, kMeanBlocks - 1) != kMeanBlocks - 1) return;
+    __threadfence();
+    double t = 0.0, tc = 0.0;
+    for (int q = 0; q < kMeanBlocks; ++q) kahan_add(t, tc, *(volatile double*)(part + q));
+    t -= tc;
+    scal[0] = (t * (dx * dx * dx)) / (L * L * L);
 }
 
 // beta = (rho - mass_offset - mean) * (-4 pi G / a) * h^2/6: one FP64 subtraction
@@ -521,8 +528,9 @@ __global__ void k_mx_resid(int n, const double* __restrict__ phi_r, const double
 
 // The same residual, two compact cells of each colour per thread (16-byte
 // loads of FP64 pairs) for rows of an even number of compact cells.  Every
-// residual is k_mx_resid's, term for term.
-__global__ void k_mx_resid2(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
+// residual is k_mx_resid's, term for term.  ints: neighbour sums on the integer
+// pipes (pm_sum6.cuh), where the FP64 pipe bounds the pass (256^3: 291 -> 190 us; 160^3: 117 -> 76).
+__global__ void __launch_bounds__(256) k_mx_resid2(int n, int ints, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
                             const double* __restrict__ beta_r, const double* __restrict__ beta_b,
                             float* r_r, float* r_b, float* rl_r, float* rl_b,
                             unsigned long long* norm)
@@ -531,6 +539,7 @@ __global__ void k_mx_resid2(int n, const double* __restrict__ phi_r, const doubl
     const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;   // compact cells 2 t2, 2 t2 + 1
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
+    const bool on_int = ints && sum6_on_int();
     unsigned long long v = 0;
     if (t2 < half / 2 && j < n) {
         const unsigned ih = 2 * t2;
@@ -560,16 +569,9 @@ __global__ void k_mx_resid2(int n, const double* __restrict__ phi_r, const doubl
             const double2 zp = __ldg(reinterpret_cast<const double2*>(other + row(j, kp) + ih));
             const double2 b = __ldg(reinterpret_cast<const double2*>(beta + t));
             const double2 m = __ldg(reinterpret_cast<const double2*>(mine + t));
-            double s0 = xm0 + xp0;
-            s0 = s0 + ym.x;
-            s0 = s0 + yp.x;
-            s0 = s0 + zm.x;
-            s0 = s0 + zp.x;
-            double s1 = xm1 + xp1;
-            s1 = s1 + ym.y;
-            s1 = s1 + yp.y;
-            s1 = s1 + zm.y;
-            s1 = s1 + zp.y;
+            const double nb0[6] = {xm0, xp0, ym.x, yp.x, zm.x, zp.x};
+            const double nb1[6] = {xm1, xp1, ym.y, yp.y, zm.y, zp.y};
+            const double s0 = sum6(nb0, on_int), s1 = sum6(nb1, on_int);
             const double r0v = b.x - fma(s0, kSixth, -m.x);
             const double r1v = b.y - fma(s1, kSixth, -m.y);
             const float h0 = f64_to_f32_rn(r0v), h1 = f64_to_f32_rn(r1v);
@@ -773,6 +775,8 @@ __global__ void __launch_bounds__(256) k_gsrb_f(int n, int color, float* __restr
 // (measured 20.6 us per half sweep; 2 planes 19.1 us, 1 plane 19.4 us)
 constexpr int kMarchZ = 2;
 constexpr int kMarchMinEdge = 256;
+// the FP64 residual of levels of at least this edge sums on the integer pipes
+constexpr int kIntMinEdge = 96;
 
 template <int MZ>
 __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __restrict__ mine,
@@ -837,12 +841,18 @@ __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __rest
 // every black neighbour is 0, so each red cell gets fmaf(0, 1/6, -beta) -- the
 // general sweep's value, without the loads, and without zeroing e beforehand
 // (the black half sweep after it reads only the red cells it overwrote).
-__global__ void k_gsrb_f_zero(long long cnt, float* __restrict__ mine, const float* __restrict__ beta)
+// Four cells per thread (a colour of a split level holds a multiple of four cells: n is
+// even); 256^3: 33.6 us with one cell per thread, 10.9 us so.
+__global__ void __launch_bounds__(256) k_gsrb_f_zero(unsigned quads, float4* __restrict__ mine,
+                                                     const float4* __restrict__ beta)
 {
     pdl_wait();
     pdl_trigger();
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < cnt) mine[t] = fmaf(0.f, kSixthF, -beta[t]);
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= quads) return;
+    const float4 b = __ldg(beta + t);
+    mine[t] = make_float4(fmaf(0.f, kSixthF, -b.x), fmaf(0.f, kSixthF, -b.y), fmaf(0.f, kSixthF, -b.z),
+                          fmaf(0.f, kSixthF, -b.w));
 }
 
 __device__ __forceinline__ float resid_f(const LevelViewF& L, int i, int j, int k)
@@ -1420,7 +1430,8 @@ nyxpm_status gsrb_sweep_f(Ctx& c, const Level& l, int fine, bool zero_start = fa
         const float* beta = color ? l.fbeta_b : l.fbeta_r;
         prof_begin(c);
         if (zero_start && color == 0)
-            launch_pdl(c, k_gsrb_f_zero, dim3(blocks_for(half_cells)), dim3(kThreads), half_cells, mine, beta);
+            launch_pdl(c, k_gsrb_f_zero, dim3(blocks_for(half_cells / 4)), dim3(kThreads), half_cells / 4,
+                       reinterpret_cast<float4*>(mine), reinterpret_cast<const float4*>(beta));
         else if (march)
             launch_pdl(c, k_gsrb_f4<kMarchZ>, dim3(g.grid), dim3(g.block), l.n, color, mine, other, beta);
         else if (vec)
@@ -1567,7 +1578,7 @@ nyxpm_status launch_mx_resid(Ctx& c, Box& b, bool low_words)
         const Geo g = geo3(l.n / 2, l.n, l.n);
         if ((l.n / 2) % 2 == 0) {
             const Geo g2 = geo3(l.n / 4, l.n, l.n);
-            k_mx_resid2<<<g2.grid, g2.block, 0, c.stream>>>(l.n, l.phi_r, l.phi_b, l.beta_r,
+            k_mx_resid2<<<g2.grid, g2.block, 0, c.stream>>>(l.n, l.n >= kIntMinEdge ? 1 : 0, l.phi_r, l.phi_b, l.beta_r,
                                                             l.beta_b, l.fbeta_r, l.fbeta_b, rl_r,
                                                             rl_b, b.norms + 1);
         } else {
@@ -1795,7 +1806,8 @@ nyxpm_status mixed_make_rhs(Ctx& c, Box& b, double a)
     prof_begin(c);
     k_mx_rowsum<<<blocks_for((long long)n * n * 32), kThreads, 0, c.stream>>>(n, b.frho,
                                                                              b.mass_offset, b.rows);
-    k_mx_mean<<<1, 1024, 0, c.stream>>>(n, dx, b.L, b.rows, b.scal);
+    k_mx_mean<<<kMeanBlocks, 32, 0, c.stream>>>(n, dx, b.L, b.rows, b.scal + 4,
+                                                reinterpret_cast<unsigned*>(b.scal + 4 + kMeanBlocks), b.scal);
     const double scale = ((-4.0 * M_PI * c.p.gconst) * (1.0 / a)) * beta_scale(b);
     k_mx_make_beta<<<g.grid, g.block, 0, c.stream>>>(n, l0.split, b.frho, b.mass_offset, b.scal,
                                                      scale, l0.beta_r, l0.beta_b);
