@@ -877,7 +877,8 @@ struct nyxpm_amr {
     int *lev = nullptr, *box = nullptr;
     double* staging = nullptr;
     unsigned long long* norms = nullptr;     // [0] ||beta||, [1] ||r||, [2] move errors
-    unsigned long long* h_norms = nullptr;
+    unsigned long long* h_norms = nullptr;   // pinned host mirror, and post's flag behind it
+    Post post;
     nyxpm_box* mg = nullptr;                 // level 0's multigrid hierarchy
     IterGraph iter_graph;                    // a composite V-cycle, its residual and the norm's copy
     std::vector<void*> allocs;
@@ -1328,6 +1329,7 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
     }
     if ((st = check_launch(c, "multilevel rhs")) != NYXPM_OK) return st;
     cudaMemsetAsync(A.phi, 0, sizeof(double) * A.ntot, c.stream);
+    post_open(c, A.post);
     cudaMemsetAsync(A.norms, 0, sizeof(unsigned long long), c.stream);
     prof_begin(c);
     k_amr_absmax0<<<norm_grid(c, n3), kT, 0, c.stream>>>(n3, A.beta, A.d_cov, A.inv_scale[0], A.norms);
@@ -1340,8 +1342,9 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
         prof_end(c, NYXPM_ST_NORM, 33.0 * A.fine_cells.count);
     }
     if ((st = comp_resid(c, A, 1)) != NYXPM_OK) return st;
-    cudaMemcpyAsync(A.h_norms, A.norms, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.stream);
-    if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "multilevel solve sync");
+    post_words(c, A.post, A.norms, 0, 2);
+    if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
+    if ((st = post_wait(c, A.post, "multilevel solve sync")) != NYXPM_OK) return st;
     const double bnorm = read_bits(A.h_norms, 0), r0 = read_bits(A.h_norms, 1);
     const double target = c.p.rel_tol * std::max(bnorm, r0);
     double r = r0;
@@ -1353,13 +1356,13 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
             nyxpm_status s;
             if ((s = vcycle(cx, A)) != NYXPM_OK) return s;
             if ((s = comp_resid(c, A, 1)) != NYXPM_OK) return s;
-            cudaMemcpyAsync(A.h_norms + 1, A.norms + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                            c.stream);
-            return check_launch(c, "norm copy");
+            post_words(c, A.post, A.norms, 1, 1);
+            return check_launch(c, "norm read-back");
         };
         for (it = 1; it <= c.p.max_vcycles; ++it) {
+            post_open(c, A.post);
             if ((st = run_iteration(c, A.iter_graph, iteration)) != NYXPM_OK) return st;
-            if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "multilevel solve sync");
+            if ((st = post_wait(c, A.post, "multilevel solve sync")) != NYXPM_OK) return st;
             r = read_bits(A.h_norms, 1);
             if (r != r) {
                 c.err = "multilevel residual is NaN";
@@ -1425,8 +1428,11 @@ nyxpm_status assign(Ctx& c, nyxpm_amr& A)
 
 nyxpm_status move_errors(nyxpm_ctx* c, nyxpm_amr& A)
 {
-    cudaMemcpyAsync(A.h_norms + 2, A.norms + 2, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream);
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) return check_launch(*c, "multilevel kick sync");
+    nyxpm_status st;
+    post_open(*c, A.post);
+    post_words(*c, A.post, A.norms, 2, 1);
+    if ((st = check_launch(*c, "norm read-back")) != NYXPM_OK) return st;
+    if ((st = post_wait(*c, A.post, "multilevel kick sync")) != NYXPM_OK) return st;
     if (A.h_norms[2] != 0) {
         c->err = "a particle's stencil left its box's ghost cells (more than 2 cells of motion in one step)";
         cudaMemsetAsync(A.norms + 2, 0, sizeof(unsigned long long), c->stream);
@@ -1588,11 +1594,8 @@ nyxpm_status nyxpm_amr_create(nyxpm_ctx* c, int n0, double L, int nlev, const in
     AALLOC(a->norms, 4);
     cudaMemsetAsync(a->norms, 0, 4 * sizeof(unsigned long long), c->stream);
 #undef AALLOC
-    if (cudaMallocHost(&a->h_norms, 4 * sizeof(unsigned long long)) != cudaSuccess) {
-        cudaGetLastError();
-        a->h_norms = nullptr;
-        return cleanup(afail(c, NYXPM_OOM, "pinned norms"));
-    }
+    if (post_alloc(a->post) != NYXPM_OK) return cleanup(afail(c, NYXPM_OOM, "pinned norms"));
+    a->h_norms = a->post.host;
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return cleanup(check_launch(*c, "hierarchy create"));
     *out = a;
     return NYXPM_OK;

@@ -43,6 +43,62 @@ nyxpm_status check_launch(Ctx& c, const char* what)
     return e == cudaErrorMemoryAllocation ? NYXPM_OOM : NYXPM_CUDA_ERROR;
 }
 
+// bound by the latency of one store to host memory; the fence orders the words before
+// the flag for the host
+__global__ void k_post(const unsigned long long* __restrict__ words, int first, int count, unsigned long long* host)
+{
+    pdl_wait();
+    pdl_trigger();
+    const int t = threadIdx.x;
+    if (t < count) {
+        reinterpret_cast<volatile unsigned long long*>(host)[first + t] = words[first + t];
+        __threadfence_system();
+    }
+    __syncwarp();
+    if (t == 0) reinterpret_cast<volatile unsigned long long*>(host)[kPostWords] = 1;
+}
+
+nyxpm_status post_alloc(Post& p)
+{
+    if (cudaMallocHost(&p.host, (kPostWords + 1) * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaGetLastError();
+        p.host = nullptr;
+        return NYXPM_OOM;
+    }
+    return NYXPM_OK;
+}
+
+void post_open(Ctx& c, Post& p)
+{
+    if (p.open) cudaStreamSynchronize(c.stream);   // a call that failed half way left one in flight
+    __atomic_store_n(p.host + kPostWords, 0ULL, __ATOMIC_RELEASE);
+    p.open = 1;
+}
+
+void post_words(Ctx& c, const Post& p, const unsigned long long* words, int first, int count)
+{
+    launch_pdl(c, k_post, dim3(1), dim3(32), words, first, count, p.host);
+    c.launches += 1;
+}
+
+nyxpm_status post_wait(Ctx& c, Post& p, const char* what)
+{
+    cudaError_t e = cudaErrorNotReady;
+    for (int i = 1; !__atomic_load_n(p.host + kPostWords, __ATOMIC_ACQUIRE); ++i) {
+        if (i & 4095) continue;
+        if (e != cudaErrorNotReady) {   // the stream ended without the words
+            const nyxpm_status st = check_launch(c, what);
+            if (st != NYXPM_OK) return st;
+            c.err = std::string(what) + ": no read-back";
+            return NYXPM_CUDA_ERROR;
+        }
+        e = cudaStreamQuery(c.stream);
+        if (e == cudaErrorNotReady) cudaGetLastError();
+    }
+    p.open = 0;
+    return NYXPM_OK;
+}
+
 nyxpm_status run_iteration(Ctx& c, IterGraph& g, const std::function<nyxpm_status()>& body)
 {
     if (c.prof_on || g.failed) return body();
@@ -380,11 +436,8 @@ nyxpm_status nyxpm_box_create(nyxpm_ctx* c, int n, double L, int64_t np, nyxpm_p
     ALLOC(b->scal, 40);
     ALLOC(b->norms, 8);
     ALLOC(b->staging, 7 * (size_t)np + 1);
-    if (cudaMallocHost(&b->h_norms, 8 * sizeof(unsigned long long)) != cudaSuccess) {
-        cudaGetLastError();
-        b->h_norms = nullptr;
-        return cleanup(fail(c, NYXPM_OOM, "cudaMallocHost"));
-    }
+    if (post_alloc(b->post) != NYXPM_OK) return cleanup(fail(c, NYXPM_OOM, "cudaMallocHost"));
+    b->h_norms = b->post.host;
     // multigrid hierarchy: split levels while n > 8, natural bottom
     const int nbot = bottom_edge(n);
     for (int nl = n;; nl /= 2) {
@@ -863,11 +916,11 @@ nyxpm_status nyxpm_est_time_step(nyxpm_ctx* c, nyxpm_box* b, double cfl, double 
     }
     if (!b->have_phi && !b->g_from_caller)
         return fail(c, NYXPM_INVALID_ARG, "no field: solve, step, set phi or set the gravity vector first");
+    post_open(*c, b->post);
     TRY(b->prec == NYXPM_MIXED ? mixed_est_dt(*c, *b) : launch_est_dt(*c, *b));
-    cudaMemcpyAsync(b->h_norms + 3, b->norms + 3, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                    c->stream);
+    post_words(*c, b->post, b->norms, 3, 3);
     TRY(check_launch(*c, "time-step readback"));
-    TRY(nyxpm_synchronize(c));
+    TRY(post_wait(*c, b->post, "time-step readback"));
     double v, g2;
     std::memcpy(&v, &b->h_norms[3], sizeof(double));
     std::memcpy(&g2, &b->h_norms[5], sizeof(double));

@@ -1844,6 +1844,7 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
     // inner right-hand side, and r_lo) and updates it from each correction
     // (k_mx_correct) instead of applying the FP64 stencil to phi.
     const bool incremental = l0.split != 0;
+    post_open(c, b.post);
     prof_begin(c);
     cudaMemsetAsync(b.norms, 0, sizeof(unsigned long long), c.stream);
     if (l0.split) {
@@ -1858,12 +1859,8 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
     if (zero_guess && incremental) {
         // r0 = beta exactly: its two words, no stencil
         if ((st = launch_mx_split_beta(c, b)) != NYXPM_OK) return st;
-        cudaMemcpyAsync(b.h_norms, b.norms, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                        c.stream);
     } else {
         if ((st = launch_mx_resid(c, b, incremental)) != NYXPM_OK) return st;
-        cudaMemcpyAsync(b.h_norms, b.norms, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                        c.stream);
     }
     // a small box: the iterations in one cluster launch (until the residual has to be
     // recomputed from phi)
@@ -1889,11 +1886,21 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
         prof_begin(c);
         launch_cluster(c, k_cluster_solve_f, ca.elems * sizeof(float), ca, P);
         prof_end(c, NYXPM_ST_SMOOTH, 0);
-        cudaMemcpyAsync(b.h_norms, b.norms, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c.stream);
         return check_launch(c, "mixed cluster solve");
     };
+    // the residual from phi with the FP64 stencil, its norm to the host
+    auto recompute = [&]() -> nyxpm_status {
+        nyxpm_status s;
+        post_open(c, b.post);
+        if ((s = launch_mx_resid(c, b, true)) != NYXPM_OK) return s;
+        post_words(c, b.post, b.norms, 1, 1);
+        if ((s = check_launch(c, "norm read-back")) != NYXPM_OK) return s;
+        return post_wait(c, b.post, "mixed sync");
+    };
     if (in_cluster && (st = cluster_solve(0, -1.0)) != NYXPM_OK) return st;
-    if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
+    post_words(c, b.post, b.norms, 0, 8);
+    if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
+    if ((st = post_wait(c, b.post, "mixed sync")) != NYXPM_OK) return st;
     const double bnorm = read_norm(b, 0);
     const double r0 = (zero_guess && incremental) ? bnorm : read_norm(b, 1);
     const double target = c.p.rel_tol * std::max(bnorm, r0);
@@ -1907,10 +1914,7 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
             err = read_norm(b, 7);
             it = (int)(b.h_norms[6] & 0xffffffffULL);
             if (b.h_norms[6] >> 32) {
-                if ((st = launch_mx_resid(c, b, true)) != NYXPM_OK) return st;
-                cudaMemcpyAsync(b.h_norms + 1, b.norms + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                c.stream);
-                if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
+                if ((st = recompute()) != NYXPM_OK) return st;
                 r = read_norm(b, 1);
                 err = 0.0;
             }
@@ -1925,8 +1929,11 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
                 c.err = "defect correction reached max_vcycles above tolerance";
                 break;
             }
+            post_open(c, b.post);
             if ((st = cluster_solve(it, target)) != NYXPM_OK) return st;
-            if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
+            post_words(c, b.post, b.norms, 0, 8);
+            if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
+            if ((st = post_wait(c, b.post, "mixed sync")) != NYXPM_OK) return st;
         }
     } else if (!(r0 <= target)) {
         auto iteration = [&]() -> nyxpm_status {
@@ -1937,20 +1944,18 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
                 if ((s = vcycle_f(c, b, 0, v == 0)) != NYXPM_OK) return s;
             if (incremental) {
                 if ((s = launch_mx_correct(c, b)) != NYXPM_OK) return s;
-                cudaMemcpyAsync(b.h_norms + 4, b.norms + 4, sizeof(unsigned long long),
-                                cudaMemcpyDeviceToHost, c.stream);
             } else {
                 if ((s = launch_mx_update(c, b)) != NYXPM_OK) return s;
                 if ((s = launch_mx_resid(c, b, false)) != NYXPM_OK) return s;
             }
-            cudaMemcpyAsync(b.h_norms + 1, b.norms + 1, sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, c.stream);
-            return check_launch(c, "norm copy");
+            post_words(c, b.post, b.norms, 1, 4);
+            return check_launch(c, "norm read-back");
         };
         for (it = 1; it <= c.p.max_vcycles; ++it) {
+            post_open(c, b.post);
             if ((st = run_iteration(c, b.iter_graph[0], iteration)) != NYXPM_OK) return st;
             inner += c.p.mixed_inner_vcycles;
-            if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "mixed sync");
+            if ((st = post_wait(c, b.post, "mixed sync")) != NYXPM_OK) return st;
             r = read_norm(b, 1);
             if (incremental) {
                 err += kDfUpdateErr * read_norm(b, 4);
@@ -1958,11 +1963,7 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
                     // the bound could hide the tolerance: recompute r from phi with
                     // the FP64 stencil (a zero-guess solve's first correction is as
                     // large as phi, so it always lands here once)
-                    if ((st = launch_mx_resid(c, b, true)) != NYXPM_OK) return st;
-                    cudaMemcpyAsync(b.h_norms + 1, b.norms + 1, sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, c.stream);
-                    if (cudaStreamSynchronize(c.stream) != cudaSuccess)
-                        return check_launch(c, "mixed sync");
+                    if ((st = recompute()) != NYXPM_OK) return st;
                     r = read_norm(b, 1);
                     err = 0.0;
                 }

@@ -912,6 +912,7 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
     nyxpm_status st;
     const Level& l0 = b.levels[0];
     const long long nc = (long long)l0.n * l0.n * l0.n;
+    post_open(c, b.post);
     // ||beta||_inf and ||r0||_inf
     prof_begin(c);
     cudaMemsetAsync(b.norms, 0, sizeof(unsigned long long), c.stream);
@@ -935,9 +936,9 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
         prof_end(c, NYXPM_ST_SMOOTH, 0);
         if ((st = check_launch(c, "cluster solve")) != NYXPM_OK) return st;
     }
-    cudaMemcpyAsync(b.h_norms, b.norms, (in_cluster ? 7 : 2) * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                    c.stream);
-    if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "solve sync");
+    post_words(c, b.post, b.norms, 0, in_cluster ? 7 : 2);
+    if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
+    if ((st = post_wait(c, b.post, "solve sync")) != NYXPM_OK) return st;
     const double bnorm = read_norm(b, 0);
     const double r0 = read_norm(b, 1);
     const double target = c.p.rel_tol * std::max(bnorm, r0);
@@ -979,15 +980,15 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
             } else if ((s = launch_resnorm(c, b, 1, red_only)) != NYXPM_OK) {
                 return s;
             }
-            cudaMemcpyAsync(b.h_norms + 1, b.norms + 1, sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, c.stream);
-            return check_launch(c, "norm copy");
+            post_words(c, b.post, b.norms, 1, 1);
+            return check_launch(c, "norm read-back");
         };
         for (it = 1; it <= c.p.max_vcycles; ++it) {
             // one graph per (opening or later iteration, physical red array)
             const int gi = (first ? 0 : 2) + (L0.phi_r == b.phi_r_alloc ? 0 : 1);
+            post_open(c, b.post);
             if ((st = run_iteration(c, b.iter_graph[gi], iteration)) != NYXPM_OK) return st;
-            if (cudaStreamSynchronize(c.stream) != cudaSuccess) return check_launch(c, "solve sync");
+            if ((st = post_wait(c, b.post, "solve sync")) != NYXPM_OK) return st;
             r = read_norm(b, 1);
             if (r != r) {
                 c.err = "multigrid residual is NaN";
