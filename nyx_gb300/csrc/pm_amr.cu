@@ -1182,14 +1182,13 @@ nyxpm_status deposit(Ctx& c, nyxpm_amr& A)
 }
 
 // the composite residual of phi into R (phi's covered cells averaged and ghosts
-// filled first); its norm into norms[slot]
+// filled first); its norm into norms[slot] (0 before)
 nyxpm_status comp_resid(Ctx& c, nyxpm_amr& A, int slot)
 {
     nyxpm_status st;
     const long long n3 = (long long)A.n0 * A.n0 * A.n0;
     if ((st = avg_down(c, A, A.phi)) != NYXPM_OK) return st;
     if ((st = ghost_fill(c, A, A.phi, A.all_ghost1)) != NYXPM_OK) return st;
-    cudaMemsetAsync(A.norms + slot, 0, sizeof(unsigned long long), c.stream);
     const Geo g = geo3(A.n0, A.n0, A.n0, kT);
     prof_begin(c);
     if (g.block.x * g.block.y == kT) {
@@ -1341,7 +1340,7 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
     if ((st = check_launch(c, "multilevel rhs")) != NYXPM_OK) return st;
     cudaMemsetAsync(A.phi, 0, sizeof(double) * A.ntot, c.stream);
     post_open(c, A.post);
-    cudaMemsetAsync(A.norms, 0, sizeof(unsigned long long), c.stream);
+    cudaMemsetAsync(A.norms, 0, 2 * sizeof(unsigned long long), c.stream);
     prof_begin(c);
     k_amr_absmax0<<<norm_grid(c, n3), kT, 0, c.stream>>>(n3, A.beta, A.d_cov, A.inv_scale[0], A.norms);
     prof_end(c, NYXPM_ST_NORM, 9.0 * n3);
@@ -1353,7 +1352,7 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
         prof_end(c, NYXPM_ST_NORM, 33.0 * A.fine_cells.count);
     }
     if ((st = comp_resid(c, A, 1)) != NYXPM_OK) return st;
-    post_words(c, A.post, A.norms, 0, 2);
+    post_words(c, A.post, A.norms, 0, 2, 1 << 1);
     if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
     if ((st = post_wait(c, A.post, "multilevel solve sync")) != NYXPM_OK) return st;
     const double bnorm = read_bits(A.h_norms, 0), r0 = read_bits(A.h_norms, 1);
@@ -1367,7 +1366,7 @@ nyxpm_status solve(nyxpm_ctx* cx, nyxpm_amr& A, double a, nyxpm_solve_info* info
             nyxpm_status s;
             if ((s = vcycle(cx, A)) != NYXPM_OK) return s;
             if ((s = comp_resid(c, A, 1)) != NYXPM_OK) return s;
-            post_words(c, A.post, A.norms, 1, 1);
+            post_words(c, A.post, A.norms, 1, 1, 1 << 1);
             return check_launch(c, "norm read-back");
         };
         for (it = 1; it <= c.p.max_vcycles; ++it) {

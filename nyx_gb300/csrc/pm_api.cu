@@ -45,13 +45,14 @@ nyxpm_status check_launch(Ctx& c, const char* what)
 
 // bound by the latency of one store to host memory; the fence orders the words before
 // the flag for the host
-__global__ void k_post(const unsigned long long* __restrict__ words, int first, int count, unsigned long long* host)
+__global__ void k_post(unsigned long long* words, int first, int count, unsigned zero, unsigned long long* host)
 {
     pdl_wait();
     pdl_trigger();
     const int t = threadIdx.x;
     if (t < count) {
         reinterpret_cast<volatile unsigned long long*>(host)[first + t] = words[first + t];
+        if (zero >> (first + t) & 1) words[first + t] = 0;
         __threadfence_system();
     }
     __syncwarp();
@@ -75,9 +76,9 @@ void post_open(Ctx& c, Post& p)
     p.open = 1;
 }
 
-void post_words(Ctx& c, const Post& p, const unsigned long long* words, int first, int count)
+void post_words(Ctx& c, const Post& p, unsigned long long* words, int first, int count, unsigned zero)
 {
-    launch_pdl(c, k_post, dim3(1), dim3(32), words, first, count, p.host);
+    launch_pdl(c, k_post, dim3(1), dim3(32), words, first, count, zero, p.host);
     c.launches += 1;
 }
 
@@ -228,11 +229,11 @@ nyxpm_status do_solve(Ctx& c, Box& b, double a, int zero_guess, nyxpm_solve_info
     const bool mixed = b.prec == NYXPM_MIXED;
     if ((st = mixed ? mixed_make_rhs(c, b, a) : launch_make_rhs(c, b, a)) != NYXPM_OK) return st;
     if (zero_guess && (st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
-    nyxpm_status solved = mixed ? mixed_solve(c, b, zero_guess, info) : mg_solve(c, b, info);
+    bool grav_done = mixed;   // the mixed solve leaves its FP32 gravity vector in g32 itself
+    nyxpm_status solved = mixed ? mixed_solve(c, b, zero_guess, info) : mg_solve(c, b, info, &grav_done);
     if (solved != NYXPM_OK && solved != NYXPM_NOT_CONVERGED) return solved;
     b.g_from_caller = 0;   // the gravity vector follows the new phi from here on
-    // the mixed solve leaves its FP32 gravity vector in g32 itself
-    if (!mixed && (st = launch_grav_vector(c, b)) != NYXPM_OK) return st;
+    if (!grav_done && (st = launch_grav_vector(c, b)) != NYXPM_OK) return st;
     return solved;
 }
 

@@ -424,6 +424,8 @@ struct ProfRec {
 
 struct Ctx;
 
+constexpr int kScalTicket = 36;        // in Box::scal
+
 // One solver iteration (V-cycle or defect-correction step, its residual norm and
 // the norm's copy to the host) captured once per box and replayed: the launches
 // of a box never change between solves, only the host reads the norm.
@@ -453,6 +455,7 @@ struct Box {
     double mscalar = 0;
     double mass_offset = 0;
     int sorted = 0;
+    int counts_dirty = 0;              // a sort that failed half way may have left cell_count nonzero
     int uploaded = 0;
     int have_phi = 0;
     int g_from_caller = 0;             // g (and g32) hold nyxpm_set_grav_vector's field
@@ -496,7 +499,7 @@ struct Box {
     double* nat = nullptr;             // n^3 natural-layout scratch for phi in/out
     double* rows = nullptr;            // n^2 row sums
     double* planes = nullptr;          // n plane sums
-    double* scal = nullptr;            // [0] mean; mixed: [4] .. [35] its partial sums, [36] their ticket
+    double* scal = nullptr;            // [0] mean; mixed: [4] .. [35] its partial sums; [36] the ticket
     unsigned long long* norms = nullptr;   // [0] ||rhs||inf, [1] ||r||inf, [2] bad uploads,
                                            // [3], [5] time-step limit, [4] mixed: max |e|,
                                            // [5] .. [7] a cluster solve's result
@@ -586,7 +589,8 @@ nyxpm_status run_iteration(Ctx& c, IterGraph& g, const std::function<nyxpm_statu
 // stream complete; an error of the stream ends it as it would end a wait for the stream.
 nyxpm_status post_alloc(Post& p);
 void post_open(Ctx& c, Post& p);
-void post_words(Ctx& c, const Post& p, const unsigned long long* words, int first, int count);
+// (bit i of `zero` set: words[i] is set to 0 once read, for a norm collected by maximum)
+void post_words(Ctx& c, const Post& p, unsigned long long* words, int first, int count, unsigned zero = 0);
 nyxpm_status post_wait(Ctx& c, Post& p, const char* what);
 
 // ---------------------------------------------------------------------------
@@ -612,7 +616,8 @@ nyxpm_status launch_est_dt(Ctx& c, Box& b);
 nyxpm_status mixed_est_dt(Ctx& c, Box& b);
 double beta_scale(const Box& b);  // (h*h)/6 of level 0: rhs -> smoother units
 nyxpm_status launch_zero_phi(Ctx& c, Box& b);
-nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info);
+// grav_done: the gravity vector of the new phi is enqueued (as launch_grav_vector does it)
+nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info, bool* grav_done);
 nyxpm_status launch_grav_vector(Ctx& c, Box& b);
 nyxpm_status launch_phi_to_natural(Ctx& c, Box& b, double* d_out);
 nyxpm_status launch_phi_from_natural(Ctx& c, Box& b, const double* d_in);
@@ -641,6 +646,7 @@ nyxpm_status mixed_g32_from_g(Ctx& c, Box& b);  // FP32 gravity vector of the FP
 nyxpm_status mixed_rho_to_double(Ctx& c, Box& b);
 
 // host-side helpers shared by the forms
+void clear_counts(Ctx& c, Box& b);            // before a sort's keys count into cell_count
 nyxpm_status scan_counts(Ctx& c, Box& b);     // cell_count -> cell_start
 nyxpm_status fix_segments(Ctx& c, Box& b);    // deterministic order inside each key segment
 nyxpm_status sort_from_keys(Ctx& c, Box& b);  // key + cell_count -> perm (scan, scatter, fix)

@@ -209,6 +209,8 @@ __global__ void k_mx_keys(long long np, int n, const int* __restrict__ cell,
                           const float* __restrict__ ox, const float* __restrict__ oy,
                           const float* __restrict__ oz, int* key, int* count)
 {
+    pdl_wait();
+    pdl_trigger();
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= np) return;
     const int c = cell[q];
@@ -229,6 +231,8 @@ __global__ void k_mx_gather(long long np, const int* __restrict__ perm, const in
                             float* ox2, float* oy2, float* oz2, float* vx2, float* vy2, float* vz2,
                             float* m2, int* id2)
 {
+    pdl_wait();
+    pdl_trigger();
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= np) return;
     const int q = perm[s];
@@ -287,6 +291,8 @@ __global__ void __launch_bounds__(256) k_mx_deposit_heavy(int n, const int* __re
                                                           const int* __restrict__ long_count,
                                                           int* key_slot, float* heavy_part)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int total = *long_count;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -340,6 +346,8 @@ __global__ void __launch_bounds__(kDepThreads) k_mx_deposit(
     const int* __restrict__ start, const int* __restrict__ key_slot,
     const float* __restrict__ heavy_part, float* rho)
 {
+    pdl_wait();
+    pdl_trigger();
     // corner-major: a warp's 32 consecutive keys (or cells) touch 32 banks
     __shared__ float part[8 * kDepKeys];
     const int i0 = blockIdx.x * kDepTx, j0 = blockIdx.y * kDepTy, k0 = blockIdx.z * kDepTz;
@@ -401,6 +409,8 @@ __device__ __forceinline__ void kahan_add(double& s, double& c, double v)
 // FP64 and n * mass_offset is taken off once per row
 __global__ void k_mx_rowsum(int n, const float* __restrict__ rho, double mo, double* rows)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= (long long)n * n) return;
@@ -425,54 +435,56 @@ __global__ void k_mx_rowsum(int n, const float* __restrict__ rho, double mo, dou
 // The partials are a chain of FP64 additions each, and one SM's FP64 pipe took 83 us for
 // them at 256^3; a block of 32 threads each on 32 SMs takes 17 us.
 constexpr int kMeanBlocks = 32;
+static_assert(4 + kMeanBlocks == kScalTicket, "the partials end before the ticket");
 
 __global__ void __launch_bounds__(32) k_mx_mean(int n, double dx, double L, const double* __restrict__ rows,
-                                                double* part, unsigned* ticket, double* scal)
+                                                double* part, unsigned* ticket, double* scal,
+                                                unsigned long long* norms)
 {
+    pdl_wait();
+    pdl_trigger();
+    if (blockIdx.x == 0 && (threadIdx.x < 2 || threadIdx.x == 4)) norms[threadIdx.x] = 0;   // maxima of the solve
     double s = 0.0, c = 0.0;
     for (long long r = blockIdx.x * 32 + threadIdx.x; r < (long long)n * n; r += 32 * kMeanBlocks)
         kahan_add(s, c, rows[r]);
     s -= c;
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if (threadIdx.x != 0) return;
-    part[blockIdx.x] = s;
+    unsigned last = 0;
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = s;
+        __threadfence();
+        last = atomicInc(ticket, kMeanBlocks - 1) == kMeanBlocks - 1;
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
-    if (atomicInc(ticket, kMeanBlocks - 1) != kMeanBlocks - 1) return;
-    __threadfence();
+    const double v = *(volatile double*)(part + threadIdx.x);
     double t = 0.0, tc = 0.0;
-    for (int q = 0; q < kMeanBlocks; ++q) kahan_add(t, tc, *(volatile double*)(part + q));
+    for (int q = 0; q < kMeanBlocks; ++q) kahan_add(t, tc, __shfl_sync(0xffffffffu, v, q));
     t -= tc;
-    scal[0] = (t * (dx * dx * dx)) / (L * L * L);
+    if (threadIdx.x == 0) scal[0] = (t * (dx * dx * dx)) / (L * L * L);
 }
 
 // beta = (rho - mass_offset - mean) * (-4 pi G / a) * h^2/6: one FP64 subtraction
-// and one product per cell (offset and scale folded once)
+// and one product per cell (offset and scale folded once); its maximum norm
 __global__ void k_mx_make_beta(int n, int split, const float* __restrict__ rho, double mo,
                                const double* __restrict__ scal, double scale, double* beta_r,
-                               double* beta_b)
+                               double* beta_b, unsigned long long* norm)
 {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
-    if (i >= n || j >= n) return;
-    const double off = mo + scal[0];
-    const double v = f32_to_f64(rho[cidx(i, j, k, n)]);
-    *lv_ptr<double>(beta_r, beta_b, n, split, i, j, k) = (v - off) * scale;
-}
-
-// ---------------------------------------------------------------------------
-// norms (max over |v| bits on the integer pipe)
-// ---------------------------------------------------------------------------
-__global__ void k_mx_absmax(long long cnt, const double* __restrict__ a, unsigned long long* out)
-{
-    unsigned long long v = 0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cnt;
-         t += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long u = absbits(a[t]);
-        v = u > v ? u : v;
+    unsigned long long u = 0;
+    if (i < n && j < n) {
+        const double off = mo + scal[0];
+        const double v = f32_to_f64(rho[cidx(i, j, k, n)]);
+        const double beta = (v - off) * scale;
+        *lv_ptr<double>(beta_r, beta_b, n, split, i, j, k) = beta;
+        u = absbits(beta);
     }
-    block_umax_store(v, out);
+    block_umax_store(u, norm);
 }
 
 // ---------------------------------------------------------------------------
@@ -501,6 +513,8 @@ __global__ void k_mx_resid(int n, const double* __restrict__ phi_r, const double
                            float* r_r, float* r_b, float* rl_r, float* rl_b,
                            unsigned long long* norm)
 {
+    pdl_wait();
+    pdl_trigger();
     const int half = n >> 1;
     const int ih = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -535,6 +549,8 @@ __global__ void __launch_bounds__(256) k_mx_resid2(int n, int ints, const double
                             float* r_r, float* r_b, float* rl_r, float* rl_b,
                             unsigned long long* norm)
 {
+    pdl_wait();
+    pdl_trigger();
     const unsigned half = (unsigned)n >> 1;
     const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;   // compact cells 2 t2, 2 t2 + 1
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -591,6 +607,8 @@ __global__ void __launch_bounds__(256) k_mx_resid2(int n, int ints, const double
 __global__ void k_mx_resid_nat(int n, const double* __restrict__ phi, const double* __restrict__ beta,
                                float* r, unsigned long long* norm)
 {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
@@ -614,6 +632,8 @@ __global__ void k_mx_resid_nat(int n, const double* __restrict__ phi, const doub
 // phi += e (FP64 update with the FP32 correction)
 __global__ void k_mx_update(long long cnt, double* phi, const float* __restrict__ e)
 {
+    pdl_wait();
+    pdl_trigger();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < cnt) phi[t] = phi[t] + f32_to_f64(e[t]);
 }
@@ -631,6 +651,8 @@ __global__ void k_mx_correct(int n, float c_hi, float c_lo, const float* __restr
                              float* r_r, float* r_b, float* rl_r, float* rl_b,
                              unsigned long long* norm, unsigned long long* enorm)
 {
+    pdl_wait();
+    pdl_trigger();
     const int half = n >> 1;
     const int ih = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -677,6 +699,8 @@ __global__ void k_mx_correct2(int n, float c_hi, float c_lo, const float* __rest
                               float* r_r, float* r_b, float* rl_r, float* rl_b,
                               unsigned long long* norm, unsigned long long* enorm)
 {
+    pdl_wait();
+    pdl_trigger();
     const unsigned half = (unsigned)n >> 1;
     const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;   // compact cells 2 t2, 2 t2 + 1
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -734,6 +758,8 @@ __global__ void k_mx_split_beta(long long cnt, const double* __restrict__ beta_r
                                 const double* __restrict__ beta_b, float* r_r, float* r_b,
                                 float* rl_r, float* rl_b)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= cnt) return;
     const double br = beta_r[t], bb = beta_b[t];
@@ -1281,6 +1307,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_f(ClArgs<float>
 // (one float4 {gx, gy, gz, 0} per cell: a CIC corner is one 16-byte load)
 __global__ void k_mx_grav(LevelView L, float half_dxi, float* g)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = L.n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1320,6 +1348,8 @@ struct MxKickArgs {
 __global__ void __launch_bounds__(256, 6) k_mx_kick(long long np, MxKickArgs A, int* cell, float* ox,
                                                  float* oy, float* oz, float* vx, float* vy, float* vz)
 {
+    pdl_wait();
+    pdl_trigger();
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= np) return;
     const int n = A.n;
@@ -1565,7 +1595,7 @@ nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false)
     return NYXPM_OK;
 }
 
-// FP64 residual of level 0 into the FP32 inner right-hand side, its norm into norms[1]
+// FP64 residual of level 0 into the FP32 inner right-hand side, its norm into norms[1] (0 before)
 nyxpm_status launch_mx_resid(Ctx& c, Box& b, bool low_words)
 {
     const Level& l = b.levels[0];
@@ -1573,22 +1603,21 @@ nyxpm_status launch_mx_resid(Ctx& c, Box& b, bool low_words)
     float* rl_r = (low_words && l.split) ? b.r_lo : nullptr;
     float* rl_b = rl_r ? b.r_lo + nc / 2 : nullptr;
     prof_begin(c);
-    cudaMemsetAsync(b.norms + 1, 0, sizeof(unsigned long long), c.stream);
     if (l.split) {
         const Geo g = geo3(l.n / 2, l.n, l.n);
         if ((l.n / 2) % 2 == 0) {
             const Geo g2 = geo3(l.n / 4, l.n, l.n);
-            k_mx_resid2<<<g2.grid, g2.block, 0, c.stream>>>(l.n, l.n >= kIntMinEdge ? 1 : 0, l.phi_r, l.phi_b, l.beta_r,
+            launch_pdl(c, k_mx_resid2, dim3(g2.grid), dim3(g2.block), l.n, l.n >= kIntMinEdge ? 1 : 0, l.phi_r, l.phi_b, l.beta_r,
                                                             l.beta_b, l.fbeta_r, l.fbeta_b, rl_r,
                                                             rl_b, b.norms + 1);
         } else {
-            k_mx_resid<<<g.grid, g.block, 0, c.stream>>>(l.n, l.phi_r, l.phi_b, l.beta_r, l.beta_b,
+            launch_pdl(c, k_mx_resid, dim3(g.grid), dim3(g.block), l.n, l.phi_r, l.phi_b, l.beta_r, l.beta_b,
                                                          l.fbeta_r, l.fbeta_b, rl_r, rl_b,
                                                          b.norms + 1);
         }
     } else {
         const Geo g = geo3(l.n, l.n, l.n);
-        k_mx_resid_nat<<<g.grid, g.block, 0, c.stream>>>(l.n, l.phi_r, l.beta_r, l.fbeta_r,
+        launch_pdl(c, k_mx_resid_nat, dim3(g.grid), dim3(g.block), l.n, l.phi_r, l.beta_r, l.fbeta_r,
                                                          b.norms + 1);
     }
     prof_end(c, NYXPM_ST_NORM, 20.0 * nc);
@@ -1603,17 +1632,15 @@ nyxpm_status launch_mx_correct(Ctx& c, Box& b)
     const float c_hi = (float)(1.0 / 6.0);
     const float c_lo = (float)(1.0 / 6.0 - (double)c_hi);
     prof_begin(c);
-    cudaMemsetAsync(b.norms + 1, 0, sizeof(unsigned long long), c.stream);
-    cudaMemsetAsync(b.norms + 4, 0, sizeof(unsigned long long), c.stream);
     if ((l.n / 2) % 2 == 0) {
         const Geo g = geo3(l.n / 4, l.n, l.n);
-        k_mx_correct2<<<g.grid, g.block, 0, c.stream>>>(l.n, c_hi, c_lo, l.fphi_r, l.fphi_b,
+        launch_pdl(c, k_mx_correct2, dim3(g.grid), dim3(g.block), l.n, c_hi, c_lo, l.fphi_r, l.fphi_b,
                                                         l.phi_r, l.phi_b, l.fbeta_r, l.fbeta_b,
                                                         b.r_lo, b.r_lo + nc / 2, b.norms + 1,
                                                         b.norms + 4);
     } else {
         const Geo g = geo3(l.n / 2, l.n, l.n);
-        k_mx_correct<<<g.grid, g.block, 0, c.stream>>>(l.n, c_hi, c_lo, l.fphi_r, l.fphi_b,
+        launch_pdl(c, k_mx_correct, dim3(g.grid), dim3(g.block), l.n, c_hi, c_lo, l.fphi_r, l.fphi_b,
                                                        l.phi_r, l.phi_b, l.fbeta_r, l.fbeta_b,
                                                        b.r_lo, b.r_lo + nc / 2, b.norms + 1,
                                                        b.norms + 4);
@@ -1627,8 +1654,7 @@ nyxpm_status launch_mx_split_beta(Ctx& c, Box& b)
     const Level& l = b.levels[0];
     const long long half_cells = (long long)l.n * l.n * l.n / 2;
     prof_begin(c);
-    k_mx_split_beta<<<blocks_for(half_cells), kThreads, 0, c.stream>>>(
-        half_cells, l.beta_r, l.beta_b, l.fbeta_r, l.fbeta_b, b.r_lo, b.r_lo + half_cells);
+    launch_pdl(c, k_mx_split_beta, dim3(blocks_for(half_cells)), dim3(kThreads), half_cells, l.beta_r, l.beta_b, l.fbeta_r, l.fbeta_b, b.r_lo, b.r_lo + half_cells);
     prof_end(c, NYXPM_ST_NORM, 32.0 * half_cells);
     return check_launch(c, "mixed split beta");
 }
@@ -1639,11 +1665,11 @@ nyxpm_status launch_mx_update(Ctx& c, Box& b)
     const long long nc = (long long)l.n * l.n * l.n;
     prof_begin(c);
     if (l.split) {
-        k_mx_update<<<blocks_for(nc / 2), kThreads, 0, c.stream>>>(nc / 2, l.phi_r, l.fphi_r);
-        k_mx_update<<<blocks_for(nc / 2), kThreads, 0, c.stream>>>(nc / 2, l.phi_b, l.fphi_b);
+        launch_pdl(c, k_mx_update, dim3(blocks_for(nc / 2)), dim3(kThreads), nc / 2, l.phi_r, l.fphi_r);
+        launch_pdl(c, k_mx_update, dim3(blocks_for(nc / 2)), dim3(kThreads), nc / 2, l.phi_b, l.fphi_b);
         c.launches += 1;
     } else {
-        k_mx_update<<<blocks_for(nc), kThreads, 0, c.stream>>>(nc, l.phi_r, l.fphi_r);
+        launch_pdl(c, k_mx_update, dim3(blocks_for(nc)), dim3(kThreads), nc, l.phi_r, l.fphi_r);
     }
     prof_end(c, NYXPM_ST_PROLONG, 20.0 * nc);
     return check_launch(c, "mixed update");
@@ -1659,6 +1685,8 @@ __global__ void __launch_bounds__(256) k_mx_est_dt(long long np, int n, const in
                                                    const float* __restrict__ g,
                                                    unsigned long long* out_v, unsigned long long* out_g)
 {
+    pdl_wait();
+    pdl_trigger();
     unsigned long long gmax = 0;
     float vmax = 0.f;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < np;
@@ -1735,17 +1763,16 @@ nyxpm_status mixed_pack(Ctx& c, Box& b, double* d_pos, double* d_vel)
 nyxpm_status mixed_sort(Ctx& c, Box& b, bool defer_vel)
 {
     nyxpm_status st;
-    cudaMemsetAsync(b.cell_count, 0, sizeof(int) * (size_t)b.n * b.n * b.n, c.stream);
+    clear_counts(c, b);
     prof_begin(c);
-    k_mx_keys<<<blocks_for(b.np), kThreads, 0, c.stream>>>(b.np, b.n, b.cell, b.ox, b.oy, b.oz,
+    launch_pdl(c, k_mx_keys, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.n, b.cell, b.ox, b.oy, b.oz,
                                                             b.key, b.cell_count);
     prof_end(c, NYXPM_ST_KEYS, 20.0 * b.np);
     if ((st = check_launch(c, "mixed keys")) != NYXPM_OK) return st;
     if ((st = sort_from_keys(c, b)) != NYXPM_OK) return st;
     const bool pm = !b.uniform_mass;
     prof_begin(c);
-    k_mx_gather<<<blocks_for(b.np), kThreads, 0, c.stream>>>(
-        b.np, b.perm, b.cell, b.ox, b.oy, b.oz, defer_vel ? nullptr : b.fvx, b.fvy, b.fvz,
+    launch_pdl(c, k_mx_gather, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.perm, b.cell, b.ox, b.oy, b.oz, defer_vel ? nullptr : b.fvx, b.fvy, b.fvz,
         pm ? b.fm : nullptr, b.id, b.cell2, b.ox2, b.oy2, b.oz2, b.fvx2, b.fvy2, b.fvz2,
         pm ? b.fm2 : nullptr, b.id2);
     prof_end(c, NYXPM_ST_GATHER, ((pm ? 76.0 : 68.0) - (defer_vel ? 24.0 : 0.0)) * b.np);
@@ -1778,10 +1805,10 @@ nyxpm_status mixed_deposit(Ctx& c, Box& b)
     // in the room of 8 doubles per slot)
     float* heavy = reinterpret_cast<float*>(b.heavy_part);
     prof_begin(c);
-    k_mx_deposit_heavy<<<c.sm_count * 4, 256, 0, c.stream>>>(n, b.cell, b.ox, b.oy, b.oz, mq,
+    launch_pdl(c, k_mx_deposit_heavy, dim3(c.sm_count * 4), dim3(256), n, b.cell, b.ox, b.oy, b.oz, mq,
                                                              b.cell_start, b.long_list, b.long_count,
                                                              b.key_slot, heavy);
-    k_mx_deposit<<<grid, kDepThreads, 0, c.stream>>>(n, scale, b.cell, b.ox, b.oy, b.oz, mq,
+    launch_pdl(c, k_mx_deposit, dim3(grid), dim3(kDepThreads), n, scale, b.cell, b.ox, b.oy, b.oz, mq,
                                                      b.cell_start, b.key_slot, heavy, b.frho);
     c.launches += 1;
     prof_end(c, NYXPM_ST_DEPOSIT, (b.uniform_mass ? 16.0 : 20.0) * b.np + 8.0 * nc);
@@ -1804,13 +1831,13 @@ nyxpm_status mixed_make_rhs(Ctx& c, Box& b, double a)
     const double dx = b.L / n;
     const Geo g = geo3(n, n, n);
     prof_begin(c);
-    k_mx_rowsum<<<blocks_for((long long)n * n * 32), kThreads, 0, c.stream>>>(n, b.frho,
+    launch_pdl(c, k_mx_rowsum, dim3(blocks_for((long long)n * n * 32)), dim3(kThreads), n, b.frho,
                                                                              b.mass_offset, b.rows);
-    k_mx_mean<<<kMeanBlocks, 32, 0, c.stream>>>(n, dx, b.L, b.rows, b.scal + 4,
-                                                reinterpret_cast<unsigned*>(b.scal + 4 + kMeanBlocks), b.scal);
+    launch_pdl(c, k_mx_mean, dim3(kMeanBlocks), dim3(32), n, dx, b.L, b.rows, b.scal + 4,
+                                                reinterpret_cast<unsigned*>(b.scal + kScalTicket), b.scal, b.norms);
     const double scale = ((-4.0 * M_PI * c.p.gconst) * (1.0 / a)) * beta_scale(b);
-    k_mx_make_beta<<<g.grid, g.block, 0, c.stream>>>(n, l0.split, b.frho, b.mass_offset, b.scal,
-                                                     scale, l0.beta_r, l0.beta_b);
+    launch_pdl(c, k_mx_make_beta, dim3(g.grid), dim3(g.block), n, l0.split, b.frho, b.mass_offset, b.scal,
+                                                     scale, l0.beta_r, l0.beta_b, b.norms);
     prof_end(c, NYXPM_ST_RHS, 20.0 * nc);
     c.launches += 2;
     return check_launch(c, "mixed rhs");
@@ -1821,7 +1848,7 @@ nyxpm_status mixed_grav32(Ctx& c, Box& b)
     const long long nc = (long long)b.n * b.n * b.n;
     const Geo g = geo3(b.n, b.n, b.n);
     prof_begin(c);
-    k_mx_grav<<<g.grid, g.block, 0, c.stream>>>(view(b.levels[0]), (float)(0.5 * b.dxi), b.g32);
+    launch_pdl(c, k_mx_grav, dim3(g.grid), dim3(g.block), view(b.levels[0]), (float)(0.5 * b.dxi), b.g32);
     prof_end(c, NYXPM_ST_KICK, 20.0 * nc);
     return check_launch(c, "mixed grav");
 }
@@ -1844,18 +1871,8 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
     // inner right-hand side, and r_lo) and updates it from each correction
     // (k_mx_correct) instead of applying the FP64 stencil to phi.
     const bool incremental = l0.split != 0;
+    constexpr unsigned kMaxima = 1 << 1 | 1 << 4;   // 0 again once read (k_mx_mean before the first)
     post_open(c, b.post);
-    prof_begin(c);
-    cudaMemsetAsync(b.norms, 0, sizeof(unsigned long long), c.stream);
-    if (l0.split) {
-        k_mx_absmax<<<norm_blocks(c, nc / 2), kThreads, 0, c.stream>>>(nc / 2, l0.beta_r, b.norms);
-        k_mx_absmax<<<norm_blocks(c, nc / 2), kThreads, 0, c.stream>>>(nc / 2, l0.beta_b, b.norms);
-        c.launches += 1;
-    } else {
-        k_mx_absmax<<<norm_blocks(c, nc), kThreads, 0, c.stream>>>(nc, l0.beta_r, b.norms);
-    }
-    prof_end(c, NYXPM_ST_NORM, 8.0 * nc);
-    if ((st = check_launch(c, "mixed rhs norm")) != NYXPM_OK) return st;
     if (zero_guess && incremental) {
         // r0 = beta exactly: its two words, no stencil
         if ((st = launch_mx_split_beta(c, b)) != NYXPM_OK) return st;
@@ -1893,12 +1910,12 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
         nyxpm_status s;
         post_open(c, b.post);
         if ((s = launch_mx_resid(c, b, true)) != NYXPM_OK) return s;
-        post_words(c, b.post, b.norms, 1, 1);
+        post_words(c, b.post, b.norms, 1, 1, kMaxima);
         if ((s = check_launch(c, "norm read-back")) != NYXPM_OK) return s;
         return post_wait(c, b.post, "mixed sync");
     };
     if (in_cluster && (st = cluster_solve(0, -1.0)) != NYXPM_OK) return st;
-    post_words(c, b.post, b.norms, 0, 8);
+    post_words(c, b.post, b.norms, 0, 8, kMaxima);
     if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
     if ((st = post_wait(c, b.post, "mixed sync")) != NYXPM_OK) return st;
     const double bnorm = read_norm(b, 0);
@@ -1931,7 +1948,7 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
             }
             post_open(c, b.post);
             if ((st = cluster_solve(it, target)) != NYXPM_OK) return st;
-            post_words(c, b.post, b.norms, 0, 8);
+            post_words(c, b.post, b.norms, 0, 8, kMaxima);
             if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
             if ((st = post_wait(c, b.post, "mixed sync")) != NYXPM_OK) return st;
         }
@@ -1948,7 +1965,7 @@ nyxpm_status mixed_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info)
                 if ((s = launch_mx_update(c, b)) != NYXPM_OK) return s;
                 if ((s = launch_mx_resid(c, b, false)) != NYXPM_OK) return s;
             }
-            post_words(c, b.post, b.norms, 1, 4);
+            post_words(c, b.post, b.norms, 1, 4, kMaxima);
             return check_launch(c, "norm read-back");
         };
         for (it = 1; it <= c.p.max_vcycles; ++it) {
@@ -2004,7 +2021,7 @@ nyxpm_status mixed_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur, 
     A.drift = (float)(dt / a_cur * b.dxi);
     A.do_move = do_move;
     prof_begin(c);
-    k_mx_kick<<<blocks_for(b.np), kThreads, 0, c.stream>>>(b.np, A, b.cell, b.ox, b.oy, b.oz, b.fvx,
+    launch_pdl(c, k_mx_kick, dim3(blocks_for(b.np)), dim3(kThreads), b.np, A, b.cell, b.ox, b.oy, b.oz, b.fvx,
                                                             b.fvy, b.fvz);
     const double nc = (double)b.n * b.n * b.n;
     prof_end(c, NYXPM_ST_KICK, (do_move ? 56.0 : 40.0) * b.np + 12.0 * nc);
@@ -2014,10 +2031,9 @@ nyxpm_status mixed_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur, 
 
 nyxpm_status mixed_est_dt(Ctx& c, Box& b)
 {
-    cudaMemsetAsync(b.norms + 3, 0, sizeof(unsigned long long), c.stream);
-    cudaMemsetAsync(b.norms + 5, 0, sizeof(unsigned long long), c.stream);
+    cudaMemsetAsync(b.norms + 3, 0, 3 * sizeof(unsigned long long), c.stream);
     const unsigned blocks = std::min(blocks_for(b.np), (unsigned)(c.sm_count * 8));
-    k_mx_est_dt<<<blocks, kThreads, 0, c.stream>>>(b.np, b.n, b.cell, b.fvx, b.fvy, b.fvz, b.g32, b.norms + 3,
+    launch_pdl(c, k_mx_est_dt, dim3(blocks), dim3(kThreads), b.np, b.n, b.cell, b.fvx, b.fvy, b.fvz, b.g32, b.norms + 3,
                                                     b.norms + 5);
     c.launches += 1;
     return check_launch(c, "mixed time-step estimate");

@@ -46,6 +46,8 @@ __device__ __forceinline__ int wrap1(int i, int n) { return i < 0 ? i + n : (i >
 // one warp per row: 32 strided lane partials, then a halving tree
 __global__ void k_rowsum(int n, const double* __restrict__ rho, double mo, double* rows)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= (long long)n * n) return;
@@ -60,50 +62,72 @@ __global__ void k_rowsum(int n, const double* __restrict__ rho, double mo, doubl
     if (lane == 0) rows[row] = s;
 }
 
-__global__ void k_planesum(int n, const double* __restrict__ rows, double* planes)
+// The n row sums of each plane in order, one plane per lane, then by whichever block ends
+// last the n plane sums in order (ticket wraps to 0).  Two serial chains of n additions:
+// the rows are read a 32 x 32 tile at a time, so that only the additions are serial.
+// It also sets the norms that the solve collects by maximum to 0.
+// (64^3: two launches, the loads in the chains, 5.4 + 4.6 us and the gap; this 6.)
+__global__ void __launch_bounds__(32) k_mean(int n, double dx, double L, const double* __restrict__ rows,
+                                             double* planes, unsigned* ticket, double* scal, unsigned long long* norms)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+    __shared__ double tile[32][33];
+    pdl_wait();
+    pdl_trigger();
+    const int lane = threadIdx.x, k0 = blockIdx.x * 32;
+    if (blockIdx.x == 0 && lane < 2) norms[lane] = 0;
     double s = 0.0;
-    for (int j = 0; j < n; ++j) s = s + rows[(long long)k * n + j];
-    planes[k] = s;
+    for (int j0 = 0; j0 < n; j0 += 32) {
+        double v[32];
+#pragma unroll
+        for (int p = 0; p < 32; ++p)
+            v[p] = k0 + p < n && j0 + lane < n ? rows[(long long)(k0 + p) * n + j0 + lane] : 0.0;
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < 32; ++p) tile[p][lane] = v[p];
+        __syncwarp();
+        const int m = min(32, n - j0);
+        for (int j = 0; j < m; ++j) s = s + tile[lane][j];
+    }
+    if (k0 + lane < n) planes[k0 + lane] = s;
+    __threadfence();
+    __syncwarp();
+    unsigned last = 0;
+    if (lane == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    s = 0.0;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+        const double v = q0 + lane < n ? *(volatile double*)(planes + q0 + lane) : 0.0;
+        const int m = min(32, n - q0);
+        for (int q = 0; q < m; ++q) s = s + __shfl_sync(0xffffffffu, v, q);
+    }
+    if (lane == 0) scal[0] = (s * (dx * dx * dx)) / (L * L * L);
 }
 
-__global__ void k_mean(int n, double dx, double L, const double* __restrict__ planes, double* scal)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int k = 0; k < n; ++k) s = s + planes[k];
-    scal[0] = (s * (dx * dx * dx)) / (L * L * L);
-}
-
+// the right-hand side and its maximum norm
 __global__ void k_make_beta(int n, int split, const double* __restrict__ rho, double mo,
                             const double* __restrict__ scal, double ggrav, double ainv, double k0,
-                            double* beta_r, double* beta_b)
+                            double* beta_r, double* beta_b, unsigned long long* norm)
 {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
-    if (i >= n || j >= n) return;
-    const double mean = scal[0];
-    const double v = rho[cidx(i, j, k, n)];
-    *lv_ptr<double>(beta_r, beta_b, n, split, i, j, k) = ((((v - mo) - mean) * ggrav) * ainv) * k0;
+    unsigned long long u = 0;
+    if (i < n && j < n) {
+        const double mean = scal[0];
+        const double v = rho[cidx(i, j, k, n)];
+        const double beta = ((((v - mo) - mean) * ggrav) * ainv) * k0;
+        *lv_ptr<double>(beta_r, beta_b, n, split, i, j, k) = beta;
+        u = absbits(beta);
+    }
+    block_umax_store(u, norm);
 }
 
 // ---------------------------------------------------------------------------
 // norms (max is order independent; non-negative doubles compare as their bits)
 // ---------------------------------------------------------------------------
-__global__ void k_absmax(long long cnt, const double* __restrict__ a, unsigned long long* out)
-{
-    unsigned long long v = 0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cnt;
-         t += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long u = absbits(a[t]);
-        v = u > v ? u : v;
-    }
-    block_umax_store(v, out);
-}
-
 // neighbour sum in the oracle's order: x-, x+, y-, y+, z-, z+
 __device__ __forceinline__ double nbr_sum(const LevelView& L, int i, int j, int k)
 {
@@ -132,6 +156,8 @@ __device__ __forceinline__ double resid_at(const LevelView& L, int i, int j, int
 // ||r_beta||_inf of a split level: one thread per (ih, j, k), both cells of the pair
 __global__ void k_resnorm_split(LevelView L, unsigned long long* out)
 {
+    pdl_wait();
+    pdl_trigger();
     const int half = L.n >> 1;
     const int ih = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -176,6 +202,8 @@ __device__ __forceinline__ double2 pair_sums(int n, const double* __restrict__ o
 // k_resnorm_split by pairs of each colour
 __global__ void __launch_bounds__(256) k_resnorm_split2(LevelView L, unsigned long long* out)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = L.n;
     const unsigned t2 = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -200,6 +228,8 @@ __global__ void __launch_bounds__(256) k_resnorm_split2(LevelView L, unsigned lo
 __global__ void k_resnorm_red(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
                               const double* __restrict__ beta_r, unsigned long long* out)
 {
+    pdl_wait();
+    pdl_trigger();
     const int half = n >> 1;
     const int ih = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -286,6 +316,8 @@ __global__ void __launch_bounds__(256) k_resnorm_red_sweep2(int n, const double*
 
 __global__ void k_resnorm_nat(LevelView L, unsigned long long* out)
 {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
@@ -648,6 +680,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_d(ClArgs<double
 // component-major output
 __global__ void k_grav(LevelView L, double dxi, double* g)
 {
+    pdl_wait();
+    pdl_trigger();
     const int n = L.n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -836,24 +870,23 @@ nyxpm_status vcycle(Ctx& c, Box& b, size_t li, int red_done = 0)
     return NYXPM_OK;
 }
 
-// launch ||r_beta||_inf of level 0 into norms[slot]: all cells, or the red
+// launch ||r_beta||_inf of level 0 into norms[slot] (0 before): all cells, or the red
 // cells only after a cycle that ended with a black half sweep
 nyxpm_status launch_resnorm(Ctx& c, Box& b, int slot, int red_only)
 {
     const Level& l = b.levels[0];
     const long long nc = (long long)l.n * l.n * l.n;
     prof_begin(c);
-    cudaMemsetAsync(b.norms + slot, 0, sizeof(unsigned long long), c.stream);
     if (l.split && red_only) {
         const Geo g = geo3(l.n / 2, l.n, l.n);
-        k_resnorm_red<<<g.grid, g.block, 0, c.stream>>>(l.n, l.phi_r, l.phi_b, l.beta_r, b.norms + slot);
+        launch_pdl(c, k_resnorm_red, dim3(g.grid), dim3(g.block), l.n, l.phi_r, l.phi_b, l.beta_r, b.norms + slot);
     } else if (l.split) {
         const bool pairs = by_pairs(l);
         const Geo g = geo3(pairs ? l.n / 4 : l.n / 2, l.n, l.n);
-        (pairs ? k_resnorm_split2 : k_resnorm_split)<<<g.grid, g.block, 0, c.stream>>>(view(l), b.norms + slot);
+        launch_pdl(c, pairs ? k_resnorm_split2 : k_resnorm_split, dim3(g.grid), dim3(g.block), view(l), b.norms + slot);
     } else {
         const Geo g = geo3(l.n, l.n, l.n);
-        k_resnorm_nat<<<g.grid, g.block, 0, c.stream>>>(view(l), b.norms + slot);
+        launch_pdl(c, k_resnorm_nat, dim3(g.grid), dim3(g.block), view(l), b.norms + slot);
     }
     prof_end(c, NYXPM_ST_NORM, (red_only ? 12.0 : 16.0) * nc);
     return check_launch(c, "resnorm");
@@ -882,15 +915,15 @@ nyxpm_status launch_make_rhs(Ctx& c, Box& b, double a)
     const double dx = b.L / n;
     const Geo g = geo3(n, n, n);
     prof_begin(c);
-    k_rowsum<<<blocks_for((long long)n * n * 32), kThreads, 0, c.stream>>>(n, b.rho, b.mass_offset,
+    launch_pdl(c, k_rowsum, dim3(blocks_for((long long)n * n * 32)), dim3(kThreads), n, b.rho, b.mass_offset,
                                                                           b.rows);
-    k_planesum<<<blocks_for(n, 128), 128, 0, c.stream>>>(n, b.rows, b.planes);
-    k_mean<<<1, 32, 0, c.stream>>>(n, dx, b.L, b.planes, b.scal);
-    k_make_beta<<<g.grid, g.block, 0, c.stream>>>(n, l0.split, b.rho, b.mass_offset, b.scal,
+    launch_pdl(c, k_mean, dim3((n + 31) / 32), dim3(32), n, dx, b.L, b.rows, b.planes,
+               reinterpret_cast<unsigned*>(b.scal + kScalTicket), b.scal, b.norms);
+    launch_pdl(c, k_make_beta, dim3(g.grid), dim3(g.block), n, l0.split, b.rho, b.mass_offset, b.scal,
                                                   -4.0 * M_PI * c.p.gconst, 1.0 / a, beta_scale(b),
-                                                  l0.beta_r, l0.beta_b);
+                                                  l0.beta_r, l0.beta_b, b.norms);
     prof_end(c, NYXPM_ST_RHS, 24.0 * nc);
-    c.launches += 3;
+    c.launches += 2;
     return check_launch(c, "make rhs");
 }
 
@@ -907,24 +940,13 @@ nyxpm_status launch_zero_phi(Ctx& c, Box& b)
     return check_launch(c, "zero phi");
 }
 
-nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
+nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info, bool* grav_done)
 {
     nyxpm_status st;
     const Level& l0 = b.levels[0];
     const long long nc = (long long)l0.n * l0.n * l0.n;
     post_open(c, b.post);
-    // ||beta||_inf and ||r0||_inf
-    prof_begin(c);
-    cudaMemsetAsync(b.norms, 0, sizeof(unsigned long long), c.stream);
-    if (l0.split) {
-        k_absmax<<<norm_blocks(c, nc / 2), kThreads, 0, c.stream>>>(nc / 2, l0.beta_r, b.norms);
-        k_absmax<<<norm_blocks(c, nc / 2), kThreads, 0, c.stream>>>(nc / 2, l0.beta_b, b.norms);
-        c.launches += 1;
-    } else {
-        k_absmax<<<norm_blocks(c, nc), kThreads, 0, c.stream>>>(nc, l0.beta_r, b.norms);
-    }
-    prof_end(c, NYXPM_ST_NORM, 8.0 * nc);
-    if ((st = check_launch(c, "rhs norm")) != NYXPM_OK) return st;
+    // ||r0||_inf (launch_make_rhs left ||beta||_inf)
     if ((st = launch_resnorm(c, b, 1, 0)) != NYXPM_OK) return st;
     // a small box: the whole solve in one cluster launch
     ClArgs<double> ca;
@@ -936,7 +958,10 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
         prof_end(c, NYXPM_ST_SMOOTH, 0);
         if ((st = check_launch(c, "cluster solve")) != NYXPM_OK) return st;
     }
-    post_words(c, b.post, b.norms, 0, in_cluster ? 7 : 2);
+    post_words(c, b.post, b.norms, 0, in_cluster ? 7 : 2, 1 << 1);
+    // the gravity vector follows every solve that ends, converged or not
+    if (in_cluster && (st = launch_grav_vector(c, b)) != NYXPM_OK) return st;
+    *grav_done = in_cluster;
     if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
     if ((st = post_wait(c, b.post, "solve sync")) != NYXPM_OK) return st;
     const double bnorm = read_norm(b, 0);
@@ -972,7 +997,6 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
                 const bool pairs = by_pairs(L0);
                 const Geo g = geo3(pairs ? L0.n / 4 : L0.n / 2, L0.n, L0.n);
                 prof_begin(c);
-                cudaMemsetAsync(b.norms + 1, 0, sizeof(unsigned long long), c.stream);
                 launch_pdl(c, pairs ? k_resnorm_red_sweep2 : k_resnorm_red_sweep, dim3(g.grid), dim3(g.block), L0.n, L0.phi_r, L0.phi_b, L0.beta_r,
                                                                       b.phi_r_spare, b.norms + 1);
                 prof_end(c, NYXPM_ST_NORM, 16.0 * nc);
@@ -980,7 +1004,7 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info)
             } else if ((s = launch_resnorm(c, b, 1, red_only)) != NYXPM_OK) {
                 return s;
             }
-            post_words(c, b.post, b.norms, 1, 1);
+            post_words(c, b.post, b.norms, 1, 1, 1 << 1);
             return check_launch(c, "norm read-back");
         };
         for (it = 1; it <= c.p.max_vcycles; ++it) {
@@ -1023,7 +1047,7 @@ nyxpm_status launch_grav_vector(Ctx& c, Box& b)
     const long long nc = (long long)b.n * b.n * b.n;
     const Geo g = geo3(b.n, b.n, b.n);
     prof_begin(c);
-    k_grav<<<g.grid, g.block, 0, c.stream>>>(view(b.levels[0]), b.dxi, b.g);
+    launch_pdl(c, k_grav, dim3(g.grid), dim3(g.block), view(b.levels[0]), b.dxi, b.g);
     prof_end(c, NYXPM_ST_KICK, 32.0 * nc);
     return check_launch(c, "grav vector");
 }

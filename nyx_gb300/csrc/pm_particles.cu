@@ -159,6 +159,8 @@ __global__ void k_keys(long long np, int n, double dxi, const double* __restrict
                        const double* __restrict__ y, const double* __restrict__ z, int* key,
                        int* count)
 {
+    pdl_wait();
+    pdl_trigger();
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= np) return;
     double f;
@@ -174,6 +176,8 @@ __global__ void k_keys(long long np, int n, double dxi, const double* __restrict
 __global__ void k_scatter(long long np, const int* __restrict__ key, const int* __restrict__ start,
                           int* count, int* perm)
 {
+    pdl_wait();
+    pdl_trigger();
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= np) return;
     const int K = key[q];
@@ -187,6 +191,8 @@ __global__ void k_scatter(long long np, const int* __restrict__ key, const int* 
 __global__ void k_fix_short(int nc, const int* __restrict__ start, int* perm, int* long_list,
                             int* long_count)
 {
+    pdl_wait();
+    pdl_trigger();
     int K = blockIdx.x * blockDim.x + threadIdx.x;
     if (K >= nc) return;
     const int s = start[K], e = start[K + 1];
@@ -205,6 +211,8 @@ constexpr int kLongSmem = 12288;
 __global__ void k_fix_long(const int* __restrict__ start, const int* __restrict__ long_list,
                            const int* __restrict__ long_count, int* perm, int* tmp)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ int sv[kLongSmem];
     const int total = *long_count;
     for (int li = blockIdx.x; li < total; li += gridDim.x) {
@@ -237,6 +245,8 @@ __global__ void k_gather(long long np, const int* __restrict__ perm, const doubl
                          const int* __restrict__ id, double* x2, double* y2, double* z2,
                          double* vx2, double* vy2, double* vz2, double* m2, int* id2)
 {
+    pdl_wait();
+    pdl_trigger();
     long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= np) return;
     const int q = perm[s];
@@ -293,6 +303,8 @@ __device__ int block_excl_scan(int v, int* total)
 
 __global__ void k_scan_reduce(const int* __restrict__ in, int n, int* tile_sums)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     int s = 0;
 #pragma unroll
@@ -303,8 +315,11 @@ __global__ void k_scan_reduce(const int* __restrict__ in, int n, int* tile_sums)
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-__global__ void k_scan_top(int* tile_sums, int ntiles)
+__global__ void k_scan_top(int* tile_sums, int ntiles, int* long_count)
 {
+    pdl_wait();
+    pdl_trigger();
+    if (threadIdx.x == 0) *long_count = 0;   // k_fix_short counts into it
     int carry = 0;
     for (int b0 = 0; b0 < ntiles; b0 += blockDim.x) {
         const int i = b0 + threadIdx.x;
@@ -319,6 +334,8 @@ __global__ void k_scan_top(int* tile_sums, int ntiles)
 __global__ void k_scan_down(const int* __restrict__ in, int n, const int* __restrict__ tile_off,
                             int* out)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     int v[kScanItems];
     int s = 0;
@@ -393,6 +410,8 @@ __global__ void __launch_bounds__(256) k_deposit_heavy(int n, double dxi,
                                                        const int* __restrict__ long_count,
                                                        int* key_slot, double* heavy_part)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int total = *long_count;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -439,6 +458,8 @@ __global__ void __launch_bounds__(32 * kKeyWarps) k_deposit_keys(long long nc, i
                                                                  const double* __restrict__ heavy_part,
                                                                  double* __restrict__ part)
 {
+    pdl_wait();
+    pdl_trigger();
     __shared__ double wbuf[kKeyWarps][32][9];   // a batch's weights (and masses)
     __shared__ double acc[kKeyWarps][32][8];    // the warp's 32 keys' corner sums
     const unsigned full = 0xffffffffu;
@@ -534,6 +555,8 @@ __global__ void __launch_bounds__(256) k_deposit_cells(int n, double scale,
                                                        const double* __restrict__ part,
                                                        double* __restrict__ rho)
 {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
@@ -570,6 +593,8 @@ struct KickArgs {
 __global__ void __launch_bounds__(256) k_kick(long long np, KickArgs A, double* x, double* y,
                                               double* z, double* vx, double* vy, double* vz)
 {
+    pdl_wait();
+    pdl_trigger();
     long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= np) return;
     const int n = A.n;
@@ -650,6 +675,8 @@ __global__ void __launch_bounds__(256) k_est_dt(long long np, int n, double dxi,
                                                 const double* __restrict__ g,
                                                 unsigned long long* out_v, unsigned long long* out_g)
 {
+    pdl_wait();
+    pdl_trigger();
     const long long nc = (long long)n * n * n;
     unsigned long long vmax = 0, gmax = 0;
     for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < np;
@@ -700,14 +727,21 @@ nyxpm_status launch_wrap(Ctx& c, Box& b)
     return check_launch(c, "wrap");
 }
 
+// the scatter leaves the counts at zero, but a sort that failed half way may not have
+void clear_counts(Ctx& c, Box& b)
+{
+    if (b.counts_dirty) cudaMemsetAsync(b.cell_count, 0, sizeof(int) * (size_t)b.n * b.n * b.n, c.stream);
+    b.counts_dirty = 1;
+}
+
 nyxpm_status scan_counts(Ctx& c, Box& b)
 {
     const int nc = b.n * b.n * b.n;
     const int nt = b.ntiles;
     prof_begin(c);
-    k_scan_reduce<<<nt, kScanThreads, 0, c.stream>>>(b.cell_count, nc, b.tile_sums);
-    k_scan_top<<<1, 1024, 0, c.stream>>>(b.tile_sums, nt);
-    k_scan_down<<<nt, kScanThreads, 0, c.stream>>>(b.cell_count, nc, b.tile_sums, b.cell_start);
+    launch_pdl(c, k_scan_reduce, dim3(nt), dim3(kScanThreads), b.cell_count, nc, b.tile_sums);
+    launch_pdl(c, k_scan_top, dim3(1), dim3(1024), b.tile_sums, nt, b.long_count);
+    launch_pdl(c, k_scan_down, dim3(nt), dim3(kScanThreads), b.cell_count, nc, b.tile_sums, b.cell_start);
     prof_end(c, NYXPM_ST_SCAN, 12.0 * nc);
     c.launches += 2;
     return check_launch(c, "scan");
@@ -717,10 +751,9 @@ nyxpm_status fix_segments(Ctx& c, Box& b)
 {
     const int nc = b.n * b.n * b.n;
     prof_begin(c);
-    cudaMemsetAsync(b.long_count, 0, sizeof(int), c.stream);
-    k_fix_short<<<blocks_for(nc), kThreads, 0, c.stream>>>(nc, b.cell_start, b.perm, b.long_list,
+    launch_pdl(c, k_fix_short, dim3(blocks_for(nc)), dim3(kThreads), nc, b.cell_start, b.perm, b.long_list,
                                                             b.long_count);
-    k_fix_long<<<c.sm_count * 2, 512, 0, c.stream>>>(b.cell_start, b.long_list, b.long_count, b.perm,
+    launch_pdl(c, k_fix_long, dim3(c.sm_count * 2), dim3(512), b.cell_start, b.long_list, b.long_count, b.perm,
                                                       b.key);
     prof_end(c, NYXPM_ST_SCATTER, 4.0 * nc + 8.0 * b.np);
     c.launches += 1;
@@ -732,20 +765,20 @@ nyxpm_status sort_from_keys(Ctx& c, Box& b)
     nyxpm_status st;
     if ((st = scan_counts(c, b)) != NYXPM_OK) return st;
     prof_begin(c);
-    k_scatter<<<blocks_for(b.np), kThreads, 0, c.stream>>>(b.np, b.key, b.cell_start, b.cell_count,
+    launch_pdl(c, k_scatter, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.key, b.cell_start, b.cell_count,
                                                             b.perm);
     prof_end(c, NYXPM_ST_SCATTER, 12.0 * b.np);
     if ((st = check_launch(c, "scatter")) != NYXPM_OK) return st;
+    b.counts_dirty = 0;
     return fix_segments(c, b);
 }
 
 nyxpm_status launch_sort(Ctx& c, Box& b, bool defer_vel)
 {
     nyxpm_status st;
-    // the scatter leaves the counts at zero, but an interrupted sort may not have
-    cudaMemsetAsync(b.cell_count, 0, sizeof(int) * (size_t)b.n * b.n * b.n, c.stream);
+    clear_counts(c, b);
     prof_begin(c);
-    k_keys<<<blocks_for(b.np), kThreads, 0, c.stream>>>(b.np, b.n, b.dxi, b.x, b.y, b.z, b.key,
+    launch_pdl(c, k_keys, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.n, b.dxi, b.x, b.y, b.z, b.key,
                                                          b.cell_count);
     prof_end(c, NYXPM_ST_KEYS, 32.0 * b.np);
     if ((st = check_launch(c, "keys")) != NYXPM_OK) return st;
@@ -754,8 +787,7 @@ nyxpm_status launch_sort(Ctx& c, Box& b, bool defer_vel)
     prof_begin(c);
     // defer_vel: the velocities are not on the device yet; launch_gather_vel
     // permutes them by the same perm once they are
-    k_gather<<<blocks_for(b.np), kThreads, 0, c.stream>>>(
-        b.np, b.perm, b.x, b.y, b.z, defer_vel ? nullptr : b.vx, b.vy, b.vz,
+    launch_pdl(c, k_gather, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.perm, b.x, b.y, b.z, defer_vel ? nullptr : b.vx, b.vy, b.vz,
         b.uniform_mass ? nullptr : b.m, b.id, b.x2, b.y2, b.z2, b.vx2, b.vy2, b.vz2,
         b.uniform_mass ? nullptr : b.m2, b.id2);
     prof_end(c, NYXPM_ST_GATHER, (16.0 * nvals + 12.0) * b.np);
@@ -829,16 +861,16 @@ nyxpm_status launch_deposit(Ctx& c, Box& b)
     const double nc = (double)n * n * n;
     const double* mq = b.uniform_mass ? nullptr : b.m;
     prof_begin(c);
-    k_deposit_heavy<<<c.sm_count * 4, 256, 0, c.stream>>>(n, b.dxi, b.x, b.y, b.z, mq, b.cell_start,
+    launch_pdl(c, k_deposit_heavy, dim3(c.sm_count * 4), dim3(256), n, b.dxi, b.x, b.y, b.z, mq, b.cell_start,
                                                           b.long_list, b.long_count, b.key_slot,
                                                           b.heavy_part);
     const long long ncl = (long long)n * n * n;
     const unsigned kb = (unsigned)((ncl + 32LL * kKeyWarps - 1) / (32LL * kKeyWarps));
-    k_deposit_keys<<<kb, 32 * kKeyWarps, 0, c.stream>>>(ncl, n, b.dxi, b.x, b.y, b.z, mq,
+    launch_pdl(c, k_deposit_keys, dim3(kb), dim3(32 * kKeyWarps), ncl, n, b.dxi, b.x, b.y, b.z, mq,
                                                          b.cell_start, b.key_slot, b.heavy_part,
                                                          b.key_part);
     const Geo g = geo3(n, n, n);
-    k_deposit_cells<<<g.grid, g.block, 0, c.stream>>>(n, scale, b.key_part, b.rho);
+    launch_pdl(c, k_deposit_cells, dim3(g.grid), dim3(g.block), n, scale, b.key_part, b.rho);
     c.launches += 2;
     prof_end(c, NYXPM_ST_DEPOSIT, (b.uniform_mass ? 24.0 : 32.0) * b.np + 12.0 * nc);
     return check_launch(c, "deposit");
@@ -859,7 +891,7 @@ nyxpm_status launch_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur,
     A.do_move = do_move;
     A.do_wrap = do_wrap;
     prof_begin(c);
-    k_kick<<<blocks_for(b.np), kThreads, 0, c.stream>>>(b.np, A, b.x, b.y, b.z, b.vx, b.vy, b.vz);
+    launch_pdl(c, k_kick, dim3(blocks_for(b.np)), dim3(kThreads), b.np, A, b.x, b.y, b.z, b.vx, b.vy, b.vz);
     const double nc = (double)b.n * b.n * b.n;
     prof_end(c, NYXPM_ST_KICK, (do_move ? 96.0 : 72.0) * b.np + 24.0 * nc);
     b.sorted = b.sorted && !do_move && !do_wrap;
@@ -868,10 +900,9 @@ nyxpm_status launch_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur,
 
 nyxpm_status launch_est_dt(Ctx& c, Box& b)
 {
-    cudaMemsetAsync(b.norms + 3, 0, sizeof(unsigned long long), c.stream);
-    cudaMemsetAsync(b.norms + 5, 0, sizeof(unsigned long long), c.stream);
+    cudaMemsetAsync(b.norms + 3, 0, 3 * sizeof(unsigned long long), c.stream);
     const unsigned blocks = std::min(blocks_for(b.np), (unsigned)(c.sm_count * 8));
-    k_est_dt<<<blocks, kThreads, 0, c.stream>>>(b.np, b.n, b.dxi, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.g, b.norms + 3,
+    launch_pdl(c, k_est_dt, dim3(blocks), dim3(kThreads), b.np, b.n, b.dxi, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.g, b.norms + 3,
                                                  b.norms + 5);
     c.launches += 1;
     return check_launch(c, "time-step estimate");
