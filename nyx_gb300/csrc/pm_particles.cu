@@ -8,6 +8,7 @@
 // (Source/Particle/DarkMatterParticleContainer.cpp:250-306) and of the CIC
 // weights (Source/Particle/NeutrinoParticles_K.H:15-45).  GB300 runs FP64 at a
 // small fraction of its FP32 rate, so every FP64 instruction saved counts.
+#include "pm_cic.cuh"
 #include "pm_common.cuh"
 
 #include <algorithm>
@@ -446,9 +447,13 @@ __global__ void __launch_bounds__(256) k_deposit_heavy(int n, double dxi,
 // summed in order, exactly as one thread would, while the expensive part (the
 // weights) is spread evenly over the lanes whatever the keys' occupancy.
 // Keys longer than a warp take their sums from k_deposit_heavy.
-constexpr int kKeyWarps = 8;
+// Measured at 256^3 with clumps: 1227 us with eight warps to a block; 1107 with the numbering read
+// off the sorted order where no key is long, the rounds limited to the batch's keys and a key's
+// first weight copied; 1063 with acc's rows 9 apart; 908 with two warps to a block (blocks over
+// clumps last longer and held the others' place) and registers for 20 of those.
+constexpr int kKeyWarps = 2;
 
-__global__ void __launch_bounds__(32 * kKeyWarps) k_deposit_keys(long long nc, int n, double dxi,
+__global__ void __launch_bounds__(32 * kKeyWarps, 40 / kKeyWarps) k_deposit_keys(long long nc, int n, double dxi,
                                                                  const double* __restrict__ x,
                                                                  const double* __restrict__ y,
                                                                  const double* __restrict__ z,
@@ -461,7 +466,7 @@ __global__ void __launch_bounds__(32 * kKeyWarps) k_deposit_keys(long long nc, i
     pdl_wait();
     pdl_trigger();
     __shared__ double wbuf[kKeyWarps][32][9];   // a batch's weights (and masses)
-    __shared__ double acc[kKeyWarps][32][8];    // the warp's 32 keys' corner sums
+    __shared__ double acc[kKeyWarps][32][9];    // the warp's 32 keys' corner sums (9: a lane per key hits other banks)
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const long long K0 = ((long long)blockIdx.x * kKeyWarps + wid) * 32;
@@ -474,15 +479,24 @@ __global__ void __launch_bounds__(32 * kKeyWarps) k_deposit_keys(long long nc, i
         cnt = start[K + 1] - b0;
     }
     const bool heavy = cnt > kDepositLanes;
-    const int ml = heavy ? 0 : cnt;
-    int incl = ml;
+    // the key's particles are numbers excl .. incl - 1; without a long key among the 32
+    // those are the sorted particles from p0 on, else a scan leaves the long keys out
+    const int p0 = __shfl_sync(full, b0, 0);
+    const bool dense = !__any_sync(full, heavy);
+    int excl = b0 - p0, incl = excl + cnt;
+    if (!valid) excl = incl = 0x7fffffff;
+    int total = __reduce_max_sync(full, valid ? incl : 0);
+    if (!dense) {
+        const int ml = heavy ? 0 : cnt;
+        incl = ml;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(full, incl, off);
-        if (lane >= off) incl += v;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(full, incl, off);
+            if (lane >= off) incl += v;
+        }
+        excl = incl - ml;
+        total = __shfl_sync(full, incl, 31);
     }
-    const int excl = incl - ml;
-    const int total = __shfl_sync(full, incl, 31);
     double* mine = acc[wid][lane];
     if (heavy) {
         const double* hp = heavy_part + 8LL * key_slot[K];
@@ -495,38 +509,34 @@ __global__ void __launch_bounds__(32 * kKeyWarps) k_deposit_keys(long long nc, i
     __syncwarp();
     const int corner = lane & 7;
     for (int base = 0; base < total; base += 32) {
-        // the lane owning particle number q: the first lane whose inclusive count exceeds q
         const int q = base + lane;
-        int o = 0;
+        int p = p0 + q;
+        if (!dense) {
+            // the lane owning particle number q: the first lane whose inclusive count exceeds q
+            int o = 0;
 #pragma unroll
-        for (int bit = 16; bit >= 1; bit >>= 1) {
-            const int v = __shfl_sync(full, incl, o + bit - 1);
-            if (v <= q) o += bit;
+            for (int bit = 16; bit >= 1; bit >>= 1) {
+                const int v = __shfl_sync(full, incl, o + bit - 1);
+                if (v <= q) o += bit;
+            }
+            const int ob0 = __shfl_sync(full, b0, o & 31);
+            const int oex = __shfl_sync(full, excl, o & 31);
+            p = ob0 + (q - oex);
         }
-        const int ob0 = __shfl_sync(full, b0, o & 31);
-        const int oex = __shfl_sync(full, excl, o & 31);
         if (q < total) {
-            const int p = ob0 + (q - oex);
-            double fx, fy, fz;
-            key1(x[p], dxi, n, &fx);
-            key1(y[p], dxi, n, &fy);
-            key1(z[p], dxi, n, &fz);
-            const double sx[2] = {1.0 - fx, fx};
-            const double sy[2] = {1.0 - fy, fy};
-            const double sz[2] = {1.0 - fz, fz};
-            double* w = wbuf[wid][lane];
+            int cell[3];
+            double w[8];
+            cic_weights(fma(x[p], dxi, 0.5), fma(y[p], dxi, 0.5), fma(z[p], dxi, 0.5), cell, w);
 #pragma unroll
-            for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-                for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-                    for (int cx = 0; cx < 2; ++cx) w[cx + 2 * cy + 4 * cz] = (sx[cx] * sy[cy]) * sz[cz];
-            if (m) w[8] = m[p];
+            for (int c = 0; c < 8; ++c) wbuf[wid][lane][c] = w[c];
+            if (m) wbuf[wid][lane][8] = m[p];
         }
         __syncwarp();
-        // eight rounds of four keys x eight corners
+        // rounds of four keys x eight corners, over the keys that have particles in the batch
+        const unsigned in = __ballot_sync(full, incl > excl && incl > base && excl < base + 32);
+        const int r1 = (31 - __clz((int)in)) >> 2;
 #pragma unroll 1
-        for (int r = 0; r < 8; ++r) {
+        for (int r = (__ffs((int)in) - 1) >> 2; r <= r1; ++r) {
             const int ow = 4 * r + (lane >> 3);
             const int oi = __shfl_sync(full, incl, ow);
             const int oe = __shfl_sync(full, excl, ow);
@@ -536,7 +546,10 @@ __global__ void __launch_bounds__(32 * kKeyWarps) k_deposit_keys(long long nc, i
                 if (m) {
                     for (int t = lo; t < hi; ++t) a = fma(wbuf[wid][t][corner], wbuf[wid][t][8], a);
                 } else {
-                    for (int t = lo; t < hi; ++t) a = a + wbuf[wid][t][corner];
+                    // a key's first weight is its sum: 0 + w = w
+                    int t = lo;
+                    if (base + lo == oe) a = wbuf[wid][t++][corner];
+                    for (; t < hi; ++t) a = a + wbuf[wid][t][corner];
                 }
                 acc[wid][ow][corner] = a;
             }
@@ -599,16 +612,10 @@ __global__ void __launch_bounds__(256) k_kick(long long np, KickArgs A, double* 
     if (q >= np) return;
     const int n = A.n;
     const long long nc = (long long)n * n * n;
-    const double lx = fma(x[q], A.dxi, 0.5);
-    const double ly = fma(y[q], A.dxi, 0.5);
-    const double lz = fma(z[q], A.dxi, 0.5);
-    int i, j, k;
-    const double fi = floor_int(lx, &i), fj = floor_int(ly, &j), fk = floor_int(lz, &k);
-    const double xint = lx - fi, yint = ly - fj, zint = lz - fk;
-    const double sx[2] = {1.0 - xint, xint};
-    const double sy[2] = {1.0 - yint, yint};
-    const double sz[2] = {1.0 - zint, zint};
-    double w[8];
+    int at[3];
+    double w[8];   // the corner t is (i - ii, j - jj, k - kk), t = ii + 2 jj + 4 kk: its weight w[7 - t]
+    cic_weights(fma(x[q], A.dxi, 0.5), fma(y[q], A.dxi, 0.5), fma(z[q], A.dxi, 0.5), at, w);
+    const int i = at[0], j = at[1], k = at[2];
     long long cell[8];
 #pragma unroll
     for (int kk = 0; kk <= 1; ++kk)
@@ -617,7 +624,6 @@ __global__ void __launch_bounds__(256) k_kick(long long np, KickArgs A, double* 
 #pragma unroll
             for (int ii = 0; ii <= 1; ++ii) {
                 const int t = ii + 2 * jj + 4 * kk;
-                w[t] = (sx[1 - ii] * sy[1 - jj]) * sz[1 - kk];
                 cell[t] = cidx(wrapi(i - ii, n), wrapi(j - jj, n), wrapi(k - kk, n), n);
             }
     double v[3] = {vx[q], vy[q], vz[q]};
@@ -626,9 +632,9 @@ __global__ void __launch_bounds__(256) k_kick(long long np, KickArgs A, double* 
         const double* gd = A.g + d * nc;
         double val = 0.0;
 #pragma unroll
-        for (int t = 0; t < 8; ++t) val = fma(w[t], __ldg(gd + cell[t]), val);
-        const double u = fma(A.a_prev, v[d], A.half_dt * val);
-        v[d] = u * A.a_cur_inv;
+        for (int t = 0; t < 8; ++t) val = fma(w[7 - t], __ldg(gd + cell[t]), val);
+        const double u = fma(A.a_prev, v[d], mul_on_int(A.half_dt, val));
+        v[d] = mul_on_int(u, A.a_cur_inv);
     }
     vx[q] = v[0];
     vy[q] = v[1];
