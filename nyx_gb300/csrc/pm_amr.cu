@@ -35,6 +35,7 @@
 // over the prefix finds the box); the other kernels walk flat lists, one thread
 // per cell, ghost cell, record or particle.
 // Built with --fmad=false: only the explicit fma() calls fuse.
+#include "pm_cic.cuh"
 #include "pm_common.cuh"
 #include "pm_sum6.cuh"
 
@@ -185,9 +186,13 @@ __global__ void k_amr_assign(BoxTab T, long long np, const double* __restrict__ 
     for (int l = T.nlev - 1; l >= 1 && B < 0; --l) {
         const double dxi = T.dxi[l];
         const int n = T.n0 << l;
-        const int i = wrapi((int)floor(x[p] * dxi), n);
-        const int j = wrapi((int)floor(y[p] * dxi), n);
-        const int k = wrapi((int)floor(z[p] * dxi), n);
+        int i, j, k;
+        floor_int(x[p] * dxi, &i);
+        floor_int(y[p] * dxi, &j);
+        floor_int(z[p] * dxi, &k);
+        i = wrapi(i, n);
+        j = wrapi(j, n);
+        k = wrapi(k, n);
         for (int b = T.first[l]; b < T.first[l] + T.count[l]; ++b)
             if (box_has(T.box[b], i, j, k)) { L = l; B = b; break; }
     }
@@ -201,15 +206,20 @@ struct PutItem {
 };
 
 // the corner mass q of level l at cell (i,j,k): coarser while not valid, then
-// finer in eighths while covered
+// finer in eighths while covered (most cells are neither)
 __device__ void amr_put(const BoxTab& T, int l, int i, int j, int k, double q, double* mass)
 {
-    while (tab_vidx(T, l, i, j, k) < 0) {
+    long long c;
+    while ((c = tab_vidx(T, l, i, j, k)) < 0) {
         const int n = T.n0 << l;
         i = wrapi(i, n) >> 1;
         j = wrapi(j, n) >> 1;
         k = wrapi(k, n) >> 1;
         --l;
+    }
+    if (!tab_covered(T, l, i, j, k)) {
+        atomicAdd(mass + c, q);
+        return;
     }
     PutItem st[8 * (kMaxLevels - 1) + 1];
     int top = 0;
@@ -228,55 +238,82 @@ __device__ void amr_put(const BoxTab& T, int l, int i, int j, int k, double q, d
     }
 }
 
+// Bound by its atomic additions (2.4 million particles on base 128^3 and two levels:
+// 401 us with a search of the boxes for each corner and weights on the FP64 pipe, 303 us).
 __global__ void k_amr_deposit(BoxTab T, long long np, const double* __restrict__ x,
                               const double* __restrict__ y, const double* __restrict__ z,
                               const double* __restrict__ m, double mscalar, const int* __restrict__ lev,
-                              double* mass)
+                              const int* __restrict__ box, double* mass)
 {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
     const int l = lev[p];
     const double dxi = T.dxi[l];
-    const double lx = fma(x[p], dxi, 0.5), ly = fma(y[p], dxi, 0.5), lz = fma(z[p], dxi, 0.5);
-    const double fi = floor(lx), fj = floor(ly), fk = floor(lz);
-    const int i = (int)fi, j = (int)fj, k = (int)fk;
-    const double fx = lx - fi, fy = ly - fj, fz = lz - fk;
-    const double sx[2] = {1.0 - fx, fx}, sy[2] = {1.0 - fy, fy}, sz[2] = {1.0 - fz, fz};
+    int at[3];
+    double w[8];
+    cic_weights(fma(x[p], dxi, 0.5), fma(y[p], dxi, 0.5), fma(z[p], dxi, 0.5), at, w);
+    const int i = at[0], j = at[1], k = at[2];
     const double mp = m ? m[p] : mscalar;
-    for (int cz = 0; cz < 2; ++cz)
-        for (int cy = 0; cy < 2; ++cy)
-            for (int cx = 0; cx < 2; ++cx)
-                amr_put(T, l, i - 1 + cx, j - 1 + cy, k - 1 + cz, ((sx[cx] * sy[cy]) * sz[cz]) * mp, mass);
+    // eight valid, uncovered cells of one box or of the base grid: no search per corner
+    const int n = T.n0 << l;
+    long long c0 = -1;
+    int sx, sxy;
+    if (l == 0) {
+        if (i >= 1 && i < n && j >= 1 && j < n && k >= 1 && k < n) c0 = cidx(i - 1, j - 1, k - 1, n);
+        sx = n;
+        sxy = n * n;
+    } else {
+        const ABox& B = T.box[box[p]];
+        if (box_has(B, i - 1, j - 1, k - 1) && box_has(B, i, j, k)) c0 = box_idx(B, i - 1, j - 1, k - 1);
+        sx = B.d[0];
+        sxy = B.d[0] * B.d[1];
+    }
+    if (l + 1 < T.nlev)
+        for (int b = T.first[l + 1]; b < T.first[l + 1] + T.count[l + 1]; ++b) {
+            const ABox& B = T.box[b];
+            if (2 * i + 1 >= B.lo[0] && 2 * i - 2 <= B.hi[0] && 2 * j + 1 >= B.lo[1] && 2 * j - 2 <= B.hi[1] &&
+                2 * k + 1 >= B.lo[2] && 2 * k - 2 <= B.hi[2])
+                c0 = -1;
+        }
+    if (c0 >= 0) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            atomicAdd(mass + c0 + (c & 1) + (long long)((c >> 1) & 1) * sx + (long long)(c >> 2) * sxy, w[c] * mp);
+        return;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) w[c] = w[c] * mp;
+#pragma unroll 1
+    for (int c = 0; c < 8; ++c)
+        amr_put(T, l, i - 1 + (c & 1), j - 1 + ((c >> 1) & 1), k - 1 + (c >> 2), w[c], mass);
 }
 
 // update_dm_particle_single (DarkMatterParticleContainer.cpp:250-306) with the
-// particle's own level's g; err counts stencils outside the box's ghost rings
+// particle's own level's g; err counts stencils outside the box's ghost rings.  Bound by
+// the FP64 pipe: 318 us with the weights and a division by a_cur on it, 191 us.
 __global__ void k_amr_move(BoxTab T, long long np, double* x, double* y, double* z, double* vx, double* vy,
                            double* vz, const int* __restrict__ lev, const int* __restrict__ box,
                            const double* __restrict__ g0, const double* __restrict__ g1,
-                           const double* __restrict__ g2, double dt, double a_prev, double a_cur,
-                           int do_move, unsigned long long* err)
+                           const double* __restrict__ g2, double half_dt, double a_prev, double a_cur_inv,
+                           double dt_a_cur_inv, int do_move, unsigned long long* err)
 {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
-    const double half_dt = 0.5 * dt;
-    const double a_cur_inv = 1.0 / a_cur;
-    const double dt_a_cur_inv = dt * a_cur_inv;
     const int l = lev[p];
     const double dxi = T.dxi[l];
-    const double lx = fma(x[p], dxi, 0.5), ly = fma(y[p], dxi, 0.5), lz = fma(z[p], dxi, 0.5);
-    const double fi = floor(lx), fj = floor(ly), fk = floor(lz);
-    const int i = (int)fi, j = (int)fj, k = (int)fk;
-    const double xint = lx - fi, yint = ly - fj, zint = lz - fk;
-    const double sx[2] = {1.0 - xint, xint}, sy[2] = {1.0 - yint, yint}, sz[2] = {1.0 - zint, zint};
-    double w[8];
+    int at[3];
+    double w[8];   // the corner t is (i - ii, j - jj, k - kk), t = ii + 2 jj + 4 kk: its weight w[7 - t]
+    cic_weights(fma(x[p], dxi, 0.5), fma(y[p], dxi, 0.5), fma(z[p], dxi, 0.5), at, w);
+    const int i = at[0], j = at[1], k = at[2];
     long long cells[8];
     bool ok = true;
+#pragma unroll
     for (int kk = 0; kk <= 1; ++kk)
+#pragma unroll
         for (int jj = 0; jj <= 1; ++jj)
+#pragma unroll
             for (int ii = 0; ii <= 1; ++ii) {
                 const int t = ii + 2 * jj + 4 * kk;
-                w[t] = (sx[1 - ii] * sy[1 - jj]) * sz[1 - kk];
                 if (l == 0) {
                     const int n = T.n0;
                     cells[t] = cidx(wrapi(i - ii, n), wrapi(j - jj, n), wrapi(k - kk, n), n);
@@ -294,17 +331,21 @@ __global__ void k_amr_move(BoxTab T, long long np, double* x, double* y, double*
             }
     if (!ok) atomicAdd(err, 1ULL);
     const double* g[3] = {g0, g1, g2};
-    double* v[3] = {vx + p, vy + p, vz + p};
+    double v[3] = {vx[p], vy[p], vz[p]};
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
         double val = 0.0;
-        for (int t = 0; t < 8; ++t) val = fma(w[t], g[d][cells[t]], val);
-        const double u = fma(a_prev, *v[d], half_dt * val);
-        *v[d] = u * a_cur_inv;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) val = fma(w[7 - t], __ldg(g[d] + cells[t]), val);
+        v[d] = mul_on_int(fma(a_prev, v[d], mul_on_int(half_dt, val)), a_cur_inv);
     }
+    vx[p] = v[0];
+    vy[p] = v[1];
+    vz[p] = v[2];
     if (do_move == 1) {
-        x[p] = fma(dt_a_cur_inv, vx[p], x[p]);
-        y[p] = fma(dt_a_cur_inv, vy[p], y[p]);
-        z[p] = fma(dt_a_cur_inv, vz[p], z[p]);
+        x[p] = fma(dt_a_cur_inv, v[0], x[p]);
+        y[p] = fma(dt_a_cur_inv, v[1], y[p]);
+        z[p] = fma(dt_a_cur_inv, v[2], z[p]);
     }
 }
 
@@ -313,13 +354,8 @@ __global__ void k_amr_wrap(long long np, double L, double* x, double* y, double*
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= np) return;
     double* c[3] = {x, y, z};
-    for (int d = 0; d < 3; ++d) {
-        double v = c[d][p];
-        if (v >= L) v = v - L;
-        else if (v < 0.0) v = v + L;
-        if (v >= L) v = 0.0;
-        c[d][p] = v;
-    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) c[d][p] = wrap_pos(c[d][p], L);
 }
 
 // counts the values that are not finite (one pass over the uploaded particles, bound by
@@ -1162,7 +1198,7 @@ nyxpm_status deposit(Ctx& c, nyxpm_amr& A)
     cudaMemsetAsync(A.mass, 0, sizeof(double) * A.ntot, c.stream);
     prof_begin(c);
     k_amr_deposit<<<nblk(A.np), kT, 0, c.stream>>>(A.tab, A.np, A.x, A.y, A.z, A.uniform_mass ? nullptr : A.m,
-                                                   A.mscalar, A.lev, A.mass);
+                                                   A.mscalar, A.lev, A.box, A.mass);
     prof_end(c, NYXPM_ST_DEPOSIT, 36.0 * A.np);
     const double h0 = A.L / A.n0;
     prof_begin(c);
@@ -1421,9 +1457,11 @@ nyxpm_status grav(Ctx& c, nyxpm_amr& A)
 
 nyxpm_status move(Ctx& c, nyxpm_amr& A, double dt, double a_prev, double a_cur, int do_move)
 {
+    const double a_cur_inv = 1.0 / a_cur;
     prof_begin(c);
     k_amr_move<<<nblk(A.np), kT, 0, c.stream>>>(A.tab, A.np, A.x, A.y, A.z, A.vx, A.vy, A.vz, A.lev, A.box, A.g[0],
-                                                A.g[1], A.g[2], dt, a_prev, a_cur, do_move, A.norms + 2);
+                                                A.g[1], A.g[2], 0.5 * dt, a_prev, a_cur_inv, dt * a_cur_inv, do_move,
+                                                A.norms + 2);
     prof_end(c, NYXPM_ST_KICK, 120.0 * A.np);
     return check_launch(c, "multilevel kick");
 }
