@@ -259,7 +259,8 @@ __device__ __forceinline__ void cl_half_sweep(const ClLevel<T>& L, int color, bo
 }
 
 // the red children's residuals of the coarse planes K with fine plane 2K in this slab,
-// into the coarse right-hand side (in the slabs of C, or in CTA 0's level at solo)
+// into the coarse right-hand side (in the slabs of C, with the opening red half sweep of
+// the coarse level, or in CTA 0's level at solo)
 template <typename T>
 __device__ __forceinline__ void cl_restrict(const ClLevel<T>& F, const ClLevel<T>* C, T* solo)
 {
@@ -283,8 +284,10 @@ __device__ __forceinline__ void cl_restrict(const ClLevel<T>& F, const ClLevel<T
         const unsigned o = (unsigned)(I >> 1) + (unsigned)chalf * J;
         if (C) {
             const int c = cl_owner(K, nc);
-            T* b = (black ? C->beta_b : C->beta_r) + (unsigned)(K - cl_first(c, nc)) * (nc * chalf) + o;
-            *cl_map(b, c) = s * T(0.5);
+            const unsigned at = (unsigned)(K - cl_first(c, nc)) * (nc * chalf) + o;
+            const T b = s * T(0.5);
+            *cl_map((black ? C->beta_b : C->beta_r) + at, c) = b;
+            if (!black) *cl_map(C->phi_r + at, c) = tail_fma(T(0), tail_sixth<T>(), -b);
         } else {
             *cl_map(solo + (2 + black) * (nc * nc * chalf) + K * (nc * chalf) + o, 0) = s * T(0.5);
         }
@@ -334,8 +337,10 @@ __device__ __forceinline__ void cl_restrict2(const ClLevel<float>& F, const ClLe
             be = solo + (2 + even_black) * nc * plane + K * plane + o;
             bo = solo + (3 - even_black) * nc * plane + K * plane + o;
         }
-        *cl_map(be, c) = s0 * 0.5f;
-        *cl_map(bo, c) = s1 * 0.5f;
+        const float b0 = s0 * 0.5f, b1 = s1 * 0.5f;
+        *cl_map(be, c) = b0;
+        *cl_map(bo, c) = b1;
+        if (C) *cl_map(C->phi_r + (K - cl_first(c, nc)) * plane + o, c) = fmaf(0.f, sixth, -(even_black ? b1 : b0));
     }
 }
 
@@ -458,17 +463,29 @@ __device__ __forceinline__ void cl_prolong_any(const ClLevel<T>& F, const T* sta
     cl_prolong<T>(F, stage, cap);
 }
 
-// One V-cycle on the slab levels, ending after a cluster barrier.  zero: the finest
-// correction is 0 on entry.
+// The opening red half sweep of a level whose correction is 0, in place of one with its
+// barrier: each thread takes the cells it has just copied (cl_copy's order).
 template <typename T>
-__device__ __forceinline__ void cl_vcycle(const ClArgs<T>& A, ClShared<T>& S, T* mem, bool zero)
+__device__ __forceinline__ void cl_open(const ClLevel<T>& L)
+{
+    const int cnt = L.n * (L.n >> 1) * L.np;
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) L.phi_r[t] = tail_fma(T(0), tail_sixth<T>(), -L.beta_r[t]);
+}
+
+// One V-cycle on the slab levels, ending after a cluster barrier.  start: the finest
+// level's correction is in place (0), is 0 throughout (1), or has had its opening red half
+// sweep from 0 (2), as the coarser ones have from the restriction (ten FP64 steps at 64^3
+// 18.65 -> 18.5 ms).
+template <typename T>
+__device__ __forceinline__ void cl_vcycle(const ClArgs<T>& A, ClShared<T>& S, T* mem, int start)
 {
     const int rank = cl_rank();
     for (int l = 0; l < A.nd; ++l) {
-        const bool fresh = l > 0 || zero;
         for (int sw = 0; sw < A.nu1; ++sw) {
-            cl_half_sweep<T>(S.lv[l], 0, fresh && sw == 0);
-            cl_barrier();
+            if (sw > 0 || (l == 0 && start < 2)) {
+                cl_half_sweep<T>(S.lv[l], 0, sw == 0 && start == 1);
+                cl_barrier();
+            }
             cl_half_sweep<T>(S.lv[l], 1, false);
             cl_barrier();
         }

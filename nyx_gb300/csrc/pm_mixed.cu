@@ -897,10 +897,20 @@ __device__ __forceinline__ float resid_f(const LevelViewF& L, int i, int j, int 
     return *lv_ptr<float>(L.beta_r, L.beta_b, n, L.split, i, j, k) - fmaf(s, kSixthF, -c);
 }
 
+// A coarse cell's right-hand side and the phi it starts from: 0, or with open (the coarse
+// level is smoothed from 0 by launches) its opening red half sweep, whose black neighbours
+// are 0; the black half sweep after it overwrites the black cells unread.
+__device__ __forceinline__ void restrict_store_f(const LevelViewF& Cv, int I, int J, int K, float beta, int open)
+{
+    *lv_ptr<float>(Cv.beta_r, Cv.beta_b, Cv.n, Cv.split, I, J, K) = beta;
+    if (open && ((I + J + K) & 1)) return;
+    *lv_ptr<float>(Cv.phi_r, Cv.phi_b, Cv.n, Cv.split, I, J, K) = open ? fmaf(0.f, kSixthF, -beta) : 0.f;
+}
+
 // RED = 1 after pre-smoothing (it ends with a black half sweep): the red
 // children only, as k_restrict_f4_red and the fused coarse V-cycle take them
 template <int RED>
-__global__ void k_restrict_f(LevelViewF F, LevelViewF Cv)
+__global__ void k_restrict_f(LevelViewF F, LevelViewF Cv, int open)
 {
     pdl_wait();
     pdl_trigger();
@@ -917,8 +927,7 @@ __global__ void k_restrict_f(LevelViewF F, LevelViewF Cv)
 #pragma unroll
             for (int di = 0; di < 2; ++di)
                 if (!RED || ((di + dj + dk) & 1) == 0) s += resid_f(F, 2 * I + di, 2 * J + dj, 2 * K + dk);
-    *lv_ptr<float>(Cv.beta_r, Cv.beta_b, nc, Cv.split, I, J, K) = s * 0.5f;
-    *lv_ptr<float>(Cv.phi_r, Cv.phi_b, nc, Cv.split, I, J, K) = 0.f;
+    restrict_store_f(Cv, I, J, K, s * 0.5f, open);
 }
 
 // The residual + restriction for a split fine level with half % 4 == 0: two
@@ -979,7 +988,7 @@ __device__ __forceinline__ void fine_row_resid(const LevelViewF& F, int j, int k
 // The restriction after pre-smoothing: the coarse right-hand side from the red
 // children only (the black ones' residuals are round-off), summed in (dk, dj)
 // order; half the loads of k_restrict_f4.
-__global__ void __launch_bounds__(256) k_restrict_f4_red(LevelViewF F, LevelViewF Cv)
+__global__ void __launch_bounds__(256) k_restrict_f4_red(LevelViewF F, LevelViewF Cv, int open)
 {
     pdl_wait();
     pdl_trigger();
@@ -1000,9 +1009,7 @@ __global__ void __launch_bounds__(256) k_restrict_f4_red(LevelViewF F, LevelView
         for (int dk = 0; dk < 2; ++dk)
 #pragma unroll
             for (int dj = 0; dj < 2; ++dj) s += r[dk][dj][u];
-        const int I = 2 * (int)t + u;
-        *lv_ptr<float>(Cv.beta_r, Cv.beta_b, nc, Cv.split, I, J, K) = s * 0.5f;
-        *lv_ptr<float>(Cv.phi_r, Cv.phi_b, nc, Cv.split, I, J, K) = 0.f;
+        restrict_store_f(Cv, 2 * (int)t + u, J, K, s * 0.5f, open);
     }
 }
 
@@ -1218,8 +1225,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_f(ClArgs<float
     pdl_trigger();
     cl_load_green(A, S);
     cl_load(S.lv[0], L, false);
+    cl_open(S.lv[0]);
     cl_barrier();
-    cl_vcycle(A, S, cl_mem_f, true);
+    cl_vcycle(A, S, cl_mem_f, 2);
     cl_store(S.lv[0], L);
 }
 
@@ -1260,7 +1268,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_f(ClArgs<float>
         cl_copy(F.beta_b, P.r_b + o, total);
         cl_barrier();
         for (it = P.first + 1;; ++it) {
-            for (int v = 0; v < P.inner; ++v) cl_vcycle(A, S, cl_mem_f, v == 0);
+            for (int v = 0; v < P.inner; ++v) cl_vcycle(A, S, cl_mem_f, v == 0 ? 1 : 0);
             float vmax = 0.f, emax = 0.f;
             for (int t = threadIdx.x; t < total; t += blockDim.x) {
                 int ih, j, q;
@@ -1440,7 +1448,7 @@ double read_norm(Box& b, int slot)
 
 // zero_start: the level's correction is 0 on entry (an inner solve's first sweep
 // on level 0): the red half sweep is k_gsrb_f_zero
-nyxpm_status gsrb_sweep_f(Ctx& c, const Level& l, int fine, bool zero_start = false)
+nyxpm_status gsrb_sweep_f(Ctx& c, const Level& l, int fine, bool zero_start = false, int black_only = 0)
 {
     const long long half_cells = (long long)l.n * l.n * l.n / 2;
     const int half = l.n / 2;
@@ -1454,7 +1462,7 @@ nyxpm_status gsrb_sweep_f(Ctx& c, const Level& l, int fine, bool zero_start = fa
     } else {
         g = geo3(half, l.n, l.n);
     }
-    for (int color = 0; color < 2; ++color) {
+    for (int color = black_only ? 1 : 0; color < 2; ++color) {
         float* mine = color ? l.fphi_b : l.fphi_r;
         const float* other = color ? l.fphi_r : l.fphi_b;
         const float* beta = color ? l.fbeta_b : l.fbeta_r;
@@ -1511,9 +1519,10 @@ bool tail_fits(const Ctx& c, const Box& b, size_t li)
            b.levels.size() - li <= (size_t)kMaxTail;
 }
 
+// red_done: the restriction made the opening red half sweep.
 // fresh: level li's correction is 0 on entry without having been zeroed (the
 // first inner V-cycle of a defect-correction step)
-nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false)
+nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false, int red_done = 0)
 {
     nyxpm_status st;
     const Level& f = b.levels[li];
@@ -1549,20 +1558,22 @@ nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false)
         cudaMemsetAsync(f.fphi_b, 0, half_bytes, c.stream);
     }
     for (int s = 0; s < c.p.nu1; ++s)
-        if ((st = gsrb_sweep_f(c, f, li == 0, fresh && s == 0)) != NYXPM_OK) return st;
+        if ((st = gsrb_sweep_f(c, f, li == 0, fresh && s == 0, s == 0 && red_done)) != NYXPM_OK) return st;
     const Level& cl = b.levels[li + 1];
     const long long ncc = (long long)cl.n * cl.n * cl.n;
     const long long ncf = (long long)f.n * f.n * f.n;
+    // a coarse level that launches smooth (not the cluster, the tail or the bottom)
+    const int open = c.p.nu1 > 0 && li + 2 < b.levels.size() && !tail_fits(c, b, li + 1) && !cluster_fits_f(c, b, li + 1, ca);
     {
         prof_begin(c);
         if ((f.n / 2) % 4 == 0) {
             const Geo g = geo3(cl.n / 2, cl.n, cl.n);
-            if (c.p.nu1 > 0) launch_pdl(c, k_restrict_f4_red, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl));
+            if (c.p.nu1 > 0) launch_pdl(c, k_restrict_f4_red, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl), open);
             else launch_pdl(c, k_restrict_f4, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl));
         } else {
             const Geo g = geo3(cl.n, cl.n, cl.n);
-            if (c.p.nu1 > 0) launch_pdl(c, k_restrict_f<1>, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl));
-            else launch_pdl(c, k_restrict_f<0>, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl));
+            if (c.p.nu1 > 0) launch_pdl(c, k_restrict_f<1>, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl), open);
+            else launch_pdl(c, k_restrict_f<0>, dim3(g.grid), dim3(g.block), viewf(f), viewf(cl), open);
         }
         // phi and beta read once, coarse beta and phi written; the red-only form reads
         // the black cells' beta not at all
@@ -1570,7 +1581,7 @@ nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false)
         prof_end(c, NYXPM_ST_RESTRICT, (red ? 6.0 : 8.0) * ncf + 8.0 * ncc);
     }
     if ((st = check_launch(c, "restrict f32")) != NYXPM_OK) return st;
-    if ((st = vcycle_f(c, b, li + 1)) != NYXPM_OK) return st;
+    if ((st = vcycle_f(c, b, li + 1, false, open)) != NYXPM_OK) return st;
     {
         prof_begin(c);
         const bool black = c.p.nu2 > 0;
