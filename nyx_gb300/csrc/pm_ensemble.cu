@@ -1099,18 +1099,18 @@ __global__ void __launch_bounds__(256) e_correct_v(const Item* __restrict__ item
                 const float2 zp = *reinterpret_cast<const float2*>(other + rzp + ih);
                 float2* rh_p = reinterpret_cast<float2*>((color ? rh_b : rh_r) + t);
                 float2* rl_p = reinterpret_cast<float2*>(rl + (color ? nh : 0u) + t);
-                float2 rh = *rh_p, rlo = *rl_p;
+                float2 rh = *rh_p, rlo = __ldcs(rl_p);
                 const float v0[6] = {xm0, xp0, ym.x, yp.x, zm.x, zp.x};
                 const float v1[6] = {xm1, xp1, ym.y, yp.y, zm.y, zp.y};
                 df_residual_update(v0, em.x, c_hi, c_lo, rh.x, rlo.x);
                 df_residual_update(v1, em.y, c_hi, c_lo, rh.y, rlo.y);
                 *rh_p = rh;
-                *rl_p = rlo;
+                __stcs(rl_p, rlo);
                 double2* pp = reinterpret_cast<double2*>((color ? p_b : p_r) + t);
-                double2 ph = *pp;
+                double2 ph = __ldcs(pp);
                 ph.x = ph.x + f32_to_f64(em.x);
                 ph.y = ph.y + f32_to_f64(em.y);
-                *pp = ph;
+                __stcs(pp, ph);
                 vmax = fmaxf(vmax, fmaxf(fabsf(rh.x), fabsf(rh.y)));
                 emax = fmaxf(emax, fmaxf(fabsf(em.x), fabsf(em.y)));
             }
@@ -1319,7 +1319,7 @@ __global__ void __launch_bounds__(256, 6) e_gsrb4(const Item* __restrict__ items
                 const float4 ym = __ldg(o4 + ((pk + rjm) >> 2));
                 const float4 yp = __ldg(o4 + ((pk + rjp) >> 2));
                 const unsigned t = pk + rj;
-                const float4 b = __ldg(b4 + (t >> 2));
+                const float4 b = __ldcs(b4 + (t >> 2));
                 const int q = (j + k + color) & 1;
                 const unsigned rowbase = t - ih;
                 float xm0, xm1, xm2, xm3, xp0, xp1, xp2, xp3;

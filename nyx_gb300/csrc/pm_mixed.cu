@@ -733,18 +733,18 @@ __global__ void k_mx_correct2(int n, float c_hi, float c_lo, const float* __rest
             const float2 zp = __ldg(reinterpret_cast<const float2*>(other + row(j, kp) + ih));
             float2* rh_p = reinterpret_cast<float2*>((color ? r_b : r_r) + t);
             float2* rl_p = reinterpret_cast<float2*>((color ? rl_b : rl_r) + t);
-            float2 rh = *rh_p, rl = *rl_p;
+            float2 rh = *rh_p, rl = __ldcs(rl_p);
             const float v0[6] = {xm0, xp0, ym.x, yp.x, zm.x, zp.x};
             const float v1[6] = {xm1, xp1, ym.y, yp.y, zm.y, zp.y};
             df_residual_update(v0, em.x, c_hi, c_lo, rh.x, rl.x);
             df_residual_update(v1, em.y, c_hi, c_lo, rh.y, rl.y);
             *rh_p = rh;
-            *rl_p = rl;
+            __stcs(rl_p, rl);
             double2* pp = reinterpret_cast<double2*>((color ? phi_b : phi_r) + t);
-            double2 ph = *pp;
+            double2 ph = __ldcs(pp);
             ph.x = ph.x + f32_to_f64(em.x);
             ph.y = ph.y + f32_to_f64(em.y);
-            *pp = ph;
+            __stcs(pp, ph);
             vmax = fmaxf(vmax, fmaxf(fabsf(rh.x), fabsf(rh.y)));
             emax = fmaxf(emax, fmaxf(fabsf(em.x), fabsf(em.y)));
         }
@@ -798,11 +798,44 @@ __global__ void __launch_bounds__(256) k_gsrb_f(int n, int color, float* __restr
 // Needs half % 4 == 0 (rows start on 16 bytes).
 // 2 planes: at 256^3 a block marching 4 planes leaves 2048 blocks, 2.25 waves
 // at 6 blocks per SM, and the last wave's tail costs a quarter of the launch
-// (measured 20.6 us per half sweep; 2 planes 19.1 us, 1 plane 19.4 us)
+// (measured 20.6 us per half sweep; 2 planes 19.1 us, 1 plane 19.4 us).
+// From kMarchMinEdge on the correction and its right-hand side (8 bytes a cell, 134 MB at
+// 256^3) exceed the L2.  There the black half sweep takes the planes from the last one down,
+// as the red one left the last ones in the L2 (five 256^3 steps 41.8 -> 41.2 ms), the
+// right-hand side is read to pass through (40.1) and the correction to stay (39.7;
+// a half sweep 17.1 -> 14.3 us).
 constexpr int kMarchZ = 2;
 constexpr int kMarchMinEdge = 256;
 // the FP64 residual of levels of at least this edge sums on the integer pipes
 constexpr int kIntMinEdge = 96;
+
+
+// L2 eviction priorities for a level whose arrays together exceed the L2: the correction is
+// read again by the next half sweep and is asked to stay, the right-hand side passes through.
+__device__ __forceinline__ unsigned long long l2_keep()
+{
+    unsigned long long p;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ unsigned long long l2_pass()
+{
+    unsigned long long p;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ float4 ld_hint(const float4* a, unsigned long long p)
+{
+    float4 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a), "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_hint(float4* a, float4 v, unsigned long long p)
+{
+    asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
+                 :: "l"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(p) : "memory");
+}
 
 template <int MZ>
 __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __restrict__ mine,
@@ -815,7 +848,7 @@ __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __rest
     const unsigned half = (unsigned)n >> 1, h4 = half >> 2;
     const unsigned t4 = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k0 = blockIdx.z * MZ;
+    const int k0 = (MZ > 1 && color ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z) * MZ;
     if (t4 >= h4 || j >= n) return;
     const unsigned ih = 4 * t4;
     const unsigned plane = (unsigned)n * half;
@@ -834,11 +867,11 @@ __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __rest
         const int k = k0 + kk;
         const int kp = k == n - 1 ? 0 : k + 1;
         const unsigned pk = (unsigned)k * plane;
-        const float4 zp = __ldg(o4 + (((unsigned)kp * plane + rj) >> 2));
+        const float4 zp = MZ > 1 ? ld_hint(o4 + (((unsigned)kp * plane + rj) >> 2), l2_keep()) : __ldg(o4 + (((unsigned)kp * plane + rj) >> 2));
         const float4 ym = __ldg(o4 + ((pk + rjm) >> 2));
         const float4 yp = __ldg(o4 + ((pk + rjp) >> 2));
         const unsigned t = pk + rj;
-        const float4 b = __ldg(b4 + (t >> 2));
+        const float4 b = MZ > 1 ? ld_hint(b4 + (t >> 2), l2_pass()) : __ldg(b4 + (t >> 2));
         const int q = (j + k + color) & 1;
         // x neighbours: q = 1 -> (ih, ih+1), q = 0 -> (ih-1, ih) of the other colour
         const unsigned rowbase = t - ih;
@@ -857,7 +890,7 @@ __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __rest
         r.y = fmaf(((((xm1 + xp1) + ym.y) + yp.y) + zm.y) + zp.y, kSixthF, -b.y);
         r.z = fmaf(((((xm2 + xp2) + ym.z) + yp.z) + zm.z) + zp.z, kSixthF, -b.z);
         r.w = fmaf(((((xm3 + xp3) + ym.w) + yp.w) + zm.w) + zp.w, kSixthF, -b.w);
-        m4[t >> 2] = r;
+        if (MZ > 1) st_hint(m4 + (t >> 2), r, l2_keep()); else m4[t >> 2] = r;
         zm = c;
         c = zp;
     }
@@ -876,7 +909,7 @@ __global__ void __launch_bounds__(256) k_gsrb_f_zero(unsigned quads, float4* __r
     pdl_trigger();
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= quads) return;
-    const float4 b = __ldg(beta + t);
+    const float4 b = __ldcs(beta + t);
     mine[t] = make_float4(fmaf(0.f, kSixthF, -b.x), fmaf(0.f, kSixthF, -b.y), fmaf(0.f, kSixthF, -b.z),
                           fmaf(0.f, kSixthF, -b.w));
 }
