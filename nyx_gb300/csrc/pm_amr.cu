@@ -843,9 +843,9 @@ __device__ __forceinline__ void grav_one(const double* __restrict__ phi, long lo
                                          double* g0, double* g1, double* g2)
 {
     const double pc = phi[q];
-    g0[q] = 0.5 * fma(phi[xp] - pc, dxi, (pc - phi[xm]) * dxi);
-    g1[q] = 0.5 * fma(phi[yp] - pc, dxi, (pc - phi[ym]) * dxi);
-    g2[q] = 0.5 * fma(phi[zp] - pc, dxi, (pc - phi[zm]) * dxi);
+    g0[q] = 0.5 * fma(phi[xp] - pc, dxi, mul_on_int(pc - phi[xm], dxi));
+    g1[q] = 0.5 * fma(phi[yp] - pc, dxi, mul_on_int(pc - phi[ym], dxi));
+    g2[q] = 0.5 * fma(phi[zp] - pc, dxi, mul_on_int(pc - phi[zm], dxi));
 }
 
 __global__ void k_amr_grav0(int n, double dxi, const double* __restrict__ phi, double* g0, double* g1, double* g2)

@@ -427,6 +427,40 @@ __device__ inline T* lv_ptr(T* r, T* b, int n, int split, int i, int j, int k)
     return base + (long long)(i >> 1) + (long long)half * ((long long)j + (long long)n * k);
 }
 
+// A row's pair of cells x = 2 ih, 2 ih + 1 of a split level with their six neighbours each:
+// phi of the even cell, the odd cell, and then c[0 .. 5], c[6 .. 11] = x-, x+, y-, y+, z-, z+ of
+// the even and of the odd one.  Twelve loads and 32-bit offsets for two cells; the gravity
+// vectors' kernels with a cell per thread were bound by their index arithmetic.
+struct CellPair {
+    double even, odd, c[12];
+};
+
+__device__ __forceinline__ CellPair cell_pair(const double* __restrict__ phi_r, const double* __restrict__ phi_b, int n,
+                                              unsigned ih, int j, int k)
+{
+    const unsigned half = (unsigned)n >> 1;
+    const int p = (j + k) & 1;   // the colour of the row's even cells; its neighbour rows' is the other
+    const double* E = p ? phi_b : phi_r;
+    const double* O = p ? phi_r : phi_b;
+    auto at = [&](int jj, int kk) -> unsigned { return ((unsigned)jj + (unsigned)n * (unsigned)kk) * half + ih; };
+    const unsigned t = at(j, k);
+    CellPair P;
+    P.even = __ldg(E + t);
+    P.odd = __ldg(O + t);
+    P.c[0] = __ldg(O + (ih == 0 ? t + half - 1 : t - 1));
+    P.c[1] = P.odd;
+    P.c[6] = P.even;
+    P.c[7] = __ldg(E + (ih + 1 == half ? t + 1 - half : t + 1));
+    const unsigned r[4] = {at(j == 0 ? n - 1 : j - 1, k), at(j == n - 1 ? 0 : j + 1, k), at(j, k == 0 ? n - 1 : k - 1),
+                           at(j, k == n - 1 ? 0 : k + 1)};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        P.c[2 + a] = __ldg(O + r[a]);
+        P.c[8 + a] = __ldg(E + r[a]);
+    }
+    return P;
+}
+
 // ---------------------------------------------------------------------------
 // box
 // ---------------------------------------------------------------------------

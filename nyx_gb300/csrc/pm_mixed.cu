@@ -487,6 +487,32 @@ __global__ void k_mx_make_beta(int n, int split, const float* __restrict__ rho, 
     block_umax_store(u, norm);
 }
 
+// the same for a split level, the cells 2 ih, 2 ih + 1 of a row per thread (256^3: 15 us less)
+__global__ void __launch_bounds__(256) k_mx_make_beta2(int n, const float* __restrict__ rho, double mo,
+                                                       const double* __restrict__ scal, double scale,
+                                                       double* __restrict__ beta_r, double* __restrict__ beta_b,
+                                                       unsigned long long* norm)
+{
+    pdl_wait();
+    pdl_trigger();
+    const unsigned half = (unsigned)n >> 1;
+    const unsigned ih = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    unsigned long long u = 0;
+    if (ih < half && j < n) {
+        const double off = mo + scal[0];
+        const unsigned t = ((unsigned)j + (unsigned)n * (unsigned)k) * half + ih;
+        const float2 v = __ldg(reinterpret_cast<const float2*>(rho) + t);
+        const double e = (f32_to_f64(v.x) - off) * scale, o = (f32_to_f64(v.y) - off) * scale;
+        const bool odd_red = (j + k) & 1;
+        beta_r[t] = odd_red ? o : e;
+        beta_b[t] = odd_red ? e : o;
+        u = max(absbits(e), absbits(o));
+    }
+    block_umax_store(u, norm);
+}
+
 // ---------------------------------------------------------------------------
 // outer FP64 residual -> FP32 inner right-hand side (+ its max norm)
 // ---------------------------------------------------------------------------
@@ -1367,6 +1393,27 @@ __global__ void k_mx_grav(LevelView L, float half_dxi, float* g)
                                                   f64_to_f32_rn(P(i, j, kp) - P(i, j, km)) * half_dxi, 0.f);
 }
 
+// the same for a split level, two cells per thread (256^3: 146 -> 100 us, the FP64 subtractions' time)
+__global__ void __launch_bounds__(256) k_mx_grav2(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
+                                                  float half_dxi, float4* __restrict__ g)
+{
+    pdl_wait();
+    pdl_trigger();
+    const unsigned half = (unsigned)n >> 1;
+    const unsigned ih = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (ih >= half || j >= n) return;
+    const CellPair P = cell_pair(phi_r, phi_b, n, ih, j, k);
+    float4* out = g + 2 * (size_t)(((unsigned)j + (unsigned)n * (unsigned)k) * half + ih);
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const double* c = P.c + 6 * o;
+        out[o] = make_float4(f64_to_f32_rn(c[1] - c[0]) * half_dxi, f64_to_f32_rn(c[3] - c[2]) * half_dxi,
+                             f64_to_f32_rn(c[5] - c[4]) * half_dxi, 0.f);
+    }
+}
+
 // a caller's FP64 gravity vector (3 n^3, component-major) as the kicks' float4 per cell
 __global__ void k_mx_g32_from_g(long long nc, const double* __restrict__ g, float* g32)
 {
@@ -1880,8 +1927,13 @@ nyxpm_status mixed_make_rhs(Ctx& c, Box& b, double a)
     launch_pdl(c, k_mx_mean, dim3(kMeanBlocks), dim3(32), n, dx, b.L, b.rows, b.scal + 4,
                                                 reinterpret_cast<unsigned*>(b.scal + kScalTicket), b.scal, b.norms);
     const double scale = ((-4.0 * M_PI * c.p.gconst) * (1.0 / a)) * beta_scale(b);
-    launch_pdl(c, k_mx_make_beta, dim3(g.grid), dim3(g.block), n, l0.split, b.frho, b.mass_offset, b.scal,
-                                                     scale, l0.beta_r, l0.beta_b, b.norms);
+    if (l0.split) {
+        const Geo g2 = geo3(n / 2, n, n);
+        launch_pdl(c, k_mx_make_beta2, dim3(g2.grid), dim3(g2.block), n, b.frho, b.mass_offset, b.scal, scale, l0.beta_r, l0.beta_b, b.norms);
+    } else {
+        launch_pdl(c, k_mx_make_beta, dim3(g.grid), dim3(g.block), n, l0.split, b.frho, b.mass_offset, b.scal,
+                   scale, l0.beta_r, l0.beta_b, b.norms);
+    }
     prof_end(c, NYXPM_ST_RHS, 20.0 * nc);
     c.launches += 2;
     return check_launch(c, "mixed rhs");
@@ -1892,7 +1944,13 @@ nyxpm_status mixed_grav32(Ctx& c, Box& b)
     const long long nc = (long long)b.n * b.n * b.n;
     const Geo g = geo3(b.n, b.n, b.n);
     prof_begin(c);
-    launch_pdl(c, k_mx_grav, dim3(g.grid), dim3(g.block), view(b.levels[0]), (float)(0.5 * b.dxi), b.g32);
+    if (b.levels[0].split) {
+        const Geo g2 = geo3(b.n / 2, b.n, b.n);
+        launch_pdl(c, k_mx_grav2, dim3(g2.grid), dim3(g2.block), b.n, b.levels[0].phi_r, b.levels[0].phi_b,
+                   (float)(0.5 * b.dxi), reinterpret_cast<float4*>(b.g32));
+    } else {
+        launch_pdl(c, k_mx_grav, dim3(g.grid), dim3(g.block), view(b.levels[0]), (float)(0.5 * b.dxi), b.g32);
+    }
     prof_end(c, NYXPM_ST_KICK, 20.0 * nc);
     return check_launch(c, "mixed grav");
 }

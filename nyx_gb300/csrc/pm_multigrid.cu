@@ -12,6 +12,7 @@
 // arithmetic uses 3-D launch geometry instead of integer division.  Built with
 // --fmad=false: only the explicit fma() calls fuse, in the same places the CPU
 // oracle fuses, so both round identically.
+#include "pm_cic.cuh"
 #include "pm_cluster.cuh"
 #include "pm_common.cuh"
 #include "pm_sum6.cuh"
@@ -689,7 +690,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_d(ClArgs<double
 }
 
 // g_d(c) = 0.5*((phi_c - phi_{c-e_d})*dxi + (phi_{c+e_d} - phi_c)*dxi), second product fused;
-// component-major output
+// component-major output; one product on the integer pipe
 __global__ void k_grav(LevelView L, double dxi, double* g)
 {
     pdl_wait();
@@ -708,9 +709,30 @@ __global__ void k_grav(LevelView L, double dxi, double* g)
     const int im = i == 0 ? n - 1 : i - 1, ip = i == n - 1 ? 0 : i + 1;
     const int jm = j == 0 ? n - 1 : j - 1, jp = j == n - 1 ? 0 : j + 1;
     const int km = k == 0 ? n - 1 : k - 1, kp = k == n - 1 ? 0 : k + 1;
-    g[c] = 0.5 * fma(P(ip, j, k) - pc, dxi, (pc - P(im, j, k)) * dxi);
-    g[nc + c] = 0.5 * fma(P(i, jp, k) - pc, dxi, (pc - P(i, jm, k)) * dxi);
-    g[2 * nc + c] = 0.5 * fma(P(i, j, kp) - pc, dxi, (pc - P(i, j, km)) * dxi);
+    auto diff = [&](double m, double p) { return 0.5 * fma(p - pc, dxi, mul_on_int(pc - m, dxi)); };
+    g[c] = diff(P(im, j, k), P(ip, j, k));
+    g[nc + c] = diff(P(i, jm, k), P(i, jp, k));
+    g[2 * nc + c] = diff(P(i, j, km), P(i, j, kp));
+}
+
+// the same for a split level, two cells per thread (256^3: 484 -> 415 us)
+__global__ void __launch_bounds__(256) k_grav2(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
+                                               double dxi, double* __restrict__ g)
+{
+    pdl_wait();
+    pdl_trigger();
+    const unsigned half = (unsigned)n >> 1;
+    const unsigned ih = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int k = blockIdx.z;
+    if (ih >= half || j >= n) return;
+    const CellPair P = cell_pair(phi_r, phi_b, n, ih, j, k);
+    auto diff = [&](double m, double c, double p) { return 0.5 * fma(p - c, dxi, mul_on_int(c - m, dxi)); };
+    const long long nc2 = (long long)n * n * half;
+    double2* out = reinterpret_cast<double2*>(g) + ((unsigned)j + (unsigned)n * (unsigned)k) * half + ih;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        out[d * nc2] = make_double2(diff(P.c[2 * d], P.even, P.c[2 * d + 1]), diff(P.c[6 + 2 * d], P.odd, P.c[7 + 2 * d]));
 }
 
 __global__ void k_to_natural(LevelView L, double* out)
@@ -1061,7 +1083,12 @@ nyxpm_status launch_grav_vector(Ctx& c, Box& b)
     const long long nc = (long long)b.n * b.n * b.n;
     const Geo g = geo3(b.n, b.n, b.n);
     prof_begin(c);
-    launch_pdl(c, k_grav, dim3(g.grid), dim3(g.block), view(b.levels[0]), b.dxi, b.g);
+    if (b.levels[0].split) {
+        const Geo g2 = geo3(b.n / 2, b.n, b.n);
+        launch_pdl(c, k_grav2, dim3(g2.grid), dim3(g2.block), b.n, b.levels[0].phi_r, b.levels[0].phi_b, b.dxi, b.g);
+    } else {
+        launch_pdl(c, k_grav, dim3(g.grid), dim3(g.block), view(b.levels[0]), b.dxi, b.g);
+    }
     prof_end(c, NYXPM_ST_KICK, 32.0 * nc);
     return check_launch(c, "grav vector");
 }
