@@ -302,15 +302,32 @@ __device__ int block_excl_scan(int v, int* total)
     return before;
 }
 
+// A thread's counts, 0 beyond n, in two 16-byte loads where all are there (the arrays start on
+// 256 bytes): k_scan_down 64 -> 25 us at 256^3.
+__device__ __forceinline__ void scan_load(const int* __restrict__ in, int n, long long base, int (&v)[kScanItems])
+{
+    static_assert(kScanItems == 8, "two int4");
+    if (base + kScanItems <= n) {
+        const int4* p = reinterpret_cast<const int4*>(in + base);
+        const int4 a = p[0], b = p[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int t = 0; t < kScanItems; ++t) v[t] = base + t < n ? in[base + t] : 0;
+    }
+}
+
 __global__ void k_scan_reduce(const int* __restrict__ in, int n, int* tile_sums)
 {
     pdl_wait();
     pdl_trigger();
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
+    int v[kScanItems];
+    scan_load(in, n, base, v);
     int s = 0;
 #pragma unroll
-    for (int t = 0; t < kScanItems; ++t)
-        if (base + t < n) s += in[base + t];
+    for (int t = 0; t < kScanItems; ++t) s += v[t];
     int total;
     block_excl_scan(s, &total);
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
@@ -339,18 +356,26 @@ __global__ void k_scan_down(const int* __restrict__ in, int n, const int* __rest
     pdl_trigger();
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     int v[kScanItems];
+    scan_load(in, n, base, v);
     int s = 0;
 #pragma unroll
-    for (int t = 0; t < kScanItems; ++t) {
-        v[t] = base + t < n ? in[base + t] : 0;
-        s += v[t];
-    }
+    for (int t = 0; t < kScanItems; ++t) s += v[t];
     int total;
     int run = block_excl_scan(s, &total) + tile_off[blockIdx.x];
 #pragma unroll
     for (int t = 0; t < kScanItems; ++t) {
-        if (base + t < n) out[base + t] = run;
-        run += v[t];
+        const int x = v[t];
+        v[t] = run;
+        run += x;
+    }
+    if (base + kScanItems <= n) {
+        int4* o = reinterpret_cast<int4*>(out + base);
+        o[0] = make_int4(v[0], v[1], v[2], v[3]);
+        o[1] = make_int4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+        for (int t = 0; t < kScanItems; ++t)
+            if (base + t < n) out[base + t] = v[t];
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = run;
 }
@@ -365,35 +390,21 @@ __global__ void k_scan_down(const int* __restrict__ in, int n, const int* __rest
 static_assert(kDepositLanes == 32, "long keys are summed by one warp; the sort queues keys > 32");
 
 // adds particle q's eight CIC weights (times its mass, fused, if m) to s
-__device__ __forceinline__ void add_weights(int q, int n, double dxi, const double* __restrict__ x,
+__device__ __forceinline__ void add_weights(int q, double dxi, const double* __restrict__ x,
                                             const double* __restrict__ y,
                                             const double* __restrict__ z,
-                                            const double* __restrict__ m, double s[8])
+                                            const double* __restrict__ m, double (&s)[8])
 {
-    double fx, fy, fz;
-    key1(x[q], dxi, n, &fx);
-    key1(y[q], dxi, n, &fy);
-    key1(z[q], dxi, n, &fz);
-    const double sx[2] = {1.0 - fx, fx};
-    const double sy[2] = {1.0 - fy, fy};
-    const double sz[2] = {1.0 - fz, fz};
+    int cell[3];
+    double w[8];
+    cic_weights(fma(x[q], dxi, 0.5), fma(y[q], dxi, 0.5), fma(z[q], dxi, 0.5), cell, w);
     if (m) {
         const double mq = m[q];
 #pragma unroll
-        for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-            for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-                for (int cx = 0; cx < 2; ++cx)
-                    s[cx + 2 * cy + 4 * cz] = fma((sx[cx] * sy[cy]) * sz[cz], mq, s[cx + 2 * cy + 4 * cz]);
+        for (int c = 0; c < 8; ++c) s[c] = fma(w[c], mq, s[c]);
     } else {
 #pragma unroll
-        for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-            for (int cy = 0; cy < 2; ++cy)
-#pragma unroll
-                for (int cx = 0; cx < 2; ++cx)
-                    s[cx + 2 * cy + 4 * cz] = s[cx + 2 * cy + 4 * cz] + (sx[cx] * sy[cy]) * sz[cz];
+        for (int c = 0; c < 8; ++c) s[c] = s[c] + w[c];
     }
 }
 
@@ -401,6 +412,9 @@ __device__ __forceinline__ void add_weights(int q, int n, double dxi, const doub
 // particles l, l+32, l+64, ... of the key in order, then the xor butterfly
 // (offsets 16, 8, 4, 2, 1) combines the lanes.  The eight corner sums go to
 // heavy_part[slot], and key_slot[K] = slot tells the tile kernel where.
+// The butterfly takes the eight corners together, each half of the lanes keeping half of
+// them (9 FP64 additions of the warp instead of 40); with that and the weights on the integer
+// pipe 185 -> 92 us at 256^3 with clumps.
 __global__ void __launch_bounds__(256) k_deposit_heavy(int n, double dxi,
                                                        const double* __restrict__ x,
                                                        const double* __restrict__ y,
@@ -422,18 +436,19 @@ __global__ void __launch_bounds__(256) k_deposit_heavy(int n, double dxi,
         double s[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) s[c] = 0.0;
-        for (int q = start[K] + lane; q < e; q += 32) add_weights(q, n, dxi, x, y, z, m, s);
+        for (int q = start[K] + lane; q < e; q += 32) add_weights(q, dxi, x, y, z, m, s);
 #pragma unroll
-        for (int off = 16; off >= 1; off >>= 1)
+        for (int off = 16; off >= 4; off >>= 1) {
+            const bool up = lane & off;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) s[c] = s[c] + __shfl_xor_sync(0xffffffffu, s[c], off);
-        if (lane < 8) {
-            double v = s[0];
-#pragma unroll
-            for (int c = 1; c < 8; ++c)
-                if (lane == c) v = s[c];
-            heavy_part[8LL * li + lane] = v;
+            for (int c = 0; c < off / 4; ++c) {
+                const double keep = up ? s[c + off / 4] : s[c], give = up ? s[c] : s[c + off / 4];
+                s[c] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+            }
         }
+        s[0] = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 2);
+        s[0] = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+        if ((lane & 3) == 0) heavy_part[8LL * li + (lane >> 2)] = s[0];
         if (lane == 0) key_slot[K] = li;
     }
 }
@@ -563,7 +578,8 @@ __global__ void __launch_bounds__(32 * kKeyWarps, 40 / kKeyWarps) k_deposit_keys
 }
 
 // Pass 2, one thread per cell: the eight keys' corners in the fixed (dk, dj, di)
-// order, times the scale -- the same sums as the tile kernel's, term for term.
+// order, times the scale -- the same sums as the tile kernel's, term for term.  Bound by the
+// FP64 additions (256^3: nine FP64 instructions a cell, 290 us; seven, 270).
 __global__ void __launch_bounds__(256) k_deposit_cells(int n, double scale,
                                                        const double* __restrict__ part,
                                                        double* __restrict__ rho)
@@ -585,9 +601,10 @@ __global__ void __launch_bounds__(256) k_deposit_cells(int n, double scale,
 #pragma unroll
             for (int di = 0; di < 2; ++di) {
                 const int corner = (1 - di) + 2 * (1 - dj) + 4 * (1 - dk);
-                acc = acc + __ldg(part + corner * nc + cidx(is[di], js[dj], ks[dk], n));
+                const double p = __ldg(part + corner * nc + cidx(is[di], js[dj], ks[dk], n));
+                acc = dk + dj + di == 0 ? p : acc + p;   // (0 + p = p)
             }
-    rho[cidx(i, j, k, n)] = acc * scale;
+    rho[cidx(i, j, k, n)] = mul_on_int(acc, scale);
 }
 
 // ---------------------------------------------------------------------------
