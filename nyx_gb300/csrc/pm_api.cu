@@ -228,9 +228,9 @@ nyxpm_status do_solve(Ctx& c, Box& b, double a, int zero_guess, nyxpm_solve_info
     nyxpm_status st;
     const bool mixed = b.prec == NYXPM_MIXED;
     if ((st = mixed ? mixed_make_rhs(c, b, a) : launch_make_rhs(c, b, a)) != NYXPM_OK) return st;
-    if (zero_guess && (st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
+    if (mixed && zero_guess && (st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
     bool grav_done = mixed;   // the mixed solve leaves its FP32 gravity vector in g32 itself
-    nyxpm_status solved = mixed ? mixed_solve(c, b, zero_guess, info) : mg_solve(c, b, info, &grav_done);
+    nyxpm_status solved = mixed ? mixed_solve(c, b, zero_guess, info) : mg_solve(c, b, zero_guess, info, &grav_done);
     if (solved != NYXPM_OK && solved != NYXPM_NOT_CONVERGED) return solved;
     b.g_from_caller = 0;   // the gravity vector follows the new phi from here on
     if (!grav_done && (st = launch_grav_vector(c, b)) != NYXPM_OK) return st;

@@ -665,7 +665,7 @@ nyxpm_status mixed_est_dt(Ctx& c, Box& b);
 double beta_scale(const Box& b);  // (h*h)/6 of level 0: rhs -> smoother units
 nyxpm_status launch_zero_phi(Ctx& c, Box& b);
 // grav_done: the gravity vector of the new phi is enqueued (as launch_grav_vector does it)
-nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info, bool* grav_done);
+nyxpm_status mg_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info, bool* grav_done);
 nyxpm_status launch_grav_vector(Ctx& c, Box& b);
 nyxpm_status launch_phi_to_natural(Ctx& c, Box& b, double* d_out);
 nyxpm_status launch_phi_from_natural(Ctx& c, Box& b, const double* d_in);

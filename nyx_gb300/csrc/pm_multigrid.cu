@@ -357,6 +357,20 @@ __global__ void __launch_bounds__(256) k_gsrb(int n, int color, double* __restri
     mine[t] = fma(s, kSixth, -beta[t]);
 }
 
+// The red half sweep from phi = 0: fma(0, 1/6, -beta) = 0 - beta by the sign bit (+0 for either
+// zero), two cells per thread.
+__global__ void __launch_bounds__(256) k_gsrb_zero(unsigned pairs, const ulonglong2* __restrict__ beta,
+                                                   ulonglong2* __restrict__ phi)
+{
+    pdl_wait();
+    pdl_trigger();
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= pairs) return;
+    const ulonglong2 b = __ldg(beta + t);
+    auto minus = [](unsigned long long u) { return (u << 1) == 0 ? 0ULL : u ^ (1ULL << 63); };
+    phi[t] = make_ulonglong2(minus(b.x), minus(b.y));
+}
+
 // k_gsrb by pairs
 __global__ void __launch_bounds__(256) k_gsrb2(int n, int color, double* __restrict__ mine,
                                                const double* __restrict__ other,
@@ -716,15 +730,17 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_nat_d(ClArgs<d
 // norms[1]) = rel_tol max(||beta||, ||r0||), with the red-cell norm of mg_solve's loop:
 // norms[5] = ||r||, norms[6] = the number of V-cycles.  Every CTA sees the same norms, so
 // all leave the loop together.
+// zero: phi is 0 on entry, whatever the arrays hold.
 __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_d(ClArgs<double> A, LevelView L, double rel_tol,
-                                                                int max_vcycles, unsigned long long* norms)
+                                                                int max_vcycles, int zero, unsigned long long* norms)
 {
     extern __shared__ __align__(16) double cl_mem_d[];
     __shared__ ClShared<double> S;
     cl_setup(A, S, cl_mem_d);
     pdl_wait();
     pdl_trigger();
-    const double bnorm = __longlong_as_double((long long)norms[0]), r0 = __longlong_as_double((long long)norms[1]);
+    const double bnorm = __longlong_as_double((long long)norms[0]);
+    const double r0 = zero ? bnorm : __longlong_as_double((long long)norms[1]);
     const double target = rel_tol * (bnorm < r0 ? r0 : bnorm);
     double r = r0;
     int it = 0;
@@ -732,10 +748,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_d(ClArgs<double
         const ClLevel<double>& F = S.lv[0];
         const int n = F.n, half = n >> 1, total = half * n * F.np;
         cl_load_green(A, S);
-        cl_load(F, L, true);
+        cl_load(F, L, !zero);
         cl_barrier();
         for (it = 1;; ++it) {
-            cl_vcycle(A, S, cl_mem_d, 0);
+            cl_vcycle(A, S, cl_mem_d, zero && it == 1 ? 1 : 0);
             unsigned long long v = 0;
             for (int t = threadIdx.x; t < total; t += blockDim.x) {
                 int ih, j, q;
@@ -749,6 +765,13 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve_d(ClArgs<double
             if (r <= target || r != r || it >= max_vcycles) break;
         }
         cl_store(F, L);
+    } else if (zero) {
+        const ClLevel<double>& F = S.lv[0];
+        const int plane = F.n * (F.n >> 1);
+        for (int t = threadIdx.x; t < plane * F.np; t += blockDim.x) {
+            L.phi_r[F.p0 * plane + t] = 0.0;
+            L.phi_b[F.p0 * plane + t] = 0.0;
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         norms[5] = absbits(r);
@@ -1042,21 +1065,32 @@ nyxpm_status launch_zero_phi(Ctx& c, Box& b)
     return check_launch(c, "zero phi");
 }
 
-nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info, bool* grav_done)
+nyxpm_status mg_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info, bool* grav_done)
 {
     nyxpm_status st;
     const Level& l0 = b.levels[0];
     const long long nc = (long long)l0.n * l0.n * l0.n;
     post_open(c, b.post);
-    // ||r0||_inf (launch_make_rhs left ||beta||_inf)
-    if ((st = launch_resnorm(c, b, 1, 0)) != NYXPM_OK) return st;
     // a small box: the whole solve in one cluster launch
     ClArgs<double> ca;
     const bool in_cluster = cluster_fits_d(c, b, 0, ca);
+    const int red_only = (c.p.nu2 > 0 && b.levels.size() > 1) ? 1 : 0;
+    // The red-cell norm after a V-cycle and the red half sweep that opens the next
+    // one share their neighbour sums: k_resnorm_red_sweep makes both, the sweep into
+    // the spare red array, which becomes level 0's red array only if the solve
+    // goes on (the next V-cycle then starts at its black half sweep).
+    Level& L0 = b.levels[0];
+    const bool fuse = red_only && c.p.nu1 > 0 && L0.split && b.phi_r_spare;
+    // From phi = 0 the residual is beta, whose norm launch_make_rhs left, and the opening red
+    // half sweep needs no neighbours, so phi is not zeroed (370 us of a 256^3 solve)
+    const bool from_zero = zero_guess && (in_cluster || fuse);
+    if (zero_guess && !from_zero && (st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
+    // ||r0||_inf
+    if (!from_zero && (st = launch_resnorm(c, b, 1, 0)) != NYXPM_OK) return st;
     if (in_cluster) {
         prof_begin(c);
         launch_cluster(c, k_cluster_solve_d, ca.elems * sizeof(double), ca, view(l0), c.p.rel_tol, c.p.max_vcycles,
-                       b.norms);
+                       from_zero ? 1 : 0, b.norms);
         prof_end(c, NYXPM_ST_SMOOTH, 0);
         if ((st = check_launch(c, "cluster solve")) != NYXPM_OK) return st;
     }
@@ -1067,18 +1101,12 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info, bool* grav_done)
     if ((st = check_launch(c, "norm read-back")) != NYXPM_OK) return st;
     if ((st = post_wait(c, b.post, "solve sync")) != NYXPM_OK) return st;
     const double bnorm = read_norm(b, 0);
-    const double r0 = read_norm(b, 1);
+    const double r0 = from_zero ? bnorm : read_norm(b, 1);
     const double target = c.p.rel_tol * std::max(bnorm, r0);
     double r = r0;
     int it = 0;
     nyxpm_status result = NYXPM_OK;
-    const int red_only = (c.p.nu2 > 0 && b.levels.size() > 1) ? 1 : 0;
-    // The red-cell norm after a V-cycle and the red half sweep that opens the next
-    // one share their neighbour sums: k_resnorm_red_sweep makes both, the sweep into
-    // the spare red array, which becomes level 0's red array only if the solve
-    // goes on (the next V-cycle then starts at its black half sweep).
-    Level& L0 = b.levels[0];
-    const bool fuse = red_only && c.p.nu1 > 0 && L0.split && b.phi_r_spare;
+    if (from_zero && !in_cluster && r0 <= target && (st = launch_zero_phi(c, b)) != NYXPM_OK) return st;
     if (in_cluster) {
         r = read_norm(b, 5);
         it = (int)b.h_norms[6];
@@ -1091,7 +1119,14 @@ nyxpm_status mg_solve(Ctx& c, Box& b, nyxpm_solve_info* info, bool* grav_done)
             c.err = "multigrid reached max_vcycles above tolerance";
         }
     } else if (!(r0 <= target)) {
-        bool first = true;
+        bool first = !from_zero;
+        if (from_zero) {
+            prof_begin(c);
+            launch_pdl(c, k_gsrb_zero, dim3(blocks_for(nc / 4)), dim3(kThreads), (unsigned)(nc / 4),
+                       reinterpret_cast<const ulonglong2*>(L0.beta_r), reinterpret_cast<ulonglong2*>(L0.phi_r));
+            prof_end(c, NYXPM_ST_SMOOTH, 8.0 * nc);
+            if ((st = check_launch(c, "opening sweep")) != NYXPM_OK) return st;
+        }
         auto iteration = [&]() -> nyxpm_status {
             nyxpm_status s;
             if ((s = vcycle(c, b, 0, fuse && !first ? 1 : 0)) != NYXPM_OK) return s;
