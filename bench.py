@@ -251,6 +251,12 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
+def fp64_adds_per_cell(n):
+    """FP64 additions per cell update of an FP64 half sweep at level edge n: five, or one warp
+    of four's where the neighbour sums are on the integer pipes."""
+    return 1.25 if n >= 128 and n % 4 == 0 else 5.0
+
+
 def ncu_traffic():
     """Per-launch DRAM bytes of the dominant kernels from the committed ncu summary."""
     p = os.path.join(REPO, "profiles", "ncu_traffic.json")
@@ -644,12 +650,14 @@ def run_amr_form(ctx, stream, n0=128, warmup=2, timed=10, cpu_n0=64, cpu_seconds
     stage_ms = sum(v["ms"] for v in prof["stages"].values())
     fp64_peak, fp64_add = ctx.measure_fp64_peak()
     updates = fs["bytes"] / 24.0
-    ops = 6.0 * updates / (fs["ms"] * 1e-3) / 1e12
-    peak_ops = 6.0 / (5.0 / fp64_add + 1.0 / (fp64_peak / 2.0))
-    roofline = {"bound": "fp64", "kernel": "red-black half sweeps of every level (k_amr_gsrbf, level 0's k_gsrb)",
+    adds = fp64_adds_per_cell(n0)
+    ops = (adds + 1.0) * updates / (fs["ms"] * 1e-3) / 1e12
+    peak_ops = (adds + 1.0) / (adds / fp64_add + 1.0 / (fp64_peak / 2.0))
+    roofline = {"bound": "fp64", "kernel": "red-black half sweeps of every level (k_amr_gsrbf, level 0's k_gsrb2)",
                 "achieved": round(ops, 4), "peak": round(peak_ops, 4), "frac": round(ops / peak_ops, 4),
-                "unit": "T FP64 op/s (an add or an FMA is one op; 6 per updated cell)",
-                "peak_source": "measured: nyxpm_measure_fp64_peak on this GPU, weighted 5 adds : 1 FMA",
+                "unit": f"T FP64 op/s (an add or an FMA is one op; {adds + 1.0:g} per updated cell, the other "
+                        "additions are on the integer pipes)",
+                "peak_source": f"measured: nyxpm_measure_fp64_peak on this GPU, weighted {adds:g} adds : 1 FMA",
                 "launches": fs["launches"], "ms": round(fs["ms"], 3),
                 "share_of_step": round(fs["ms"] / stage_ms, 3) if stage_ms > 0 else None}
     H.close()
@@ -814,7 +822,8 @@ def run_ours(args):
         fs = prof["fine_smooth"]
         per_launch = fs["bytes"] / fs["launches"]
         avg_ms = fs["ms"] / fs["launches"]
-        kname = ("k_gsrb (finest-level FP64 red-black half sweep)" if args.precision == "fp64" else
+        kname = (f"{'k_gsrb2' if fp64_adds_per_cell(n) < 5 else 'k_gsrb'} (finest-level FP64 red-black half sweep)"
+                 if args.precision == "fp64" else
                  "k_gsrb_f4 (finest-level FP32 red-black half sweep)")
         tr = traffic.get("k_gsrb_fine") if args.precision == "fp64" else None
     else:
@@ -829,26 +838,30 @@ def run_ours(args):
     share = round(stages[dom]["ms"] / sum(v["ms"] for v in stages.values()), 3)
     traffic_launch = tr * (n / traffic.get("n", n)) ** 3 if tr else None
     if args.precision == "fp64" and dom == "smooth" and prof["fine_smooth"]["launches"]:
-        # the finest FP64 half sweep updates n^3/2 cells with 6 FP64 operations each
-        # (5 additions of the neighbour sum and one fused multiply-add), 24 algorithmic
-        # bytes per cell.  The bound is the time the FP64 pipe needs for that mix at the
-        # rates measured on this GPU: 5 / add rate + 1 / FMA rate per cell, i.e. a peak
-        # of 6 / (5 / R_add + 1 / R_fma) operations per second
+        # the finest FP64 half sweep updates n^3/2 cells, 24 algorithmic bytes each, with 5
+        # additions of the neighbour sum and one fused multiply-add.  From 128^3 on three
+        # warps of four add on the integer pipes (k_gsrb2), which share the issue slots
+        # with the FP64 pipe: adds = 1.25 of the additions are FP64 instructions.  The
+        # peak is the FP64 pipe's time for its part of the mix at the rates measured on
+        # this GPU: (adds + 1) / (adds / R_add + 1 / R_fma) operations per second
         cells = per_launch / 24.0
-        ops = 6.0 * cells / (avg_ms * 1e-3) / 1e12
+        adds = fp64_adds_per_cell(n)
+        ops = (adds + 1.0) * cells / (avg_ms * 1e-3) / 1e12
         r_fma = fp64_peak / 2.0
-        peak_ops = 6.0 / (5.0 / fp64_add + 1.0 / r_fma)
+        peak_ops = (adds + 1.0) / (adds / fp64_add + 1.0 / r_fma)
         roofline = {"bound": "fp64", "kernel": kname,
                     "achieved": round(ops, 4), "peak": round(peak_ops, 4),
                     "peak_source": "measured: nyxpm_measure_fp64_peak on this GPU (chains of FP64 "
-                                   "additions and of FMAs, CUDA events), weighted 5 adds : 1 FMA",
-                    "unit": "T FP64 op/s (an add or an FMA is one op)",
+                                   f"additions and of FMAs, CUDA events), weighted {adds:g} adds : 1 FMA",
+                    "unit": "T FP64 op/s (an add or an FMA is one op; additions made on the "
+                            "integer pipes are not counted)",
+                    "cell_updates_G_per_s": round(cells / (avg_ms * 1e-3) / 1e9, 2),
                     "frac": round(ops / peak_ops, 4), "traffic": traffic_launch,
                     "fp64_rates_measured": {"fma_T_per_s": round(r_fma, 4),
                                             "add_T_per_s": round(fp64_add, 4)},
-                    "flops": {"achieved_TFLOPs": round(7.0 * cells / (avg_ms * 1e-3) / 1e12, 4),
+                    "flops": {"achieved_TFLOPs": round((adds + 2.0) * cells / (avg_ms * 1e-3) / 1e12, 4),
                               "peak_TFLOPs": round(fp64_peak, 4),
-                              "note": "FMA = 2 flops: 7 flops per updated cell; peak = FMA chains"},
+                              "note": f"FMA = 2 flops: {adds + 2.0:g} FP64 flops per updated cell; peak = FMA chains"},
                     "hbm": hbm,
                     "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": avg_ms,
                     "fp64_pipe_active_ncu": traffic.get("k_gsrb_fine_fp64_pipe_active"),

@@ -1512,13 +1512,6 @@ __global__ void __launch_bounds__(256, 6) k_mx_kick(long long np, MxKickArgs A, 
     }
 }
 
-inline unsigned norm_blocks(Ctx& c, long long cnt)
-{
-    long long b = (cnt + kThreads - 1) / kThreads;
-    long long cap = (long long)c.sm_count * 8;
-    return (unsigned)std::max<long long>(1, std::min(b, cap));
-}
-
 double read_norm(Box& b, int slot)
 {
     double v;

@@ -869,13 +869,6 @@ __global__ void k_beta_from_natural(LevelView L, const double* __restrict__ in, 
 constexpr int kPairMinEdge = 128;
 inline bool by_pairs(const Level& l) { return l.split && l.n >= kPairMinEdge && l.n % 4 == 0; }
 
-inline unsigned norm_blocks(Ctx& c, long long cnt)
-{
-    long long b = (cnt + kThreads - 1) / kThreads;
-    long long cap = (long long)c.sm_count * 8;
-    return (unsigned)std::max<long long>(1, std::min(b, cap));
-}
-
 nyxpm_status gsrb_sweep(Ctx& c, const Level& l, int fine, int black_only = 0)
 {
     const long long half_cells = (long long)l.n * l.n * l.n / 2;
