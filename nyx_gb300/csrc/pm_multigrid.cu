@@ -895,9 +895,16 @@ bool tail_fits_d(const Ctx& c, const Box& b, size_t li)
            b.levels.size() - li <= (size_t)kMaxTail;
 }
 
-// whether the levels from li on are taken by one cluster, and how they lie in it
+// whether the levels from li on are taken by one cluster, and how they lie in it.  Below a
+// box's finest level only from 16^3 down: a pass over 32^3 takes the FP64 pipes of 16 SMs as long
+// as a launch takes all of them and its launch (four steps at 64^3 7.48 ms with level 32 in the
+// cluster, 7.19 without; 7.8 with level 16 out too).  A box of up to 32^3 is solved in one
+// launch (3.64 ms; its V-cycles by launches down to 16^3 3.82).
+constexpr int kClusterEdgeD = 16, kClusterSolveEdgeD = 32;
+
 bool cluster_fits_d(Ctx& c, const Box& b, size_t li, ClArgs<double>& A)
 {
+    if (b.levels[li].n > (li > 0 ? kClusterEdgeD : kClusterSolveEdgeD)) return false;
     if (!cl_args<double>(c, b, li, A)) return false;
     if (c.cluster_d < 0) {
         const size_t most = cl_max_bytes<double>();
