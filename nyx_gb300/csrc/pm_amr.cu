@@ -532,11 +532,12 @@ __device__ __forceinline__ void block_umax(unsigned long long v, unsigned long l
         const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, off);
         v = o > v ? o : v;
     }
-    const unsigned tid = threadIdx.x + blockDim.x * threadIdx.y;   // blocks of kT threads
+    const unsigned tid = threadIdx.x + blockDim.x * threadIdx.y;   // whole warps, at most kT threads
     if ((tid & 31) == 0) part[tid >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-        for (int w = 1; w < kT / 32; ++w) v = part[w] > v ? part[w] : v;
+        const int warps = (int)(blockDim.x * blockDim.y) >> 5;
+        for (int w = 1; w < warps; ++w) v = part[w] > v ? part[w] : v;
         if (v != 0ULL) atomicMax(out, v);
     }
 }
@@ -1237,13 +1238,8 @@ nyxpm_status comp_resid(Ctx& c, nyxpm_amr& A, int slot)
     if ((st = ghost_fill(c, A, A.phi, A.all_ghost1)) != NYXPM_OK) return st;
     const Geo g = geo3(A.n0, A.n0, A.n0, kT);
     prof_begin(c);
-    if (g.block.x * g.block.y == kT) {
-        launch_pdl(c, on_int(n3) ? k_amr_resid0<true> : k_amr_resid0<false>, dim3(g.grid), dim3(g.block), A.n0, A.phi,
-                   A.beta, A.d_cov, A.inv_scale[0], A.R, A.norms + slot);
-    } else {   // a tiny level 0: whole blocks of kT threads all the same
-        launch_pdl(c, k_amr_resid0<false>, dim3(1, 1, A.n0), dim3(kT / 16, 16), A.n0, A.phi, A.beta, A.d_cov,
-                   A.inv_scale[0], A.R, A.norms + slot);
-    }
+    launch_pdl(c, on_int(n3) ? k_amr_resid0<true> : k_amr_resid0<false>, dim3(g.grid), dim3(g.block), A.n0, A.phi,
+               A.beta, A.d_cov, A.inv_scale[0], A.R, A.norms + slot);
     prof_end(c, NYXPM_ST_NORM, 25.0 * n3);
     if (A.fine_cells.count) {
         prof_begin(c);
