@@ -254,7 +254,7 @@ def measured_peaks():
 def fp64_adds_per_cell(n):
     """FP64 additions per cell update of an FP64 half sweep at level edge n: five, or one warp
     of four's where the neighbour sums are on the integer pipes."""
-    return 1.25 if n >= 128 and n % 4 == 0 else 5.0
+    return 1.25 if n >= 96 and n % 4 == 0 else 5.0
 
 
 def ncu_traffic():
@@ -839,7 +839,7 @@ def run_ours(args):
     traffic_launch = tr * (n / traffic.get("n", n)) ** 3 if tr else None
     if args.precision == "fp64" and dom == "smooth" and prof["fine_smooth"]["launches"]:
         # the finest FP64 half sweep updates n^3/2 cells, 24 algorithmic bytes each, with 5
-        # additions of the neighbour sum and one fused multiply-add.  From 128^3 on three
+        # additions of the neighbour sum and one fused multiply-add.  From 96^3 on three
         # warps of four add on the integer pipes (k_gsrb2), which share the issue slots
         # with the FP64 pipe: adds = 1.25 of the additions are FP64 instructions.  The
         # peak is the FP64 pipe's time for its part of the mix at the rates measured on

@@ -863,10 +863,10 @@ __global__ void k_beta_from_natural(LevelView L, const double* __restrict__ in, 
 }
 
 // Levels of at least this edge work by pairs of cells, their sums on the integer pipes
-// (pm_sum6.cuh): there the FP64 pipe is the bound (128^3: a half sweep 16.4 -> 12.3 us,
-// a whole solve 3.21 -> 2.82 ms).  On 64^3 a half sweep is latency: integer sums gave
-// a ten-step 64^3 run 23.8 ms against 24.0 ms, and with them on every level 25.4 ms.
-constexpr int kPairMinEdge = 128;
+// (pm_sum6.cuh): there the FP64 pipe is the bound (four steps at 96^3 12.3 -> 11.5 ms, at 112^3
+// 18.3 -> 17.1).  Below, a half sweep is latency: with integer sums on level 64 four 64^3 steps take
+// 7.24 ms against 7.10, on level 80 four 160^3 steps 31.1 against 30.5.
+constexpr int kPairMinEdge = 96;
 inline bool by_pairs(const Level& l) { return l.split && l.n >= kPairMinEdge && l.n % 4 == 0; }
 
 nyxpm_status gsrb_sweep(Ctx& c, const Level& l, int fine, int black_only = 0)
