@@ -1180,8 +1180,9 @@ nyxpm_status build_lists(nyxpm_ctx* c, nyxpm_amr* a)
 // launch sequences
 // ---------------------------------------------------------------------------
 // passes over at least this many cells sum on the integer pipes (the FP64 pipe bounds them;
-// smaller ones are latency, as on the single level)
-inline bool on_int(long long cells) { return cells >= (1LL << 20); }
+// smaller ones are latency, as on the single level): a zoom step on base 80^3 7.87 ms with 2^20,
+// 7.71 with 2^17, on 96^3 10.12 and 9.91, on 64^3 5.29 and 5.21
+inline bool on_int(long long cells) { return cells >= (1LL << 17); }
 
 nyxpm_status ghost_fill(Ctx& c, nyxpm_amr& A, double* f, const Range& r)
 {
