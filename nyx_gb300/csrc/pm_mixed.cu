@@ -719,8 +719,9 @@ __global__ void k_mx_correct(int n, float c_hi, float c_lo, const float* __restr
 
 // k_mx_correct with two compact cells of each colour per thread (8- and 16-byte
 // accesses) for rows of an even number of compact cells; every cell's update is
-// k_mx_correct's, term for term.
-__global__ void k_mx_correct2(int n, float c_hi, float c_lo, const float* __restrict__ e_r,
+// k_mx_correct's, term for term.  Bound by HBM (36 bytes a cell); six blocks an SM asked for:
+// 124 -> 113 us at 256^3.
+__global__ void __launch_bounds__(256, 6) k_mx_correct2(int n, float c_hi, float c_lo, const float* __restrict__ e_r,
                               const float* __restrict__ e_b, double* phi_r, double* phi_b,
                               float* r_r, float* r_b, float* rl_r, float* rl_b,
                               unsigned long long* norm, unsigned long long* enorm)
@@ -1047,7 +1048,7 @@ __device__ __forceinline__ void fine_row_resid(const LevelViewF& F, int j, int k
 // The restriction after pre-smoothing: the coarse right-hand side from the red
 // children only (the black ones' residuals are round-off), summed in (dk, dj)
 // order; half the loads of k_restrict_f4.
-__global__ void __launch_bounds__(256) k_restrict_f4_red(LevelViewF F, LevelViewF Cv, int open)
+__global__ void __launch_bounds__(256, 6) k_restrict_f4_red(LevelViewF F, LevelViewF Cv, int open)
 {
     pdl_wait();
     pdl_trigger();
