@@ -865,7 +865,9 @@ __global__ void k_beta_from_natural(LevelView L, const double* __restrict__ in, 
 // Levels of at least this edge work by pairs of cells, their sums on the integer pipes
 // (pm_sum6.cuh): there the FP64 pipe is the bound (four steps at 96^3 12.3 -> 11.5 ms, at 112^3
 // 18.3 -> 17.1).  Below, a half sweep is latency: with integer sums on level 64 four 64^3 steps take
-// 7.24 ms against 7.10, on level 80 four 160^3 steps 31.1 against 30.5.
+// 7.24 ms against 7.10, on level 80 four 160^3 steps 31.1 against 30.5.  Their half sweeps and
+// restrictions go by blocks of 128 threads, whose four warps are one on the FP64 pipe and three on the
+// integer pipes (256^3: 101.5 ms with 256 threads, 100.2; with 64 106.6).
 constexpr int kPairMinEdge = 96;
 inline bool by_pairs(const Level& l) { return l.split && l.n >= kPairMinEdge && l.n % 4 == 0; }
 
@@ -873,7 +875,7 @@ nyxpm_status gsrb_sweep(Ctx& c, const Level& l, int fine, int black_only = 0)
 {
     const long long half_cells = (long long)l.n * l.n * l.n / 2;
     const bool pairs = by_pairs(l);
-    const Geo g = geo3(pairs ? l.n / 4 : l.n / 2, l.n, l.n);
+    const Geo g = geo3(pairs ? l.n / 4 : l.n / 2, l.n, l.n, pairs ? 128 : 256);
     for (int color = black_only ? 1 : 0; color < 2; ++color) {
         double* mine = color ? l.phi_b : l.phi_r;
         const double* other = color ? l.phi_r : l.phi_b;
@@ -966,7 +968,7 @@ nyxpm_status vcycle(Ctx& c, Box& b, size_t li, int red_done = 0)
     const int open = nu1 > 0 && li + 2 < b.levels.size() && !tail_fits_d(c, b, li + 1) && !cluster_fits_d(c, b, li + 1, ca);
     {
         const bool pairs = c.p.nu1 > 0 && by_pairs(f);
-        const Geo g = geo3(pairs ? cl.n / 2 : cl.n, cl.n, cl.n);
+        const Geo g = geo3(pairs ? cl.n / 2 : cl.n, cl.n, cl.n, pairs ? 128 : 256);
         prof_begin(c);
         if (c.p.nu1 > 0)
             launch_pdl(c, pairs ? k_restrict_red2 : k_restrict<1>, dim3(g.grid), dim3(g.block), view(f), view(cl), open);
