@@ -1689,13 +1689,7 @@ nyxpm_status nyxpm_amr_upload(nyxpm_ctx* c, nyxpm_amr* a, const double* pos, con
     const nyxpm_status sent = check_launch(*c, "hierarchy upload");
     double total = mass_scalar * (double)a->np;
     bool bad_mass = !mass && (!(mass_scalar >= 0) || !std::isfinite(mass_scalar));
-    if (mass) {
-        total = 0.0;
-        for (int64_t p = 0; p < a->np; ++p) {
-            bad_mass = bad_mass || !(mass[p] >= 0) || !std::isfinite(mass[p]);
-            total = total + mass[p];
-        }
-    }
+    if (mass) bad_mass = !sum_masses(mass, a->np, total);
     if (sent != NYXPM_OK) {
         cudaStreamSynchronize(c->stream);   // the caller's arrays are the caller's again
         return sent;

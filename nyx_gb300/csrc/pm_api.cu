@@ -529,13 +529,7 @@ nyxpm_status nyxpm_box_upload(nyxpm_ctx* c, nyxpm_box* b, const double* pos, con
         double* dm = b->staging + 6 * np;
         cudaMemcpyAsync(dm, mass, sizeof(double) * np, cudaMemcpyHostToDevice, c->stream);
         d_mass = dm;
-        bool ok = true;
-        total = 0.0;
-        for (int64_t q = 0; q < np; ++q) {
-            ok = ok && mass[q] >= 0 && std::isfinite(mass[q]);
-            total = total + mass[q];
-        }
-        if (!ok) {
+        if (!sum_masses(mass, np, total)) {
             cudaStreamSynchronize(c->stream);   // the caller's arrays are the caller's again
             return fail(c, NYXPM_INVALID_ARG, "bad mass");
         }
@@ -762,10 +756,7 @@ nyxpm_status nyxpm_step_host(nyxpm_ctx* c, nyxpm_box* b, double* pos, double* ve
     const int64_t np = b->np;
     double total = 0.0;
     if (mass) {
-        for (int64_t q = 0; q < np; ++q) {
-            if (!(mass[q] >= 0) || !std::isfinite(mass[q])) return fail(c, NYXPM_INVALID_ARG, "bad mass");
-            total = total + mass[q];
-        }
+        if (!sum_masses(mass, np, total)) return fail(c, NYXPM_INVALID_ARG, "bad mass");
     } else {
         if (!(mass_scalar >= 0) || !std::isfinite(mass_scalar)) return fail(c, NYXPM_INVALID_ARG, "bad mass");
         total = mass_scalar * (double)np;

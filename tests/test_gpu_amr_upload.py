@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from nyx_gb300.amr import AmrHierarchy
-from nyx_gb300.pm import Context, NyxPMError
+from nyx_gb300.pm import Box, Context, NyxPMError
 from tests.conftest import gpu_available
 
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="no GPU")]
@@ -44,3 +44,17 @@ def test_refused_upload_names_the_first_fault_and_keeps_the_particles(np_):
     np.testing.assert_array_equal(v, vel)
     H.upload(pos, vel * 3, 2.0)
     np.testing.assert_array_equal(H.download()[1], vel * 3)
+
+
+def test_masses_of_minus_zero_pass_and_others_out_of_range_do_not():
+    """sum_masses: -0 is not negative; the largest number is finite (FP64 box and hierarchy)."""
+    ctx = Context()
+    rng = np.random.default_rng(3)
+    pos, vel = rng.random((512, 3)), np.zeros((512, 3))
+    box, H = Box(ctx, 8, 1.0, 512), AmrHierarchy(ctx, 8, 1.0, [], 512)
+    for up in (box.upload, H.upload):
+        for good in (-0.0, 0.0, 5e-324, 1.7e308):
+            up(pos, vel, np.where(np.arange(512) == 300, good, 0.0))
+        for bad in (-5e-324, -1.0, -np.inf, np.inf, np.nan, -np.nan):
+            with pytest.raises(NyxPMError, match="bad mass"):
+                up(pos, vel, np.where(np.arange(512) == 300, bad, 1.0))
