@@ -1,7 +1,7 @@
 // V-cycles of small levels by one cluster of 16 CTAs, every level in shared memory.
 //
-// Why.  Below 64^3 (FP32) or 32^3 (FP64) a pass over a level is a few thousand cells:
-// as a launch of its own it takes 2 to 4 us, nearly all of it launch and memory latency,
+// Why.  On small levels a pass is a few thousand cells: as a launch of its own it takes 1.5
+// to 4 us, nearly all of it launch and memory latency,
 // and a V(2,2) cycle has ten passes per level.  One CTA is too slow for these levels,
 // and a cluster that passes its values through L2 as well.  Here the levels of a V-cycle
 // stay in the CTAs' shared memory: a level is cut into slabs of whole z planes, the CTA
@@ -13,8 +13,8 @@
 // Measured on GB300 (SM clocks): a cluster barrier 526; a half sweep of 64^3 in FP32
 // 2800 and of 32^3 in FP64 3800, against 2.3 us and 2.2 us (4700 and 4500 clocks) of a
 // launch.  Whole solves from phi = 0: FP64 32^3 0.83 -> 0.55 ms, FP32 32^3 0.63 -> 0.28,
-// 64^3 0.80 -> 0.59 ms.  The limits on the edge: FP32 64^3 is what 16 CTAs' shared memory
-// holds; FP64 issues at 19 clocks per warp instruction and SM, so that 16 SMs smooth 48^3
+// 64^3 0.80 -> 0.59 ms.  Since then the launches overlap and fit the row, and the edges were
+// measured again (cluster_fits_f, cluster_fits_d).  FP64 issues at 19 clocks per warp instruction and SM, so that 16 SMs smooth 48^3
 // in 6 us, twice a launch over the whole chip.  (Integer sums, pm_sum6.cuh, lose here: on
 // coarse levels some lane of a warp nearly always needs the FP64 additions as well, a
 // 32^3 solve took 0.64 ms.)
@@ -36,7 +36,7 @@ constexpr int kClCtas = 16;         // CTAs of the cluster
 constexpr int kClThreads = 512;   // a cluster barrier of 16 x 512 threads takes 526 cycles, of 16 x 1024 682
 constexpr int kClMaxPlanes = 4;     // planes of a level a CTA owns at most
 constexpr int kClMaxLevels = 4;     // levels in slabs
-constexpr int kClEdgeF = 64;        // largest level taken, FP32 and FP64
+constexpr int kClEdgeF = 48;        // largest level taken, FP32 and FP64 (whole boxes; see cluster_fits_f, _d)
 constexpr int kClEdgeD = 32;
 constexpr int kClSoloF = 16;        // levels up to this edge belong to one CTA
 constexpr int kClSoloD = 8;

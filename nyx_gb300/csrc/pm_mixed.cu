@@ -1581,11 +1581,11 @@ nyxpm_status vcycle_tail_f(Ctx& c, Box& b, size_t li)
 // finest level from 32^3 down (four steps at 128^3 8.28 ms with level 64 in the cluster, 7.50
 // without, 8.60 with level 32 out too; at 112^3 8.87 with level 56, 7.92 without), whole boxes
 // of up to 48^3 (3.35 ms against 3.47 by launches; at 64^3 4.08 against 3.83)
-constexpr int kClusterEdgeF = 32, kClusterSolveEdgeF = 48;
+constexpr int kClusterEdgeF = 32;   // (whole boxes: kClEdgeF)
 
 bool cluster_fits_f(Ctx& c, const Box& b, size_t li, ClArgs<float>& A)
 {
-    if (b.levels[li].n > (li > 0 ? kClusterEdgeF : kClusterSolveEdgeF)) return false;
+    if (li > 0 && b.levels[li].n > kClusterEdgeF) return false;
     if (!cl_args<float>(c, b, li, A)) return false;
     if (c.cluster_f < 0)
         c.cluster_f = cl_prepare(k_cluster_vcycle_f, cl_max_bytes<float>()) &&

@@ -902,11 +902,11 @@ bool tail_fits_d(const Ctx& c, const Box& b, size_t li)
 // as a launch takes all of them and its launch (four steps at 64^3 7.48 ms with level 32 in the
 // cluster, 7.19 without; 7.8 with level 16 out too).  A box of up to 32^3 is solved in one
 // launch (3.64 ms; its V-cycles by launches down to 16^3 3.82).
-constexpr int kClusterEdgeD = 16, kClusterSolveEdgeD = 32;
+constexpr int kClusterEdgeD = 16;   // (whole boxes: kClEdgeD)
 
 bool cluster_fits_d(Ctx& c, const Box& b, size_t li, ClArgs<double>& A)
 {
-    if (b.levels[li].n > (li > 0 ? kClusterEdgeD : kClusterSolveEdgeD)) return false;
+    if (li > 0 && b.levels[li].n > kClusterEdgeD) return false;
     if (!cl_args<double>(c, b, li, A)) return false;
     if (c.cluster_d < 0) {
         const size_t most = cl_max_bytes<double>();
