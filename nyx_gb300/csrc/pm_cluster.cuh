@@ -593,9 +593,9 @@ inline bool cl_args(const Ctx& c, const Box& b, size_t li, ClArgs<T>& A)
     return true;
 }
 
-// host: whether a kernel can run here as one cluster with that much shared memory
+// host: whether a kernel can run here as one cluster with that much dynamic shared memory
 template <typename K>
-inline bool cl_prepare(K kernel, size_t bytes)
+inline bool cl_prepare(K kernel, size_t bytes, int threads = kClThreads)
 {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
@@ -608,7 +608,7 @@ inline bool cl_prepare(K kernel, size_t bytes)
     at[0].val.clusterDim.x = kClCtas;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(kClCtas);
-    cfg.blockDim = dim3(kClThreads);
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = bytes;
     cfg.attrs = at;
     cfg.numAttrs = 1;

@@ -37,9 +37,10 @@ constexpr int kNaScanT = 512, kNaScanIPT = 8, kNaScanTile = kNaScanT * kNaScanIP
 constexpr long long kNaTiles = (kNaMaxCells + kNaScanTile - 1) / kNaScanTile;
 
 // Up to this many particles and cells the sort is one cluster launch (na_sort), beyond it
-// ten launches over the whole chip.  Measured, a call from the host, particles on a
-// lattice: 8^3 77 -> 40 us, 32^3 95 -> 61 us, 48^3 112 -> 87 us; 64^3 with 262,144 particles 134 us by launches,
-// 136 by the cluster, 155 before the deposit below.
+// and where the device or the stream cannot place that cluster ten launches over the whole
+// chip.  Measured, a call from the host, particles on a lattice: 8^3 77 -> 40 us, 32^3
+// 95 -> 61 us, 48^3 112 -> 87 us; 64^3 with 262,144 particles 134 us by launches, 136 by the
+// cluster, 155 before the deposit below.
 constexpr long long kNaClusterMax = 131072;
 // scratch layout, each part rounded up to 256 bytes
 constexpr size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -63,17 +64,20 @@ __global__ void na_sort(int np, int n, double dxi, const double* __restrict__ x,
                         const double* __restrict__ z, int* key, int* count, int* start, int* perm, int* long_list,
                         int* long_count, int* bad);
 
+constexpr int kNaThreads = 1024;   // of a CTA of the cluster sort
+
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 unsigned char* g_scratch_addr[kMaxDevices] = {};
 int g_sm_count[kMaxDevices] = {};
+int g_cluster[kMaxDevices] = {};   // the device can place the cluster sort: 1 yes, -1 no, 0 not asked yet
 
 // The device address of the scratch on the current device (the host-side name
 // of the array is not a device address).  It is looked up again on every call
 // whose stream is not capturing -- a device reset reloads the module and may
 // move the array -- and the last address found is used while a capture runs.
-nyxpm_status scratch_address(cudaStream_t stream, unsigned char** out, int* sm_count, bool* capturing,
-                             char* errbuf, size_t errlen)
+nyxpm_status scratch_address(cudaStream_t stream, unsigned char** out, int* sm_count, bool* cluster,
+                             bool* capturing, char* errbuf, size_t errlen)
 {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
@@ -104,11 +108,14 @@ nyxpm_status scratch_address(cudaStream_t stream, unsigned char** out, int* sm_c
             sms = 1;
         }
         g_sm_count[dev] = sms > 0 ? sms : 1;
-        if (cudaFuncSetAttribute(na_sort, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-            cudaGetLastError();   // the launch reports it
+        if (!g_cluster[dev])
+            g_cluster[dev] = cl_prepare(na_sort, 0, kNaThreads) ? 1 : -1;
+        else if (cudaFuncSetAttribute(na_sort, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            cudaGetLastError();   // (a device reset forgets it) the launch reports it
     }
     *out = g_scratch_addr[dev];
     *sm_count = g_sm_count[dev];
+    *cluster = g_cluster[dev] > 0;
     *capturing = cap != cudaStreamCaptureStatusNone;
     return NYXPM_OK;
 }
@@ -322,7 +329,6 @@ __device__ __forceinline__ void na_add_weights(int q, int n, double dxi,
 // for a few microseconds of work.  The particles are not permuted: the deposit reads them
 // through perm.  Same keys, counts and order as the kernels above.
 // ---------------------------------------------------------------------------
-constexpr int kNaThreads = 1024;
 constexpr int kNaSeg = 512;   // longer segments are ranked by a block
 
 // Corner sums of the keys longer than a warp, a warp each: lane l sums particles l, l + 32,
@@ -579,8 +585,8 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
     unsigned char* base = nullptr;
     int sm_count = 1;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    bool capturing = false;
-    const nyxpm_status st = scratch_address(s, &base, &sm_count, &capturing, errbuf, errlen);
+    bool cluster = false, capturing = false;
+    const nyxpm_status st = scratch_address(s, &base, &sm_count, &cluster, &capturing, errbuf, errlen);
     if (st != NYXPM_OK) return st;
     int* count = reinterpret_cast<int*>(base + kOffCount);
     int* start = reinterpret_cast<int*>(base + kOffStart);
@@ -600,10 +606,11 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
     const unsigned pb = (unsigned)((np + 255) / 256);
     const unsigned cb = (unsigned)((nc + 255) / 256);
     const dim3 grid((n + kTx - 1) / kTx, (n + kTy - 1) / kTy, (n + kTz - 1) / kTz);
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
-    if (np <= kNaClusterMax && nc <= kNaClusterMax) {
+    bool sorted = false;
+    if (cluster && np <= kNaClusterMax && nc <= kNaClusterMax) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = kClCtas;
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
@@ -612,16 +619,17 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
         cfg.stream = s;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, na_sort, (int)np, n, dxi, d_x, d_y, d_z, key, count, start, perm, long_list,
-                               long_count, bad);
-        if (e == cudaSuccess) {
-            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.gridDim = grid;
-            cfg.blockDim = dim3(256);
-            e = cudaLaunchKernelEx(&cfg, na_deposit, n, dxi, scale, d_x, d_y, d_z,
-                                   (const int*)perm, (const int*)start, (const int*)count, (const double*)key, d_rho);
-        }
+        sorted = cudaLaunchKernelEx(&cfg, na_sort, (int)np, n, dxi, d_x, d_y, d_z, key, count, start, perm, long_list,
+                                    long_count, bad) == cudaSuccess;
+        if (!sorted) cudaGetLastError();   // this stream cannot place it (an SM partition, say): by launches
+    }
+    if (sorted) {
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(256);
+        e = cudaLaunchKernelEx(&cfg, na_deposit, n, dxi, scale, d_x, d_y, d_z, (const int*)perm, (const int*)start,
+                               (const int*)count, (const double*)key, d_rho);
     } else {
         const int ntiles = (nc + kNaScanTile - 1) / kNaScanTile;
         // the counts, the long-segment counter and the non-finite count must start at
@@ -637,9 +645,7 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
         na_fix_long<<<2 * sm_count, 512, 0, s>>>(start, long_list, long_count, perm, key);
         na_gather<<<pb, 256, 0, s>>>(np, perm, d_x, d_y, d_z, xs, ys, zs);
         na_heavy<<<4 * sm_count, 256, 0, s>>>(n, dxi, xs, ys, zs, start, long_list, long_count, count, (double*)key);
-        na_deposit<<<grid, 256, 0, s>>>(n, dxi, scale, xs, ys, zs, nullptr, start, count,
-                                                                   (const double*)key, d_rho);
-        e = cudaSuccess;
+        na_deposit<<<grid, 256, 0, s>>>(n, dxi, scale, xs, ys, zs, nullptr, start, count, (const double*)key, d_rho);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     else cudaGetLastError();
