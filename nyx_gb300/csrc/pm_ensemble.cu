@@ -2935,13 +2935,28 @@ nyxpm_status nyxpm_ensemble_remove(nyxpm_ctx* c, nyxpm_ensemble* E, int slot)
 
 size_t nyxpm_ensemble_arena_used(const nyxpm_ensemble* E) { return E ? E->arena.used_bytes() : 0; }
 
-// Particles in and out are converted on the device.  The caller's arrays pass through
-// the box's FP64 right-hand side in pieces (8 bytes a cell in two arrays, rewritten by
-// every solve), so neither needs arena space beyond the box itself: positions of n^3 / 6
-// particles in the red array, their velocities in the black one.  Measured: sixteen boxes
-// of 9.8 M particles in, ten steps and out, 187 ms with the conversion on one host thread
-// and 73 ms so (the steps take 50).
-static long long piece_of(const EDesc& d) { return std::max<long long>(1, (long long)d.n * d.n * d.n / 6); }
+// Particles in and out are converted on the device.  The caller's arrays pass in pieces
+// through memory of the box that holds nothing between calls, so neither needs arena space
+// beyond the box itself: up to a particle per cell through the FP64 right-hand side (rewritten
+// by every solve), positions of n^3 / 6 particles in the red array and their velocities in the
+// black one; above, through the particle buffer that is not current (rewritten by every sort),
+// np / 6 in its x offsets and its x velocities.  So there are six or seven pieces at most from
+// a particle per cell on: a download looks through all ids for each piece, an upload pays two
+// copies.  Measured: sixteen boxes of 9.8 M particles in, ten steps and out, 187 ms with the
+// conversion on one host thread and 73 ms so (the steps take 50); a million particles on 16^3
+// in and out, 12.1 and 43.8 ms in 1466 pieces of n^3 / 6.
+struct Pieces {
+    long long count;     // particles of a piece
+    double *pos, *vel;   // where they pass, 3 count values each
+};
+
+static Pieces pieces_of(const EDesc& d, int parity)
+{
+    const long long nc = (long long)d.n * d.n * d.n;
+    if (d.np <= nc) return Pieces{nc / 6, d.beta_r, d.beta_b};
+    const PArr P = parr(d, parity ^ 1);
+    return Pieces{d.np / 6, reinterpret_cast<double*>(P.ox), reinterpret_cast<double*>(P.vx)};
+}
 
 nyxpm_status nyxpm_ensemble_upload(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, const double* pos,
                                    const double* vel, double mass)
@@ -2951,14 +2966,15 @@ nyxpm_status nyxpm_ensemble_upload(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, co
     if (E->dirty) ETRY(rebuild(c, E));
     EnsSlot& s = E->slots[slot];
     EDesc& d = s.desc;
-    const long long np = d.np, piece = piece_of(d);
+    const long long np = d.np;
+    const Pieces by = pieces_of(d, 0);
     cudaMemsetAsync(d.norms + 2, 0, sizeof(unsigned long long), c->stream);
-    for (long long q0 = 0; q0 < np; q0 += piece) {
-        const long long m = std::min(piece, np - q0);
-        cudaMemcpyAsync(d.beta_r, pos + 3 * q0, 24 * m, cudaMemcpyHostToDevice, c->stream);
-        cudaMemcpyAsync(d.beta_b, vel + 3 * q0, 24 * m, cudaMemcpyHostToDevice, c->stream);
-        e_unpack<<<(unsigned)((m + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, d.beta_r, d.beta_b, d.n, d.dxi,
-                                                                         parr(d, 0), d.norms + 2);
+    for (long long q0 = 0; q0 < np; q0 += by.count) {
+        const long long m = std::min(by.count, np - q0);
+        cudaMemcpyAsync(by.pos, pos + 3 * q0, 24 * m, cudaMemcpyHostToDevice, c->stream);
+        cudaMemcpyAsync(by.vel, vel + 3 * q0, 24 * m, cudaMemcpyHostToDevice, c->stream);
+        e_unpack<<<(unsigned)((m + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, by.pos, by.vel, d.n, d.dxi, parr(d, 0),
+                                                                         d.norms + 2);
     }
     ETRY(echeck(c, "ensemble upload"));
     unsigned long long bad = 0;
@@ -2986,16 +3002,18 @@ nyxpm_status nyxpm_ensemble_download(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, 
     if (!E->slots[slot].uploaded) return efail(c, NYXPM_INVALID_ARG, "slot has no particles");
     ETRY(pull_state(c, E));
     const EDesc& d = E->slots[slot].desc;
-    const long long np = d.np, piece = piece_of(d);
+    const long long np = d.np;
+    const int parity = E->h_state[slot].parity;
+    const Pieces by = pieces_of(d, parity);
     touch_pages(pos, 24 * np);
     touch_pages(vel, 24 * np);
     cudaMemsetAsync(d.norms + 2, 0, sizeof(unsigned long long), c->stream);
-    for (long long q0 = 0; q0 < np; q0 += piece) {
-        const long long m = std::min(piece, np - q0);
-        e_pack<<<(unsigned)((np + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, np, d.dx, parr(d, E->h_state[slot].parity),
-                                                                        d.beta_r, d.beta_b, d.norms + 2);
-        cudaMemcpyAsync(pos + 3 * q0, d.beta_r, 24 * m, cudaMemcpyDeviceToHost, c->stream);
-        cudaMemcpyAsync(vel + 3 * q0, d.beta_b, 24 * m, cudaMemcpyDeviceToHost, c->stream);
+    for (long long q0 = 0; q0 < np; q0 += by.count) {
+        const long long m = std::min(by.count, np - q0);
+        e_pack<<<(unsigned)((np + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, np, d.dx, parr(d, parity), by.pos, by.vel,
+                                                                        d.norms + 2);
+        cudaMemcpyAsync(pos + 3 * q0, by.pos, 24 * m, cudaMemcpyDeviceToHost, c->stream);
+        cudaMemcpyAsync(vel + 3 * q0, by.vel, 24 * m, cudaMemcpyDeviceToHost, c->stream);
     }
     ETRY(echeck(c, "ensemble download"));
     unsigned long long bad = 0;
