@@ -18,50 +18,12 @@
 #include <cstring>
 #include <functional>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/nyxpm.h"
-
-#include <unistd.h>
+#include "pm_pages.h"
 
 namespace nyxpm {
-
-// One write to every page of a host buffer that a device-to-host copy will fill.  On a
-// host whose page tables the GPU shares, a copy into pages the process has not touched
-// yet takes a GPU page fault for each (measured 1.4 to 25 GB/s against 190 GB/s into
-// touched pages); one host thread faults them in at 30 to 40 GB/s, four a buffer of 50 MB
-// at 96 GB/s (8 MB: 59 against 42, less than the threads are worth).
-inline void touch_range(volatile char* c, size_t bytes, size_t page)
-{
-    for (size_t o = 0; o < bytes; o += page) c[o] = 0;
-    if (bytes) c[bytes - 1] = 0;
-}
-
-inline void touch_pages(void* p, size_t bytes)
-{
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    volatile char* c = static_cast<volatile char*>(p);
-    constexpr int kThreads = 4;
-    size_t done = 0;
-    if (bytes >= ((size_t)16 << 20)) {
-        const size_t part = bytes / kThreads;
-        std::thread t[kThreads - 1];
-        try {
-            for (std::thread& x : t) {
-                x = std::thread(touch_range, c + done, part, page);
-                done += part;
-            }
-        } catch (const std::system_error&) {   // no more threads: the rest here
-        }
-        touch_range(c + done, bytes - done, page);
-        for (std::thread& x : t)
-            if (x.joinable()) x.join();
-        return;
-    }
-    touch_range(c, bytes, page);
-}
 
 constexpr int kMaxBottom = 8;          // largest coarsest-grid edge (solved exactly)
 // A deposit key with more particles than this is summed by a whole warp in

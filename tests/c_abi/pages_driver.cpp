@@ -1,0 +1,76 @@
+// What touch_pages (pm_pages.h) does to a buffer: its pages are there afterwards, its bytes
+// are as they were, and an address that cannot be written is left alone.
+#include "pm_pages.h"
+
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#define CHECK(x) \
+    do { \
+        if (!(x)) { \
+            std::printf("line %d: %s\n", __LINE__, #x); \
+            std::exit(1); \
+        } \
+    } while (0)
+
+static const size_t kPage = (size_t)sysconf(_SC_PAGESIZE);
+
+static char* map(size_t bytes, int prot)
+{
+    void* p = mmap(nullptr, bytes, prot, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    CHECK(p != MAP_FAILED);
+    return static_cast<char*>(p);
+}
+
+static size_t present(char* p, size_t bytes)
+{
+    std::vector<unsigned char> v(bytes / kPage);
+    CHECK(mincore(p, bytes, v.data()) == 0);
+    size_t n = 0;
+    for (unsigned char c : v) n += c & 1;
+    return n;
+}
+
+static unsigned char at(size_t i) { return (unsigned char)(i * 131 + (i >> 12) * 7 + 1); }
+
+// bytes of [off, off + len) of a mapping half of whose pages hold data
+static void keeps(size_t bytes, size_t off, size_t len)
+{
+    char* p = map(bytes, PROT_READ | PROT_WRITE);
+    for (size_t i = 0; i < bytes; ++i)
+        if (i / kPage % 2) p[i] = (char)at(i);
+    nyxpm::touch_pages(p + off, len);
+    const size_t a = off / kPage * kPage, e = (off + len + kPage - 1) / kPage * kPage;
+    CHECK(present(p + a, e - a) == (e - a) / kPage);
+    for (size_t i = 0; i < bytes; ++i) CHECK((unsigned char)p[i] == (i / kPage % 2 ? at(i) : 0));
+    munmap(p, bytes);
+}
+
+int main(int argc, char** argv)
+{
+    const size_t M = (size_t)1 << 20;
+    const char* what = argc > 1 ? argv[1] : "";
+    if (!std::strcmp(what, "keeps")) {
+        for (size_t len : {(size_t)1, kPage - 1, kPage, kPage + 1, 3 * M + 17, 20 * M + 5, 150 * M + 9})
+            for (size_t off : {(size_t)0, (size_t)8, kPage - 8}) keeps((len + 3 * kPage) / kPage * kPage, off, len);
+    } else if (!std::strcmp(what, "refused")) {
+        for (int prot : {PROT_NONE, PROT_READ}) {
+            char* p = map(40 * M, prot);
+            nyxpm::touch_pages(p + 100, 40 * M - 200);
+            munmap(p, 40 * M);
+            nyxpm::touch_pages(p + 100, 40 * M - 200);   // nothing there any more
+        }
+        char* p = map(40 * M, PROT_READ | PROT_WRITE);
+        CHECK(munmap(p + 20 * M, 10 * M) == 0);   // a hole
+        nyxpm::touch_pages(p, 40 * M);
+        CHECK(present(p, 20 * M) * kPage == 20 * M);
+        nyxpm::touch_pages(nullptr, 1);
+        nyxpm::touch_pages(p, 0);
+    } else {
+        return 2;
+    }
+    std::printf("ok\n");
+    return 0;
+}
