@@ -18,7 +18,6 @@
 
 #include <cstddef>
 #include <cstdint>
-#include <system_error>
 #include <thread>
 
 #include <sys/mman.h>
@@ -77,7 +76,7 @@ inline void touch_pages(void* p, size_t bytes)
                 t[k] = std::thread(missing_pages, at, at + part, page, true);
                 at += part;
             }
-        } catch (const std::system_error&) {   // no more threads: the rest here
+        } catch (...) {   // no more threads, or no memory for one: the rest here
         }
     }
     missing_pages(at, end, page, true);

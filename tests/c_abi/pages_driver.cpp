@@ -1,11 +1,37 @@
 // What touch_pages (pm_pages.h) does to a buffer: its pages are there afterwards, its bytes
-// are as they were, and an address that cannot be written is left alone.
+// are as they were, an address that cannot be written is left alone, and neither memory nor
+// threads that cannot be had end the process.
 #include "pm_pages.h"
 
+#include <cerrno>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <vector>
+
+#include <dlfcn.h>
+#include <pthread.h>
+
+// the n-th thread from now on, or the memory it takes, cannot be had (-1: all can)
+static int memory_after = -1, threads_after = -1;
+
+void* operator new(size_t n)
+{
+    if (memory_after >= 0 && memory_after-- == 0) throw std::bad_alloc();
+    if (void* p = std::malloc(n)) return p;
+    throw std::bad_alloc();
+}
+
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x)
+{
+    using Create = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+    static Create create = reinterpret_cast<Create>(dlsym(RTLD_NEXT, "pthread_create"));
+    return threads_after >= 0 && threads_after-- == 0 ? EAGAIN : create(t, a, f, x);
+}
 
 #define CHECK(x) \
     do { \
@@ -68,6 +94,17 @@ int main(int argc, char** argv)
         CHECK(present(p, 20 * M) * kPage == 20 * M);
         nyxpm::touch_pages(nullptr, 1);
         nyxpm::touch_pages(p, 0);
+    } else if (!std::strcmp(what, "memory") || !std::strcmp(what, "threads")) {
+        for (int after = 0; after < 4; ++after) {
+            char* p = map(200 * M, PROT_READ | PROT_WRITE);
+            int& left = what[0] == 'm' ? memory_after : threads_after;
+            left = after;
+            nyxpm::touch_pages(p, 200 * M);
+            CHECK((left == -1) == (after < 3));   // three threads beside the caller's
+            left = -1;
+            CHECK(present(p, 200 * M) * kPage == 200 * M);
+            munmap(p, 200 * M);
+        }
     } else {
         return 2;
     }

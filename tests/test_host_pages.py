@@ -13,8 +13,10 @@ from tests.conftest import REPO
 @pytest.fixture(scope="module")
 def driver(tmp_path_factory):
     exe = tmp_path_factory.mktemp("pages") / "pages_driver"
-    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-rdynamic", f"-I{os.path.join(REPO, 'nyx_gb300', 'csrc')}",
-                    os.path.join(REPO, "tests", "c_abi", "pages_driver.cpp"), "-o", str(exe), "-lpthread"], check=True)
+    src = os.path.join(REPO, "tests", "c_abi", "pages_driver.cpp")
+    include = os.path.join(REPO, "nyx_gb300", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-Wall", "-rdynamic", f"-I{include}", src, "-o", str(exe),
+                    "-lpthread", "-ldl"], check=True)
 
     def run(what):
         r = subprocess.run([str(exe), what], capture_output=True, text=True, timeout=120)
@@ -24,4 +26,9 @@ def driver(tmp_path_factory):
 
 @pytest.mark.parametrize("what", ["keeps", "refused"])
 def test_pages_come_in_and_nothing_is_written(driver, what):
+    assert driver(what) == (0, "ok\n")
+
+
+@pytest.mark.parametrize("what", ["memory", "threads"])
+def test_threads_that_cannot_be_had(driver, what):
     assert driver(what) == (0, "ok\n")
