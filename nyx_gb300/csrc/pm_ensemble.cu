@@ -1730,13 +1730,19 @@ __global__ void __launch_bounds__(256, 4) e_prolong4_black(const Item* __restric
 
 // The coarse end of every box's V-cycle (levels tail_l .. bottom), one CTA per box: the
 // per-pass kernels' arithmetic (pm_tail.cuh), so the same bits.  Levels of up to 16^3
-// with pre- and post-smoothing are cycled in shared memory (vcycle_solo).
-constexpr int kETailThreads = 512;
+// with pre- and post-smoothing are cycled in shared memory (vcycle_solo), bound by latency:
+// 512 threads.  Others go through global memory (vcycle_tail); where mg_fused_edge lets in
+// larger ones they want more loads in flight: eight boxes of 32^3 to 128^3 with levels of up
+// to 32^3 here 4.06 ms a step with 512 threads, 3.83 with 1024 (without pre-smoothing 4.38 and
+// 4.16); at 16^3 without pre- or post-smoothing both widths take the same time.
+constexpr int kETailThreads = 512, kETailWide = kTailThreads;
+constexpr int kETailSolo = 16;
 constexpr int kETailLevels = 2 * (16 * 16 * 16 + 8 * 8 * 8 + 4 * 4 * 4);   // no level chain from 16 down holds more
 constexpr int kETailGreen = 7 * 7 * 7, kETailTmp = 16 * 16 * 16 / 2;
 
-__global__ void __launch_bounds__(kETailThreads) e_tail(int nbox, const EDesc* __restrict__ D,
-                                                        const EState* __restrict__ S, int nu1, int nu2)
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) e_tail(int nbox, const EDesc* __restrict__ D, const EState* __restrict__ S,
+                                                   int nu1, int nu2)
 {
     pdl_wait();
     pdl_trigger();
@@ -1748,7 +1754,7 @@ __global__ void __launch_bounds__(kETailThreads) e_tail(int nbox, const EDesc* _
     const EDesc& d = D[b];
     const int nl = d.nlev - d.tail_l;
     const ELevel& top = d.lv[d.tail_l];
-    if (top.split && top.n <= 16 && nu1 > 0 && nu2 > 0) {
+    if (top.split && top.n <= kETailSolo && nu1 > 0 && nu2 > 0) {
         const int half = top.n * top.n * top.n / 2;
         float *tmp = mem + kETailLevels, *g = tmp + kETailTmp;
         if (threadIdx.x == 0) {
@@ -2516,7 +2522,9 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
                 c->launches += 1;
             }
             ep_begin(c);
-            launch_pdl(*c, e_tail, dim3(nbox), dim3(kETailThreads), nbox, D, S, c->p.nu1, c->p.nu2);
+            const bool wide = c->p.mg_fused_edge > kETailSolo;
+            launch_pdl(*c, wide ? e_tail<kETailWide> : e_tail<kETailThreads>, dim3(nbox),
+                       dim3(wide ? kETailWide : kETailThreads), nbox, D, S, c->p.nu1, c->p.nu2);
             ep_end(c, NYXPM_ST_BOTTOM);
             c->launches += 1;
             for (int l = E->max_lev - 2; l >= 0; --l) {
