@@ -257,12 +257,13 @@ def fp64_adds_per_cell(n):
     return 1.25 if n >= 96 and n % 4 == 0 else 5.0
 
 
-def ncu_traffic():
-    """Per-launch DRAM bytes of the dominant kernels from the committed ncu summary."""
+def ncu_capture(kernel, n):
+    """The committed ncu figures of one kernel's launch at level edge n (DRAM bytes, FP64 pipe
+    activity); empty where none was taken at that size: what stays in the L2 depends on it."""
     p = os.path.join(REPO, "profiles", "ncu_traffic.json")
     if os.path.exists(p):
         with open(p) as f:
-            return json.load(f)
+            return json.load(f).get(kernel, {}).get(str(n), {})
     return {}
 
 
@@ -817,26 +818,24 @@ def run_ours(args):
                   for k, v in stages.items() if v["launches"]}
     dom = max(stages, key=lambda k: stages[k]["ms"])
     peak, peak_kind = measured_peaks()
-    traffic = ncu_traffic()
+    capture = {}
     if dom == "smooth" and prof["fine_smooth"]["launches"]:
         fs = prof["fine_smooth"]
         per_launch = fs["bytes"] / fs["launches"]
         avg_ms = fs["ms"] / fs["launches"]
-        kname = (f"{'k_gsrb2' if fp64_adds_per_cell(n) < 5 else 'k_gsrb'} (finest-level FP64 red-black half sweep)"
-                 if args.precision == "fp64" else
-                 "k_gsrb_f4 (finest-level FP32 red-black half sweep)")
-        tr = traffic.get("k_gsrb_fine") if args.precision == "fp64" else None
+        kernel = "k_gsrb_f4" if args.precision != "fp64" else "k_gsrb2" if fp64_adds_per_cell(n) < 5 else "k_gsrb"
+        kname = f"{kernel} (finest-level {'FP64' if args.precision == 'fp64' else 'FP32'} red-black half sweep)"
+        capture = ncu_capture(kernel, n)
     else:
         st = stages[dom]
         per_launch = st["bytes"] / max(st["launches"], 1)
         avg_ms = st["ms"] / max(st["launches"], 1)
         kname = dom
-        tr = traffic.get(dom)
     achieved = per_launch / (avg_ms * 1e6)
     hbm = {"achieved": round(achieved, 1), "peak": peak, "peak_source": peak_kind, "unit": "GB/s",
            "frac": round(achieved / peak, 4)}
     share = round(stages[dom]["ms"] / sum(v["ms"] for v in stages.values()), 3)
-    traffic_launch = tr * (n / traffic.get("n", n)) ** 3 if tr else None
+    traffic_launch = capture.get("dram_bytes")
     if args.precision == "fp64" and dom == "smooth" and prof["fine_smooth"]["launches"]:
         # the finest FP64 half sweep updates n^3/2 cells, 24 algorithmic bytes each, with 5
         # additions of the neighbour sum and one fused multiply-add.  From 96^3 on three
@@ -864,7 +863,7 @@ def run_ours(args):
                               "note": f"FMA = 2 flops: {adds + 2.0:g} FP64 flops per updated cell; peak = FMA chains"},
                     "hbm": hbm,
                     "algorithmic_bytes_per_launch": per_launch, "avg_launch_ms": avg_ms,
-                    "fp64_pipe_active_ncu": traffic.get("k_gsrb_fine_fp64_pipe_active"),
+                    "fp64_pipe_active_ncu": capture.get("fp64_pipe_active"),
                     "dominant_stage_share": share}
     else:
         roofline = dict(hbm, bound="hbm", kernel=kname, traffic=traffic_launch,
