@@ -840,7 +840,8 @@ __global__ void k_amr_absmaxf(long long n, int b0, int nb, const long long* __re
                               unsigned long long* out)
 {
     unsigned long long v = 0ULL;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const long long all = (long long)gridDim.x * blockDim.x;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += all) {
         int b;
         const long long q = fine_cell(boxes, pref, b0, nb, t, b);
         if (!(cov[q] & kCovered)) v = umax_bits(v, fabs(f[q]) * inv_scale[boxes[b].lev]);

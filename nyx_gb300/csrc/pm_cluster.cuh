@@ -165,12 +165,16 @@ __device__ __forceinline__ void cl_setup(const ClArgs<T>& A, ClShared<T>& S, T* 
             L.br[q] = cl_map(L.beta_r + o, c);
         }
     }
-    if ((int)threadIdx.x < A.ns) S.solo[threadIdx.x] = SoloLevel<T>{A.n[A.nd + threadIdx.x], mem + A.at[A.nd + threadIdx.x]};
+    if ((int)threadIdx.x < A.ns)
+        S.solo[threadIdx.x] = SoloLevel<T>{A.n[A.nd + threadIdx.x], mem + A.at[A.nd + threadIdx.x]};
     __syncthreads();
 }
 
 // t -> (x, y, plane)
-__device__ __forceinline__ void cl_split(int t, int nx, int ny, int& x, int& y, int& z) { tail_split3(t, nx, ny, x, y, z); }
+__device__ __forceinline__ void cl_split(int t, int nx, int ny, int& x, int& y, int& z)
+{
+    tail_split3(t, nx, ny, x, y, z);
+}
 
 // neighbour sum of the cell at column ih of row j of the own plane q (q = 1 is p0), from
 // the planes z of the other colour; odd: the cell's x is 2 ih + 1
@@ -440,7 +444,8 @@ __device__ __forceinline__ void cl_prolong4(const ClLevel<float>& F, const float
                 const float w[4] = {e.x, o.x, e.y, o.y};
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    const float side = odd ? (r == 3 ? z : w[r == 3 ? 3 : r + 1]) : (r == 0 ? z : w[r == 0 ? 0 : r - 1]);
+                    const float side = odd ? (r == 3 ? z : w[r == 3 ? 3 : r + 1])
+                                           : (r == 0 ? z : w[r == 0 ? 0 : r - 1]);
                     s[r] = fmaf(tail_prolong_w<float>(2 * a + 4 * b), w[r], s[r]);
                     s[r] = fmaf(tail_prolong_w<float>(1 + 2 * a + 4 * b), side, s[r]);
                 }

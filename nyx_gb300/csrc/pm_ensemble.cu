@@ -793,7 +793,8 @@ __global__ void __launch_bounds__(256) e_resid(const Item* __restrict__ items, i
                     const double r = beta[t] - fma(s, kSixth, -mine[t]);
                     const float h = f64_to_f32_rn(r);
                     (color ? d.lv[0].beta_b : d.lv[0].beta_r)[t] = h;
-                    if (low_words) d.r_lo[(color ? (long long)n * n * half : 0LL) + t] = f64_to_f32_rn(r - f32_to_f64(h));
+                    if (low_words)
+                        d.r_lo[(color ? (long long)n * n * half : 0LL) + t] = f64_to_f32_rn(r - f32_to_f64(h));
                     (color ? d.lv[0].phi_b : d.lv[0].phi_r)[t] = 0.f;
                     const unsigned long long u = absbits(r);
                     vmax = u > vmax ? u : vmax;
@@ -1729,7 +1730,9 @@ __global__ void __launch_bounds__(256, 4) e_prolong4_black(const Item* __restric
 }
 
 // The coarse end of every box's V-cycle (levels tail_l .. bottom), one CTA per box: the
-// per-pass kernels' arithmetic (pm_tail.cuh), so the same bits.  Levels of up to 16^3
+// per-pass kernels' arithmetic (pm_tail.cuh), so the same bits (but for e_restrict, which takes
+// all eight children of levels whose rows hold no multiple of four compact cells, and this
+// after pre-smoothing the four red ones: phi's constant differs then).  Levels of up to 16^3
 // with pre- and post-smoothing are cycled in shared memory (vcycle_solo), bound by latency:
 // 512 threads.  Others go through global memory (vcycle_tail); where mg_fused_edge lets in
 // larger ones they want more loads in flight: eight boxes of 32^3 to 128^3 with levels of up
@@ -1838,7 +1841,8 @@ __global__ void __launch_bounds__(256) e_grav_v(const Item* __restrict__ items, 
             const int j = it.c + (int)(task / half);
             const unsigned ih = task % half;
             const CellPair P = cell_pair(d.phi_r, d.phi_b, n, ih, j, k);
-            float4* out = reinterpret_cast<float4*>(d.g32) + 2 * (size_t)(((unsigned)j + (unsigned)n * (unsigned)k) * half + ih);
+            const unsigned t = ((unsigned)j + (unsigned)n * (unsigned)k) * half + ih;
+            float4* out = reinterpret_cast<float4*>(d.g32) + 2 * (size_t)t;
 #pragma unroll
             for (int o = 0; o < 2; ++o) {
                 const double* c = P.c + 6 * o;
@@ -2413,7 +2417,7 @@ void enqueue_solve_head(nyxpm_ctx* c, nyxpm_ensemble* E)
     ep_begin(c);
     launch_pdl(*c, e_sort_reset, dim3(bb), dim3(128), nbox, D, S);
     launch_pdl(*c, e_keys, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), it + E->r_part.off, E->r_part.cnt, D, S,
-                                                   E->tune.sort_bucket);
+               E->tune.sort_bucket);
     ep_end(c, NYXPM_ST_KEYS);
     ep_begin(c);
     launch_pdl(*c, e_scan_reduce, dim3(pgrid(E, E->r_scan.cnt)), dim3(kScanT), it + E->r_scan.off, E->r_scan.cnt, D, S);
@@ -2422,13 +2426,13 @@ void enqueue_solve_head(nyxpm_ctx* c, nyxpm_ensemble* E)
     ep_end(c, NYXPM_ST_SCAN);
     ep_begin(c);
     launch_pdl(*c, e_scatter, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), it + E->r_part.off, E->r_part.cnt, D, S,
-                                                      E->tune.sort_bucket);
+               E->tune.sort_bucket);
     launch_pdl(*c, e_fix_short, dim3(pgrid(E, E->r_keys.cnt)), dim3(256), it + E->r_keys.off, E->r_keys.cnt, D, S);
     launch_pdl(*c, e_fix_long, dim3(E->sm * 2), dim3(512), nbox, D, S);
     ep_end(c, NYXPM_ST_SCATTER);
     ep_begin(c);
     launch_pdl(*c, e_gather, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), it + E->r_part.off, E->r_part.cnt, D, S,
-                                                     E->tune.sort_bucket);
+               E->tune.sort_bucket);
     launch_pdl(*c, e_flip, dim3(bb), dim3(128), nbox, S);
     ep_end(c, NYXPM_ST_GATHER);
     ep_begin(c);
@@ -2441,7 +2445,8 @@ void enqueue_solve_head(nyxpm_ctx* c, nyxpm_ensemble* E)
         launch_pdl(*c, e_deposit<8, 8, 8>, dim3(gt), dim3(256), it + E->r_tile.off, E->r_tile.cnt, D, S);
     ep_end(c, NYXPM_ST_DEPOSIT);
     ep_begin(c);
-    launch_pdl(*c, e_rowsum, dim3(pgrid(E, E->r_rows_rho.cnt)), dim3(256), it + E->r_rows_rho.off, E->r_rows_rho.cnt, D, S);
+    launch_pdl(*c, e_rowsum, dim3(pgrid(E, E->r_rows_rho.cnt)), dim3(256), it + E->r_rows_rho.off, E->r_rows_rho.cnt,
+               D, S);
     const double ggrav = -4.0 * M_PI * c->p.gconst;
     launch_pdl(*c, e_mean, dim3(nbox * kMeanWarps), dim3(32), D, S, ggrav);
     const dim3 rb(32, E->tune.smooth_rows);
@@ -2538,14 +2543,18 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
                 if (black && E->tune.prolong_quad) {
                     const auto& pq = E->r_prolong_quad[l];
                     const auto& pe = E->r_prolong_rest[l];
-                    if (pq.cnt) launch_pdl(*c, e_prolong4_black, dim3(pgrid(E, pq.cnt, 4)), dim3(256), it + pq.off, pq.cnt, D, S);
-                    if (pe.cnt) launch_pdl(*c, e_prolong4, dim3(pgrid(E, pe.cnt)), dim3(rb), it + pe.off, pe.cnt, D, S, black);
+                    if (pq.cnt) launch_pdl(*c, e_prolong4_black, dim3(pgrid(E, pq.cnt, 4)), dim3(256), it + pq.off,
+                                           pq.cnt, D, S);
+                    if (pe.cnt) launch_pdl(*c, e_prolong4, dim3(pgrid(E, pe.cnt)), dim3(rb), it + pe.off, pe.cnt, D,
+                                           S, black);
                     nk += (pq.cnt ? 1 : 0) + (pe.cnt ? 1 : 0);
                 } else {
-                    if (pv.cnt) launch_pdl(*c, e_prolong4, dim3(pgrid(E, pv.cnt)), dim3(rb), it + pv.off, pv.cnt, D, S, black);
+                    if (pv.cnt) launch_pdl(*c, e_prolong4, dim3(pgrid(E, pv.cnt)), dim3(rb), it + pv.off, pv.cnt, D,
+                                           S, black);
                     nk += pv.cnt ? 1 : 0;
                 }
-                if (pr.cnt) launch_pdl(*c, e_prolong, dim3(pgrid(E, pr.cnt)), dim3(rb), it + pr.off, pr.cnt, D, S, black);
+                if (pr.cnt) launch_pdl(*c, e_prolong, dim3(pgrid(E, pr.cnt)), dim3(rb), it + pr.off, pr.cnt, D, S,
+                                       black);
                 ep_end(c, NYXPM_ST_PROLONG);
                 c->launches += nk + (pr.cnt ? 1 : 0) - 1;
                 for (int sw = 0; sw < c->p.nu2; ++sw)
@@ -2567,8 +2576,10 @@ void enqueue_iterations(nyxpm_ctx* c, nyxpm_ensemble* E, int outer, int first)
             const float c_lo = (float)(1.0 / 6.0 - (double)c_hi);
             const auto& cv = E->r_correct_vec;
             const auto& cr = E->r_correct_rest;
-            if (cv.cnt) launch_pdl(*c, e_correct_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S, c_hi, c_lo);
-            if (cr.cnt) launch_pdl(*c, e_correct, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, c_hi, c_lo);
+            if (cv.cnt) launch_pdl(*c, e_correct_v, dim3(pgrid(E, cv.cnt)), dim3(rb), it + cv.off, cv.cnt, D, S, c_hi,
+                                   c_lo);
+            if (cr.cnt) launch_pdl(*c, e_correct, dim3(pgrid(E, cr.cnt)), dim3(rb), it + cr.off, cr.cnt, D, S, c_hi,
+                                   c_lo);
             c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0) - 1;
             const auto& rz = c->p.nu1 > 0 ? E->r_rows_tail0 : r0;
             if (rz.cnt) launch_pdl(*c, e_zero_inner, dim3(pgrid(E, rz.cnt)), dim3(rb), it + rz.off, rz.cnt, D, S);
@@ -2587,8 +2598,10 @@ void enqueue_grav(nyxpm_ctx* c, nyxpm_ensemble* E)
     const auto& cv = E->r_correct_vec;
     const auto& cr = E->r_correct_rest;
     ep_begin(c);
-    if (cv.cnt) launch_pdl(*c, e_grav_v, dim3(pgrid(E, cv.cnt)), dim3(rb), E->d_items + cv.off, cv.cnt, E->d_desc, E->d_state);
-    if (cr.cnt) launch_pdl(*c, e_grav, dim3(pgrid(E, cr.cnt)), dim3(rb), E->d_items + cr.off, cr.cnt, E->d_desc, E->d_state);
+    if (cv.cnt) launch_pdl(*c, e_grav_v, dim3(pgrid(E, cv.cnt)), dim3(rb), E->d_items + cv.off, cv.cnt, E->d_desc,
+                           E->d_state);
+    if (cr.cnt) launch_pdl(*c, e_grav, dim3(pgrid(E, cr.cnt)), dim3(rb), E->d_items + cr.off, cr.cnt, E->d_desc,
+                           E->d_state);
     ep_end(c, NYXPM_ST_KICK);
     c->launches += (cv.cnt ? 1 : 0) + (cr.cnt ? 1 : 0);
 }
@@ -2597,8 +2610,7 @@ void enqueue_kick(nyxpm_ctx* c, nyxpm_ensemble* E, int phase)
 {
     ep_begin(c);
     launch_pdl(*c, e_kick, dim3(pgrid(E, E->r_part.cnt)), dim3(kPT), E->d_items + E->r_part.off, E->r_part.cnt,
-                                                            E->d_desc, E->d_state, phase,
-                                                            E->tune.sort_bucket);
+               E->d_desc, E->d_state, phase, E->tune.sort_bucket);
     ep_end(c, NYXPM_ST_KICK);
     c->launches += 1;
 }
@@ -3018,8 +3030,8 @@ nyxpm_status nyxpm_ensemble_download(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, 
     cudaMemsetAsync(d.norms + 2, 0, sizeof(unsigned long long), c->stream);
     for (long long q0 = 0; q0 < np; q0 += by.count) {
         const long long m = std::min(by.count, np - q0);
-        e_pack<<<(unsigned)((np + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, np, d.dx, parr(d, parity), by.pos, by.vel,
-                                                                        d.norms + 2);
+        e_pack<<<(unsigned)((np + kPT - 1) / kPT), kPT, 0, c->stream>>>(q0, m, np, d.dx, parr(d, parity), by.pos,
+                                                                        by.vel, d.norms + 2);
         cudaMemcpyAsync(pos + 3 * q0, by.pos, 24 * m, cudaMemcpyDeviceToHost, c->stream);
         cudaMemcpyAsync(vel + 3 * q0, by.vel, 24 * m, cudaMemcpyDeviceToHost, c->stream);
     }

@@ -570,10 +570,11 @@ __global__ void k_mx_resid(int n, const double* __restrict__ phi_r, const double
 // loads of FP64 pairs) for rows of an even number of compact cells.  Every
 // residual is k_mx_resid's, term for term.  ints: neighbour sums on the integer
 // pipes (pm_sum6.cuh), where the FP64 pipe bounds the pass (256^3: 291 -> 190 us; 160^3: 117 -> 76).
-__global__ void __launch_bounds__(256) k_mx_resid2(int n, int ints, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
-                            const double* __restrict__ beta_r, const double* __restrict__ beta_b,
-                            float* r_r, float* r_b, float* rl_r, float* rl_b,
-                            unsigned long long* norm)
+__global__ void __launch_bounds__(256) k_mx_resid2(int n, int ints, const double* __restrict__ phi_r,
+                                                   const double* __restrict__ phi_b,
+                                                   const double* __restrict__ beta_r,
+                                                   const double* __restrict__ beta_b, float* r_r, float* r_b,
+                                                   float* rl_r, float* rl_b, unsigned long long* norm)
 {
     pdl_wait();
     pdl_trigger();
@@ -894,7 +895,8 @@ __global__ void __launch_bounds__(256) k_gsrb_f4(int n, int color, float* __rest
         const int k = k0 + kk;
         const int kp = k == n - 1 ? 0 : k + 1;
         const unsigned pk = (unsigned)k * plane;
-        const float4 zp = MZ > 1 ? ld_hint(o4 + (((unsigned)kp * plane + rj) >> 2), l2_keep()) : __ldg(o4 + (((unsigned)kp * plane + rj) >> 2));
+        const float4* above = o4 + (((unsigned)kp * plane + rj) >> 2);
+        const float4 zp = MZ > 1 ? ld_hint(above, l2_keep()) : __ldg(above);
         const float4 ym = __ldg(o4 + ((pk + rjm) >> 2));
         const float4 yp = __ldg(o4 + ((pk + rjp) >> 2));
         const unsigned t = pk + rj;
@@ -1395,8 +1397,9 @@ __global__ void k_mx_grav(LevelView L, float half_dxi, float* g)
 }
 
 // the same for a split level, two cells per thread (256^3: 146 -> 100 us, the FP64 subtractions' time)
-__global__ void __launch_bounds__(256) k_mx_grav2(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
-                                                  float half_dxi, float4* __restrict__ g)
+__global__ void __launch_bounds__(256) k_mx_grav2(int n, const double* __restrict__ phi_r,
+                                                  const double* __restrict__ phi_b, float half_dxi,
+                                                  float4* __restrict__ g)
 {
     pdl_wait();
     pdl_trigger();
@@ -1643,7 +1646,8 @@ nyxpm_status vcycle_f(Ctx& c, Box& b, size_t li, bool fresh = false, int red_don
     const long long ncc = (long long)cl.n * cl.n * cl.n;
     const long long ncf = (long long)f.n * f.n * f.n;
     // a coarse level that launches smooth (not the cluster, the tail or the bottom)
-    const int open = c.p.nu1 > 0 && li + 2 < b.levels.size() && !tail_fits(c, b, li + 1) && !cluster_fits_f(c, b, li + 1, ca);
+    const int open = c.p.nu1 > 0 && li + 2 < b.levels.size() && !tail_fits(c, b, li + 1) &&
+                     !cluster_fits_f(c, b, li + 1, ca);
     {
         prof_begin(c);
         if ((f.n / 2) % 4 == 0) {
@@ -1698,18 +1702,15 @@ nyxpm_status launch_mx_resid(Ctx& c, Box& b, bool low_words)
         const Geo g = geo3(l.n / 2, l.n, l.n);
         if ((l.n / 2) % 2 == 0) {
             const Geo g2 = geo3(l.n / 4, l.n, l.n);
-            launch_pdl(c, k_mx_resid2, dim3(g2.grid), dim3(g2.block), l.n, l.n >= kIntMinEdge ? 1 : 0, l.phi_r, l.phi_b, l.beta_r,
-                                                            l.beta_b, l.fbeta_r, l.fbeta_b, rl_r,
-                                                            rl_b, b.norms + 1);
+            launch_pdl(c, k_mx_resid2, dim3(g2.grid), dim3(g2.block), l.n, l.n >= kIntMinEdge ? 1 : 0, l.phi_r,
+                       l.phi_b, l.beta_r, l.beta_b, l.fbeta_r, l.fbeta_b, rl_r, rl_b, b.norms + 1);
         } else {
             launch_pdl(c, k_mx_resid, dim3(g.grid), dim3(g.block), l.n, l.phi_r, l.phi_b, l.beta_r, l.beta_b,
-                                                         l.fbeta_r, l.fbeta_b, rl_r, rl_b,
-                                                         b.norms + 1);
+                       l.fbeta_r, l.fbeta_b, rl_r, rl_b, b.norms + 1);
         }
     } else {
         const Geo g = geo3(l.n, l.n, l.n);
-        launch_pdl(c, k_mx_resid_nat, dim3(g.grid), dim3(g.block), l.n, l.phi_r, l.beta_r, l.fbeta_r,
-                                                         b.norms + 1);
+        launch_pdl(c, k_mx_resid_nat, dim3(g.grid), dim3(g.block), l.n, l.phi_r, l.beta_r, l.fbeta_r, b.norms + 1);
     }
     prof_end(c, NYXPM_ST_NORM, 20.0 * nc);
     return check_launch(c, "mixed residual");
@@ -1725,16 +1726,12 @@ nyxpm_status launch_mx_correct(Ctx& c, Box& b)
     prof_begin(c);
     if ((l.n / 2) % 2 == 0) {
         const Geo g = geo3(l.n / 4, l.n, l.n);
-        launch_pdl(c, k_mx_correct2, dim3(g.grid), dim3(g.block), l.n, c_hi, c_lo, l.fphi_r, l.fphi_b,
-                                                        l.phi_r, l.phi_b, l.fbeta_r, l.fbeta_b,
-                                                        b.r_lo, b.r_lo + nc / 2, b.norms + 1,
-                                                        b.norms + 4);
+        launch_pdl(c, k_mx_correct2, dim3(g.grid), dim3(g.block), l.n, c_hi, c_lo, l.fphi_r, l.fphi_b, l.phi_r,
+                   l.phi_b, l.fbeta_r, l.fbeta_b, b.r_lo, b.r_lo + nc / 2, b.norms + 1, b.norms + 4);
     } else {
         const Geo g = geo3(l.n / 2, l.n, l.n);
-        launch_pdl(c, k_mx_correct, dim3(g.grid), dim3(g.block), l.n, c_hi, c_lo, l.fphi_r, l.fphi_b,
-                                                       l.phi_r, l.phi_b, l.fbeta_r, l.fbeta_b,
-                                                       b.r_lo, b.r_lo + nc / 2, b.norms + 1,
-                                                       b.norms + 4);
+        launch_pdl(c, k_mx_correct, dim3(g.grid), dim3(g.block), l.n, c_hi, c_lo, l.fphi_r, l.fphi_b, l.phi_r,
+                   l.phi_b, l.fbeta_r, l.fbeta_b, b.r_lo, b.r_lo + nc / 2, b.norms + 1, b.norms + 4);
     }
     prof_end(c, NYXPM_ST_NORM, 36.0 * nc);
     return check_launch(c, "mixed correction");
@@ -1745,7 +1742,8 @@ nyxpm_status launch_mx_split_beta(Ctx& c, Box& b)
     const Level& l = b.levels[0];
     const long long half_cells = (long long)l.n * l.n * l.n / 2;
     prof_begin(c);
-    launch_pdl(c, k_mx_split_beta, dim3(blocks_for(half_cells)), dim3(kThreads), half_cells, l.beta_r, l.beta_b, l.fbeta_r, l.fbeta_b, b.r_lo, b.r_lo + half_cells);
+    launch_pdl(c, k_mx_split_beta, dim3(blocks_for(half_cells)), dim3(kThreads), half_cells, l.beta_r, l.beta_b,
+               l.fbeta_r, l.fbeta_b, b.r_lo, b.r_lo + half_cells);
     prof_end(c, NYXPM_ST_NORM, 32.0 * half_cells);
     return check_launch(c, "mixed split beta");
 }
@@ -1856,16 +1854,16 @@ nyxpm_status mixed_sort(Ctx& c, Box& b, bool defer_vel)
     nyxpm_status st;
     clear_counts(c, b);
     prof_begin(c);
-    launch_pdl(c, k_mx_keys, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.n, b.cell, b.ox, b.oy, b.oz,
-                                                            b.key, b.cell_count);
+    launch_pdl(c, k_mx_keys, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.n, b.cell, b.ox, b.oy, b.oz, b.key,
+               b.cell_count);
     prof_end(c, NYXPM_ST_KEYS, 20.0 * b.np);
     if ((st = check_launch(c, "mixed keys")) != NYXPM_OK) return st;
     if ((st = sort_from_keys(c, b)) != NYXPM_OK) return st;
     const bool pm = !b.uniform_mass;
     prof_begin(c);
-    launch_pdl(c, k_mx_gather, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.perm, b.cell, b.ox, b.oy, b.oz, defer_vel ? nullptr : b.fvx, b.fvy, b.fvz,
-        pm ? b.fm : nullptr, b.id, b.cell2, b.ox2, b.oy2, b.oz2, b.fvx2, b.fvy2, b.fvz2,
-        pm ? b.fm2 : nullptr, b.id2);
+    launch_pdl(c, k_mx_gather, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.perm, b.cell, b.ox, b.oy, b.oz,
+               defer_vel ? nullptr : b.fvx, b.fvy, b.fvz, pm ? b.fm : nullptr, b.id, b.cell2, b.ox2, b.oy2, b.oz2,
+               b.fvx2, b.fvy2, b.fvz2, pm ? b.fm2 : nullptr, b.id2);
     prof_end(c, NYXPM_ST_GATHER, ((pm ? 76.0 : 68.0) - (defer_vel ? 24.0 : 0.0)) * b.np);
     if ((st = check_launch(c, "mixed gather")) != NYXPM_OK) return st;
     std::swap(b.cell, b.cell2);
@@ -1896,11 +1894,10 @@ nyxpm_status mixed_deposit(Ctx& c, Box& b)
     // in the room of 8 doubles per slot)
     float* heavy = reinterpret_cast<float*>(b.heavy_part);
     prof_begin(c);
-    launch_pdl(c, k_mx_deposit_heavy, dim3(c.sm_count * 4), dim3(256), n, b.cell, b.ox, b.oy, b.oz, mq,
-                                                             b.cell_start, b.long_list, b.long_count,
-                                                             b.key_slot, heavy);
-    launch_pdl(c, k_mx_deposit, dim3(grid), dim3(kDepThreads), n, scale, b.cell, b.ox, b.oy, b.oz, mq,
-                                                     b.cell_start, b.key_slot, heavy, b.frho);
+    launch_pdl(c, k_mx_deposit_heavy, dim3(c.sm_count * 4), dim3(256), n, b.cell, b.ox, b.oy, b.oz, mq, b.cell_start,
+               b.long_list, b.long_count, b.key_slot, heavy);
+    launch_pdl(c, k_mx_deposit, dim3(grid), dim3(kDepThreads), n, scale, b.cell, b.ox, b.oy, b.oz, mq, b.cell_start,
+               b.key_slot, heavy, b.frho);
     c.launches += 1;
     prof_end(c, NYXPM_ST_DEPOSIT, (b.uniform_mass ? 16.0 : 20.0) * b.np + 8.0 * nc);
     return check_launch(c, "mixed deposit");
@@ -1922,14 +1919,15 @@ nyxpm_status mixed_make_rhs(Ctx& c, Box& b, double a)
     const double dx = b.L / n;
     const Geo g = geo3(n, n, n);
     prof_begin(c);
-    launch_pdl(c, k_mx_rowsum, dim3(blocks_for((long long)n * n * 32)), dim3(kThreads), n, b.frho,
-                                                                             b.mass_offset, b.rows);
+    launch_pdl(c, k_mx_rowsum, dim3(blocks_for((long long)n * n * 32)), dim3(kThreads), n, b.frho, b.mass_offset,
+               b.rows);
     launch_pdl(c, k_mx_mean, dim3(kMeanBlocks), dim3(32), n, dx, b.L, b.rows, b.scal + 4,
-                                                reinterpret_cast<unsigned*>(b.scal + kScalTicket), b.scal, b.norms);
+               reinterpret_cast<unsigned*>(b.scal + kScalTicket), b.scal, b.norms);
     const double scale = ((-4.0 * M_PI * c.p.gconst) * (1.0 / a)) * beta_scale(b);
     if (l0.split) {
         const Geo g2 = geo3(n / 2, n, n);
-        launch_pdl(c, k_mx_make_beta2, dim3(g2.grid), dim3(g2.block), n, b.frho, b.mass_offset, b.scal, scale, l0.beta_r, l0.beta_b, b.norms);
+        launch_pdl(c, k_mx_make_beta2, dim3(g2.grid), dim3(g2.block), n, b.frho, b.mass_offset, b.scal, scale,
+                   l0.beta_r, l0.beta_b, b.norms);
     } else {
         launch_pdl(c, k_mx_make_beta, dim3(g.grid), dim3(g.block), n, l0.split, b.frho, b.mass_offset, b.scal,
                    scale, l0.beta_r, l0.beta_b, b.norms);
@@ -2123,8 +2121,8 @@ nyxpm_status mixed_kick(Ctx& c, Box& b, double dt, double a_prev, double a_cur, 
     A.drift = (float)(dt / a_cur * b.dxi);
     A.do_move = do_move;
     prof_begin(c);
-    launch_pdl(c, k_mx_kick, dim3(blocks_for(b.np)), dim3(kThreads), b.np, A, b.cell, b.ox, b.oy, b.oz, b.fvx,
-                                                            b.fvy, b.fvz);
+    launch_pdl(c, k_mx_kick, dim3(blocks_for(b.np)), dim3(kThreads), b.np, A, b.cell, b.ox, b.oy, b.oz, b.fvx, b.fvy,
+               b.fvz);
     const double nc = (double)b.n * b.n * b.n;
     prof_end(c, NYXPM_ST_KICK, (do_move ? 56.0 : 40.0) * b.np + 12.0 * nc);
     if (do_move) b.sorted = 0;
@@ -2135,8 +2133,8 @@ nyxpm_status mixed_est_dt(Ctx& c, Box& b)
 {
     cudaMemsetAsync(b.norms + 3, 0, 3 * sizeof(unsigned long long), c.stream);
     const unsigned blocks = std::min(blocks_for(b.np), (unsigned)(c.sm_count * 8));
-    launch_pdl(c, k_mx_est_dt, dim3(blocks), dim3(kThreads), b.np, b.n, b.cell, b.fvx, b.fvy, b.fvz, b.g32, b.norms + 3,
-                                                    b.norms + 5);
+    launch_pdl(c, k_mx_est_dt, dim3(blocks), dim3(kThreads), b.np, b.n, b.cell, b.fvx, b.fvy, b.fvz, b.g32,
+               b.norms + 3, b.norms + 5);
     c.launches += 1;
     return check_launch(c, "mixed time-step estimate");
 }

@@ -698,8 +698,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_d(ClArgs<doubl
 }
 
 // the same with both in natural layout
-__global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_nat_d(ClArgs<double> A, const double* __restrict__ beta,
-                                                                     double* __restrict__ e)
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_vcycle_nat_d(ClArgs<double> A,
+                                                                        const double* __restrict__ beta,
+                                                                        double* __restrict__ e)
 {
     extern __shared__ __align__(16) double cl_mem_d[];
     __shared__ ClShared<double> S;
@@ -806,8 +807,8 @@ __global__ void k_grav(LevelView L, double dxi, double* g)
 }
 
 // the same for a split level, two cells per thread (256^3: 484 -> 415 us)
-__global__ void __launch_bounds__(256) k_grav2(int n, const double* __restrict__ phi_r, const double* __restrict__ phi_b,
-                                               double dxi, double* __restrict__ g)
+__global__ void __launch_bounds__(256) k_grav2(int n, const double* __restrict__ phi_r,
+                                               const double* __restrict__ phi_b, double dxi, double* __restrict__ g)
 {
     pdl_wait();
     pdl_trigger();
@@ -822,7 +823,8 @@ __global__ void __launch_bounds__(256) k_grav2(int n, const double* __restrict__
     double2* out = reinterpret_cast<double2*>(g) + ((unsigned)j + (unsigned)n * (unsigned)k) * half + ih;
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-        out[d * nc2] = make_double2(diff(P.c[2 * d], P.even, P.c[2 * d + 1]), diff(P.c[6 + 2 * d], P.odd, P.c[7 + 2 * d]));
+        out[d * nc2] = make_double2(diff(P.c[2 * d], P.even, P.c[2 * d + 1]),
+                                    diff(P.c[6 + 2 * d], P.odd, P.c[7 + 2 * d]));
 }
 
 __global__ void k_to_natural(LevelView L, double* out)
@@ -965,13 +967,15 @@ nyxpm_status vcycle(Ctx& c, Box& b, size_t li, int red_done = 0)
     const long long ncf = (long long)f.n * f.n * f.n;
     const bool quads = f.split && (f.n / 2) % 4 == 0;
     // a coarse level that launches smooth (not the cluster, the tail or the bottom)
-    const int open = nu1 > 0 && li + 2 < b.levels.size() && !tail_fits_d(c, b, li + 1) && !cluster_fits_d(c, b, li + 1, ca);
+    const int open = nu1 > 0 && li + 2 < b.levels.size() && !tail_fits_d(c, b, li + 1) &&
+                     !cluster_fits_d(c, b, li + 1, ca);
     {
         const bool pairs = c.p.nu1 > 0 && by_pairs(f);
         const Geo g = geo3(pairs ? cl.n / 2 : cl.n, cl.n, cl.n, pairs ? 128 : 256);
         prof_begin(c);
         if (c.p.nu1 > 0)
-            launch_pdl(c, pairs ? k_restrict_red2 : k_restrict<1>, dim3(g.grid), dim3(g.block), view(f), view(cl), open);
+            launch_pdl(c, pairs ? k_restrict_red2 : k_restrict<1>, dim3(g.grid), dim3(g.block), view(f), view(cl),
+                       open);
         else
             launch_pdl(c, k_restrict<0>, dim3(g.grid), dim3(g.block), view(f), view(cl), open);
         prof_end(c, NYXPM_ST_RESTRICT, 16.0 * ncf + 16.0 * ncc);
@@ -1042,13 +1046,11 @@ nyxpm_status launch_make_rhs(Ctx& c, Box& b, double a)
     const double dx = b.L / n;
     const Geo g = geo3(n, n, n);
     prof_begin(c);
-    launch_pdl(c, k_rowsum, dim3(blocks_for((long long)n * n * 32)), dim3(kThreads), n, b.rho, b.mass_offset,
-                                                                          b.rows);
+    launch_pdl(c, k_rowsum, dim3(blocks_for((long long)n * n * 32)), dim3(kThreads), n, b.rho, b.mass_offset, b.rows);
     launch_pdl(c, k_mean, dim3((n + 31) / 32), dim3(32), n, dx, b.L, b.rows, b.planes,
                reinterpret_cast<unsigned*>(b.scal + kScalTicket), b.scal, b.norms);
     launch_pdl(c, k_make_beta, dim3(g.grid), dim3(g.block), n, l0.split, b.rho, b.mass_offset, b.scal,
-                                                  -4.0 * M_PI * c.p.gconst, 1.0 / a, beta_scale(b),
-                                                  l0.beta_r, l0.beta_b, b.norms);
+               -4.0 * M_PI * c.p.gconst, 1.0 / a, beta_scale(b), l0.beta_r, l0.beta_b, b.norms);
     prof_end(c, NYXPM_ST_RHS, 24.0 * nc);
     c.launches += 2;
     return check_launch(c, "make rhs");
@@ -1136,8 +1138,8 @@ nyxpm_status mg_solve(Ctx& c, Box& b, int zero_guess, nyxpm_solve_info* info, bo
                 const bool pairs = by_pairs(L0);
                 const Geo g = geo3(pairs ? L0.n / 4 : L0.n / 2, L0.n, L0.n);
                 prof_begin(c);
-                launch_pdl(c, pairs ? k_resnorm_red_sweep2 : k_resnorm_red_sweep, dim3(g.grid), dim3(g.block), L0.n, L0.phi_r, L0.phi_b, L0.beta_r,
-                                                                      b.phi_r_spare, b.norms + 1);
+                launch_pdl(c, pairs ? k_resnorm_red_sweep2 : k_resnorm_red_sweep, dim3(g.grid), dim3(g.block), L0.n,
+                           L0.phi_r, L0.phi_b, L0.beta_r, b.phi_r_spare, b.norms + 1);
                 prof_end(c, NYXPM_ST_NORM, 16.0 * nc);
                 if ((s = check_launch(c, "red norm + sweep")) != NYXPM_OK) return s;
             } else if ((s = launch_resnorm(c, b, 1, red_only)) != NYXPM_OK) {

@@ -775,9 +775,9 @@ nyxpm_status fix_segments(Ctx& c, Box& b)
     const int nc = b.n * b.n * b.n;
     prof_begin(c);
     launch_pdl(c, k_fix_short, dim3(blocks_for(nc)), dim3(kThreads), nc, b.cell_start, b.perm, b.long_list,
-                                                            b.long_count);
+               b.long_count);
     launch_pdl(c, k_fix_long, dim3(c.sm_count * 2), dim3(512), b.cell_start, b.long_list, b.long_count, b.perm,
-                                                      b.key);
+               b.key);
     prof_end(c, NYXPM_ST_SCATTER, 4.0 * nc + 8.0 * b.np);
     c.launches += 1;
     return check_launch(c, "fix segments");
@@ -788,8 +788,7 @@ nyxpm_status sort_from_keys(Ctx& c, Box& b)
     nyxpm_status st;
     if ((st = scan_counts(c, b)) != NYXPM_OK) return st;
     prof_begin(c);
-    launch_pdl(c, k_scatter, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.key, b.cell_start, b.cell_count,
-                                                            b.perm);
+    launch_pdl(c, k_scatter, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.key, b.cell_start, b.cell_count, b.perm);
     prof_end(c, NYXPM_ST_SCATTER, 12.0 * b.np);
     if ((st = check_launch(c, "scatter")) != NYXPM_OK) return st;
     b.counts_dirty = 0;
@@ -802,7 +801,7 @@ nyxpm_status launch_sort(Ctx& c, Box& b, bool defer_vel)
     clear_counts(c, b);
     prof_begin(c);
     launch_pdl(c, k_keys, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.n, b.dxi, b.x, b.y, b.z, b.key,
-                                                         b.cell_count);
+               b.cell_count);
     prof_end(c, NYXPM_ST_KEYS, 32.0 * b.np);
     if ((st = check_launch(c, "keys")) != NYXPM_OK) return st;
     if ((st = sort_from_keys(c, b)) != NYXPM_OK) return st;
@@ -810,9 +809,9 @@ nyxpm_status launch_sort(Ctx& c, Box& b, bool defer_vel)
     prof_begin(c);
     // defer_vel: the velocities are not on the device yet; launch_gather_vel
     // permutes them by the same perm once they are
-    launch_pdl(c, k_gather, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.perm, b.x, b.y, b.z, defer_vel ? nullptr : b.vx, b.vy, b.vz,
-        b.uniform_mass ? nullptr : b.m, b.id, b.x2, b.y2, b.z2, b.vx2, b.vy2, b.vz2,
-        b.uniform_mass ? nullptr : b.m2, b.id2);
+    launch_pdl(c, k_gather, dim3(blocks_for(b.np)), dim3(kThreads), b.np, b.perm, b.x, b.y, b.z,
+               defer_vel ? nullptr : b.vx, b.vy, b.vz, b.uniform_mass ? nullptr : b.m, b.id, b.x2, b.y2, b.z2, b.vx2,
+               b.vy2, b.vz2, b.uniform_mass ? nullptr : b.m2, b.id2);
     prof_end(c, NYXPM_ST_GATHER, (16.0 * nvals + 12.0) * b.np);
     if ((st = check_launch(c, "gather")) != NYXPM_OK) return st;
     std::swap(b.x, b.x2);
@@ -885,13 +884,11 @@ nyxpm_status launch_deposit(Ctx& c, Box& b)
     const double* mq = b.uniform_mass ? nullptr : b.m;
     prof_begin(c);
     launch_pdl(c, k_deposit_heavy, dim3(c.sm_count * 4), dim3(256), n, b.dxi, b.x, b.y, b.z, mq, b.cell_start,
-                                                          b.long_list, b.long_count, b.key_slot,
-                                                          b.heavy_part);
+               b.long_list, b.long_count, b.key_slot, b.heavy_part);
     const long long ncl = (long long)n * n * n;
     const unsigned kb = (unsigned)((ncl + 32LL * kKeyWarps - 1) / (32LL * kKeyWarps));
-    launch_pdl(c, k_deposit_keys, dim3(kb), dim3(32 * kKeyWarps), ncl, n, b.dxi, b.x, b.y, b.z, mq,
-                                                         b.cell_start, b.key_slot, b.heavy_part,
-                                                         b.key_part);
+    launch_pdl(c, k_deposit_keys, dim3(kb), dim3(32 * kKeyWarps), ncl, n, b.dxi, b.x, b.y, b.z, mq, b.cell_start,
+               b.key_slot, b.heavy_part, b.key_part);
     const Geo g = geo3(n, n, n);
     launch_pdl(c, k_deposit_cells, dim3(g.grid), dim3(g.block), n, scale, b.key_part, b.rho);
     c.launches += 2;
@@ -925,8 +922,8 @@ nyxpm_status launch_est_dt(Ctx& c, Box& b)
 {
     cudaMemsetAsync(b.norms + 3, 0, 3 * sizeof(unsigned long long), c.stream);
     const unsigned blocks = std::min(blocks_for(b.np), (unsigned)(c.sm_count * 8));
-    launch_pdl(c, k_est_dt, dim3(blocks), dim3(kThreads), b.np, b.n, b.dxi, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.g, b.norms + 3,
-                                                 b.norms + 5);
+    launch_pdl(c, k_est_dt, dim3(blocks), dim3(kThreads), b.np, b.n, b.dxi, b.x, b.y, b.z, b.vx, b.vy, b.vz, b.g,
+               b.norms + 3, b.norms + 5);
     c.launches += 1;
     return check_launch(c, "time-step estimate");
 }
