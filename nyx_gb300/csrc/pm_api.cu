@@ -84,7 +84,6 @@ void post_words(Ctx& c, const Post& p, unsigned long long* words, int first, int
 
 nyxpm_status post_wait(Ctx& c, Post& p, const char* what)
 {
-    if (waits_give_way()) cudaStreamSynchronize(c.stream);   // an error is found below
     cudaError_t e = cudaErrorNotReady;
     for (int i = 1; !__atomic_load_n(p.host + kPostWords, __ATOMIC_ACQUIRE); ++i) {
         if (i & 4095) continue;
@@ -94,7 +93,7 @@ nyxpm_status post_wait(Ctx& c, Post& p, const char* what)
             c.err = std::string(what) + ": no read-back";
             return NYXPM_CUDA_ERROR;
         }
-        e = cudaStreamQuery(c.stream);
+        e = i == 4096 && waits_give_way() ? cudaStreamSynchronize(c.stream) : cudaStreamQuery(c.stream);
         if (e == cudaErrorNotReady) cudaGetLastError();
     }
     p.open = 0;

@@ -461,7 +461,7 @@ inline bool waits_give_way()
 
 // A read-back of a few words that the host is waiting for: one small kernel at the end
 // of the work writes them and then a flag to pinned host memory, and the host polls the
-// flag (waits for the stream first where waits_give_way).  A copy plus a wait for the
+// flag (some microseconds only where waits_give_way).  A copy plus a wait for the
 // stream costs 12 us between a V-cycle's last kernel and the next V-cycle's first, this
 // 3 us (measured, ten short kernels a graph: 34.6 -> 24.0 us; 22.5 back to back).
 constexpr int kPostWords = 8;

@@ -659,12 +659,12 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
     // alone, and the check is the caller's (every replay's positions finite).
     if (capturing) return NYXPM_OK;
     // Where the device can write the caller's stack, one kernel writes the count there and
-    // the host polls for it (32^3: the call 61 -> 48 us against the copy and the wait), unless
-    // the application wants waits that give the CPU away.
+    // the host polls for it (32^3: the call 61 -> 48 us against the copy and the wait); some
+    // microseconds only, where the application wants waits that give the CPU away.
     int h_bad = 0, dev = 0, pageable = 0;
     cudaError_t es = cudaGetDevice(&dev);
     if (es == cudaSuccess) es = cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev);
-    if (es == cudaSuccess && pageable && !waits_give_way()) {
+    if (es == cudaSuccess && pageable) {
         unsigned long long word = 0;
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(1);
@@ -677,8 +677,11 @@ extern "C" nyxpm_status nyxpm_deposit_noalloc(const double* d_x, const double* d
         if (es == cudaSuccess) {
             cudaError_t q = cudaErrorNotReady;
             int i = 1;
-            while (!__atomic_load_n(&word, __ATOMIC_ACQUIRE) && q == cudaErrorNotReady)
-                if ((i++ & 4095) == 0 && (q = cudaStreamQuery(s)) == cudaErrorNotReady) cudaGetLastError();
+            while (!__atomic_load_n(&word, __ATOMIC_ACQUIRE) && q == cudaErrorNotReady) {
+                if (i++ & 4095) continue;
+                q = i == 4097 && waits_give_way() ? cudaStreamSynchronize(s) : cudaStreamQuery(s);
+                if (q == cudaErrorNotReady) cudaGetLastError();
+            }
             // a stream that ended (or failed) first: nothing writes the word any more
             if (q != cudaErrorNotReady) es = cudaStreamSynchronize(s);
             h_bad = (int)(word >> 32);
