@@ -1732,8 +1732,8 @@ nyxpm_status nyxpm_amr_download(nyxpm_ctx* c, nyxpm_amr* a, double* pos, double*
                                                    a->staging + 3 * a->np);
     prof_end(*c, NYXPM_ST_GATHER, 96.0 * a->np);
     ATRY(check_launch(*c, "hierarchy download"));
-    touch_pages(pos, sizeof(double) * 3 * a->np);
-    touch_pages(vel, sizeof(double) * 3 * a->np);
+    touch_host(pos, sizeof(double) * 3 * a->np);
+    touch_host(vel, sizeof(double) * 3 * a->np);
     cudaMemcpyAsync(pos, a->staging, sizeof(double) * 3 * a->np, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(vel, a->staging + 3 * a->np, sizeof(double) * 3 * a->np, cudaMemcpyDeviceToHost, c->stream);
     return nyxpm_synchronize(c);

@@ -578,8 +578,8 @@ nyxpm_status nyxpm_box_download(nyxpm_ctx* c, nyxpm_box* b, double* pos, double*
     double* d_vel = b->staging + 3 * np;
     if (b->prec == NYXPM_MIXED) TRY(mixed_pack(*c, *b, d_pos, d_vel));
     else TRY(launch_pack(*c, *b, d_pos, d_vel));
-    touch_pages(pos, sizeof(double) * 3 * np);
-    touch_pages(vel, sizeof(double) * 3 * np);
+    touch_host(pos, sizeof(double) * 3 * np);
+    touch_host(vel, sizeof(double) * 3 * np);
     cudaMemcpyAsync(pos, d_pos, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(vel, d_vel, sizeof(double) * 3 * np, cudaMemcpyDeviceToHost, c->stream);
     return nyxpm_synchronize(c);
@@ -610,7 +610,7 @@ nyxpm_status nyxpm_deposit(nyxpm_ctx* c, nyxpm_box* b, double* rho_out)
     if (rho_out) {
         const size_t nc = (size_t)b->n * b->n * b->n;
         if (b->prec == NYXPM_MIXED) TRY(mixed_rho_to_double(*c, *b));
-        touch_pages(rho_out, sizeof(double) * nc);
+        touch_host(rho_out, sizeof(double) * nc);
         cudaMemcpyAsync(rho_out, b->rho, sizeof(double) * nc, cudaMemcpyDeviceToHost, c->stream);
         TRY(check_launch(*c, "rho copy"));
         return nyxpm_synchronize(c);
@@ -632,7 +632,7 @@ nyxpm_status nyxpm_get_phi(nyxpm_ctx* c, nyxpm_box* b, double* phi)
     if (!phi) return fail(c, NYXPM_INVALID_ARG, "null phi");
     const size_t nc = (size_t)b->n * b->n * b->n;
     TRY(launch_phi_to_natural(*c, *b, b->nat));
-    touch_pages(phi, sizeof(double) * nc);
+    touch_host(phi, sizeof(double) * nc);
     cudaMemcpyAsync(phi, b->nat, sizeof(double) * nc, cudaMemcpyDeviceToHost, c->stream);
     TRY(check_launch(*c, "phi copy"));
     return nyxpm_synchronize(c);
@@ -675,7 +675,7 @@ nyxpm_status nyxpm_grav_vector(nyxpm_ctx* c, nyxpm_box* b, double* g_out)
     if (b->prec == NYXPM_MIXED && !b->g_from_caller) TRY(launch_grav_vector(*c, *b));
     if (g_out) {
         const size_t nc = (size_t)b->n * b->n * b->n;
-        touch_pages(g_out, sizeof(double) * 3 * nc);
+        touch_host(g_out, sizeof(double) * 3 * nc);
         cudaMemcpyAsync(g_out, b->g, sizeof(double) * 3 * nc, cudaMemcpyDeviceToHost, c->stream);
         TRY(check_launch(*c, "g copy"));
         return nyxpm_synchronize(c);

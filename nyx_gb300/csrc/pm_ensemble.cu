@@ -3025,8 +3025,8 @@ nyxpm_status nyxpm_ensemble_download(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, 
     const long long np = d.np;
     const int parity = E->h_state[slot].parity;
     const Pieces by = pieces_of(d, parity);
-    touch_pages(pos, 24 * np);
-    touch_pages(vel, 24 * np);
+    touch_host(pos, 24 * np);
+    touch_host(vel, 24 * np);
     cudaMemsetAsync(d.norms + 2, 0, sizeof(unsigned long long), c->stream);
     for (long long q0 = 0; q0 < np; q0 += by.count) {
         const long long m = std::min(by.count, np - q0);
@@ -3051,7 +3051,7 @@ nyxpm_status nyxpm_ensemble_get_phi(nyxpm_ctx* c, nyxpm_ensemble* E, int slot, d
     if (!tmp) return efail(c, NYXPM_OOM, "ensemble phi staging");
     const Geo g = geo3(d.n, d.n, d.n);
     e_phi_to_natural<<<g.grid, g.block, 0, c->stream>>>(d.n, d.phi_r, d.phi_b, (double*)tmp);
-    touch_pages(phi, 8 * nc);
+    touch_host(phi, 8 * nc);
     cudaMemcpyAsync(phi, tmp, 8 * nc, cudaMemcpyDeviceToHost, c->stream);
     const cudaError_t e = cudaStreamSynchronize(c->stream);
     E->arena.release(tmp);
@@ -3067,7 +3067,7 @@ nyxpm_status nyxpm_ensemble_grav_vector(nyxpm_ctx* c, nyxpm_ensemble* E, int slo
     void* tmp = E->arena.alloc(8 * cnt);
     if (tmp) {
         e_g32_to_double<<<(unsigned)((ncell + 255) / 256), 256, 0, c->stream>>>(ncell, d.g32, (double*)tmp);
-        touch_pages(g_out, 8 * cnt);
+        touch_host(g_out, 8 * cnt);
         cudaMemcpyAsync(g_out, tmp, 8 * cnt, cudaMemcpyDeviceToHost, c->stream);
         const cudaError_t e = cudaStreamSynchronize(c->stream);
         E->arena.release(tmp);

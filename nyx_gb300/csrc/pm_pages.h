@@ -6,13 +6,14 @@
 // until the copy runs the buffer holds what it held, whatever the call's outcome.  Missing
 // pages come in by the kernel (MADV_POPULATE_WRITE), which refuses an address the process
 // cannot write (a read-only mapping, device memory) where a store would end the process.
-// Which are missing says mincore (3.5 us for 50 MB of 64 KB pages).  Pages that are there are
+// Which are missing says mincore (0.35 us and 3.5 us for 50 MB of 64 KB pages).  Pages that are there are
 // read: without it a read-back of 470 MB into them took 20 to 60 ms instead of 6 about every
 // half second, as if their entries had been closed in between.
 //
-// Measured on fresh pages, GB/s: one thread 48 (a store to each page 42); 16 MB by three threads
-// 79 and 50 MB 103 (four threads 72 and 84: they wait for one another in the kernel); 400 MB by
-// four 113, by three 92.  In steps of 1 MB: in one step per thread 64 GB/s for 50 MB by four.
+// Measured on fresh pages: 8 MB 161 us (186 by a store to each page), 20 MB 221 (198), 50 MB 500
+// (456), 400 MB 3440 (3890); three threads up to 128 MB, as four wait for one another in the
+// kernel (50 MB 84 GB/s against 103; 400 MB 113 against 92), in steps of 1 MB (in one step per
+// thread 64 GB/s).  Pages that are there: 8 MB 0.9 us, 50 MB 40, 400 MB 87 (0.2, 35, 49).
 // (A page that was read before its first write counts as there: the copy faults it.)
 #pragma once
 
@@ -29,7 +30,8 @@
 
 namespace nyxpm {
 
-constexpr size_t kPageStep = (size_t)1 << 20;            // bytes per system call
+constexpr size_t kPageStep = (size_t)1 << 20;            // bytes brought in per system call
+constexpr size_t kPageLook = (size_t)16 << 20;           // bytes asked about per system call
 constexpr size_t kPageMin = 4096;
 constexpr size_t kTouchThreadsFrom = (size_t)16 << 20;   // bytes worth threads
 constexpr size_t kTouchThreeTo = (size_t)128 << 20;      // missing bytes better by three than by four
@@ -37,26 +39,42 @@ constexpr size_t kTouchThreeTo = (size_t)128 << 20;      // missing bytes better
 // the missing pages of [at, end), whole pages; touch: fault them in and read the others
 inline size_t missing_pages(uintptr_t at, uintptr_t end, size_t page, bool touch)
 {
-    unsigned char there[kPageStep / kPageMin];
-    size_t missing = 0;
+    unsigned char there[kPageLook / kPageMin];
+    const size_t step = kPageStep / page;
+    size_t missing = 0, look = kPageLook;
     while (at < end) {
-        const size_t len = end - at < kPageStep ? end - at : kPageStep, pages = len / page;
-        if (mincore(reinterpret_cast<void*>(at), len, there) != 0) return missing;   // not mapped
-        size_t first = pages, last = 0;
-        for (size_t i = 0; i < pages; ++i) {
-            if (there[i] & 1) {
-                if (touch) (void)*reinterpret_cast<volatile char*>(at + i * page);
-                continue;
-            }
-            ++missing;
-            if (first == pages) first = i;
-            last = i;
+        const size_t len = end - at < look ? end - at : look, pages = len / page;
+        if (mincore(reinterpret_cast<void*>(at), len, there) != 0) {
+            if (look == kPageStep) return missing;   // not mapped
+            look = kPageStep;
+            continue;
         }
-        if (touch && first < pages)
-            madvise(reinterpret_cast<void*>(at + first * page), (last + 1 - first) * page, MADV_POPULATE_WRITE);
+        for (size_t i0 = 0; i0 < pages; i0 += step) {
+            const size_t i1 = i0 + step < pages ? i0 + step : pages;
+            size_t first = i1, last = 0;
+            for (size_t i = i0; i < i1; ++i) {
+                if (there[i] & 1) {
+                    if (touch) (void)*reinterpret_cast<volatile char*>(at + i * page);
+                    continue;
+                }
+                ++missing;
+                if (first == i1) first = i;
+                last = i;
+            }
+            if (touch && first < i1)
+                madvise(reinterpret_cast<void*>(at + first * page), (last + 1 - first) * page, MADV_POPULATE_WRITE);
+        }
         at += len;
     }
     return missing;
+}
+
+inline void read_pages(const void* p, size_t bytes)
+{
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const volatile char* c = static_cast<const volatile char*>(p);
+    for (size_t o = 0; o < bytes; o += page) (void)c[o];
+    if (bytes) (void)c[bytes - 1];
 }
 
 inline void touch_pages(void* p, size_t bytes)
