@@ -65,10 +65,10 @@ typedef struct nyxpm_params {
                                (the FP64 ones of at most half as many, below the finest) run
                                as one launch (one CTA per box) per V-cycle, same results;
                                with any value above 0 and nu1, nu2 > 0, a single box's FP32
-                               levels of at most 32 and FP64 levels of at most 16 cells per
-                               edge (a whole box: 48 and 32) run as one launch of a 16-CTA
-                               cluster where their planes fit in its shared memory, same
-                               results;
+                               levels of at most 32 cells per edge (a whole box: 48) and, on
+                               grids of 4 * 2^k and 6 * 2^k cells, its FP64 levels of at most
+                               16 (a whole box: 32) run as one launch of a 16-CTA cluster,
+                               same results;
                                0: one launch per pass on every level (default 16) */
 } nyxpm_params;
 

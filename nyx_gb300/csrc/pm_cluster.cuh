@@ -1,23 +1,26 @@
 // V-cycles of small levels by one cluster of 16 CTAs, every level in shared memory.
 //
 // Why.  On small levels a pass is a few thousand cells: as a launch of its own it takes 1.5
-// to 4 us, nearly all of it launch and memory latency,
-// and a V(2,2) cycle has ten passes per level.  One CTA is too slow for these levels,
-// and a cluster that passes its values through L2 as well.  Here the levels of a V-cycle
-// stay in the CTAs' shared memory: a level is cut into slabs of whole z planes, the CTA
-// that owns a plane updates it, the neighbour planes of a slab are read from the other
-// CTAs' shared memory, and a hardware cluster barrier stands between two passes.  The
-// levels small enough for one CTA (8^3 in FP64, 16^3 in FP32) are cycled by the
-// cluster's first CTA (vcycle_solo, pm_tail.cuh) in its shared memory.
+// to 4 us, nearly all of it launch and memory latency, and a V(2,2) cycle has ten passes per
+// level.  One CTA is too slow for these levels, and a cluster that passes its values through
+// L2 as well.  Here the levels of a V-cycle stay in the CTAs' shared memory: a level is cut
+// into slabs of whole z planes, the CTA that owns a plane updates it, the neighbour planes of
+// a slab are read from the other CTAs' shared memory, and a hardware cluster barrier stands
+// between two passes.  The levels small enough for one CTA (8^3 in FP64, 16^3 in FP32) are
+// cycled by the cluster's first CTA (vcycle_solo, pm_tail.cuh) in its shared memory, two
+// levels at least, the bottom and a split one: in FP64 the chains 20-10-5 and 28-14-7 have the
+// bottom only, and grids of 5 * 2^k and 7 * 2^k cells an edge go by launches at every level.
 //
-// Measured on GB300 (SM clocks): a cluster barrier 526; a half sweep of 64^3 in FP32
-// 2800 and of 32^3 in FP64 3800, against 2.3 us and 2.2 us (4700 and 4500 clocks) of a
-// launch.  Whole solves from phi = 0: FP64 32^3 0.83 -> 0.55 ms, FP32 32^3 0.63 -> 0.28,
-// 64^3 0.80 -> 0.59 ms.  Since then the launches overlap and fit the row, and the edges were
-// measured again (cluster_fits_f, cluster_fits_d).  FP64 issues at 19 clocks per warp instruction and SM, so that 16 SMs smooth 48^3
-// in 6 us, twice a launch over the whole chip.  (Integer sums, pm_sum6.cuh, lose here: on
-// coarse levels some lane of a warp nearly always needs the FP64 additions as well, a
-// 32^3 solve took 0.64 ms.)
+// Measured on GB300 (SM clocks): a cluster barrier 526; a half sweep of 32^3 in FP64 3800,
+// against 2.2 us (4500 clocks) of a launch.  FP64 issues at 19 clocks per warp instruction and
+// SM, so that a pass over 32^3 takes the FP64 pipes of 16 SMs about as long as a launch over
+// the whole chip.  Where the edges lie (launches overlap by programmatic dependent launch):
+//   whole boxes             FP64 to 32^3: four steps 3.64 ms, by launches down to 16^3 3.82;
+//                           FP32 to 48^3: 3.35 against 3.47; at 64^3 4.08 against 3.83
+//   below a finest level    FP64 from 16^3: 64^3 7.10, with level 32 7.48, without any 7.8;
+//                           FP32 from 32^3: 128^3 7.50, with level 64 8.28, without level 32 8.60
+// (Integer sums, pm_sum6.cuh, lose here: on coarse levels some lane of a warp nearly always
+// needs the FP64 additions as well, a 32^3 solve of 0.55 ms took 0.64.)
 //
 // Every cell's arithmetic is that of the per-pass kernels (k_gsrb, k_restrict<1>,
 // k_prolong<1> and their FP32 forms), in the same order, so the bits are theirs.
@@ -34,7 +37,7 @@ namespace nyxpm {
 
 constexpr int kClCtas = 16;         // CTAs of the cluster
 constexpr int kClThreads = 512;   // a cluster barrier of 16 x 512 threads takes 526 cycles, of 16 x 1024 682
-constexpr int kClMaxPlanes = 4;     // planes of a level a CTA owns at most
+constexpr int kClMaxPlanes = 3;     // planes of a level a CTA owns at most: kClEdgeF / kClCtas
 constexpr int kClMaxLevels = 4;     // levels in slabs
 constexpr int kClEdgeF = 48;        // largest level taken, FP32 and FP64 (whole boxes; see cluster_fits_f, _d)
 constexpr int kClEdgeD = 32;
@@ -116,7 +119,7 @@ inline bool cl_layout(ClArgs<T>& A, const int* n, int levels)
             at += 2u * nl * nl * nl;
         }
     }
-    if (A.ns < 2) return false;   // the first one-CTA level is a split one
+    if (A.ns < 2) return false;   // vcycle_solo takes a split level over the bottom
     stage = std::max(stage, (unsigned)(A.n[A.nd] * A.n[A.nd] * A.n[A.nd]) / 2u);
     A.stage = (at + 3u) & ~3u;
     A.elems = A.stage + stage;

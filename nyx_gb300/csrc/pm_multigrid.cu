@@ -903,7 +903,8 @@ bool tail_fits_d(const Ctx& c, const Box& b, size_t li)
 // box's finest level only from 16^3 down: a pass over 32^3 takes the FP64 pipes of 16 SMs as long
 // as a launch takes all of them and its launch (four steps at 64^3 7.48 ms with level 32 in the
 // cluster, 7.19 without; 7.8 with level 16 out too).  A box of up to 32^3 is solved in one
-// launch (3.64 ms; its V-cycles by launches down to 16^3 3.82).
+// launch (3.64 ms; its V-cycles by launches down to 16^3 3.82).  Grids of 4 * 2^k and 6 * 2^k
+// cells only (cl_layout).
 constexpr int kClusterEdgeD = 16;   // (whole boxes: kClEdgeD)
 
 bool cluster_fits_d(Ctx& c, const Box& b, size_t li, ClArgs<double>& A)
