@@ -446,10 +446,10 @@ struct IterGraph {
     int failed = 0;                    // capture refused: enqueue eagerly from then on
 };
 
-// touch_pages before a copy into a caller's array.  Pinned pages are there: those of a small
-// array are read, as a copy into pages no CPU has used yet takes longer (2 x 2.4 MB: 51 us, 57
-// without); large ones are left (2 x 50 MB: 583 us, 588 with a read, 690 with a store by four
-// threads).  Device memory is not the host's to touch.
+// touch_pages before a copy into a caller's array.  Pinned pages are there and are read only (2 x
+// 50 MB: a read-back of 588 us, 690 with a store to each by four threads; 2 x 2.4 MB not used by a
+// CPU before 51, 57 without; 2 x 400 MB without 25 to 115 ms instead of 4.5 about every half
+// second).  Device memory is not the host's to touch.
 inline void touch_host(void* p, size_t bytes)
 {
     cudaPointerAttributes a{};
@@ -457,8 +457,8 @@ inline void touch_host(void* p, size_t bytes)
         cudaGetLastError();
         a.type = cudaMemoryTypeUnregistered;
     }
-    if (a.type == cudaMemoryTypeUnregistered) touch_pages(p, bytes);
-    if (a.type == cudaMemoryTypeHost && bytes < kTouchThreadsFrom) read_pages(p, bytes);
+    if (a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost)
+        touch_pages(p, bytes, a.type == cudaMemoryTypeHost);
 }
 
 // Whether the application has asked that a thread waiting for the device gives its CPU away

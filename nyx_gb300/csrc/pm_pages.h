@@ -35,6 +35,7 @@ constexpr size_t kPageLook = (size_t)16 << 20;           // bytes asked about pe
 constexpr size_t kPageMin = 4096;
 constexpr size_t kTouchThreadsFrom = (size_t)16 << 20;   // bytes worth threads
 constexpr size_t kTouchThreeTo = (size_t)128 << 20;      // missing bytes better by three than by four
+constexpr size_t kReadThreadsFrom = (size_t)128 << 20;   // bytes worth threads to read only
 
 // the missing pages of [at, end), whole pages; touch: fault them in and read the others
 inline size_t missing_pages(uintptr_t at, uintptr_t end, size_t page, bool touch)
@@ -69,37 +70,45 @@ inline size_t missing_pages(uintptr_t at, uintptr_t end, size_t page, bool touch
     return missing;
 }
 
-inline void read_pages(const void* p, size_t bytes)
+inline void fill_pages(uintptr_t at, uintptr_t end, size_t page) { missing_pages(at, end, page, true); }
+
+inline void read_pages(uintptr_t at, uintptr_t end, size_t page)
 {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    const volatile char* c = static_cast<const volatile char*>(p);
-    for (size_t o = 0; o < bytes; o += page) (void)c[o];
-    if (bytes) (void)c[bytes - 1];
+    for (; at < end; at += page) (void)*reinterpret_cast<volatile char*>(at);
 }
 
-inline void touch_pages(void* p, size_t bytes)
+// work on the whole pages of [at, end) in up to four threads, the caller's among them
+inline void pages_by_threads(void (*work)(uintptr_t, uintptr_t, size_t), uintptr_t at, uintptr_t end, size_t page,
+                             int threads)
+{
+    std::thread t[3];
+    const size_t part = (end - at) / threads & ~(kPageStep - 1);
+    try {
+        for (int k = 0; k + 1 < threads; ++k) {
+            t[k] = std::thread(work, at, at + part, page);
+            at += part;
+        }
+    } catch (...) {   // no more threads, or no memory for one: the rest here
+    }
+    work(at, end, page);
+    for (std::thread& x : t)
+        if (x.joinable()) x.join();
+}
+
+// there: no page is missing, as of pinned memory
+inline void touch_pages(void* p, size_t bytes, bool there = false)
 {
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     if (!p || !bytes || page < kPageMin || page > kPageStep) return;
-    uintptr_t at = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)(page - 1);
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)(page - 1);
     const uintptr_t end = (reinterpret_cast<uintptr_t>(p) + bytes + page - 1) & ~(uintptr_t)(page - 1);
-    constexpr int kMost = 4;
-    std::thread t[kMost - 1];
+    if (there) return pages_by_threads(read_pages, at, end, page, end - at < kReadThreadsFrom ? 1 : 4);
+    int threads = 1;
     if (end - at >= kTouchThreadsFrom) {
         const size_t missing = missing_pages(at, end, page, false) * page;
-        const int threads = missing >= kTouchThreadsFrom && missing < kTouchThreeTo ? 3 : kMost;
-        const size_t part = (end - at) / threads & ~(kPageStep - 1);
-        try {
-            for (int k = 0; k + 1 < threads; ++k) {
-                t[k] = std::thread(missing_pages, at, at + part, page, true);
-                at += part;
-            }
-        } catch (...) {   // no more threads, or no memory for one: the rest here
-        }
+        threads = missing >= kTouchThreadsFrom && missing < kTouchThreeTo ? 3 : 4;
     }
-    missing_pages(at, end, page, true);
-    for (std::thread& x : t)
-        if (x.joinable()) x.join();
+    pages_by_threads(fill_pages, at, end, page, threads);
 }
 
 }  // namespace nyxpm
