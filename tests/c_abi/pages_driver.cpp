@@ -81,6 +81,17 @@ int main(int argc, char** argv)
     if (!std::strcmp(what, "keeps")) {
         for (size_t len : {(size_t)1, kPage - 1, kPage, kPage + 1, 3 * M + 17, 20 * M + 5, 150 * M + 9})
             for (size_t off : {(size_t)0, (size_t)8, kPage - 8}) keeps((len + 3 * kPage) / kPage * kPage, off, len);
+    } else if (!std::strcmp(what, "there")) {   // every page in place: read only, by threads from 128 MB on
+        for (size_t len : {(size_t)1, kPage + 1, 127 * M + 3, 128 * M, 200 * M + 11}) {
+            const size_t bytes = (len + 2 * kPage) / kPage * kPage;
+            char* p = map(bytes, PROT_READ | PROT_WRITE);
+            for (size_t i = 0; i < bytes; ++i) p[i] = (char)at(i);
+            CHECK(mprotect(p, bytes, PROT_READ) == 0);
+            nyxpm::touch_pages(p + 5, len - 1, true);
+            nyxpm::touch_pages(p, len, true);
+            for (size_t i = 0; i < bytes; ++i) CHECK((unsigned char)p[i] == at(i));
+            munmap(p, bytes);
+        }
     } else if (!std::strcmp(what, "refused")) {
         for (int prot : {PROT_NONE, PROT_READ}) {
             char* p = map(40 * M, prot);

@@ -24,7 +24,7 @@ def driver(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("what", ["keeps", "refused"])
+@pytest.mark.parametrize("what", ["keeps", "there", "refused"])
 def test_pages_come_in_and_nothing_is_written(driver, what):
     assert driver(what) == (0, "ok\n")
 
